@@ -49,13 +49,17 @@ FALLBACK_HBM_GBS = 6800.0
 #   pointwise reads two transforms and writes one, the CRT scan reads the
 #   residues and writes the product limbs.
 def kernel_bytes(name: str, na: int, nb: int, L: int) -> float:
-    if name.startswith("ntt_fwd_load"):
-        return 4.0 * (na + nb) + 24.0 * L  # mean operand length: one launch per operand
-    if name.startswith("ntt_fwd_") or name.startswith("ntt_inv_"):
+    """Bytes a launch must move once (six 4-byte residues a coefficient; the
+    forward passes of both operands share a launch)."""
+    if name == "six_load_col_pass":
+        return 8.0 * (na + nb) + 48.0 * L
+    if name == "six_fwd_col_pass":
+        return 96.0 * L
+    if name == "six_fused_row_pass":
+        return 72.0 * L
+    if name.startswith("six_inv_"):
         return 48.0 * L
-    if name in ("ntt_pointwise", "ntt_fused_row_pass"):
-        return 72.0 * L  # fused: reads both transforms, writes one
-    if name == "crt_carry_scan":
+    if name == "six_crt_scan":
         return 24.0 * L + 8.0 * (na + nb)
     return 0.0
 

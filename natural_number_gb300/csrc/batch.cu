@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(256, 3) batch_kernel(const BatchJob* __restric
           CrtProducerT<true> prod{J.res_a, L, size - 1};
           scan_tile(prod, it.tile, size, J.out, size, nullptr, flags + J.flag_base, err);
         } else {
-          PieceCrtProducer prod{J.res_a, L, J.piece, J.pieces, J.nb, size - 1};
+          ThreePieceCrtProducer prod{J.res_a, L, J.piece, J.pieces, J.nb, size - 1};
           scan_tile(prod, it.tile, size, J.out, size, nullptr, flags + J.flag_base, err);
         }
         break;

@@ -112,7 +112,8 @@ struct nn_context {
   cudaEvent_t ev_first = nullptr, ev_second = nullptr, ev_chunk = nullptr, ev_in = nullptr;
   u64 budget = 0;
   u64 held = 0;  // bytes of live allocations made through the context
-  nn::Tables tables;
+  nn::Tables tables;   // three-prime transforms (nn_transform_*, nn_ntt_mul)
+  nn::SixTables six;   // products
   nn::Scan scan;
   std::string err;
   u64* scratch[3] = {nullptr, nullptr, nullptr};  // grow-only device staging for host calls
@@ -268,25 +269,6 @@ nn_status inverse_save(nn_context* c, nn_transform* t, u64* d_out, u64 size, u64
   return NN_OK;
 }
 
-// inverse_save(skip_last_pass) in normal mode, with the product's limbs
-// copied to h_out on the copy stream range by range as the carry scan
-// finishes them, so the copy-back overlaps the scan.
-constexpr int kCopyChunks = 8;
-nn_status inverse_save_to_host(nn_context* c, nn_transform* t, u64* d_out, u64 size, u64* h_out) {
-  const std::vector<nn::Pass> plan = c->passes(t->scale);
-  NN_CK(c, nn::ntt_inverse(t->res, t->scale, c->tables, c->stream, &plan, true), "inverse NTT");
-  const cudaError_t e =
-      nn::ntt_save_chunks(t->res, t->scale, d_out, size, c->scan, c->stream, kCopyChunks, [&](u64 lo, u64 hi) {
-        cudaError_t r = cudaEventRecord(c->ev_chunk, c->stream);
-        if (r == cudaSuccess) r = cudaStreamWaitEvent(c->copy, c->ev_chunk, 0);
-        if (r == cudaSuccess)
-          r = cudaMemcpyAsync(h_out + lo, d_out + lo, (hi - lo) * 8, cudaMemcpyDeviceToHost, c->copy);
-        return r;
-      });
-  NN_CK(c, e, "CRT/carry with copy-back");
-  return NN_OK;
-}
-
 nn_status pointwise(nn_context* c, nn_transform* dst, const nn_transform* a, const nn_transform* b) {
   if (a->scale != b->scale || a->scale < 2) {
     c->err = "pointwise: transforms differ in scale";
@@ -312,27 +294,14 @@ nn_status forward_fused(nn_context* c, nn_transform* t, const u64* d_limbs, u64 
   return NN_OK;
 }
 
-// Balanced NTT product at scale s into d_out (size limbs, or wrap).
-// b_ready (optional): an event b's contents wait for; the stream waits for it
-// only after a's forward transform.  h_out (optional): host memory the
-// product is also copied to, overlapping the carry scan; *h_done tells
-// whether that happened (fused pipelines only).
+// Three-prime product at scale s into d_out (size limbs, or wrap).
 nn_status ntt_product(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b, u64 nb, int s, u64 size,
-                      u64* written, cudaEvent_t b_ready = nullptr, u64* h_out = nullptr, bool* h_done = nullptr) {
+                      u64* written) {
   nn_transform xa, xb;
   nn_status st = forward(c, &xa, a, na, s);
-  if (st == NN_OK && b_ready) {
-    const cudaError_t e = cudaStreamWaitEvent(c->stream, b_ready, 0);
-    if (e != cudaSuccess) st = fail(c, e, "wait for the second operand");
-  }
   if (st == NN_OK && c->passes(s).size() >= 2) {
     st = forward_fused(c, &xb, b, nb, s, &xa);
-    if (st == NN_OK && h_out && size - 1 <= (1ull << s)) {
-      st = inverse_save_to_host(c, &xb, d_out, size, h_out);
-      if (st == NN_OK && h_done) *h_done = true;
-    } else if (st == NN_OK) {
-      st = inverse_save(c, &xb, d_out, size, written, true);
-    }
+    if (st == NN_OK) st = inverse_save(c, &xb, d_out, size, written, true);
   } else {
     if (st == NN_OK) st = forward(c, &xb, b, nb, s);
     if (st == NN_OK) st = pointwise(c, &xb, &xa, &xb);
@@ -343,33 +312,59 @@ nn_status ntt_product(nn_context* c, u64* d_out, const u64* a, u64 na, const u64
   return st;
 }
 
-// Balanced NTT product of host operands (ha: na limbs, hb: nb limbs, na >=
-// nb) into d_out and h_out.  a's copy to da goes a range of columns at a time
-// (kInChunks ranges: a 2-D copy of the range in every full row of the first
-// pass, plus its part of a last, partial row) on the copy stream, and the
-// first forward pass runs each range's tiles as soon as it has arrived, so
-// the copy overlaps that pass; b's copy follows on the same stream while a's
-// other passes run.  *used is false, and nothing is done, when the plan's
-// first pass cannot run by ranges.
-constexpr int kInChunks = 8;
-nn_status ntt_product_from_host(nn_context* c, u64* d_out, u64* da, const u64* ha, u64 na, u64* db, const u64* hb,
+// Residues of a product over six primes: ra, then rb unless the transforms
+// are squared or take one pass.
+nn_status six_residues(nn_context* c, DBuf& buf, nn::SixOperands& op, const nn::SixPlan& pl) {
+  NN_CK(c, nn::six_tables_ensure(c->six, pl.s, c->stream, &c->retired_tables), "twiddle tables");
+  const u64 each = 3ull << pl.s;  // 6 words of 32 bits a coefficient
+  const bool two = op.b && pl.n > 1;
+  nn_status st = buf.alloc((op.pieces + (two ? 1 : 0)) * each);
+  if (st != NN_OK) return st;
+  op.ra = reinterpret_cast<nn::u32*>(buf.p);
+  op.rb = two ? reinterpret_cast<nn::u32*>(buf.p + op.pieces * each) : nullptr;
+  return NN_OK;
+}
+
+// op's product over six primes at scale s (op.b nullptr: the square).
+nn_status six_product(nn_context* c, u64* d_out, nn::SixOperands op, int s) {
+  const nn::SixPlan pl = nn::six_plan(std::max(s, nn::kSixMinScale));
+  DBuf buf(c);
+  nn_status st = six_residues(c, buf, op, pl);
+  if (st != NN_OK) return st;
+  NN_CK(c, nn::six_load(op, pl, c->six, c->stream), "first pass");
+  NN_CK(c, nn::six_finish(op, pl, c->six, c->stream), "passes");
+  NN_CK(c, nn::six_save(op, pl, d_out, c->scan, c->stream), "CRT/carry");
+  return NN_OK;
+}
+
+// Product of host operands (ha: na limbs, hb: nb limbs, na >= nb) into d_out
+// and h_out.  a's copy to da goes a range of columns at a time (kInChunks
+// ranges: a 2-D copy of the range in every full row of the first pass, plus
+// its part of a last, partial row) on the copy stream, and the first pass
+// runs each range's tiles as soon as it has arrived, so the copy overlaps
+// that pass; b's copy follows on the same stream.  The product's limbs go
+// back range by range (kCopyChunks) behind the carry scan.  *used is false,
+// and nothing is done, for transforms of one pass.
+constexpr int kInChunks = 8, kCopyChunks = 8;
+nn_status six_product_from_host(nn_context* c, u64* d_out, u64* da, const u64* ha, u64 na, u64* db, const u64* hb,
                                 u64 nb, int s, u64* h_out, bool* used) {
   *used = false;
-  const std::vector<nn::Pass> plan = c->passes(s);
-  u64 tiles = 0;
-  if (plan.size() < 2 || !nn::ntt_first_pass_tiles(s, plan[0], &tiles)) return NN_OK;
+  const nn::SixPlan pl = nn::six_plan(std::max(s, nn::kSixMinScale));
+  const u64 tiles = nn::six_first_pass_tiles(pl), width = nn::six_first_pass_columns(pl);
+  if (pl.n < 2) return NN_OK;
   *used = true;
-  NN_CK(c, nn::tables_ensure(c->tables, s, c->stream, &c->retired_tables), "twiddle tables");
-  nn_transform xa, xb;
-  nn_status st = xform_reserve(c, &xa, s);
+  nn::SixOperands op{da, na, na, 1, db, nb, nullptr, nullptr};
+  DBuf buf(c);
+  nn_status st = six_residues(c, buf, op, pl);
   if (st != NN_OK) return st;
-  const u64 row = 1ull << (s - plan[0].R);           // limbs a row of the first pass
+  const nn::SixOperands first{da, na, na, 1, nullptr, 0, op.ra, nullptr}, second{db, nb, nb, 1, nullptr, 0, op.rb, nullptr};
+  const u64 row = 1ull << (pl.s - pl.R[0]);            // limbs a row of the first pass
   const u64 full = na / row, part = na - full * row;  // full rows, limbs of the partial row
   const u64 k = std::min<u64>(kInChunks, tiles);
   cudaError_t e = cudaEventRecord(c->ev_first, c->stream);  // da and db are reused: after earlier work
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->copy, c->ev_first, 0);
   for (u64 j = 0; j < k && e == cudaSuccess; ++j) {
-    const u64 t0 = tiles * j / k, t1 = tiles * (j + 1) / k, c0 = 16 * t0, c1 = 16 * t1;
+    const u64 t0 = tiles * j / k, t1 = tiles * (j + 1) / k, c0 = width * t0, c1 = width * t1;
     if (full)
       e = cudaMemcpy2DAsync(da + c0, row * 8, ha + c0, row * 8, (c1 - c0) * 8, full, cudaMemcpyHostToDevice, c->copy);
     if (e == cudaSuccess && part > c0)
@@ -377,24 +372,57 @@ nn_status ntt_product_from_host(nn_context* c, u64* d_out, u64* da, const u64* h
                           cudaMemcpyHostToDevice, c->copy);
     if (e == cudaSuccess) e = cudaEventRecord(c->ev_in, c->copy);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_in, 0);
-    if (e == cudaSuccess) e = nn::ntt_first_pass_range(da, na, xa.res, s, c->tables, plan[0], t0, t1, c->stream);
+    if (e == cudaSuccess) e = nn::six_load(first, pl, c->six, c->stream, (nn::u32)t0, (nn::u32)t1);
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(db, hb, nb * 8, cudaMemcpyHostToDevice, c->copy);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev_second, c->copy);
-  if (e == cudaSuccess) e = nn::ntt_forward_tail(xa.res, s, c->tables, c->stream, plan);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_second, 0);
-  if (e != cudaSuccess) st = fail(c, e, "first operand by column ranges");
-  if (st == NN_OK) st = forward_fused(c, &xb, db, nb, s, &xa);
-  if (st == NN_OK) st = inverse_save_to_host(c, &xb, d_out, na + nb, h_out);
-  dev_free(c, xa.res, xa.words);
-  dev_free(c, xb.res, xb.words);
-  return st;
+  if (e == cudaSuccess) e = nn::six_load(second, pl, c->six, c->stream);
+  if (e == cudaSuccess) e = nn::six_finish(op, pl, c->six, c->stream);
+  if (e == cudaSuccess)
+    e = nn::six_save(op, pl, d_out, c->scan, c->stream, kCopyChunks, [&](u64 lo, u64 hi) {
+      cudaError_t r = cudaEventRecord(c->ev_chunk, c->stream);
+      if (r == cudaSuccess) r = cudaStreamWaitEvent(c->copy, c->ev_chunk, 0);
+      if (r == cudaSuccess)
+        r = cudaMemcpyAsync(h_out + lo, d_out + lo, (hi - lo) * 8, cudaMemcpyDeviceToHost, c->copy);
+      return r;
+    });
+  if (e != cudaSuccess) return fail(c, e, "product from host operands");
+  return NN_OK;
 }
 
-// b_ready (optional): an event the contents of b wait for; the balanced NTT
-// product waits for it after a's forward transform, the other paths at once.
-nn_status mul_impl(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b, u64 nb,
-                   cudaEvent_t b_ready = nullptr, u64* h_out = nullptr, bool* h_done = nullptr) {
+// An unbalanced product nx x ny (nx >= ny) at scale s may run as P pieces of k
+// limbs of the longer operand, each through a transform of scale s2 < s
+// sharing the shorter operand's: 2P + 1 transforms of 2^s2 words and s2 - 3
+// levels against 3 of 2^s.  k is the most that keeps a piece's product within
+// its transform (k + ny - 1 <= 2^s2), rounded down to a multiple of 8 (the CRT
+// scan's vector loads stay within a piece), and at least ny, so that at most
+// two pieces overlap at any position.  The cost of a word is its levels plus
+// about four levels' worth of load, block products and CRT.
+int six_split(u64 nx, u64 ny, int s, u64* k, u64* P) {
+  double best = 3.0 * (double)(1ull << s) * (s + 1);
+  int s_best = s;
+  *k = nx;
+  *P = 1;
+  for (int s2 = s - 1; s2 >= nn::kSixMinScale; --s2) {
+    const u64 L2 = 1ull << s2;
+    if (L2 + 1 < 2 * ny) break;
+    const u64 kk = (L2 - ny + 1) & ~7ull;
+    if (kk < ny || kk >= nx) continue;
+    const u64 pieces = (nx + kk - 1) / kk;
+    if (pieces > 32768) break;  // a grid dimension of the passes
+    const double cost = (2.0 * pieces + 1.0) * (double)L2 * (s2 + 1);
+    if (cost < 0.95 * best) {
+      best = cost;
+      s_best = s2;
+      *k = kk;
+      *P = pieces;
+    }
+  }
+  return s_best;
+}
+
+nn_status mul_impl(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b, u64 nb) {
   if (!d_out || !a || !b || na == 0 || nb == 0) {
     c->err = "mul: null pointer or empty operand";
     return NN_ERR_INVALID;
@@ -402,45 +430,17 @@ nn_status mul_impl(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b
   if (na < nb) {
     std::swap(a, b);
     std::swap(na, nb);
-    if (b_ready) NN_CK(c, cudaStreamWaitEvent(c->stream, b_ready, 0), "wait for an operand");
-    b_ready = nullptr;
-  }
-  const u64 a0 = (na + 1) >> 1;
-  const bool balanced = nb >= kNttMulThreshold && ntt_scale(na, nb) == ntt_scale(a0, nb);
-  if (b_ready && !balanced) {
-    NN_CK(c, cudaStreamWaitEvent(c->stream, b_ready, 0), "wait for an operand");
-    b_ready = nullptr;
   }
   if (nb < kNttMulThreshold) {  // natural.h:445-446 -> _mul_base
     NN_CK(c, nn::school_mul(a, na, b, nb, d_out, c->scan, c->stream), "base-case product");
     return NN_OK;
   }
-  // natural::_mul_NTT (natural.h:391-419)
-  const int s = ntt_scale(na, nb), s_opt = ntt_scale(a0, nb);
-  if (s == s_opt) return ntt_product(c, d_out, a, na, b, nb, s, na + nb, nullptr, b_ready, h_out, h_done);
-  // Unbalanced: b's transform is made once at s_opt and reused for both
-  // halves of a (mul_save_NTT_info / mul_load_NTT_info, natural.h:452-515).
-  const u64 a1 = na - a0;
-  nn_transform xb, x0, x1;
-  DBuf p0(c), p1(c);
-  nn_status st = p0.alloc(a0 + nb);
-  if (st == NN_OK) st = p1.alloc(a1 + nb);
-  if (st == NN_OK) st = forward(c, &xb, b, nb, s_opt);
-  if (st == NN_OK) st = forward(c, &x0, a, a0, s_opt);
-  if (st == NN_OK) st = pointwise(c, &x0, &xb, &x0);
-  if (st == NN_OK) st = inverse_save(c, &x0, p0.p, a0 + nb, nullptr);
-  if (st == NN_OK) st = forward(c, &x1, a + a0, a1, s_opt);
-  if (st == NN_OK) st = pointwise(c, &x1, &xb, &x1);
-  if (st == NN_OK) st = inverse_save(c, &x1, p1.p, a1 + nb, nullptr);
-  // (a1*b << a0 limbs) + a0*b  (natural.h:417)
-  if (st == NN_OK) {
-    cudaError_t e = nn::add_shifted(p0.p, a0 + nb, p1.p, a1 + nb, a0, d_out, na + nb, c->scan, c->stream);
-    if (e != cudaSuccess) st = fail(c, e, "split combine");
-  }
-  dev_free(c, xb.res, xb.words);
-  dev_free(c, x0.res, x0.words);
-  dev_free(c, x1.res, x1.words);
-  return st;
+  // natural::_mul_NTT (natural.h:391-419) cuts the longer operand in two when
+  // that lowers the scale; here it may go in any number of pieces.
+  u64 piece, pieces;
+  const int s = six_split(na, nb, ntt_scale(na, nb), &piece, &pieces);
+  if (s > nn::kSixMaxScale) return ntt_product(c, d_out, a, na, b, nb, s, na + nb, nullptr);
+  return six_product(c, d_out, nn::SixOperands{a, na, piece, (nn::u32)pieces, b, nb, nullptr, nullptr}, s);
 }
 
 nn_status sqr_impl(nn_context* c, u64* d_out, const u64* a, u64 n) {
@@ -452,20 +452,10 @@ nn_status sqr_impl(nn_context* c, u64* d_out, const u64* a, u64 n) {
     NN_CK(c, nn::school_mul(a, n, a, n, d_out, c->scan, c->stream), "base-case square");
     return NN_OK;
   }
-  // natural::_sqr_NTT (natural.h:433-442): one transform, squared pointwise.
+  // natural::_sqr_NTT (natural.h:433-442): one transform.
   const int s = ntt_scale(n, n);
-  nn_transform x;
-  nn_status st;
-  if (c->passes(s).size() >= 2) {
-    st = forward_fused(c, &x, a, n, s, nullptr);
-    if (st == NN_OK) st = inverse_save(c, &x, d_out, 2 * n, nullptr, true);
-  } else {
-    st = forward(c, &x, a, n, s);
-    if (st == NN_OK) st = pointwise(c, &x, &x, &x);
-    if (st == NN_OK) st = inverse_save(c, &x, d_out, 2 * n, nullptr);
-  }
-  dev_free(c, x.res, x.words);
-  return st;
+  if (s > nn::kSixMaxScale) return ntt_product(c, d_out, a, n, a, n, s, 2 * n, nullptr);
+  return six_product(c, d_out, nn::SixOperands{a, n, n, 1, nullptr, n, nullptr, nullptr}, s);
 }
 
 // Grow-only device staging buffer `slot` of at least `words` limbs.
@@ -913,6 +903,7 @@ nn_status nn_context_destroy(nn_context* c) {
   for (int i = 0; i < 3; ++i) dev_free(c, c->scratch[i], c->scratch_words[i]);
   cudaStreamSynchronize(c->own);
   nn::tables_free(c->tables);
+  nn::six_tables_free(c->six);
   for (u64* p : c->retired_tables) cudaFree(p);
   c->retired_tables.clear();
   nn::scan_free(c->scan);
@@ -965,7 +956,8 @@ const char* nn_last_error(const nn_context* c) { return c ? c->err.c_str() : "no
 
 uint64_t nn_context_device_bytes(const nn_context* c) {
   if (!c) return 0;
-  return c->held + 2 * 3 * c->tables.cap * sizeof(u64) + (c->scan.max_tiles + 1) * 4;
+  return c->held + 2 * 3 * c->tables.cap * sizeof(u64) + 2 * 6 * c->six.cap * sizeof(int2) +
+         (c->scan.max_tiles + 1) * 4;
 }
 
 nn_status nn_transform_create(nn_context* c, nn_transform** out) {
@@ -1047,34 +1039,26 @@ nn_status nn_mul_host(nn_context* c, uint64_t* out, uint64_t* out_n, const uint6
   if (st == NN_OK) st = scratch(c, 1, nb, &db);
   if (st == NN_OK) st = scratch(c, 2, na + nb, &dout);
   if (st != NN_OK) return st;
-  const int s = ntt_scale(na, nb);
-  if (nb >= kNttMulThreshold && s == ntt_scale((na + 1) >> 1, nb)) {  // balanced NTT product
+  u64 piece, pieces;
+  const int s = nb >= kNttMulThreshold ? six_split(na, nb, ntt_scale(na, nb), &piece, &pieces) : 0;
+  if (s && s <= nn::kSixMaxScale && pieces == 1) {
     bool used = false;
-    st = ntt_product_from_host(c, dout, da, a, na, db, b, nb, s, out, &used);
-    if (used || st != NN_OK) {
+    st = six_product_from_host(c, dout, da, a, na, db, b, nb, s, out, &used);
+    if (used) {
       if (st == NN_OK) st = nn_context_synchronize(c);
       const cudaError_t e = cudaStreamSynchronize(c->copy);
       if (st == NN_OK && e != cudaSuccess) st = fail(c, e, "copy-back");
       if (st == NN_OK && out_n) *out_n = normalized(out, na + nb);
       return st;
     }
+    if (st != NN_OK) return st;
   }
-  // a on the context's stream; b on the copy stream once a is in, so that
-  // b's copy runs while a is transformed.
   NN_CK(c, cudaMemcpyAsync(da, a, na * 8, cudaMemcpyHostToDevice, c->stream), "H2D");
-  NN_CK(c, cudaEventRecord(c->ev_first, c->stream), "event record");
-  NN_CK(c, cudaStreamWaitEvent(c->copy, c->ev_first, 0), "copy stream wait");
-  NN_CK(c, cudaMemcpyAsync(db, b, nb * 8, cudaMemcpyHostToDevice, c->copy), "H2D");
-  NN_CK(c, cudaEventRecord(c->ev_second, c->copy), "event record");
-  bool copied = false;  // the balanced NTT path copies the product back while its carry scan runs
-  st = mul_impl(c, dout, da, na, db, nb, c->ev_second, out, &copied);
-  if (st != NN_OK) {
-    cudaStreamSynchronize(c->copy);
-    return st;
-  }
-  if (!copied) NN_CK(c, cudaMemcpyAsync(out, dout, (na + nb) * 8, cudaMemcpyDeviceToHost, c->stream), "D2H");
+  NN_CK(c, cudaMemcpyAsync(db, b, nb * 8, cudaMemcpyHostToDevice, c->stream), "H2D");
+  st = mul_impl(c, dout, da, na, db, nb);
+  if (st != NN_OK) return st;
+  NN_CK(c, cudaMemcpyAsync(out, dout, (na + nb) * 8, cudaMemcpyDeviceToHost, c->stream), "D2H");
   st = nn_context_synchronize(c);
-  NN_CK(c, cudaStreamSynchronize(c->copy), "copy-back");
   if (st == NN_OK && out_n) *out_n = normalized(out, na + nb);
   return st;
 }

@@ -51,6 +51,54 @@ inline size_t tile_smem_bytes(int C, int R) {
   return C == 2 ? tile + (((size_t)1 << R) - 1) * 16 : tile;
 }
 
+// ---- The product pipeline over six 32-bit primes (six.cu) ----
+
+// W[b] pairs (w, round(w 2^32 / p)) of the six primes, then of the inverses:
+// [2][6][cap].  Grow-only; a table for scale s serves every smaller one.
+struct SixTables {
+  int2* tab = nullptr;
+  u64 cap = 0;
+};
+cudaError_t six_tables_ensure(SixTables& t, int s, cudaStream_t st, std::vector<u64*>* retired = nullptr);
+void six_tables_free(SixTables& t);
+
+constexpr int kSixMinScale = 4, kSixMaxScale = 31;
+// The passes of a transform of scale s: levels R[k] from lambda0[k], the last
+// pass over contiguous tiles, down to blocks of 2^lgm coefficients.
+struct SixPlan {
+  int s, lgm, n;
+  int R[3], lambda0[3];
+  // more than 18 levels: the lazy words are reduced at the last pass's start
+  bool reduce_in() const { return lambda0[n - 1] + R[n - 1] > 18; }
+};
+SixPlan six_plan(int s);
+
+// Operands of a product: a in `pieces` pieces of `piece` limbs (one piece of
+// na limbs: not split), residues ra [pieces][6][2^s]; b (nullptr: a square),
+// residues rb [6][2^s].  One-pass transforms leave rb untouched.
+struct SixOperands {
+  const u64* a;
+  u64 na, piece;
+  u32 pieces;
+  const u64* b;
+  u64 nb;
+  u32* ra;
+  u32* rb;
+};
+// The first pass (tiles [tile0, tile1) of it: tile j covers
+// six_first_pass_columns() columns of every row of 2^(s - R[0]) limbs), and
+// the rest: products of the pieces with b, as residues in ra for the CRT.
+u32 six_first_pass_tiles(const SixPlan& pl);
+u32 six_first_pass_columns(const SixPlan& pl);
+cudaError_t six_load(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st, u32 tile0 = 0,
+                     u32 tile1 = ~0u);
+cudaError_t six_finish(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st);
+// The multipliers of the CRT after a transform of scale s.
+struct SixCrt {
+  int w[6], wp[6];
+};
+SixCrt six_crt(int s);
+
 // Scratch for the carry scan.
 struct Scan {
   u32* flags = nullptr;  // per-tile status words
@@ -123,16 +171,6 @@ struct AddJob {
 };
 cudaError_t add_batch(const AddJob* d_jobs, u64 m, cudaStream_t st);
 
-// The first forward pass a range of tiles at a time, so that it can start
-// on the columns of an operand already copied: *tiles receives the pass's
-// tile count, tile j covering columns [16 j, 16 j + 16) of every row of
-// 2^(s - R) limbs (false when the pass does not take this form).  Then
-// ntt_forward_tail runs the plan's other passes.
-bool ntt_first_pass_tiles(int s, const Pass& ps, u64* tiles);
-cudaError_t ntt_first_pass_range(const u64* limbs, u64 n, u64* res, int s, const Tables& t, const Pass& ps, u64 tile0,
-                                 u64 tile1, cudaStream_t st);
-cudaError_t ntt_forward_tail(u64* res, int s, const Tables& t, cudaStream_t st, const std::vector<Pass>& plan);
-
 // Forward transform: limbs (n <= 2^s) -> residues [3][2^s] equal to
 // NTT_info::load + NTT (ntt_info.h:147-198) modulo each prime; lazy values in
 // [0, 4p) for p0 and p1, [0, 2p) for p2.
@@ -150,15 +188,15 @@ cudaError_t ntt_forward_head(const u64* limbs, u64 n, u64* res, int s, const Tab
 // (a complete forward transform; nullptr squares) and the first inverse pass.
 cudaError_t ntt_fused_last(u64* res, const u64* other, int s, const Tables& t, cudaStream_t st,
                            const std::vector<Pass>& plan);
+// CRT + carry of six_finish's residues: op's product in out[0..na+nb).
+// chunks > 1: in that many ranges of scan tiles, calling done(limb_begin,
+// limb_end) after each range's launch (for instance to queue its copy-back).
+cudaError_t six_save(const SixOperands& op, const SixPlan& pl, u64* out, Scan& sc, cudaStream_t st, int chunks = 1,
+                     const std::function<cudaError_t(u64, u64)>& done = nullptr);
 // CRT + carry into `size` limbs (normal mode) or the wrapped product mod
 // B^L - 1 in L limbs when size-1 > L (ntt_info.h:237-248).  Returns the
 // number of limbs written through *written (host value).
 cudaError_t ntt_save(const u64* res, int s, u64* out, u64 size, Scan& sc, u64* written, cudaStream_t st);
-// ntt_save in normal mode, run as `chunks` consecutive ranges of scan tiles;
-// after each range is launched, done(limb_begin, limb_end) is called with the
-// limbs that range writes (for instance to queue their copy to the host).
-cudaError_t ntt_save_chunks(const u64* res, int s, u64* out, u64 size, Scan& sc, cudaStream_t st, int chunks,
-                            const std::function<cudaError_t(u64, u64)>& done);
 // Schoolbook product by column sums + carry scan: out[0..na+nb).
 cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Scan& sc, cudaStream_t st);
 // out[0..n) = x (nx limbs) + y (ny limbs) shifted up by `shift` limbs; the

@@ -6,6 +6,7 @@
 
 #include "nn_device.cuh"
 #include "nn_internal.h"
+#include "six_tiles.cuh"
 
 namespace nn {
 
@@ -118,16 +119,183 @@ struct CrtProducerT {
 typedef CrtProducerT<false> CrtProducer;
 
 
+// CRT of the six-prime residues (six_tiles.cuh): with t_i = r_i * k_i mod p_i
+// (k_i = (M/p_i)^-1 and the transform's scale; any representative in (0, 2p)),
+// the coefficient is sum t_i (M/p_i) - q M for q = floor(sum t_i / p_i): it is
+// below 2^160 (two overlapping pieces, up to 2^31 limbs each), under a quarter
+// of M = 2^162.25, so a sum of 15-bit fractions tells q.  Column j of the sum
+// adds the t_i times word j of M/p_i in 64 bits without carries (six terms
+// below 2^61), then one pass propagates them; q M enters as q times 2^192 - M.
+// 42 multiply-adds, none dependent on another before the columns, where
+// Garner's mixed radix has fifteen dependent modular products.
+struct SixWords {
+  u32 w[6];
+};
+constexpr SixWords six_times(SixWords a, u32 b) {
+  u64 c = 0;
+  for (int i = 0; i < 6; ++i) {
+    c += (u64)a.w[i] * b;
+    a.w[i] = (u32)c;
+    c >>= 32;
+  }
+  return a;
+}
+constexpr SixWords six_modulus_without(int skip) {  // the product of the primes but one (6: all)
+  SixWords m{{1, 0, 0, 0, 0, 0}};
+  for (int i = 0; i < six::kPrimes; ++i)
+    if (i != skip) m = six_times(m, six::prime_of(i));
+  return m;
+}
+constexpr SixWords six_negated(SixWords a) {
+  u64 c = 1;
+  for (int i = 0; i < 6; ++i) {
+    c += (u32)~a.w[i];
+    a.w[i] = (u32)c;
+    c >>= 32;
+  }
+  return a;
+}
+template <int I>
+__device__ __forceinline__ void six_crt_term(int y, const SixCrt& k, u64 (&col)[6], u32& frac) {
+  constexpr u32 p = six::prime_of(I);
+  constexpr SixWords m = six_modulus_without(I);
+  constexpr u32 f = (u32)(((1ull << 39) + p / 2) / p);
+  const u32 t = (u32)six::mul_mod(y, k.w[I], k.wp[I], (int)p) + p;
+  frac += (t >> 12) * f;  // t / p in units of 2^-27, within 2^-11
+#pragma unroll
+  for (int j = 0; j < 5; ++j) col[j] += (u64)t * m.w[j];
+}
+__device__ __forceinline__ W3 six_garner(const int (&y)[six::kPrimes], const SixCrt& k) {
+  static_assert(six::kPrimes == 6);
+  constexpr SixWords neg = six_negated(six_modulus_without(six::kPrimes));
+  u64 col[6] = {0, 0, 0, 0, 0, 0};
+  u32 frac = 1u << 24;  // an eighth: the coefficient's own fraction is below a quarter
+  six_crt_term<0>(y[0], k, col, frac);
+  six_crt_term<1>(y[1], k, col, frac);
+  six_crt_term<2>(y[2], k, col, frac);
+  six_crt_term<3>(y[3], k, col, frac);
+  six_crt_term<4>(y[4], k, col, frac);
+  six_crt_term<5>(y[5], k, col, frac);
+  const u32 q = frac >> 27;
+  u32 w[6];
+  u64 c = 0;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {
+    c += col[j] + (u64)q * neg.w[j];
+    w[j] = (u32)c;
+    c >>= 32;
+  }
+  return W3{(u64)w[1] << 32 | w[0], (u64)w[3] << 32 | w[2], (u64)w[5] << 32 | w[4]};
+}
+__device__ __forceinline__ void six_garner4(const int4 (&v)[six::kPrimes], const SixCrt& k, W3 (&x)[kScanE], int e0) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    int y[six::kPrimes];
+#pragma unroll
+    for (int q = 0; q < six::kPrimes; ++q) y[q] = e == 0 ? v[q].x : e == 1 ? v[q].y : e == 2 ? v[q].z : v[q].w;
+    x[e0 + e] = six_garner(y, k);
+  }
+}
+template <bool CG>
+struct SixCrtProducer {
+  const u32* res;  // [6][L]
+  u64 L, count;
+  SixCrt k;
+  static constexpr bool kBulk = true;
+  // One position: the ends of a product only, so a call rather than sixteen
+  // inlined copies in the scan.
+  __device__ __noinline__ W3 operator()(u64 i) const {
+    if (i >= count) return W3{0, 0, 0};
+    int y[six::kPrimes];
+#pragma unroll
+    for (int q = 0; q < six::kPrimes; ++q) {
+      const u32* r = res + q * L + i;
+      y[q] = (int)(CG ? __ldcg(r) : *r);
+    }
+    return six_garner(y, k);
+  }
+  // Eight consecutive positions from k0 (a multiple of 8) with 16-byte loads.
+  __device__ __forceinline__ void bulk(u64 k0, W3 (&x)[kScanE]) const {
+    if (k0 + kScanE > count) {
+#pragma unroll
+      for (int e = 0; e < kScanE; ++e) x[e] = (*this)(k0 + e);
+      return;
+    }
+#pragma unroll
+    for (int e0 = 0; e0 < kScanE; e0 += 4) {
+      int4 v[six::kPrimes];
+#pragma unroll
+      for (int q = 0; q < six::kPrimes; ++q) v[q] = six::ld4<CG>(res + q * L + k0 + e0);
+      six_garner4(v, k, x, e0);
+    }
+  }
+};
+
 // A product split into pieces: the longer operand x (nx limbs) cut into P
 // pieces of k limbs (the last one shorter), each multiplied by the shorter
 // operand y (ny <= k + 1 limbs) through its own transform of L words, laid
-// out [P][3][L].  Product coefficient j is the sum of coefficient j - i*k of
+// out [P][6][L].  Product coefficient j is the sum of coefficient j - i*k of
 // piece i = floor(j/k) (the last piece for j beyond it) and coefficient
 // j - (i-1)*k of piece i-1 when that is below k + ny - 1: at most two terms
 // (k >= ny - 1), each below 2^160, so the sum fits three limbs.  k is a
 // multiple of 8, so eight positions starting at a multiple of 8 lie in one
 // piece.  Batch work items read other CTAs' results: .cg loads.
+template <bool CG>
 struct PieceCrtProducer {
+  const u32* res;
+  u64 L, k, P, ny, count;
+  SixCrt crt;
+  static constexpr bool kBulk = true;
+  __device__ __forceinline__ u64 piece_of(u64 j) const {
+    const u64 i = j / k;
+    return i < P ? i : P - 1;
+  }
+  __device__ __noinline__ W3 operator()(u64 j) const {
+    if (j >= count) return W3{0, 0, 0};
+    const u64 i = piece_of(j), r = j - i * k;
+    const u32* c = res + i * six::kPrimes * L + r;
+    const u32* b = c - six::kPrimes * L + k;  // the piece before, at r + k
+    const bool ov = i > 0 && r + 1 < ny;
+    int y[six::kPrimes];
+#pragma unroll
+    for (int q = 0; q < six::kPrimes; ++q) {
+      y[q] = (int)(CG ? __ldcg(c + q * L) : c[q * L]);
+      if (ov) y[q] += (int)(CG ? __ldcg(b + q * L) : b[q * L]);
+    }
+    return six_garner(y, crt);
+  }
+  __device__ __forceinline__ void bulk(u64 k0, W3 (&x)[kScanE]) const {
+    const u64 i = piece_of(k0), r = k0 - i * k;  // one piece for the eight positions
+    if (k0 + kScanE > count) {
+#pragma unroll
+      for (int e = 0; e < kScanE; ++e) x[e] = (*this)(k0 + e);
+      return;
+    }
+    const u32* c = res + i * six::kPrimes * L + r;
+    const u32* b = c - six::kPrimes * L + k;
+    const u64 ov = i > 0 && r + 1 < ny ? ny - 1 - r : 0;  // so many of them overlap
+#pragma unroll
+    for (int e0 = 0; e0 < kScanE; e0 += 4) {
+      int4 v[six::kPrimes];
+#pragma unroll
+      for (int q = 0; q < six::kPrimes; ++q) v[q] = six::ld4<CG>(c + q * L + e0);
+      if (ov > e0) {
+#pragma unroll
+        for (int q = 0; q < six::kPrimes; ++q) {
+          const int4 w = six::ld4<CG>(b + q * L + e0);
+          v[q].x += w.x;
+          v[q].y += ov > e0 + 1 ? w.y : 0;
+          v[q].z += ov > e0 + 2 ? w.z : 0;
+          v[q].w += ov > e0 + 3 ? w.w : 0;
+        }
+      }
+      six_garner4(v, crt, x, e0);
+    }
+  }
+};
+
+// The same over three-prime residues [P][3][L] (batch work items: .cg loads).
+struct ThreePieceCrtProducer {
   const u64* res;
   u64 L, k, P, ny, count;
   static constexpr bool kBulk = true;

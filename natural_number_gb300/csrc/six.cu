@@ -1,0 +1,337 @@
+// six.cu — the product pipeline over six 32-bit primes on sm_103a: twiddle
+// tables, the tiled passes and their launches (six_tiles.cuh has the
+// arithmetic and the tiles).
+//
+// A transform of scale s runs T = min(s - 3, 22) levels: strided passes of up
+// to 9 levels (tiles of 2^R rows x 128 bytes), then one pass over contiguous
+// tiles of 4096 words, which takes both operands through their last levels,
+// multiplies them block by block and runs the first inverse levels, so
+// neither operand's finished transform goes through memory:
+//   scale  4-12  1 pass   limbs -> product residues
+//   scale 13-21  2 passes load, fused, inverse
+//   scale 22-31  3 passes load, strided, fused, inverse strided, inverse
+// Both operands' strided passes share a launch (and the pieces of a split
+// operand do).  Groups of at most three levels run in registers (eight rows of
+// four columns a thread); the first group of a pass reads global memory
+// directly and the last one writes it, so a pass of eight levels crosses
+// shared memory twice.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "nn_device.cuh"
+#include "nn_internal.h"
+#include "six_tiles.cuh"
+
+namespace nn {
+
+namespace {
+
+using namespace six;
+typedef unsigned __int128 h128;
+
+u64 h_pow(u64 b, u64 e, u64 p) {
+  u64 r = 1;
+  for (b %= p; e; e >>= 1, b = b * b % p)
+    if (e & 1) r = r * b % p;
+  return r;
+}
+i32 h_center(u64 w, u64 p) { return (i32)(w > p / 2 ? (i64)w - (i64)p : (i64)w); }
+i32 h_companion(i32 w, u64 p) {  // round(w 2^32 / p)
+  const i64 n = (i64)w * (1ll << 32), h = (i64)p / 2;
+  return (i32)((n + (n < 0 ? -h : h)) / (i64)p);
+}
+// An element of order 2^22 modulo each p.
+u64 h_root(u64 p) {
+  for (u64 a = 2;; ++a) {
+    const u64 g = h_pow(a, (p - 1) >> kRootLog, p);
+    if (h_pow(g, 1ull << (kRootLog - 1), p) == p - 1) return g;
+  }
+}
+
+// rho_t and its inverse for every prime: the factors of the table entries.
+struct Factors {
+  int2 f[2][kPrimes][kRootLog - 1];  // (w, companion)
+};
+Factors make_factors() {
+  Factors F;
+  for (int i = 0; i < kPrimes; ++i) {
+    const u64 p = prime_of(i), g = h_root(p);
+    for (int t = 0; t < kRootLog - 1; ++t) {  // rho_t has order 2^(t+2)
+      const u64 r = h_pow(g, 1ull << (kRootLog - 2 - t), p);
+      const i32 w = h_center(r, p), v = h_center(h_pow(r, p - 2, p), p);
+      F.f[0][i][t] = make_int2(w, h_companion(w, p));
+      F.f[1][i][t] = make_int2(v, h_companion(v, p));
+    }
+  }
+  return F;
+}
+
+// W[b] = the product of rho_t over the bits t of b (and of the inverses in
+// the second direction), centred, with its companion.  One launch writes
+// every entry of the 12 tables; an entry is at most 21 products.
+__global__ void __launch_bounds__(256) six_table_kernel(int2* tab, u64 cap, const Factors F) {
+  const u64 b = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= cap) return;
+  const int dir = blockIdx.y / kPrimes, prime = blockIdx.y % kPrimes;
+  const i32 p = c_primes[prime].p;
+  i32 w = 1;
+  for (int t = 0; t < kRootLog - 1; ++t)
+    if ((b >> t) & 1) w = mul_mod(w, F.f[dir][prime][t].x, F.f[dir][prime][t].y, p);
+  const i32 h = p >> 1;
+  if (w > h) w -= p;
+  if (w < -h) w += p;
+  const i64 n = (i64)w << 32;
+  tab[blockIdx.y * cap + b] = make_int2(w, (i32)((n + (n < 0 ? -(i64)h : (i64)h)) / p));
+}
+
+// Threads of a CTA: one unit of eight rows x four columns each.
+constexpr int col_threads(int R) { return std::max(32, (col_width(R) / 4) << (R - 3)); }
+constexpr int col_smem(int R) { return groups_of(R) > 1 ? (int)tile_words32<32>(R) * (col_width(R) / 32) * 4 : 0; }
+// Registers: 64 a thread; tiles of up to 2^8 rows as many CTAs as that allows.
+constexpr int col_blocks(int R) { return std::min(16, 1024 / col_threads(R)); }
+
+// First pass of up to two operands, the first in pieces: CTA (6 tile + prime,
+// y): piece y of a, or b for y = pieces.  The CTAs of one tile's six primes
+// run together, so its limbs cross HBM about once.
+template <int R>
+__global__ void __launch_bounds__(col_threads(R), col_blocks(R))
+    six_load_kernel(SixOperands op, int s, const int2* __restrict__ tab, u64 cap, u32 tile0) {
+  extern __shared__ __align__(16) u32 sm6[];
+  const int prime = (int)(blockIdx.x % kPrimes);
+  const u32 tile = tile0 + blockIdx.x / kPrimes;
+  if (blockIdx.y < op.pieces) {
+    const u64 at0 = blockIdx.y * op.piece;
+    load_tile<R, col_threads(R), false>(sm6, op.a + at0, min(op.piece, op.na - at0),
+                                        op.ra + ((u64)blockIdx.y * kPrimes << s), s, tile, prime, tab, cap);
+  } else {
+    load_tile<R, col_threads(R), false>(sm6, op.b, op.nb, op.rb, s, tile, prime, tab, cap);
+  }
+}
+
+template <int R, bool INV>
+__global__ void __launch_bounds__(col_threads(R), col_blocks(R))
+    six_col_kernel(u32* ra, u32* rb, u32 pieces, int s, int lambda0, const int2* __restrict__ tab, u64 cap, bool raw) {
+  extern __shared__ __align__(16) u32 sm6[];
+  u32* res = blockIdx.z < pieces ? ra + ((u64)blockIdx.z * kPrimes << s) : rb;
+  col_tile<R, col_threads(R), INV, false>(sm6, res, s, lambda0, blockIdx.x, blockIdx.y, tab, cap, raw);
+}
+
+constexpr int fused_threads(int R, int LGM) { return std::max(32, (1 << (R + LGM)) / 32); }
+// Two tiles of 4096 words in shared memory let six CTAs of 128 threads share
+// an SM (80 registers a thread); smaller tiles keep that register budget.
+constexpr int fused_blocks(int R, int LGM) { return std::min(16, 768 / fused_threads(R, LGM)); }
+template <int R, int LGM, bool FIRST>
+__global__ void __launch_bounds__(fused_threads(R, LGM), fused_blocks(R, LGM))
+    six_fused_kernel(SixOperands op, int s, const int2* __restrict__ tab, u64 cap, bool reduce_in) {
+  extern __shared__ __align__(16) u32 sm6[];
+  constexpr int NT = fused_threads(R, LGM);
+  u32* out = op.ra + ((u64)blockIdx.z * kPrimes << s);
+  const int2* itab = tab + kPrimes * cap;
+  if constexpr (FIRST) {
+    const u64 at0 = blockIdx.z * op.piece;
+    fused_tile<R, LGM, NT, true, false>(sm6, op.a + at0, min(op.piece, op.na - at0), op.b, op.nb, out, s, 0, blockIdx.y,
+                                        tab, itab, cap, false, op.pieces == 1);
+  } else {
+    fused_tile<R, LGM, NT, false, false>(sm6, out, 0, op.b ? op.rb : nullptr, 0, out, s, blockIdx.x, blockIdx.y, tab,
+                                         itab, cap, reduce_in, false);
+  }
+}
+
+template <class Kernel>
+cudaError_t allow_smem(Kernel k, int bytes) {
+  return bytes > 48 * 1024 ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
+}
+
+template <int R>
+cudaError_t launch_load(const SixOperands& op, int s, const SixTables& t, u32 tile0, u32 tile1, cudaStream_t st) {
+  constexpr int smem = col_smem(R);
+  static const cudaError_t ok = allow_smem(six_load_kernel<R>, smem);
+  if (ok != cudaSuccess) return ok;
+  const u32 tiles = (u32)((1ull << s) / ((u64)col_width(R) << R));
+  tile1 = std::min(tile1, tiles);
+  const dim3 grid(kPrimes * (tile1 - tile0), op.pieces + (op.b ? 1 : 0));
+  launch_begin("six_load_col_pass", st);
+  six_load_kernel<R><<<grid, col_threads(R), smem, st>>>(op, s, t.tab, t.cap, tile0);
+  launch_end(st);
+  return cudaGetLastError();
+}
+template <int R, bool INV>
+cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, int s, int lambda0, const SixTables& t, cudaStream_t st) {
+  constexpr int smem = col_smem(R);
+  static const cudaError_t ok = allow_smem(six_col_kernel<R, INV>, smem);
+  if (ok != cudaSuccess) return ok;
+  const dim3 grid((unsigned)((1ull << s) / ((u64)col_width(R) << R)), kPrimes, pieces + (rb ? 1 : 0));
+  launch_begin(INV ? (lambda0 == 0 ? "six_inv_last_col_pass" : "six_inv_col_pass") : "six_fwd_col_pass", st);
+  six_col_kernel<R, INV><<<grid, col_threads(R), smem, st>>>(
+      ra, rb, pieces, s, lambda0, t.tab + (INV ? kPrimes * t.cap : 0), t.cap, INV && lambda0 == 0 && pieces == 1);
+  launch_end(st);
+  return cudaGetLastError();
+}
+template <int R, int LGM, bool FIRST>
+cudaError_t launch_fused(const SixOperands& op, int s, const SixTables& t, bool reduce_in, cudaStream_t st) {
+  constexpr int tile = (int)tile_words32<1 << LGM>(R) * 4;
+  static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, FIRST>, 2 * tile);
+  if (ok != cudaSuccess) return ok;
+  const int smem = (op.b ? 2 : 1) * tile;
+  const dim3 grid(FIRST ? 1u : (unsigned)((1ull << s) >> (R + LGM)), kPrimes, op.pieces);
+  launch_begin(FIRST ? "six_small_pass" : "six_fused_row_pass", st);
+  six_fused_kernel<R, LGM, FIRST><<<grid, fused_threads(R, LGM), smem, st>>>(op, s, t.tab, t.cap, reduce_in);
+  launch_end(st);
+  return cudaGetLastError();
+}
+
+cudaError_t load_pass(const SixOperands& op, int s, int R, const SixTables& t, u32 t0, u32 t1, cudaStream_t st) {
+  switch (R) {
+    case 4: return launch_load<4>(op, s, t, t0, t1, st);
+    case 5: return launch_load<5>(op, s, t, t0, t1, st);
+    case 6: return launch_load<6>(op, s, t, t0, t1, st);
+    case 7: return launch_load<7>(op, s, t, t0, t1, st);
+    case 8: return launch_load<8>(op, s, t, t0, t1, st);
+    case 9: return launch_load<9>(op, s, t, t0, t1, st);
+  }
+  return cudaErrorInvalidValue;
+}
+template <bool INV>
+cudaError_t col_pass(u32* ra, u32* rb, u32 pieces, int s, int lambda0, int R, const SixTables& t, cudaStream_t st) {
+  switch (R) {
+    case 4: return launch_col<4, INV>(ra, rb, pieces, s, lambda0, t, st);
+    case 5: return launch_col<5, INV>(ra, rb, pieces, s, lambda0, t, st);
+    case 6: return launch_col<6, INV>(ra, rb, pieces, s, lambda0, t, st);
+    case 7: return launch_col<7, INV>(ra, rb, pieces, s, lambda0, t, st);
+    case 8: return launch_col<8, INV>(ra, rb, pieces, s, lambda0, t, st);
+    case 9: return launch_col<9, INV>(ra, rb, pieces, s, lambda0, t, st);
+  }
+  return cudaErrorInvalidValue;
+}
+cudaError_t fused_pass(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  const int R = pl.R[pl.n - 1], s = pl.s;
+  const bool red = pl.reduce_in();
+  if (pl.n == 1) {
+    switch (R) {
+      case 1: return launch_fused<1, 3, true>(op, s, t, red, st);
+      case 2: return launch_fused<2, 3, true>(op, s, t, red, st);
+      case 3: return launch_fused<3, 3, true>(op, s, t, red, st);
+      case 4: return launch_fused<4, 3, true>(op, s, t, red, st);
+      case 5: return launch_fused<5, 3, true>(op, s, t, red, st);
+      case 6: return launch_fused<6, 3, true>(op, s, t, red, st);
+      case 7: return launch_fused<7, 3, true>(op, s, t, red, st);
+      case 8: return launch_fused<8, 3, true>(op, s, t, red, st);
+      case 9: return launch_fused<9, 3, true>(op, s, t, red, st);
+    }
+    return cudaErrorInvalidValue;
+  }
+  switch (pl.lgm) {
+    case 4: return launch_fused<8, 4, false>(op, s, t, red, st);
+    case 5: return launch_fused<7, 5, false>(op, s, t, red, st);
+    case 6: return launch_fused<6, 6, false>(op, s, t, red, st);
+    case 7: return launch_fused<5, 7, false>(op, s, t, red, st);
+    case 8: return launch_fused<4, 8, false>(op, s, t, red, st);
+    case 9: return launch_fused<4, 9, false>(op, s, t, red, st);
+  }
+  switch (R) {
+    case 5: return launch_fused<5, 3, false>(op, s, t, red, st);
+    case 6: return launch_fused<6, 3, false>(op, s, t, red, st);
+    case 7: return launch_fused<7, 3, false>(op, s, t, red, st);
+    case 8: return launch_fused<8, 3, false>(op, s, t, red, st);
+    case 9: return launch_fused<9, 3, false>(op, s, t, red, st);
+  }
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace
+
+SixPlan six_plan(int s) {
+  SixPlan pl{};
+  pl.s = s;
+  const int T = std::min(s - 3, kRootLog);
+  pl.lgm = s - T;
+  const int row_max = std::max(12 - pl.lgm, 4);  // contiguous tiles of 4096 words (8192 at scale 31)
+  pl.n = T <= row_max ? 1 : T <= row_max + 9 ? 2 : 3;
+  int row = T;
+  if (pl.n > 1) row = pl.lgm > 3 ? row_max : (T + pl.n - 1) / pl.n;
+  for (int k = 0, left = T - row; k + 1 < pl.n; ++k) {
+    pl.R[k] = left / (pl.n - 1 - k);
+    pl.lambda0[k + 1] = pl.lambda0[k] + pl.R[k];
+    left -= pl.R[k];
+  }
+  pl.R[pl.n - 1] = row;
+  return pl;
+}
+
+cudaError_t six_tables_ensure(SixTables& t, int s, cudaStream_t st, std::vector<u64*>* retired) {
+  const u64 need = std::max<u64>(8, 1ull << (std::min(s - 3, kRootLog) - 1));
+  if (t.cap >= need) return cudaSuccess;
+  // from the size of one-pass transforms at once, then doubling: a handful of
+  // growths in a context's life
+  const u64 cap = std::max<u64>(need, 1 << 12);
+  int2* tab = nullptr;
+  cudaError_t e = cudaMallocAsync((void**)&tab, 2 * kPrimes * cap * sizeof(int2), st);
+  if (e != cudaSuccess) return e;
+  static const Factors F = make_factors();
+  launch_begin("six_table", st);
+  six_table_kernel<<<dim3((unsigned)((cap + 255) / 256), 2 * kPrimes), 256, 0, st>>>(tab, cap, F);
+  launch_end(st);
+  e = cudaGetLastError();
+  // other streams of the context read the table from the next launch on
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    cudaFreeAsync(tab, st);
+    return e;
+  }
+  if (t.tab) {
+    if (retired)
+      retired->push_back(reinterpret_cast<u64*>(t.tab));
+    else
+      cudaFreeAsync(t.tab, st);
+  }
+  t.tab = tab;
+  t.cap = cap;
+  return cudaSuccess;
+}
+
+void six_tables_free(SixTables& t) {
+  if (t.tab) cudaFree(t.tab);
+  t = SixTables{};
+}
+
+u32 six_first_pass_tiles(const SixPlan& pl) {
+  return pl.n == 1 ? 0 : (u32)((1ull << pl.s) / ((u64)col_width(pl.R[0]) << pl.R[0]));
+}
+u32 six_first_pass_columns(const SixPlan& pl) { return (u32)col_width(pl.R[0]); }
+
+cudaError_t six_load(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st, u32 tile0,
+                     u32 tile1) {
+  return pl.n == 1 ? cudaSuccess : load_pass(op, pl.s, pl.R[0], t, tile0, tile1, st);
+}
+
+cudaError_t six_finish(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  for (int k = 1; k + 1 < pl.n && e == cudaSuccess; ++k)
+    e = col_pass<false>(op.ra, op.b ? op.rb : nullptr, op.pieces, pl.s, pl.lambda0[k], pl.R[k], t, st);
+  if (e == cudaSuccess) e = fused_pass(op, pl, t, st);
+  for (int k = pl.n - 2; k >= 0 && e == cudaSuccess; --k)
+    e = col_pass<true>(op.ra, nullptr, op.pieces, pl.s, pl.lambda0[k], pl.R[k], t, st);
+  return e;
+}
+
+// The product residues are the coefficients times 2^T (the inverse's sums)
+// and 2^-96 (the Montgomery steps of the two operands' limbs and of the
+// blocks' products); the CRT multiplies them by the inverse of that and of
+// the other primes' product.
+SixCrt six_crt(int s) {
+  SixCrt c;
+  const int T = std::min(s - 3, kRootLog);
+  for (int i = 0; i < kPrimes; ++i) {
+    const u64 p = prime_of(i);
+    u64 m = 1;
+    for (int j = 0; j < kPrimes; ++j)
+      if (j != i) m = m * (prime_of(j) % p) % p;
+    const u64 k = h_pow(2, 96 - T, p) * h_pow(m, p - 2, p) % p;
+    c.w[i] = h_center(k, p);
+    c.wp[i] = h_companion(c.w[i], p);
+  }
+  return c;
+}
+
+}  // namespace nn

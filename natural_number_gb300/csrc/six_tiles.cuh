@@ -1,0 +1,549 @@
+// six_tiles.cuh — tile-level device code of the six-prime 32-bit NTT, shared
+// by the per-call kernels (six.cu) and the persistent batch kernel (batch.cu).
+//
+// A product of limbs is a convolution of 64-bit digits whose coefficients
+// stay below min(n_a, n_b) * 2^128.  It is computed modulo six primes
+// p = m * 2^22 + 1 just below 2^27.4 (product 2^162) instead of three 62-bit
+// ones: the same 24 bytes a coefficient, but a butterfly is one
+// multiply-high and two multiply-adds of 32 bits (8 cycles of the multiply
+// pipe a warp and scheduler on GB300, 8.9 measured in a register-only loop,
+// so 53 for the six primes) where a 64-bit Shoup butterfly takes 46 a prime,
+// 137 for the three.
+//
+// Residues are signed 32-bit words, lazy: |x| < 2^31, at least 12.8 p.  With
+// a twiddle pair (w, wp = round(w 2^32 / p)), |w| < p/2, the product y w - q p
+// with q = round(y wp / 2^32) is at most (1/2 + |y| / 2^33) p in magnitude, so
+//  - a forward butterfly (x, y) -> (x + w y, x - w y) adds at most
+//    p (1/2 + |y|/2^33): from |x| <= p, 18 levels stay below 12.1 p (and a
+//    transform of more levels reduces its values once on the way);
+//  - an inverse butterfly (x, y) -> (x + y, (x - y) w) doubles its sums: a
+//    group of three levels takes values of at most 1.5 p to sums of at most
+//    12 p; the first two of its eight outputs (one for shorter groups) are
+//    then reduced and the others are below 1.5 p again.
+//
+// The transform is the CRT tree of x^L - 1: block b at any level is taken
+// modulo x^h - c_b and splits with w = W[b] = sqrt(c_b) into x^(h/2) - w (child
+// 2b) and x^(h/2) + w (child 2b + 1); W[b] is the product of rho_t over the
+// bits t of b, rho_t a primitive 2^(t+2)-th root, so one table serves every
+// level and length.  The tree stops at blocks of m = 2^lgm coefficients
+// (m = 8 up to L = 2^25; 2^22 is the order of the roots), which are multiplied
+// directly modulo x^m - c_b: at m = 8 the eight multiply-adds a coefficient
+// cost less than the three levels they replace.
+#pragma once
+
+#include <cstdint>
+#include <type_traits>
+
+#include "nn_device.cuh"
+
+namespace nn {
+namespace six {
+
+typedef int i32;
+
+constexpr int kPrimes = 6;
+constexpr int kRootLog = 22;    // 2^22 divides every p - 1
+constexpr u32 kMul[kPrimes] = {25, 27, 33, 37, 39, 40};  // p = m * 2^22 + 1
+
+struct Prime {
+  i32 p;
+  u32 pinv;  // p^-1 mod 2^32 = 1 - m 2^22
+  i32 u;     // round(2^32 / p)
+  u32 c32;   // 2^32 mod p
+};
+constexpr u32 prime_of(int i) { return kMul[i] << 22 | 1; }
+constexpr Prime make_prime(int i) {
+  const u64 p = prime_of(i), two32 = 1ull << 32;
+  return Prime{(i32)p, (u32)(1u - (kMul[i] << 22)), (i32)((two32 + p / 2) / p), (u32)(two32 % p)};
+}
+static __constant__ Prime c_primes[kPrimes] = {make_prime(0), make_prime(1), make_prime(2),
+                                               make_prime(3), make_prime(4), make_prime(5)};
+
+// round(y * wp / 2^32)
+__device__ __forceinline__ i32 mulhi_round(i32 y, i32 wp) {
+  return (i32)(((i64)y * wp + 0x80000000ll) >> 32);
+}
+// y * w mod p, at most (1/2 + |y|/2^33) p in magnitude.
+__device__ __forceinline__ i32 mul_mod(i32 y, i32 w, i32 wp, i32 p) {
+  return (i32)((u32)y * (u32)w - (u32)mulhi_round(y, wp) * (u32)p);
+}
+// Any word to at most 0.75 p in magnitude.
+__device__ __forceinline__ i32 reduce(i32 x, const Prime& P) {
+  return (i32)((u32)x - (u32)mulhi_round(x, P.u) * (u32)P.p);
+}
+// x, y -> x + w y, x - w y: the product enters the first sum as its
+// multiply-adds' addend, the second is 2 x minus the first.
+__device__ __forceinline__ void fwd_bfly(i32& x, i32& y, i32 w, i32 wp, i32 p) {
+  const u32 q = (u32)mulhi_round(y, wp);
+  const u32 s = (u32)y * (u32)w + (u32)x - q * (u32)p;
+  y = (i32)(2u * (u32)x - s);
+  x = (i32)s;
+}
+__device__ __forceinline__ void inv_bfly(i32& x, i32& y, i32 w, i32 wp, i32 p) {
+  const i32 d = (i32)((u32)x - (u32)y);
+  x = (i32)((u32)x + (u32)y);
+  y = mul_mod(d, w, wp, p);
+}
+// limb * 2^-32 mod p, below p in magnitude (Montgomery step on hi * 2^32 mod
+// p * + lo, which is below 2^32 p).
+__device__ __forceinline__ i32 limb_residue(u64 limb, const Prime& P) {
+  const u64 t = (u64)(u32)(limb >> 32) * P.c32 + (u32)limb;
+  const u32 m = (u32)t * P.pinv;
+  return (i32)((u32)(t >> 32) - __umulhi(m, (u32)P.p));
+}
+// c * 2^-32 mod p, at most |c| / 2^32 + p/2 in magnitude.
+__device__ __forceinline__ i32 mont(i64 c, const Prime& P) {
+  const i32 m = (i32)((u32)c * P.pinv);
+  return (i32)((u32)(c >> 32) - (u32)__mulhi(m, P.p));
+}
+
+// A twiddle pair and two neighbouring ones (16-byte load).
+template <bool CG>
+__device__ __forceinline__ int4 ld4(const void* p) {
+  const int4* q = reinterpret_cast<const int4*>(p);
+  if (CG) return __ldcg(q);
+  return *q;
+}
+template <bool CG>
+__device__ __forceinline__ void st4(void* p, int4 v) {
+  int4* q = reinterpret_cast<int4*>(p);
+  if (CG)
+    __stcg(q, v);
+  else
+    *q = v;
+}
+
+// A unit: 2^K rows of four neighbouring columns in registers.
+template <int K>
+struct Unit {
+  i32 x[1 << K][4];
+  __device__ __forceinline__ void set(int m, int4 v) {
+    x[m][0] = v.x;
+    x[m][1] = v.y;
+    x[m][2] = v.z;
+    x[m][3] = v.w;
+  }
+  __device__ __forceinline__ int4 get(int m) const { return make_int4(x[m][0], x[m][1], x[m][2], x[m][3]); }
+};
+
+// The twiddle pairs of local level lv of a unit whose block index at the
+// unit's first level is b: W[b 2^lv + g], g < 2^lv.
+template <int LV>
+__device__ __forceinline__ void twiddles(int2 (&w)[1 << LV], const int2* __restrict__ tw, u32 b) {
+  if constexpr (LV == 0) {
+    w[0] = __ldg(tw + b);
+  } else {
+    const int4* t = reinterpret_cast<const int4*>(tw + ((u64)b << LV));
+#pragma unroll
+    for (int g = 0; g < (1 << LV); g += 2) {
+      const int4 v = __ldg(t + g / 2);
+      w[g] = make_int2(v.x, v.y);
+      w[g + 1] = make_int2(v.z, v.w);
+    }
+  }
+}
+
+template <int K, int LV>
+__device__ __forceinline__ void fwd_level(Unit<K>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+  int2 w[1 << LV];
+  twiddles<LV>(w, tw, b);
+  constexpr int half = (1 << K) >> (LV + 1);
+#pragma unroll
+  for (int g = 0; g < (1 << LV); ++g)
+#pragma unroll
+    for (int m = 0; m < half; ++m)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        fwd_bfly(u.x[g * 2 * half + m][c], u.x[g * 2 * half + m + half][c], w[g].x, w[g].y, p);
+}
+// Levels [LV0, K) of a unit.
+template <int K, int LV = 0>
+__device__ __forceinline__ void fwd_levels(Unit<K>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+  if constexpr (LV < K) {
+    fwd_level<K, LV>(u, tw, b, p);
+    fwd_levels<K, LV + 1>(u, tw, b, p);
+  }
+}
+
+template <int K, int LV>
+__device__ __forceinline__ void inv_level(Unit<K>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+  int2 w[1 << LV];
+  twiddles<LV>(w, tw, b);
+  constexpr int half = (1 << K) >> (LV + 1);
+#pragma unroll
+  for (int g = 0; g < (1 << LV); ++g)
+#pragma unroll
+    for (int m = 0; m < half; ++m)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        inv_bfly(u.x[g * 2 * half + m][c], u.x[g * 2 * half + m + half][c], w[g].x, w[g].y, p);
+}
+template <int K, int LV = K - 1>
+__device__ __forceinline__ void inv_levels(Unit<K>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+  if constexpr (LV >= 0) {
+    inv_level<K, LV>(u, tw, b, p);
+    inv_levels<K, LV - 1>(u, tw, b, p);
+  }
+}
+// The outputs of an inverse group above 1.5 p: row 0, and row 1 of three levels.
+template <int K>
+__device__ __forceinline__ void inv_fold(Unit<K>& u, const Prime& P) {
+#pragma unroll
+  for (int m = 0; m < (K == 3 ? 2 : 1); ++m)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) u.x[m][c] = reduce(u.x[m][c], P);
+}
+
+// Levels of a tile of R levels go in groups of at most three, one
+// shared-memory exchange between groups: groups_of(R) of them, the longer
+// ones first (forward order).
+constexpr int groups_of(int R) { return (R + 2) / 3; }
+constexpr int group_size(int R, int g) {
+  int left = R, k = 0;
+  for (int i = 0; i <= g; ++i) {
+    const int n = groups_of(R) - i;
+    k = (left + n - 1) / n;
+    left -= k;
+  }
+  return k;
+}
+constexpr int group_start(int R, int g) {
+  int l = 0;
+  for (int i = 0; i < g; ++i) l += group_size(R, i);
+  return l;
+}
+
+// Word of (row, column) in a tile of C columns: dense 128-byte rows from C =
+// 32; narrower rows are padded by one row's length every eight rows, which
+// spreads the units of the deepest group over the banks.  A unit's rows are
+// 2^nsub apart and their offsets from the first are the same for every unit.
+template <int C>
+__device__ __forceinline__ constexpr u32 at(u32 row) {
+  return row * C + (C < 32 ? (row >> 3) * C : 0);
+}
+template <int C>
+constexpr u32 tile_words32(int R) {
+  return ((u32)C << R) + (C < 32 ? ((((u32)1 << R) + 7) / 8) * C : 0);
+}
+// Columns of a strided tile: 32 (128 bytes), more where few rows would leave
+// the CTA with few units.
+constexpr int col_width(int R) { return R >= 7 ? 32 : R == 6 ? 64 : 128; }
+
+// Forward levels [0, R) of one tile of C columns x 2^R rows, block index ksb
+// at its first level.  load(row, col) gives the four words at (row, col ..
+// col + 3), store puts four finished words; between groups the words go
+// through sm.  HALF: the rows from 2^(R-1) are zero, so level 0 copies.
+// START: a reduction of the loaded words; LAST: one of the stored words.
+template <int R, int C, int NT, bool START, bool LAST, class Load, class Store>
+__device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const Store& store, bool half_zero,
+                                             const int2* __restrict__ tw, u32 ksb, const Prime& P, bool start_red) {
+  constexpr int G = groups_of(R);
+  auto group = [&](auto gc) {
+    constexpr int g = decltype(gc)::value;
+    constexpr int K = group_size(R, g), l = group_start(R, g), nsub = R - l - K;
+    constexpr u32 units = (u32)(C / 4) << (R - K);
+    if (g > 0) __syncthreads();
+#pragma unroll 1
+    for (u32 i = threadIdx.x; i < units; i += NT) {
+      const u32 col = (i % (C / 4)) * 4, v = i / (C / 4);
+      const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
+      Unit<K> u;
+      const u32 b = (ksb << l) + rb;
+      u32* sp = sm + at<C>(row0) + col;
+      if constexpr (g == 0) {
+        if (half_zero) {
+#pragma unroll
+          for (int m = 0; m < (1 << K) / 2; ++m) {
+            u.set(m, load(row0 + ((u32)m << nsub), col));
+            u.set(m + (1 << K) / 2, u.get(m));
+          }
+          fwd_levels<K, 1>(u, tw, b, P.p);
+        } else {
+#pragma unroll
+          for (int m = 0; m < (1 << K); ++m) u.set(m, load(row0 + ((u32)m << nsub), col));
+          if (START) {
+            if (start_red) {
+#pragma unroll
+              for (int m = 0; m < (1 << K); ++m)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) u.x[m][c] = reduce(u.x[m][c], P);
+            }
+          }
+          fwd_levels<K>(u, tw, b, P.p);
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < (1 << K); ++m) u.set(m, *reinterpret_cast<const int4*>(sp + at<C>((u32)m << nsub)));
+        fwd_levels<K>(u, tw, b, P.p);
+      }
+      if constexpr (g + 1 == G) {
+#pragma unroll
+        for (int m = 0; m < (1 << K); ++m) {
+          if (LAST) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) u.x[m][c] = reduce(u.x[m][c], P);
+          }
+          store(row0 + ((u32)m << nsub), col, u.get(m));
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < (1 << K); ++m) *reinterpret_cast<int4*>(sp + at<C>((u32)m << nsub)) = u.get(m);
+      }
+    }
+  };
+  group(std::integral_constant<int, 0>{});
+  if constexpr (G > 1) group(std::integral_constant<int, 1>{});
+  if constexpr (G > 2) group(std::integral_constant<int, 2>{});
+}
+
+// Inverse levels R-1 .. 0 of one tile; the groups in the opposite order.
+// raw: the outputs of the last group go out unreduced (up to 12 p, for the
+// CRT; overlapping pieces are added there and want at most 1.5 p).
+template <int R, int C, int NT, class Load, class Store>
+__device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const Store& store,
+                                             const int2* __restrict__ tw, u32 ksb, const Prime& P, bool raw) {
+  constexpr int G = groups_of(R);
+  auto group = [&](auto gc) {
+    constexpr int g = decltype(gc)::value;
+    constexpr int K = group_size(R, g), l = group_start(R, g), nsub = R - l - K;
+    constexpr u32 units = (u32)(C / 4) << (R - K);
+    if (g + 1 < G) __syncthreads();
+#pragma unroll 1
+    for (u32 i = threadIdx.x; i < units; i += NT) {
+      const u32 col = (i % (C / 4)) * 4, v = i / (C / 4);
+      const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
+      Unit<K> u;
+      const u32 b = (ksb << l) + rb;
+      u32* sp = sm + at<C>(row0) + col;
+#pragma unroll
+      for (int m = 0; m < (1 << K); ++m) {
+        if constexpr (g + 1 == G)
+          u.set(m, load(row0 + ((u32)m << nsub), col));
+        else
+          u.set(m, *reinterpret_cast<const int4*>(sp + at<C>((u32)m << nsub)));
+      }
+      inv_levels<K>(u, tw, b, P.p);
+      if (g > 0 || !raw) inv_fold<K>(u, P);
+#pragma unroll
+      for (int m = 0; m < (1 << K); ++m) {
+        if constexpr (g == 0)
+          store(row0 + ((u32)m << nsub), col, u.get(m));
+        else
+          *reinterpret_cast<int4*>(sp + at<C>((u32)m << nsub)) = u.get(m);
+      }
+    }
+  };
+  if constexpr (G > 2) group(std::integral_constant<int, 2>{});
+  if constexpr (G > 1) group(std::integral_constant<int, 1>{});
+  group(std::integral_constant<int, 0>{});
+}
+
+// Four limbs from position pos as residues (zero at and beyond n).
+__device__ __forceinline__ int4 limbs4(const u64* __restrict__ in, u64 n, u64 pos, bool vec, const Prime& P) {
+  u64 x[4] = {0, 0, 0, 0};
+  if (pos + 4 <= n && vec) {
+    const ulonglong2 v0 = __ldg(reinterpret_cast<const ulonglong2*>(in + pos));
+    const ulonglong2 v1 = __ldg(reinterpret_cast<const ulonglong2*>(in + pos) + 1);
+    x[0] = v0.x;
+    x[1] = v0.y;
+    x[2] = v1.x;
+    x[3] = v1.y;
+  } else {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (pos + c < n) x[c] = __ldg(in + pos + c);
+  }
+  return make_int4(limb_residue(x[0], P), limb_residue(x[1], P), limb_residue(x[2], P), limb_residue(x[3], P));
+}
+
+// The first pass of one operand: levels [0, R) from its limbs, columns
+// [tile * C, tile * C + C) of every row of 2^(s-R).
+template <int R, int NT, bool CG>
+__device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u64 n, u32* res, int s, u32 tile,
+                                          int prime, const int2* __restrict__ tab, u64 cap) {
+  constexpr int C = col_width(R);
+  const Prime P = c_primes[prime];
+  const int lg_s = s - R;
+  u32* out = res + ((u64)prime << s) + (u64)tile * C;
+  const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+  const u64 col0 = (u64)tile * C;
+  forward_tile<R, C, NT, false, false>(
+      sm, [&](u32 row, u32 col) { return limbs4(in, n, ((u64)row << lg_s) + col0 + col, vec, P); },
+      [&](u32 row, u32 col, int4 v) { st4<CG>(out + ((u64)row << lg_s) + col, v); }, n <= (1ull << (s - 1)),
+      tab + prime * cap, 0, P, false);
+}
+
+// Levels [lambda0, lambda0 + R) of residues in place: forward or inverse.
+template <int R, int NT, bool INV, bool CG>
+__device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, u32 tile, int prime,
+                                         const int2* __restrict__ tab, u64 cap, bool raw = false) {
+  constexpr int C = col_width(R);
+  const Prime P = c_primes[prime];
+  const int lg_s = s - lambda0 - R;
+  const u32 per = (u32)((1ull << lg_s) / C);  // tiles a block
+  const u32 ksb = tile / per;
+  u32* g = res + ((u64)prime << s) + ((u64)ksb << (lg_s + R)) + (u64)(tile % per) * C;
+  const int2* tw = tab + prime * cap;
+  auto ld = [&](u32 row, u32 col) { return ld4<CG>(g + ((u64)row << lg_s) + col); };
+  auto st = [&](u32 row, u32 col, int4 v) { st4<CG>(g + ((u64)row << lg_s) + col, v); };
+  if constexpr (INV)
+    inverse_tile<R, C, NT>(sm, ld, st, tw, ksb, P, raw);
+  else
+    forward_tile<R, C, NT, false, false>(sm, ld, st, false, tw, ksb, P, false);
+}
+
+// Products of the blocks of 8 coefficients of a tile: block row r of A times
+// that of B modulo x^8 - c, times 2^-32, into A.  Words at most 0.75 p in
+// magnitude, so the sums of eight products stay below 2^57.
+template <int R, int NT>
+__device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const int2* __restrict__ tw, u32 ksb,
+                                               const Prime& P) {
+#pragma unroll 1
+  for (u32 r = threadIdx.x; r < (1u << R); r += NT) {
+    const u32 blk = (ksb << R) + r;
+    int2 c = __ldg(tw + (blk >> 1));
+    if (blk & 1) c = make_int2(-c.x, -c.y);
+    i32 a[8], b[8], bw[8];
+    int4* pa = reinterpret_cast<int4*>(sa + at<8>(r));
+    const int4* pb = reinterpret_cast<const int4*>(sb + at<8>(r));
+    *reinterpret_cast<int4*>(a) = pa[0];
+    *reinterpret_cast<int4*>(a + 4) = pa[1];
+    *reinterpret_cast<int4*>(b) = pb[0];
+    *reinterpret_cast<int4*>(b + 4) = pb[1];
+#pragma unroll
+    for (int j = 1; j < 8; ++j) bw[j] = mul_mod(b[j], c.x, c.y, P.p);
+    i32 o[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      i64 t = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t += (i64)a[i] * (i <= j ? b[j - i] : bw[8 + j - i]);
+      o[j] = mont(t, P);
+    }
+    pa[0] = *reinterpret_cast<int4*>(o);
+    pa[1] = *reinterpret_cast<int4*>(o + 4);
+  }
+}
+
+// The same for blocks of m = 8 G coefficients (transforms above 2^25), seen as
+// polynomials of degree below G in x over Z_p[z] / (z^8 - c), z = x^G (word
+// g + G i is the z^i coefficient of x^g): a thread forms one x^g of one block
+// from G products of 8 coefficients each, with z b in the place of b where
+// the power of x wraps.  The results go out through `put` after every thread
+// of the CTA has read the block.
+template <int R, int LGM, int NT>
+__device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const int2* __restrict__ tw, u32 ksb,
+                                              const Prime& P) {
+  constexpr int C = 1 << LGM, G = C / 8;
+  constexpr u32 items = (u32)G << R;
+  constexpr u32 rounds = (items + NT - 1) / NT;
+  for (u32 it = 0; it < rounds; ++it) {
+    const u32 q = it * NT + threadIdx.x;  // whole blocks a round: items of a block lie in one round
+    const bool on = q < items;
+    const u32 r = on ? q / G : 0, g = q % G;
+    const u32 blk = (ksb << R) + r;
+    int2 c = __ldg(tw + (blk >> 1));
+    if (blk & 1) c = make_int2(-c.x, -c.y);
+    i64 t[15];
+#pragma unroll
+    for (int i = 0; i < 15; ++i) t[i] = 0;
+    u32* pa = sa + at<C>(r);
+    const u32* pb = sb + at<C>(r);
+#pragma unroll 1
+    for (int h = 0; h < G; ++h) {
+      const u32 k = (g - h) % G;
+      const bool wrap = (u32)h > g;
+      i32 a[8], b[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        a[i] = (i32)pa[h + G * i];
+        b[i] = (i32)pb[k + G * i];
+      }
+      const i32 top = mul_mod(b[7], c.x, c.y, P.p);
+#pragma unroll
+      for (int i = 7; i > 0; --i) b[i] = wrap ? b[i - 1] : b[i];
+      b[0] = wrap ? top : b[0];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t[i + j] += (i64)a[i] * b[j];
+    }
+    __syncthreads();  // the blocks of this round have been read
+    if (on) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        i32 o = mont(t[i], P);
+        if (i < 7) o = (i32)((u32)o + (u32)mul_mod(mont(t[i + 8 < 15 ? i + 8 : 14], P), c.x, c.y, P.p));
+        pa[g + G * i] = (u32)reduce(o, P);
+      }
+    }
+  }
+}
+
+// The last pass: tile `tile` (block index ksb at level lambda0, 2^R blocks of
+// 2^LGM coefficients) of both operands forward, the blocks' products, and the
+// first inverse levels.  a and b are residues after the strided passes (b
+// nullptr: a square), or, FIRST, limbs (na, nb of them; a transform of one
+// pass).  The inverse goes to out.  Modes for a batch run step by step:
+// kAll everything; kForward only a's forward levels, written back to a;
+// kProduct products and inverse of operands whose forward levels are done.
+enum : int { kAll = 0, kForward = 1, kProduct = 2 };
+template <int R, int LGM, int NT, bool FIRST, bool CG>
+__device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const void* b, u64 nb, u32* out, int s,
+                                           u32 tile, int prime, const int2* __restrict__ tab,
+                                           const int2* __restrict__ itab, u64 cap, bool reduce_in, bool raw, int mode = kAll) {
+  constexpr int C = 1 << LGM;
+  constexpr u32 W = tile_words32<C>(R);
+  const Prime P = c_primes[prime];
+  const int2* tw = tab + prime * cap;
+  const int2* itw = itab + prime * cap;
+  const u64 off = FIRST ? 0 : ((u64)prime << s) + ((u64)tile << (R + LGM));
+  u32* sa = sm;
+  u32* sb = b ? sm + W : sm;
+  auto to = [&](u32* t) { return [t](u32 row, u32 col, int4 v) { *reinterpret_cast<int4*>(t + at<C>(row) + col) = v; }; };
+  auto forward = [&](const void* src, u64 n, u32* t) {
+    if constexpr (FIRST) {
+      const u64* in = static_cast<const u64*>(src);
+      const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+      forward_tile<R, C, NT, false, true>(
+          t, [&](u32 row, u32 col) { return limbs4(in, n, (u64)row * C + col, vec, P); }, to(t), n <= (1ull << (s - 1)),
+          tw, 0, P, false);
+    } else {
+      const u32* in = static_cast<const u32*>(src) + off;
+      forward_tile<R, C, NT, true, true>(
+          t, [&](u32 row, u32 col) { return ld4<CG>(in + row * C + col); }, to(t), false, tw, tile, P, reduce_in);
+    }
+  };
+  auto fetch = [&](const void* src, u32* t) {  // kProduct: words whose forward levels are done
+    const u32* in = static_cast<const u32*>(src) + off;
+    for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT)
+      *reinterpret_cast<int4*>(t + at<C>(i / C) + i % C) = ld4<CG>(in + i);
+  };
+  if (FIRST || mode != kProduct) {
+    forward(a, na, sa);
+    if (!FIRST && mode == kForward) {
+      __syncthreads();
+      u32* back = out + off;
+      for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT)
+        st4<CG>(back + i, *reinterpret_cast<const int4*>(sa + at<C>(i / C) + i % C));
+      return;
+    }
+    if (b) forward(b, nb, sb);
+  } else if constexpr (!FIRST) {
+    fetch(a, sa);
+    if (b) fetch(b, sb);
+  }
+  __syncthreads();
+  if constexpr (LGM == 3)
+    leaf_products8<R, NT>(sa, sb, tw, FIRST ? 0 : tile, P);
+  else
+    leaf_products<R, LGM, NT>(sa, sb, tw, FIRST ? 0 : tile, P);
+  u32* dst = out + ((u64)prime << s) + (FIRST ? 0 : (u64)tile << (R + LGM));
+  __syncthreads();
+  inverse_tile<R, C, NT>(
+      sa, [&](u32 row, u32 col) { return *reinterpret_cast<const int4*>(sa + at<C>(row) + col); },
+      [&](u32 row, u32 col, int4 v) { st4<CG>(dst + row * C + col, v); }, itw, FIRST ? 0 : tile, P, FIRST && raw);
+}
+
+}  // namespace six
+}  // namespace nn

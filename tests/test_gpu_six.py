@@ -1,0 +1,88 @@
+"""The six-prime products on the GPU at the edges of their shapes: every
+transform scale with the fewest and the most coefficients it holds (half and
+whole first-pass tiles, one, two and three passes, blocks of 8 to 64
+coefficients), pieces of an unbalanced operand, operands at odd 8-byte
+addresses, limbs of all ones (the largest coefficients)."""
+import numpy as np
+import pytest
+
+from gpu_util import mod_checks, to_dev, to_host
+from natural_number_gb300.synth import limbs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import natural_number_gb300 as nn
+    c = nn.Context(0)
+    yield c
+    c.close()
+
+
+def product(ctx, a, b):
+    import torch
+    out = torch.empty(a.numel() + b.numel(), dtype=torch.uint64, device="cuda")
+    ctx.mul_device(out, a, b)
+    ctx.synchronize()
+    return out
+
+
+def check_mod(ctx, a, b, out):
+    ma, mb, mp = mod_checks(to_host(a)), mod_checks(to_host(b)), mod_checks(to_host(out))
+    assert mp[0] == ma[0] * mb[0] % (2**64 - 1) and mp[1] == ma[1] * mb[1] % (2**64 + 1)
+
+
+@pytest.mark.parametrize("s", range(10, 20))
+def test_every_scale_vs_oracle(ctx, oracle, s):
+    half = 1 << (s - 1)
+    for na, nb in [(half // 2 + 1, half // 2 + 1), (half, half + 1), (half + 1, half), (half - 3, half - 130)]:
+        a, b = limbs(s * 11 + na, na), limbs(s * 13 + nb, nb)
+        got = to_host(product(ctx, to_dev(a), to_dev(b)))
+        want = oracle.mul(a, b)
+        assert np.array_equal(got[: want.size], want) and not got[want.size:].any()
+        import torch
+        sq = torch.empty(2 * na, dtype=torch.uint64, device="cuda")
+        ctx.sqr_device(sq, to_dev(a))
+        got, want = to_host(sq), oracle.sqr(a)
+        assert np.array_equal(got[: want.size], want) and not got[want.size:].any()
+
+
+@pytest.mark.parametrize("s", [20, 21, 22, 23, 24, 25, 26, 27, 28])
+def test_long_scales_by_residues(ctx, s):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(s)
+    half = 1 << (s - 1)
+    for na, nb in [(half // 2 + 1, half // 2 + 7), (half, half + 1)]:
+        a, b = (torch.randint(-(2**63), 2**63 - 1, (n,), dtype=torch.int64, device="cuda", generator=g)
+                .view(torch.uint64) for n in (na, nb))
+        check_mod(ctx, a, b, product(ctx, a, b))
+        if s % 2 == 0:
+            out = torch.empty(2 * na, dtype=torch.uint64, device="cuda")
+            ctx.sqr_device(out, a)
+            ctx.synchronize()
+            check_mod(ctx, a, a, out)
+
+
+@pytest.mark.parametrize("na,nb", [(5000, 384), (70001, 400), (300007, 2049), (1 << 20, 5003), (40000, 12001)])
+def test_pieces_vs_oracle(ctx, oracle, na, nb):
+    a, b = limbs(na, na), limbs(nb, nb)
+    a[: na // 2] = np.uint64(0xFFFFFFFFFFFFFFFF)  # largest overlaps
+    b[:] = np.uint64(0xFFFFFFFFFFFFFFFF)
+    for x, y in ((a, b), (b, a)):
+        got, want = to_host(product(ctx, to_dev(x), to_dev(y))), oracle.mul(a, b)
+        assert np.array_equal(got[: want.size], want) and not got[want.size:].any()
+
+
+@pytest.mark.parametrize("n", [600, 5000, 1 << 17, (1 << 24) + 5])
+def test_odd_addresses_and_all_ones(ctx, n):
+    import torch
+    a = torch.full((n + 3,), -1, dtype=torch.int64, device="cuda").view(torch.uint64)
+    out = torch.empty(2 * n + 1, dtype=torch.uint64, device="cuda")
+    for oa, ob, oo in ((0, 0, 0), (1, 2, 1), (3, 1, 0)):
+        ctx.mul_device(out[oo:oo + 2 * n], a[oa:oa + n], a[ob:ob + n])
+        ctx.synchronize()
+        got = to_host(out[oo:oo + 2 * n])  # (B^n - 1)^2 = B^2n - 2 B^n + 1
+        ones = np.uint64(0xFFFFFFFFFFFFFFFF)
+        assert got[0] == 1 and not got[1:n].any() and got[n] == ones - np.uint64(1) and (got[n + 1:] == ones).all()
