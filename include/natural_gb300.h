@@ -151,19 +151,18 @@ nn_status nn_batch_mul(nn_context* ctx, const nn_mul_job* jobs, uint64_t count);
 /* Tunables: "r_last" (levels of the contiguous NTT pass, 3..12, default 11),
  * "r_col" (most levels of a strided pass, 1..9, default 9), "r_last@<s>" and
  * "r_col@<s>" (the same for transforms of scale s only; 0 = default),
- * "batch_r_last@<s>" (r_last for batched transforms of scale s; 0 = as for
- * one product),
+ * "batch_r_last@<s>" (levels of the contiguous last pass of two-pass batched
+ * products of scale s, where it can have that many; 0 = the built-in split),
  * "batch_ntt_min" (default 384), "batch_school_balanced" (default 256: a
  * product whose longer operand is at most twice its shorter also takes the
  * schoolbook route while the shorter is below this; 0 = off),
  * "batch_blocks_per_sm" (0 = occupancy limit),
  * "batch_item_words" (residues per prime a batch pass item covers at least,
  * in consecutive tiles; default 8192), "batch_fused" (1, the default: a
- * batched transform of two passes or more runs the second operand's last
- * forward pass, the pointwise product and the first inverse pass as one
- * step; 0: as separate steps), "batch_merge" (1, the default: a batched
- * pass whose tiles hold fewer than 2048 words works on several of them as one
- * tile; 0: tile by tile), "batch_split" (1, the default: an unbalanced
+ * batched transform of two passes or more runs both operands' last forward
+ * levels, their products and the first inverse levels as one step; 0: the
+ * forward levels as a step of their own), "batch_merge" (0 or 1; kept for
+ * callers that set it, every batch tile fills its CTA), "batch_split" (1, the default: an unbalanced
  * product may run as pieces of its longer operand, each through a smaller
  * transform sharing the shorter operand's, when that is estimated faster;
  * 0: one transform per product), "batch_solo_scale" (default 22: a batched

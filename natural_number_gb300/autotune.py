@@ -3,9 +3,8 @@
 Sweeps, on the GPU it runs on:
   - the NTT pass split: levels of the contiguous pass ("r_last") and the most
     levels of a strided column pass ("r_col"), timed on one product per
-    scale; and for batched transforms at scales 13-17 ("batch_r_last@s"),
-    timed on a batch of balanced products (a batch merges small tiles, so
-    its best split differs);
+    scale (these passes serve nn_ntt_mul and the cached transforms); and the
+    levels of the contiguous pass of batched products ("batch_r_last@s");
   - the batch shapes: persistent CTAs per SM ("batch_blocks_per_sm") and the
     shortest operand sent down the NTT route in a batch ("batch_ntt_min"),
     timed on the uneven-size workload.
@@ -44,7 +43,7 @@ def _time(fn, reps: int) -> float:
 
 
 def tune_passes(ctx, n_exps) -> tuple[dict, dict]:
-    """Per transform scale s = n_exp + 1: the pass split of one balanced
+    """Per transform scale s = n_exp + 1: the pass split of the three-prime
     2^n_exp x 2^n_exp product (ties keep the default split)."""
     import torch
 
@@ -63,7 +62,7 @@ def tune_passes(ctx, n_exps) -> tuple[dict, dict]:
             for r_col in (9, 8, 7):
                 ctx.set_tunable("r_last@%d" % s, r_last)
                 ctx.set_tunable("r_col@%d" % s, r_col)
-                ms = _time(lambda: ctx.mul_device(out, a, b), reps)
+                ms = _time(lambda: ctx.ntt_mul_device(out, a, b, s, 2 * n), reps)
                 if ref is None:
                     ref = out.clone()
                 elif not torch.equal(ref, out):
@@ -82,10 +81,9 @@ def tune_passes(ctx, n_exps) -> tuple[dict, dict]:
 
 
 def tune_batch_scales(ctx, scales) -> tuple[dict, dict]:
-    """The pass split at the scales where products are usually batched
-    (2^12-2^16-limb operands): timed on a batch of balanced products at each
-    scale, 2^24 transform words in all (with the small-tile merging a batch
-    does, the best split differs from a lone product's)."""
+    """Levels of the contiguous pass of two-pass batched transforms (5 to 9),
+    timed on a batch of balanced products at each scale, 2^24 transform words
+    in all."""
     import torch
 
     from .workloads import MulJob
@@ -103,8 +101,8 @@ def tune_batch_scales(ctx, scales) -> tuple[dict, dict]:
             jobs[j] = MulJob(a.data_ptr() + 8 * n * j, n, b.data_ptr() + 8 * n * j, n, out.data_ptr() + 16 * n * j)
         sizes = np.full(count, n, dtype=np.uint64)
         results, ref = {}, None
-        for r_last in (11, 10, 9, 8, 7, 6, 5):
-            if r_last > s - 2:
+        for r_last in (9, 8, 7, 6, 5):
+            if not 4 <= s - 3 - r_last <= 9:
                 continue
             ctx.set_tunable("batch_r_last@%d" % s, r_last)
             plan = ctx.batch(sizes, sizes)
@@ -135,8 +133,8 @@ def tune_batch(ctx, jobs: int) -> tuple[dict, dict]:
     W = UnevenProducts(jobs, seed=5)
     results = {}
     ref = None
-    for per_sm in (2, 3):
-        for ntt_min in (64, 128, 256, 384):
+    for per_sm in (5, 6):
+        for ntt_min in (48, 64, 96, 128):
             for item in (8192, 16384, 32768):
                 ctx.set_tunable("batch_blocks_per_sm", per_sm)
                 ctx.set_tunable("batch_ntt_min", ntt_min)

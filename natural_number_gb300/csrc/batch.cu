@@ -1,16 +1,15 @@
 // batch.cu — thousands of products of uneven lengths in one persistent launch.
 //
 // The host (engine.cpp) turns a batch into a work queue: every product is a
-// job with a short pipeline of steps — for an NTT job at scale s: the forward
-// passes of both operands (step k = pass k), the pointwise product, the
-// inverse passes, the CRT + carry scan; for a short operand (schoolbook job):
-// one column-sum scan — and every step is cut into tiles (items).  When the
-// transform has two passes or more, the first operand's last forward pass,
-// the pointwise product and the first inverse pass are one step (fused
-// items), after the second operand's last pass.  An unbalanced product may
-// be split: the longer operand (operand 0) in pieces, each with its own
-// transform, sharing the shorter operand's; the CRT + carry scan sums the
-// pieces' overlapping coefficients.  Items are
+// job with a short pipeline of steps — for an NTT job: the strided forward
+// passes of both operands, the fused last pass (both operands' last levels,
+// block products, first inverse levels), the strided inverse passes, the CRT +
+// carry scan; for a short operand (schoolbook job): one column-sum scan — and
+// every step is cut into tiles (items).  Transforms of one pass (up to 4096
+// words) are a fused item a prime, from limbs, and the CRT.  An unbalanced
+// product may be split: the longer operand (operand 0) in pieces, each with
+// its own transform, sharing the shorter operand's; the CRT + carry scan adds
+// the pieces' overlapping residues.  Items are
 // sorted by step, then job, then tile.  A fixed grid of CTAs (all resident)
 // pulls items from an atomic head; an item of step k of job j waits until all
 // items of step k-1 of job j have completed (a per-(job, step) counter).
@@ -19,14 +18,15 @@
 // other CTAs wrote in the same launch is read around L1 (.cg).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <array>
+
 #include "nn_device.cuh"
 #include "nn_internal.h"
-#include "ntt_tiles.cuh"
 #include "scan_tiles.cuh"
+#include "six_tiles.cuh"
 
 namespace nn {
-
-NN_DEFINE_PRIME_UPLOADER(upload_primes_batch)
 
 namespace {
 
@@ -38,21 +38,8 @@ __device__ __forceinline__ u32 ld_acquire(const u32* p) {
   return v;
 }
 
-// Wide strided tiles (32, 64 or 128 columns) of a transform's first pass:
-// the forward pass that loads limbs, or the last inverse pass, which scales.
-template <bool INV>
-__device__ __forceinline__ void wide_tile(int C, u64* sm, const u64* in, u64* out, u64 n_in, int s, int l0, int R,
-                                          const u64* tab, const Tables& t, int prime, u64 tile) {
-  if (C == 32)
-    pass_tile<32, !INV, INV, INV, true>(sm, in, out, n_in, s, l0, R, tab, t.cap, prime, tile);
-  else if (C == 64)
-    pass_tile<64, !INV, INV, INV, true>(sm, in, out, n_in, s, l0, R, tab, t.cap, prime, tile);
-  else
-    pass_tile<128, !INV, INV, INV, true>(sm, in, out, n_in, s, l0, R, tab, t.cap, prime, tile);
-}
-
 // A base-case item: the column sums of one scan tile's positions and of the
-// kScanE positions before them (the scan reads those too), all 256 threads
+// kScanE positions before them (the scan reads those too), all threads
 // at once, eight lanes a position, into shared memory as three word arrays
 // of kColumnTileWords; the scan then reads them from there.  (With one
 // thread computing its scan positions' sums in turn, a product of a few
@@ -74,10 +61,10 @@ struct SmemSumsProducer {
 };
 
 __device__ __forceinline__ void column_tile_sums(u64* sm, const BatchJob& J, u64 tile) {
-  constexpr u32 kLanes = 8, kGroups = 256 / kLanes;
+  constexpr u32 kLanes = 8, kGroups = kBatchThreads / kLanes;
   const u64 size = J.na + J.nb;
-  const long long first = (long long)(tile * kScanTile) - kScanE;
-  const u64 end = min(size, (tile + 1) * kScanTile);
+  const long long first = (long long)(tile * kBatchScanTile) - kScanE;
+  const u64 end = min(size, (tile + 1) * kBatchScanTile);
   const u32 npos = (u32)((long long)end - first);  // at most kColumnTileWords
   const u32 g = threadIdx.x / kLanes, j = threadIdx.x % kLanes;
   const u32 rounds = (npos + kGroups - 1) / kGroups;  // the same for every thread
@@ -119,73 +106,129 @@ __device__ __forceinline__ PieceTile piece_tile(const BatchJob& J, u64 g, u64 ti
   return {i, g - i * tiles_per_transform};
 }
 
-// One pass item: forward passes of operand 0 (the pieces of the longer
+using namespace six;
+
+// The multipliers of the CRT by scale, and the twiddle tables.
+struct BatchConst {
+  SixTables t;
+  SixCrt crt[kSixMaxScale + 1];
+};
+
+template <int R>
+__device__ __forceinline__ void strided(u32* sm, const BatchJob& J, const BatchItem& it, const BatchConst& k, u32* res,
+                                        const u64* in, u64 n, u32 tile) {
+  constexpr int C = batch_col_width(R);
+  const int s = J.plan.s;
+  if (it.kind == kItemInv)  // the pieces' residues are added in the CRT: folded
+    col_tile<R, C, kBatchThreads, true, true>(sm, res, s, J.plan.lambda0[it.pass], tile, it.prime,
+                                              k.t.tab + kPrimes * k.t.cap, k.t.cap);
+  else if (it.pass == 0)
+    load_tile<R, C, kBatchThreads, true>(sm, in, n, res, s, tile, it.prime, k.t.tab, k.t.cap);
+  else
+    col_tile<R, C, kBatchThreads, false, true>(sm, res, s, J.plan.lambda0[it.pass], tile, it.prime, k.t.tab, k.t.cap);
+}
+
+// A strided pass: forward passes of operand 0 (the pieces of the longer
 // operand) or 1 (the shorter), inverse passes of operand 0.
-template <bool INV, bool SCALE>
-__device__ __forceinline__ void run_pass(u64* sm, const BatchJob& J, const BatchItem& it, int operand,
-                                         const Tables& t, bool first) {
-  const int pk = it.pass;
-  const int s = J.s, l0 = J.lambda0[pk], R = J.R[pk], C = J.C[pk], skip = J.skip[pk];
-  const u64 L = 1ull << s;
-  const u64* tab = INV ? t.iroot : t.root;
-  for (u32 k = 0; k < it.ntile; ++k) {
-    if (k) __syncthreads();  // the previous tile's write-back has read shared memory
-    const u64* in;
-    u64* out;
-    u64 n_in = 0, tile = (u64)it.tile + k;
-    if (operand == 0) {
-      const PieceTile pt = piece_tile(J, tile, L / ((u64)C << R));
-      tile = pt.tile;
-      out = J.res_a + pt.piece * 3 * L;
-      in = out;
-      if (first) {
-        in = J.a + pt.piece * J.piece;
-        n_in = min(J.piece, J.na - pt.piece * J.piece);
+__device__ __forceinline__ void run_pass(u32* sm, const BatchJob& J, const BatchItem& it, const BatchConst& k,
+                                         u32 per_transform) {
+  const u64 words = (u64)kPrimes << J.plan.s;
+  for (u32 q = 0; q < it.ntile; ++q) {
+    if (q) __syncthreads();  // the previous tile has been read from shared memory
+    PieceTile pt{0, (u64)it.tile + q};
+    u32* res = J.res_b;
+    const u64* in = J.b;
+    u64 n = J.nb;
+    if (it.operand == 0) {
+      pt = piece_tile(J, pt.tile, per_transform);
+      res = J.res_a + pt.piece * words;
+      in = J.a + pt.piece * J.piece;
+      n = min(J.piece, J.na - pt.piece * J.piece);
+    }
+    const u32 tile = (u32)pt.tile;
+    switch (J.plan.R[it.pass]) {
+      case 4: strided<4>(sm, J, it, k, res, in, n, tile); break;
+      case 5: strided<5>(sm, J, it, k, res, in, n, tile); break;
+      case 6: strided<6>(sm, J, it, k, res, in, n, tile); break;
+      case 7: strided<7>(sm, J, it, k, res, in, n, tile); break;
+      case 8: strided<8>(sm, J, it, k, res, in, n, tile); break;
+      case 9: strided<9>(sm, J, it, k, res, in, n, tile); break;
+    }
+  }
+}
+
+template <int R, int LGM>
+__device__ __forceinline__ void fused(u32* sm, const BatchJob& J, const BatchItem& it, const BatchConst& k, u32* res,
+                                      u32 tile, int mode) {
+  u32* b = J.square ? nullptr : J.res_b;
+  fused_tile<R, LGM, kBatchThreads, false, true>(sm, res, 0, b, 0, res, J.plan.s, tile, it.prime, k.t.tab,
+                                                 k.t.tab + kPrimes * k.t.cap, k.t.cap, J.plan.reduce_in(), false, mode);
+}
+template <int R>
+__device__ __forceinline__ void small(u32* sm, const BatchJob& J, const BatchItem& it, const BatchConst& k, u32* res,
+                                      const u64* a, u64 na) {
+  const u64* b = J.square ? nullptr : J.b;
+  fused_tile<R, 3, kBatchThreads, true, true>(sm, a, na, b, J.nb, res, J.plan.s, 0, it.prime, k.t.tab,
+                                              k.t.tab + kPrimes * k.t.cap, k.t.cap, false, false);
+}
+
+// The contiguous last pass, tile by tile; transforms of one pass run it from
+// limbs, a piece an index.
+__device__ __forceinline__ void run_fused(u32* sm, const BatchJob& J, const BatchItem& it, const BatchConst& k) {
+  const SixPlan& pl = J.plan;
+  const u64 words = (u64)kPrimes << pl.s;
+  const int R = pl.R[pl.n - 1];
+  const u32 per = (u32)((1ull << pl.s) >> (R + pl.lgm));
+  const int mode = it.kind == kItemRow ? kForward : J.rows ? kProduct : kAll;
+  for (u32 q = 0; q < it.ntile; ++q) {
+    if (q) __syncthreads();
+    if (pl.n == 1) {
+      const u64 piece = (u64)it.tile + q;
+      u32* res = J.res_a + piece * words;
+      const u64* a = J.a + piece * J.piece;
+      const u64 na = min(J.piece, J.na - piece * J.piece);
+      switch (R) {
+        case 1: small<1>(sm, J, it, k, res, a, na); break;
+        case 2: small<2>(sm, J, it, k, res, a, na); break;
+        case 3: small<3>(sm, J, it, k, res, a, na); break;
+        case 4: small<4>(sm, J, it, k, res, a, na); break;
+        case 5: small<5>(sm, J, it, k, res, a, na); break;
+        case 6: small<6>(sm, J, it, k, res, a, na); break;
+        case 7: small<7>(sm, J, it, k, res, a, na); break;
+        case 8: small<8>(sm, J, it, k, res, a, na); break;
+        case 9: small<9>(sm, J, it, k, res, a, na); break;
       }
-    } else {
-      out = J.res_b;
-      in = first ? J.b : out;
-      n_in = J.nb;
+      continue;
     }
-    if (C == 16) {
-      if (first)
-        pass_tile<16, true, INV, SCALE, true>(sm, in, out, n_in, s, l0, R, tab, t.cap, it.prime, tile);
-      else
-        pass_tile<16, false, INV, SCALE, true>(sm, in, out, n_in, s, l0, R, tab, t.cap, it.prime, tile);
-    } else if (C == 2) {
-      if (first)
-        pass_tile<2, true, INV, SCALE, true>(sm, in, out, n_in, s, l0, R, tab, t.cap, it.prime, tile);
-      else
-        pass_tile<2, false, INV, SCALE, true>(sm, in, out, n_in, s, l0, R, tab, t.cap, it.prime, tile, nullptr,
-                                              nullptr, skip);
-    } else if constexpr (INV == SCALE) {  // the planner widens pass 0 only
-      wide_tile<INV>(C, sm, in, out, n_in, s, l0, R, tab, t, it.prime, tile);
+    const PieceTile pt = it.operand == 0 ? piece_tile(J, (u64)it.tile + q, per) : PieceTile{0, (u64)it.tile + q};
+    u32* res = it.operand == 0 ? J.res_a + pt.piece * words : J.res_b;
+    const u32 tile = (u32)pt.tile;
+    switch (pl.lgm) {
+      case 4: fused<8, 4>(sm, J, it, k, res, tile, mode); continue;
+      case 5: fused<7, 5>(sm, J, it, k, res, tile, mode); continue;
+      case 6: fused<6, 6>(sm, J, it, k, res, tile, mode); continue;
+      case 7: fused<5, 7>(sm, J, it, k, res, tile, mode); continue;
+      case 8: fused<4, 8>(sm, J, it, k, res, tile, mode); continue;
+      case 9: fused<4, 9>(sm, J, it, k, res, tile, mode); continue;
+    }
+    switch (R) {
+      case 5: fused<5, 3>(sm, J, it, k, res, tile, mode); break;
+      case 6: fused<6, 3>(sm, J, it, k, res, tile, mode); break;
+      case 7: fused<7, 3>(sm, J, it, k, res, tile, mode); break;
+      case 8: fused<8, 3>(sm, J, it, k, res, tile, mode); break;
+      case 9: fused<9, 3>(sm, J, it, k, res, tile, mode); break;
     }
   }
 }
 
-// The last forward pass of the first operand's pieces (or of the only
-// operand, for a square), the pointwise product with the second operand's
-// finished residues and the first inverse pass, tile by tile (the contiguous
-// pass only).
-__device__ __forceinline__ void run_fused(u64* sm, const BatchJob& J, const BatchItem& it, const Tables& t) {
-  const int pk = it.pass;
-  const u64 L = 1ull << J.s;
-  const u64* other = J.square ? nullptr : J.res_b;
-  for (u32 k = 0; k < it.ntile; ++k) {
-    if (k) __syncthreads();
-    const PieceTile pt = piece_tile(J, (u64)it.tile + k, L / (2ull << J.R[pk]));
-    u64* r = J.res_a + pt.piece * 3 * L;
-    pass_tile<2, false, false, false, true, true>(sm, r, r, 0, J.s, J.lambda0[pk], J.R[pk], t.root, t.cap, it.prime,
-                                                  pt.tile, t.iroot, other, J.skip[pk]);
-  }
-}
-
-__global__ void __launch_bounds__(256, 3) batch_kernel(const BatchJob* __restrict__ jobs,
+// Six CTAs of 128 threads an SM (80 registers a thread, two padded tiles of
+// 4096 words of shared memory).
+__global__ void __launch_bounds__(kBatchThreads, 6) batch_kernel(const BatchJob* __restrict__ jobs,
                                                     const BatchItem* __restrict__ items, u32 n_items,
                                                     const u32* __restrict__ need, u32* done, u32* head, u32* flags,
-                                                    u32* err, Tables t) {
-  extern __shared__ u64 sm[];
+                                                    u32* err, const __grid_constant__ BatchConst k) {
+  extern __shared__ __align__(16) u64 sm[];
+  u32* const sm32 = reinterpret_cast<u32*>(sm);
   __shared__ u32 s_item;
   // Thread 0 claims the next item while the current one runs, so the queue
   // atomic's latency is hidden.  Items are claimed in queue order and depend
@@ -215,48 +258,32 @@ __global__ void __launch_bounds__(256, 3) batch_kernel(const BatchJob* __restric
       __threadfence();
     }
     __syncthreads();
-    const u64 L = 1ull << J.s;
     switch (it.kind) {
       case kItemFwd:
-        run_pass<false, false>(sm, J, it, it.operand, t, it.pass == 0);
-        break;
-      case kItemPointwise: {  // piece i's residues times the other operand's, in place
-        const u64 groups = L / 4;
-        const u64 chunks = (groups + kBatchPointwiseChunk - 1) / kBatchPointwiseChunk;
-        const PieceTile pt = piece_tile(J, it.tile, chunks);
-        const u64 g0 = pt.tile * kBatchPointwiseChunk;
-        u64* d = J.res_a + pt.piece * 3 * L;
-        const u64* b = J.square ? d : J.res_b;
-        for (u64 g = g0 + threadIdx.x; g < g0 + kBatchPointwiseChunk && g < groups; g += blockDim.x)
-          pointwise_group<true>(d, d, b, L, t.root, t.cap, it.prime, g);
+      case kItemInv: {
+        const u32 R = J.plan.R[it.pass];
+        run_pass(sm32, J, it, k, (u32)((1ull << J.plan.s) / ((u64)batch_col_width((int)R) << R)));
         break;
       }
-      case kItemInv:
-        if (it.pass == 0)
-          run_pass<true, true>(sm, J, it, 0, t, false);
-        else
-          run_pass<true, false>(sm, J, it, 0, t, false);
-        break;
+      case kItemRow:
       case kItemFused:
-        run_fused(sm, J, it, t);
+        run_fused(sm32, J, it, k);
         break;
       case kItemCrt: {
-        const u64 size = J.na + J.nb;
-        if (J.pieces == 1) {
-          CrtProducerT<true> prod{J.res_a, L, size - 1};
-          scan_tile(prod, it.tile, size, J.out, size, nullptr, flags + J.flag_base, err);
-        } else {
-          ThreePieceCrtProducer prod{J.res_a, L, J.piece, J.pieces, J.nb, size - 1};
-          scan_tile(prod, it.tile, size, J.out, size, nullptr, flags + J.flag_base, err);
-        }
+        const u64 size = J.na + J.nb, L = 1ull << J.plan.s;
+        const SixCrt crt = k.crt[J.plan.s];
+        const PieceCrtProducer<true> prod{J.res_a, L, J.piece, J.pieces, J.nb, size - 1, crt};
+        scan_tile<PieceCrtProducer<true>, true, kBatchThreads>(prod, it.tile, size, J.out, size, nullptr,
+                                                               flags + J.flag_base, err);
         break;
       }
       case kItemColumn: {
         const u64 size = J.na + J.nb;
         column_tile_sums(sm, J, it.tile);
         __syncthreads();
-        const SmemSumsProducer prod{sm, (u64)it.tile * kScanTile - kScanE, size};
-        scan_tile(prod, it.tile, size, J.out, size, nullptr, flags + J.flag_base, err);
+        const SmemSumsProducer prod{sm, (u64)it.tile * kBatchScanTile - kScanE, size};
+        scan_tile<SmemSumsProducer, true, kBatchThreads>(prod, it.tile, size, J.out, size, nullptr,
+                                                         flags + J.flag_base, err);
         break;
       }
     }
@@ -270,17 +297,39 @@ __global__ void __launch_bounds__(256, 3) batch_kernel(const BatchJob* __restric
 
 }  // namespace
 
+u32 batch_pass_tiles(const SixPlan& pl, int k) {
+  const u64 L = 1ull << pl.s;
+  if (k == pl.n - 1) return (u32)(L >> (pl.R[k] + pl.lgm));
+  return (u32)(L / ((u64)batch_col_width(pl.R[k]) << pl.R[k]));
+}
+size_t batch_pass_smem(const SixPlan& pl, int k, bool square) {
+  const int R = pl.R[k];
+  if (k == pl.n - 1) {
+    const size_t rows = (size_t)1 << R, C = (size_t)1 << pl.lgm;
+    return (square ? 4 : 8) * (rows * C + (C < 32 ? (rows + 7) / 8 * C : 0));
+  }
+  return 4 * (R == 9 ? tile_words32<16>(9) : ((size_t)batch_col_width(R) << R));
+}
+
 cudaError_t batch_configure(int* blocks_per_sm, size_t smem) {
   cudaError_t e = cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, batch_kernel, 256, smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, batch_kernel, kBatchThreads, smem);
 }
 
 cudaError_t batch_launch(const BatchJob* jobs, const BatchItem* items, u32 n_items, const u32* need, u32* done,
-                         u32* head, u32* flags, u32* err, const Tables& t, int grid, size_t smem, cudaStream_t st) {
+                         u32* head, u32* flags, u32* err, const SixTables& t, int grid, size_t smem, cudaStream_t st) {
   // Recorded into a CUDA graph by the caller, which accounts for the launch
   // at each replay.
-  batch_kernel<<<grid, 256, smem, st>>>(jobs, items, n_items, need, done, head, flags, err, t);
+  BatchConst k;
+  k.t = t;
+  static const auto crt = [] {
+    std::array<SixCrt, kSixMaxScale + 1> c{};
+    for (int s = kSixMinScale; s <= kSixMaxScale; ++s) c[s] = six_crt(s);
+    return c;
+  }();
+  std::copy(crt.begin(), crt.end(), k.crt);
+  batch_kernel<<<grid, kBatchThreads, smem, st>>>(jobs, items, n_items, need, done, head, flags, err, k);
   return cudaGetLastError();
 }
 

@@ -12,6 +12,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <unordered_map>
 #include <unordered_set>
@@ -25,7 +26,6 @@ using nn::u64;
 
 namespace {
 constexpr u64 kNttMulThreshold = 384;  // ntt_info.h:6
-constexpr int kMergedTileWords = 2048;  // batch tiles: 256 threads x radix-8 units
 
 int ntt_scale(u64 n1, u64 n2) {  // get_NTT_scale (natural.h:384-386)
   u64 v = n1 + n2 - 2;
@@ -128,23 +128,17 @@ struct nn_context {
   int r_col = 9;              // most levels of a strided column pass
   int r_last_at[64] = {};     // per-scale overrides (0: use r_last / r_col)
   int r_col_at[64] = {};
-  int batch_r_last_at[64] = {};  // per-scale overrides for batched transforms (0: as above)
+  int batch_r_last_at[64] = {};  // levels of a two-pass batched transform's last pass (0: six_plan's)
   std::vector<nn::Pass> passes(int s) const {
     const int rl = (s >= 0 && s < 64 && r_last_at[s]) ? r_last_at[s] : r_last;
     const int rc = (s >= 0 && s < 64 && r_col_at[s]) ? r_col_at[s] : r_col;
     return nn::plan_passes(s, rl, rc);
   }
-  // Batched transforms merge small tiles, which favours other splits at the
-  // scales where products are usually batched.
-  std::vector<nn::Pass> batch_passes(int s) const {
-    if (s < 0 || s >= 64 || !batch_r_last_at[s]) return passes(s);
-    return nn::plan_passes(s, batch_r_last_at[s], r_col_at[s] ? r_col_at[s] : r_col);
-  }
   u64 batch_ntt_min = 384;    // batches: schoolbook when min(n_a, n_b) is below this
   u64 batch_school_balanced = 256;  // ... or below this when max(n_a, n_b) <= 2 min(n_a, n_b) (0: off)
   u64 batch_item_words = nn::kBatchItemWords;  // residues a pass item covers at least
-  int batch_fused = 1;        // batches: fused last pass (forward + pointwise + inverse)
-  int batch_merge = 1;        // batches: small tiles worked on 2048 words at a time
+  int batch_fused = 1;        // batches: last forward levels, products and first inverse levels in one item
+  int batch_merge = 1;        // kept for callers that set it: every batch tile fills its CTA
   int batch_split = 1;        // batches: unbalanced products in pieces sharing one transform
   int batch_blocks_per_sm = 0;  // persistent CTAs per SM (0: occupancy limit)
   int batch_solo_scale = 22;    // batches: products of this scale and up run one at a time (0: never)
@@ -477,45 +471,6 @@ nn_status scratch(nn_context* c, int slot, u64 words, u64** p) {
 // Batches: a work queue over all jobs' pipeline steps (batch.cu).
 // ---------------------------------------------------------------------------
 
-// Batched transform time per word at each scale, relative (GB300: 10^9
-// transform words per second of whole batched products at that scale, tiles
-// merged, last pass fused; scales below 9 and above 20 estimated).
-double batch_word_rate(int s) {
-  static const double rate[] = {1.0, 1.0, 1.0, 1.0, 1.2, 1.4, 1.7, 2.0, 2.3, 2.57, 4.77, 6.94,
-                                7.51, 6.9, 6.9, 6.66, 6.39, 6.08, 5.63, 5.66, 5.65};
-  return s < (int)(sizeof rate / sizeof rate[0]) ? rate[s] : 5.0;
-}
-
-// An unbalanced product nx x ny (nx >= ny) may run as P pieces of k limbs of
-// the longer operand, each through a transform of scale s2 < s sharing the
-// shorter operand's: 2P + 1 transforms of 2^s2 words against 3 of 2^s.  The
-// piece length is the most that keeps each piece's product within its
-// transform (k + ny - 1 <= 2^s2), rounded down to a multiple of 8 (the CRT
-// scan's vector loads stay within a piece), and at least ny, so that at most
-// two pieces overlap at any product position.  Returns the scale; sets k, P
-// (k = nx, P = 1: not split).
-int batch_split(u64 nx, u64 ny, int s, u64* k, u64* P) {
-  double best = 3.0 * (double)(1ull << s) / batch_word_rate(s);
-  int s_best = s;
-  *k = nx;
-  *P = 1;
-  for (int s2 = s - 1; s2 >= 2; --s2) {
-    const u64 L2 = 1ull << s2;
-    if (L2 + 1 < 2 * ny) break;
-    const u64 kk = (L2 - ny + 1) & ~7ull;
-    if (kk < ny || kk >= nx) continue;
-    const u64 pieces = (nx + kk - 1) / kk;
-    const double cost = (2.0 * pieces + 1.0) * (double)L2 / batch_word_rate(s2);
-    if (cost < 0.95 * best) {
-      best = cost;
-      s_best = s2;
-      *k = kk;
-      *P = pieces;
-    }
-  }
-  return s_best;
-}
-
 nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, const int* square, u64 count) {
   if (count >= 0xffffffffull) {  // BatchItem::job is 32-bit
     c->err = "batch: too many products";
@@ -529,8 +484,7 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
   B->off_b.assign(count, 0);
   B->swap.assign(count, 0);
   std::vector<int> steps(count, 0);
-  std::vector<int> fused_at(count, -1);  // step of the fused items, -1 without
-  int max_s = 2;
+  int max_s = nn::kSixMinScale;
   size_t smem = 8;
   for (u64 j = 0; j < count; ++j) {
     if (!na[j] || !nb[j]) {
@@ -545,10 +499,9 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
     J.pieces = 1;
     J.ctr_base = B->n_ctrs;
     J.flag_base = B->n_flags;
-    B->n_flags += (nn::u32)nn::scan_tiles(na[j] + nb[j]);
+    B->n_flags += (nn::u32)nn::batch_scan_tiles(na[j] + nb[j]);
     const u64 mn = std::min(na[j], nb[j]), mx = std::max(na[j], nb[j]);
     if (mn < c->batch_ntt_min || (mn < c->batch_school_balanced && mx <= 2 * mn)) {
-      J.s = 0;
       steps[j] = 1;
       smem = std::max(smem, nn::kColumnTileSmem);  // the item's column sums
     } else {
@@ -562,59 +515,30 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
       J.na = std::max(na[j], nb[j]);
       J.nb = std::min(na[j], nb[j]);
       J.piece = J.na;
-      int s = ntt_scale(J.na, J.nb);
+      int s = std::max(ntt_scale(J.na, J.nb), nn::kSixMinScale);
       if (c->batch_solo_scale > 0 && s >= c->batch_solo_scale) {
-        // From this scale on the one-product passes (TMA tiles, fused last
-        // pass) beat the batch kernel's generic tiles (GB300, 4 products of
-        // 2^21 limbs: 4.65 ms against 5.55 ms), and one product already fills
-        // the GPU: no items, no arena; the launch runs it alone.
+        // From this scale on one product fills the GPU by itself and the
+        // one-product passes beat the batch kernel's: no items, no arena; the
+        // launch runs it alone.
         B->solo.push_back(j);
         continue;
       }
-      if (c->batch_split && !J.square) s = batch_split(J.na, J.nb, s, &J.piece, &J.pieces);
-      J.s = s;
-      max_s = std::max(max_s, s);
-      const std::vector<nn::Pass> plan = c->batch_passes(s);
-      if (plan.size() > 4) {
+      if (c->batch_split && !J.square) s = six_split(J.na, J.nb, s, &J.piece, &J.pieces);
+      if (s > nn::kSixMaxScale) {
         c->err = "batch: transform too long for one batch";
         return NN_ERR_INVALID;
       }
-      J.n_pass = (int)plan.size();
-      for (int k = 0; k < J.n_pass; ++k) {
-        J.lambda0[k] = plan[k].lambda0;
-        J.R[k] = plan[k].R;
-        J.C[k] = plan[k].C;
-        J.skip[k] = 0;
-        if (c->batch_merge) {
-          // Small tiles leave most of a CTA's 256 threads idle and cut the
-          // levels into radix-2 and radix-4 sweeps; work on 2048 words at once:
-          // pass 0's strided tiles get up to 128 columns (as many as its
-          // column blocks hold), later contiguous passes take 2^skip
-          // consecutive tiles as one tile of R + skip levels.
-          const int lg_s = s - plan[k].lambda0 - plan[k].R;
-          if (k == 0 && plan[k].C == 16)
-            while ((J.C[k] << J.R[k]) < kMergedTileWords && J.C[k] < 128 && 2 * J.C[k] <= (1 << lg_s)) J.C[k] *= 2;
-          if (k > 0 && plan[k].C == 2)
-            while ((2 << J.R[k]) < kMergedTileWords && J.skip[k] < plan[k].lambda0) {
-              ++J.skip[k];
-              ++J.R[k];
-              --J.lambda0[k];
-            }
-        }
-        smem = std::max(smem, nn::tile_smem_bytes(J.C[k], J.R[k]));
-      }
-      const int m = J.n_pass;
-      if (c->batch_fused && m >= 2 && J.C[m - 1] == 2) {
-        // forward passes 0..m-2 of both operands, the second operand's last
-        // pass (not for a square), the fused step, inverse passes m-2..0, CRT
-        fused_at[j] = J.square ? m - 1 : m;
-        steps[j] = fused_at[j] + m + 1;
-      } else {
-        steps[j] = 2 * m + 2;
-      }
+      J.plan = nn::six_plan(s, s < 64 ? c->batch_r_last_at[s] : 0);
+      max_s = std::max(max_s, s);
+      for (int k = 0; k < J.plan.n; ++k) smem = std::max(smem, nn::batch_pass_smem(J.plan, k, J.square));
+      const int m = J.plan.n;
+      J.rows = m > 1 && !c->batch_fused;
+      // forward strided passes, (the last forward levels alone,) the fused
+      // pass, inverse strided passes, CRT
+      steps[j] = (m - 1) + J.rows + 1 + (m - 1) + 1;
       B->off_a[j] = B->arena_words;
       B->arena_words += J.pieces * (3ull << s);
-      if (!J.square) {
+      if (!J.square && m > 1) {
         B->off_b[j] = B->arena_words;
         B->arena_words += 3ull << s;
       }
@@ -624,8 +548,14 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
   B->need.assign(B->n_ctrs, 0);
   const int max_steps = *std::max_element(steps.begin(), steps.end());  // 0 when every job runs alone
   B->items.clear();
+  // Within a step, jobs of one scale one after another, the longest first:
+  // CTAs that share an SM then mostly run the same tile's code, and the step
+  // ends with its smallest items.
+  std::vector<u64> order(count);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](u64 x, u64 y) { return B->jobs[x].plan.s > B->jobs[y].plan.s; });
   for (int st = 0; st < max_steps; ++st) {
-    for (u64 j = 0; j < count; ++j) {
+    for (u64 j : order) {
       if (st >= steps[j]) continue;
       const nn::BatchJob& J = B->jobs[j];
       auto push = [&](unsigned char kind, int pass, int prime, int operand, u64 tile, u64 ntile = 1) {
@@ -641,46 +571,31 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
         B->items.push_back(it);
         B->need[J.ctr_base + st] += 1;
       };
-      if (J.s == 0) {
-        for (u64 t = 0; t < nn::scan_tiles(J.na + J.nb); ++t) push(nn::kItemColumn, 0, 0, 0, t);
+      const nn::SixPlan& pl = J.plan;
+      if (pl.s == 0) {
+        for (u64 t = 0; t < nn::batch_scan_tiles(J.na + J.nb); ++t) push(nn::kItemColumn, 0, 0, 0, t);
         continue;
       }
-      const int m = J.n_pass;
-      const u64 L = 1ull << J.s;
+      const int m = pl.n, fused_at = m - 1 + J.rows;
       // items of pass k over operand 0's pieces (tiles numbered across them) or operand 1
       auto pass_items = [&](unsigned char kind, int k, int operand) {
-        const u64 tw = (u64)J.C[k] << J.R[k], tiles = (L / tw) * (operand == 0 ? J.pieces : 1);
+        const u64 each = nn::batch_pass_tiles(pl, k), tiles = each * (operand == 0 ? J.pieces : 1);
+        const u64 tw = (1ull << pl.s) / each;
         const u64 per = std::clamp<u64>(c->batch_item_words / tw, 1, 0xffff);  // BatchItem::ntile is 16-bit
-        for (int pr = 0; pr < 3; ++pr)
+        for (int pr = 0; pr < 6; ++pr)
           for (u64 t = 0; t < tiles; t += per) push(kind, k, pr, operand, t, std::min(per, tiles - t));
       };
-      auto crt_items = [&] {
-        for (u64 t = 0; t < nn::scan_tiles(J.na + J.nb); ++t) push(nn::kItemCrt, 0, 0, 0, t);
-      };
-      if (const int f = fused_at[j]; f >= 0) {
-        if (st < m - 1) {
-          for (int op = 0; op < (J.square ? 1 : 2); ++op) pass_items(nn::kItemFwd, st, op);
-        } else if (st < f) {
-          pass_items(nn::kItemFwd, m - 1, 1);  // the second operand's last pass
-        } else if (st == f) {
-          pass_items(nn::kItemFused, m - 1, 0);
-        } else if (st < f + m) {
-          pass_items(nn::kItemInv, f + m - 1 - st, 0);  // inverse passes m-2 .. 0
-        } else {
-          crt_items();
-        }
-        continue;
-      }
-      if (st < m) {  // forward pass st of each operand
-        for (int op = 0; op < (J.square ? 1 : 2); ++op) pass_items(nn::kItemFwd, st, op);
-      } else if (st == m) {
-        const u64 chunks = (L / 4 + nn::kBatchPointwiseChunk - 1) / nn::kBatchPointwiseChunk * J.pieces;
-        for (int pr = 0; pr < 3; ++pr)
-          for (u64 t = 0; t < chunks; ++t) push(nn::kItemPointwise, 0, pr, 0, t);
-      } else if (st < 2 * m + 1) {  // inverse passes m-1 .. 0
-        pass_items(nn::kItemInv, 2 * m - st, 0);
+      const int operands = J.square ? 1 : 2;
+      if (st < m - 1) {
+        for (int op = 0; op < operands; ++op) pass_items(nn::kItemFwd, st, op);
+      } else if (st < fused_at) {
+        for (int op = 0; op < operands; ++op) pass_items(nn::kItemRow, m - 1, op);
+      } else if (st == fused_at) {
+        pass_items(nn::kItemFused, m - 1, 0);
+      } else if (st < fused_at + m) {
+        pass_items(nn::kItemInv, fused_at + m - 1 - st, 0);  // inverse passes m-2 .. 0
       } else {
-        crt_items();
+        for (u64 t = 0; t < nn::batch_scan_tiles(J.na + J.nb); ++t) push(nn::kItemCrt, 0, 0, 0, t);
       }
     }
   }
@@ -689,7 +604,7 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
     return NN_ERR_INVALID;
   }
   B->smem = smem;
-  NN_CK(c, nn::tables_ensure(c->tables, max_s, c->stream, &c->retired_tables), "twiddle tables");
+  NN_CK(c, nn::six_tables_ensure(c->six, max_s, c->stream, &c->retired_tables), "twiddle tables");
   int per_sm = 0;
   NN_CK(c, nn::batch_configure(&per_sm, smem), "batch kernel attributes");
   if (c->batch_blocks_per_sm > 0) per_sm = std::min(per_sm, c->batch_blocks_per_sm);
@@ -729,7 +644,7 @@ nn_status batch_capture(nn_context* c, nn_batch* B) {
   cudaMemsetAsync(B->d_state, 0, (B->n_ctrs + 4) * 4, cs);
   cudaMemsetAsync(B->d_flags, 0, (B->n_flags + 2) * 4, cs);
   cudaError_t le = nn::batch_launch(B->d_jobs, B->d_items, (nn::u32)B->items.size(), B->d_need, B->d_state,
-                                    B->d_state + B->n_ctrs, B->d_flags, c->scan.err, c->tables, B->grid, B->smem, cs);
+                                    B->d_state + B->n_ctrs, B->d_flags, c->scan.err, c->six, B->grid, B->smem, cs);
   cudaError_t e = cudaStreamEndCapture(cs, &B->graph);
   if (le != cudaSuccess) return fail(c, le, "batch launch (capture)");
   NN_CK(c, e, "end capture");
@@ -1215,8 +1130,8 @@ nn_status batch_fill(nn_context* c, nn_batch* B, const nn_mul_job* jobs, nn::Bat
     J.a = B->swap[j] ? jobs[j].d_b : jobs[j].d_a;
     J.b = B->swap[j] ? jobs[j].d_a : jobs[j].d_b;
     J.out = jobs[j].d_out;
-    J.res_a = B->d_arena + B->off_a[j];
-    J.res_b = B->d_arena + B->off_b[j];
+    J.res_a = reinterpret_cast<nn::u32*>(B->d_arena + B->off_a[j]);
+    J.res_b = reinterpret_cast<nn::u32*>(B->d_arena + B->off_b[j]);
     dst[j] = J;
   }
   return NN_OK;
@@ -1251,7 +1166,7 @@ nn_status nn_batch_launch(nn_context* c, nn_batch* B, const nn_mul_job* jobs) {
     NN_CK(c, cudaMemsetAsync(B->d_flags, 0, (B->n_flags + 2) * 4, c->stream), "reset flags");
     nn::launch_begin("batch_persistent", c->stream);
     cudaError_t le = nn::batch_launch(B->d_jobs, B->d_items, (nn::u32)B->items.size(), B->d_need, B->d_state,
-                                      B->d_state + B->n_ctrs, B->d_flags, c->scan.err, c->tables, B->grid,
+                                      B->d_state + B->n_ctrs, B->d_flags, c->scan.err, c->six, B->grid,
                                       B->smem, c->stream);
     nn::launch_end(c->stream);
     NN_CK(c, le, "batch launch");

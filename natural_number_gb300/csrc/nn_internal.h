@@ -69,9 +69,11 @@ struct SixPlan {
   int s, lgm, n;
   int R[3], lambda0[3];
   // more than 18 levels: the lazy words are reduced at the last pass's start
-  bool reduce_in() const { return lambda0[n - 1] + R[n - 1] > 18; }
+  constexpr bool reduce_in() const { return lambda0[n - 1] + R[n - 1] > 18; }
 };
-SixPlan six_plan(int s);
+// row_levels: levels of the last pass of a two-pass transform, where it can
+// have that many (0: as even as possible).
+SixPlan six_plan(int s, int row_levels = 0);
 
 // Operands of a product: a in `pieces` pieces of `piece` limbs (one piece of
 // na limbs: not split), residues ra [pieces][6][2^s]; b (nullptr: a square),
@@ -113,36 +115,38 @@ struct Scan {
 constexpr int kScanThreads = 256;
 constexpr int kScanE = 8;  // limbs per thread
 constexpr u64 kScanTile = (u64)kScanThreads * kScanE;
-// A batched base-case item's column sums in shared memory: a scan tile's
-// positions and the kScanE before them, three words each.
-constexpr u64 kColumnTileWords = kScanTile + kScanE;
-constexpr size_t kColumnTileSmem = 3 * kColumnTileWords * 8;
 
-// Batched products (batch.cu): jobs, their work items, and the launch.  A
-// pass item covers consecutive tiles worth at least kBatchItemWords residues
-// and a pointwise item kBatchPointwiseChunk groups of 4, so an item's fixed
-// cost (queue, dependency check, barriers) stays small beside its work.
+// Batched products (batch.cu): jobs, their work items, and the launch.  CTAs
+// of 128 threads: a unit of eight rows x four columns a thread is a tile of
+// 4096 words, the contiguous passes' tile.  A pass item covers consecutive
+// tiles worth at least kBatchItemWords residues, so an item's fixed cost
+// (queue, dependency check, barriers) stays small beside its work.
+constexpr int kBatchThreads = 128;
+constexpr u64 kBatchScanTile = (u64)kBatchThreads * kScanE;
+inline u64 batch_scan_tiles(u64 positions) { return (positions + kBatchScanTile - 1) / kBatchScanTile; }
+// A base-case item's column sums in shared memory: a scan tile's positions
+// and the kScanE before them, three words each.
+constexpr u64 kColumnTileWords = kBatchScanTile + kScanE;
+constexpr size_t kColumnTileSmem = 3 * kColumnTileWords * 8;
 constexpr u64 kBatchItemWords = 8192;
-constexpr u64 kBatchPointwiseChunk = 4096;
-enum : unsigned char { kItemFwd = 0, kItemPointwise = 1, kItemInv = 2, kItemCrt = 3, kItemColumn = 4, kItemFused = 5 };
+// Forward (load or strided) pass, fused last pass, inverse strided pass, CRT
+// and base-case items; kItemRow: the last pass's forward levels alone, before
+// a fused item that runs only the products and inverse levels (batch_fused 0).
+enum : unsigned char { kItemFwd = 0, kItemRow = 1, kItemInv = 2, kItemCrt = 3, kItemColumn = 4, kItemFused = 5 };
 struct BatchJob {
   const u64* a;  // NTT jobs: the longer operand (split into pieces)
   const u64* b;
   u64* out;      // na + nb limbs
   u64 na, nb;
-  u64* res_a;    // [pieces][3][2^s] residues (NTT jobs)
-  u64* res_b;    // [3][2^s]
+  u32* res_a;    // [pieces][6][2^s] residues (NTT jobs)
+  u32* res_b;    // [6][2^s]
   u64 piece;     // limbs of a per piece (na when not split)
   u64 pieces;
   u32 ctr_base;  // first (job, step) completion counter
   u32 flag_base; // first carry-scan status word
-  int s;         // transform scale; 0 for a schoolbook job
   int square;    // a == b: one transform
-  int n_pass;
-  // Pass k covers levels [lambda0 + skip, lambda0 + R) in tiles of C columns x
-  // 2^R rows: the batch widens pass 0's strided tiles (C up to 128) and runs
-  // later contiguous passes in tiles of 2^skip consecutive tiles.
-  int lambda0[4], R[4], C[4], skip[4];
+  int rows;      // kItemRow steps ran: the fused items start at the products
+  SixPlan plan;  // plan.s 0 for a schoolbook job
 };
 struct BatchItem {
   u32 job;
@@ -151,9 +155,12 @@ struct BatchItem {
   unsigned short ntile;  // consecutive tiles (pass items) handled by this item
   u32 tile;
 };
+// Tiles a transform has in pass k of its plan, and a CTA's shared memory for them.
+u32 batch_pass_tiles(const SixPlan& pl, int k);
+size_t batch_pass_smem(const SixPlan& pl, int k, bool square);
 cudaError_t batch_configure(int* blocks_per_sm, size_t smem);
 cudaError_t batch_launch(const BatchJob* jobs, const BatchItem* items, u32 n_items, const u32* need, u32* done,
-                         u32* head, u32* flags, u32* err, const Tables& t, int grid, size_t smem, cudaStream_t st);
+                         u32* head, u32* flags, u32* err, const SixTables& t, int grid, size_t smem, cudaStream_t st);
 
 // Many sums at once (carry.cu): job j writes out = x + y in nout >=
 // max(nx, ny) + 1 limbs, or with `sub` out = x - y mod B^nout (x >= y: the

@@ -547,9 +547,8 @@ void primes_host(u64 p[3]) {
 
 cudaError_t upload_primes() {
   PrimeSet ps = make_primes();
-  cudaError_t e = upload_primes_ntt(ps);
-  if (e == cudaSuccess) e = upload_primes_carry(ps);
-  return e == cudaSuccess ? upload_primes_batch(ps) : e;
+  const cudaError_t e = upload_primes_ntt(ps);
+  return e == cudaSuccess ? upload_primes_carry(ps) : e;
 }
 
 cudaError_t tables_ensure(Tables& t, int s, cudaStream_t st, std::vector<u64*>* retired) {

@@ -294,42 +294,6 @@ struct PieceCrtProducer {
   }
 };
 
-// The same over three-prime residues [P][3][L] (batch work items: .cg loads).
-struct ThreePieceCrtProducer {
-  const u64* res;
-  u64 L, k, P, ny, count;
-  static constexpr bool kBulk = true;
-  __device__ __forceinline__ CrtProducerT<true> piece(u64 i) const { return {res + i * 3 * L, L, L}; }
-  __device__ __forceinline__ u64 piece_of(u64 j) const {
-    const u64 i = j / k;
-    return i < P ? i : P - 1;
-  }
-  __device__ __forceinline__ W3 operator()(u64 j) const {
-    if (j >= count) return W3{0, 0, 0};
-    const u64 i = piece_of(j), r = j - i * k;
-    W3 x = piece(i)(r);
-    if (i > 0 && r + 1 < ny) x = add_w3(x, piece(i - 1)(r + k));
-    return x;
-  }
-  __device__ __forceinline__ void bulk(u64 k0, W3 (&x)[kScanE]) const {
-    if (k0 + kScanE > count) {
-#pragma unroll
-      for (int e = 0; e < kScanE; ++e) x[e] = (*this)(k0 + e);
-      return;
-    }
-    // one piece lookup for the eight positions; scalar loads keep fewer
-    // values live than two eight-position vector loads
-    const u64 i = piece_of(k0), r = k0 - i * k;
-    const CrtProducerT<true> cur = piece(i), prev = piece(i > 0 ? i - 1 : 0);
-    const bool ov = i > 0;
-#pragma unroll
-    for (int e = 0; e < kScanE; ++e) {
-      x[e] = cur(r + e);
-      if (ov && r + e + 1 < ny) x[e] = add_w3(x[e], prev(r + e + k));
-    }
-  }
-};
-
 // Column sums of a schoolbook product (asmMul1's column order, asmLinux.asm:188-278).
 struct ColumnProducer {
   static constexpr bool kBulk = false;
@@ -456,29 +420,33 @@ __device__ __forceinline__ u32 wait_flag(const u32* f, int limit) {
 // The scan's shared scratch: one block per kernel, whatever producers its
 // scan_tile instances take (a function's __shared__ variables exist once per
 // CTA, while each instance of a template would get its own).
+template <int NT>
 struct ScanShared {
-  u64 h0[kScanThreads], h1[kScanThreads];
-  u32 wg[kScanThreads / 32], wp[kScanThreads / 32];
+  u64 h0[NT], h1[NT];
+  u32 wg[NT / 32], wp[NT / 32];
   u32 cin;
   u64 x[kScanE][3];
 };
-__device__ __forceinline__ ScanShared& scan_shared() {
-  __shared__ ScanShared sh;
+template <int NT>
+__device__ __forceinline__ ScanShared<NT>& scan_shared() {
+  __shared__ ScanShared<NT> sh;
   return sh;
 }
 
-template <class Prod, bool LOOKBACK = true>
+// NT: threads of the CTA; a tile is NT * kScanE positions.
+template <class Prod, bool LOOKBACK = true, int NT = kScanThreads>
 __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total, u64* out, u64 out_limit, u64* side,
                                           u32* flags, u32* err) {
   constexpr int E = kScanE;
-  ScanShared& sh = scan_shared();
+  constexpr u64 kTile = (u64)NT * E;
+  ScanShared<NT>& sh = scan_shared<NT>();
   u64* const s_h0 = sh.h0;
   u64* const s_h1 = sh.h1;
   u32* const s_wg = sh.wg;
   u32* const s_wp = sh.wp;
   u32& s_cin = sh.cin;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const u64 k0 = tile * kScanTile + (u64)tid * E;
+  const u64 k0 = tile * kTile + (u64)tid * E;
 
   u64 y[E];
   u64 c0 = 0, c1 = 0;
@@ -503,7 +471,7 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
   u64(&s_x)[E][3] = sh.x;
   if (warp == 0) {
     if (lane < E && tile != 0) {
-      const W3 x = prod(tile * kScanTile - E + lane);
+      const W3 x = prod(tile * kTile - E + lane);
       s_x[lane][0] = x.w0;
       s_x[lane][1] = x.w1;
       s_x[lane][2] = x.w2;
@@ -544,7 +512,7 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
   __syncthreads();
   if (tid == 0) {
     u32 c_if0 = 0, c_if1 = 1;
-    for (int w = 0; w < kScanThreads / 32; ++w) {
+    for (int w = 0; w < NT / 32; ++w) {
       c_if0 = s_wg[w] | (s_wp[w] & c_if0);
       c_if1 = s_wg[w] | (s_wp[w] & c_if1);
     }

@@ -102,10 +102,10 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
   const u32 tile = tile0 + blockIdx.x / kPrimes;
   if (blockIdx.y < op.pieces) {
     const u64 at0 = blockIdx.y * op.piece;
-    load_tile<R, col_threads(R), false>(sm6, op.a + at0, min(op.piece, op.na - at0),
+    load_tile<R, col_width(R), col_threads(R), false>(sm6, op.a + at0, min(op.piece, op.na - at0),
                                         op.ra + ((u64)blockIdx.y * kPrimes << s), s, tile, prime, tab, cap);
   } else {
-    load_tile<R, col_threads(R), false>(sm6, op.b, op.nb, op.rb, s, tile, prime, tab, cap);
+    load_tile<R, col_width(R), col_threads(R), false>(sm6, op.b, op.nb, op.rb, s, tile, prime, tab, cap);
   }
 }
 
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
     six_col_kernel(u32* ra, u32* rb, u32 pieces, int s, int lambda0, const int2* __restrict__ tab, u64 cap, bool raw) {
   extern __shared__ __align__(16) u32 sm6[];
   u32* res = blockIdx.z < pieces ? ra + ((u64)blockIdx.z * kPrimes << s) : rb;
-  col_tile<R, col_threads(R), INV, false>(sm6, res, s, lambda0, blockIdx.x, blockIdx.y, tab, cap, raw);
+  col_tile<R, col_width(R), col_threads(R), INV, false>(sm6, res, s, lambda0, blockIdx.x, blockIdx.y, tab, cap, raw);
 }
 
 constexpr int fused_threads(int R, int LGM) { return std::max(32, (1 << (R + LGM)) / 32); }
@@ -241,15 +241,21 @@ cudaError_t fused_pass(const SixOperands& op, const SixPlan& pl, const SixTables
 
 }  // namespace
 
-SixPlan six_plan(int s) {
+SixPlan six_plan(int s, int row_levels) {
   SixPlan pl{};
   pl.s = s;
   const int T = std::min(s - 3, kRootLog);
   pl.lgm = s - T;
   const int row_max = std::max(12 - pl.lgm, 4);  // contiguous tiles of 4096 words (8192 at scale 31)
   pl.n = T <= row_max ? 1 : T <= row_max + 9 ? 2 : 3;
+  // The contiguous tile as long as the strided passes keep four levels (two
+  // passes: batched products of 2^14 limbs 0.084 ns a limb with 9 levels there,
+  // 0.126 with 6) or six (three passes: 2^24 x 2^24 limbs 2.80 ms with 6 + 7 +
+  // 9 levels, 2.86 with 7 + 7 + 8; at 2^21 7 levels and 9 read 378 and 394 us).
   int row = T;
-  if (pl.n > 1) row = pl.lgm > 3 ? row_max : (T + pl.n - 1) / pl.n;
+  if (pl.n == 2) row = std::min(9, T - 4);
+  if (pl.n == 3) row = pl.lgm > 3 ? row_max : std::min(9, T - 12);
+  if (pl.n == 2 && row_levels >= 5 && row_levels <= 9 && T - row_levels >= 4 && T - row_levels <= 9) row = row_levels;
   for (int k = 0, left = T - row; k + 1 < pl.n; ++k) {
     pl.R[k] = left / (pl.n - 1 - k);
     pl.lambda0[k + 1] = pl.lambda0[k] + pl.R[k];

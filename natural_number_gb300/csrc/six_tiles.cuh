@@ -227,7 +227,10 @@ constexpr u32 tile_words32(int R) {
 }
 // Columns of a strided tile: 32 (128 bytes), more where few rows would leave
 // the CTA with few units.
-constexpr int col_width(int R) { return R >= 7 ? 32 : R == 6 ? 64 : 128; }
+constexpr int col_width(int R) { return R >= 7 ? 32 : 4096 >> R; }
+// In the batch kernel: 16 (64 bytes) at 9 levels, so that every tile stays
+// within the shared memory of the two tiles of a fused item.
+constexpr int batch_col_width(int R) { return R == 9 ? 16 : col_width(R); }
 
 // Forward levels [0, R) of one tile of C columns x 2^R rows, block index ksb
 // at its first level.  load(row, col) gives the four words at (row, col ..
@@ -358,10 +361,9 @@ __device__ __forceinline__ int4 limbs4(const u64* __restrict__ in, u64 n, u64 po
 
 // The first pass of one operand: levels [0, R) from its limbs, columns
 // [tile * C, tile * C + C) of every row of 2^(s-R).
-template <int R, int NT, bool CG>
+template <int R, int C, int NT, bool CG>
 __device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u64 n, u32* res, int s, u32 tile,
                                           int prime, const int2* __restrict__ tab, u64 cap) {
-  constexpr int C = col_width(R);
   const Prime P = c_primes[prime];
   const int lg_s = s - R;
   u32* out = res + ((u64)prime << s) + (u64)tile * C;
@@ -374,10 +376,9 @@ __device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u
 }
 
 // Levels [lambda0, lambda0 + R) of residues in place: forward or inverse.
-template <int R, int NT, bool INV, bool CG>
+template <int R, int C, int NT, bool INV, bool CG>
 __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, u32 tile, int prime,
                                          const int2* __restrict__ tab, u64 cap, bool raw = false) {
-  constexpr int C = col_width(R);
   const Prime P = c_primes[prime];
   const int lg_s = s - lambda0 - R;
   const u32 per = (u32)((1ull << lg_s) / C);  // tiles a block
