@@ -11,19 +11,21 @@
 // carries are one bit each (propagate p_t = u_t is all ones; g_t and p_t are
 // exclusive), resolved by warp ballots inside a tile.
 //
-// Between tiles the per-call scans of more than 1024 tiles take three
+// Between tiles the per-call scans of more than kLookbackTiles tiles take two
 // launches and never wait:
 //  1. every tile runs with carry-in 0, writes its limbs and records its
 //     one-bit generate and propagate (no tile waits for another);
-//  2. one CTA composes those bits over the tiles (a scan of the maps
-//     carry-in -> carry-out) and records each tile's carry-in;
-//  3. each tile whose carry-in is 1 adds it at its first limb, where it
-//     ripples only while limbs wrap to zero.
+//  2. each CTA takes the carry into its range of tiles from the nearest tile
+//     before it that does not propagate, resolves the carries inside its range
+//     with ballots, and adds a tile's carry-in of 1 at its first limb, where
+//     it ripples only while limbs wrap to zero.
 // Smaller per-call scans, the persistent batch kernel and the
 // allocation-free entry point take the decoupled lookback instead (scan_tile
 // with LOOKBACK: one launch, each tile's carry-in from its predecessors'
 // status words), whose waits are bounded and record an error instead of
-// hanging.
+// hanging.  A per-call lookback leaves its status words and counters zero for
+// the next scan: the CTA that finishes last clears them, so a scan is one
+// launch with nothing to reset before it.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,19 +42,40 @@ NN_DEFINE_PRIME_UPLOADER(upload_primes_carry)
 namespace {
 
 // Scans of at most kLookbackTiles tiles take one launch: tile ids come from
-// an atomic counter (from tile_base), so every predecessor of a tile has
-// started before it, and each tile takes its carry-in by the decoupled
-// lookback.  Their tiles fit in one or two waves, so a lookback waits about
-// one tile's work; larger scans take the three steps below, which never wait.
+// an atomic counter, so every predecessor of a tile has started before it,
+// and each tile takes its carry-in by the decoupled lookback.  Their tiles fit
+// in one or two waves, so a lookback waits about one tile's work; larger
+// scans never wait.
 constexpr u64 kLookbackTiles = 1024;
+
+// The next tile of the scan, for every thread.
+__device__ __forceinline__ u32 next_tile(u32* counter) {
+  __shared__ u32 s_tile;
+  if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
+  __syncthreads();
+  return s_tile;
+}
+// The last tile of a scan to finish (of all its launches) clears the status
+// words and counters: every other tile's lookback is over by then.
+__device__ __forceinline__ void finish_tile(u32* flags, u32* counter, u32 tiles) {
+  __shared__ u32 s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(counter + 1, 1u) + 1 == tiles;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  for (u32 i = threadIdx.x; i < tiles; i += blockDim.x) flags[i] = 0;
+  if (threadIdx.x < 2) counter[threadIdx.x] = 0;
+}
+
 template <class Prod>
 __global__ void __launch_bounds__(kScanThreads, 3) scan_lookback_kernel(Prod prod, u64 total, u64* out, u64 out_limit,
                                                                      u64* side, u32* flags, u32* counter, u32* err,
-                                                                     u32 tile_base) {
-  __shared__ u32 s_tile;
-  if (threadIdx.x == 0) s_tile = tile_base + atomicAdd(counter, 1u);
-  __syncthreads();
-  scan_tile(prod, s_tile, total, out, out_limit, side, flags, err);
+                                                                     u32 tiles) {
+  scan_tile(prod, next_tile(counter), total, out, out_limit, side, flags, err);
+  finish_tile(flags, counter, tiles);
 }
 
 // Step 1: tile tile_base + blockIdx.x with carry-in 0; flags[tile] receives
@@ -63,85 +86,55 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_kernel(Prod prod, u64 to
   scan_tile<Prod, false>(prod, tile_base + blockIdx.x, total, out, out_limit, side, flags, nullptr);
 }
 
-// Step 2: the carries between tiles [t0, t1), in chunks of kCarryChunk
-// tiles.  The chunk's status words come into shared memory with coalesced
-// loads; each thread folds kCarryPer consecutive tiles into the map carry-in
-// -> carry-out (the pair of outputs for carry-in 0 and 1); a scan over the
-// threads composes the maps; each thread walks its tiles again and sets bit 2
-// to the tile's carry-in; the words go back with coalesced stores.  The
-// carry into t0 is *chain (left there by the previous range of the same
-// scan) or 0 when t0 = 0; the carry out of t1 - 1 is left in *chain.
-constexpr int kCarryThreads = 1024, kCarryPer = 32, kCarryChunk = kCarryThreads * kCarryPer;
-__global__ void __launch_bounds__(kCarryThreads) tile_carry_kernel(u32* flags, u64 t0, u64 t1, u32* chain) {
-  __shared__ unsigned char sb[kCarryChunk];
-  __shared__ unsigned char m0[kCarryThreads], m1[kCarryThreads];
-  __shared__ u32 s_carry;
-  const int j = threadIdx.x;
-  if (j == 0) s_carry = t0 > 0 ? *chain : 0u;
-  for (u64 c0 = t0; c0 < t1; c0 += kCarryChunk) {
-    const u64 n = min((u64)kCarryChunk, t1 - c0);
-#pragma unroll 8
-    for (int i = 0; i < kCarryPer; ++i) {
-      const u64 k = (u64)i * kCarryThreads + j;
-      sb[k] = k < n ? (unsigned char)flags[c0 + k] : 2;  // past the range: propagates (the identity map)
-    }
-    __syncthreads();
-    u32 f0 = 0, f1 = 1;
-#pragma unroll 8
-    for (int i = 0; i < kCarryPer; ++i) {
-      const u32 v = sb[j * kCarryPer + i], g = v & 1, p = (v >> 1) & 1;
-      f0 = g | (p & f0);
-      f1 = g | (p & f1);
-    }
-    // inclusive scan: thread j ends with the map of the tiles of threads 0..j
-    for (int d = 1; d < kCarryThreads; d <<= 1) {
-      m0[j] = (unsigned char)f0;
-      m1[j] = (unsigned char)f1;
-      __syncthreads();
-      if (j >= d) {  // the earlier threads' map first, then this one's
-        const u32 e0 = m0[j - d], e1 = m1[j - d];
-        const u32 h0 = e0 ? f1 : f0, h1 = e1 ? f1 : f0;
-        f0 = h0;
-        f1 = h1;
-      }
-      __syncthreads();
-    }
-    m0[j] = (unsigned char)f0;
-    m1[j] = (unsigned char)f1;
-    __syncthreads();
-    const u32 cin = s_carry;
-    u32 c = j == 0 ? cin : (cin ? m1[j - 1] : m0[j - 1]);
-#pragma unroll 8
-    for (int i = 0; i < kCarryPer; ++i) {
-      const u32 v = sb[j * kCarryPer + i];
-      sb[j * kCarryPer + i] = (unsigned char)((v & 3) | (c << 2));
-      c = (v & 1) | ((v >> 1) & c);
-    }
-    __syncthreads();  // every thread has read s_carry and written its tiles
-    if (j == kCarryThreads - 1) s_carry = c;  // tiles past the range propagate: c is the carry out of c0 + n - 1
-#pragma unroll 8
-    for (int i = 0; i < kCarryPer; ++i) {
-      const u64 k = (u64)i * kCarryThreads + j;
-      if (k < n) flags[c0 + k] = sb[k];
-    }
-    __syncthreads();
-  }
-  if (j == 0) *chain = s_carry;
-}
-
-// Step 3: a tile whose carry-in is 1 adds it at its first limb; it ripples
-// while limbs wrap to zero, at most to the tile's end (a tile of all-ones
-// limbs passes the carry on through its propagate bit instead).
+// Step 2: 32 tiles a CTA.  The carry into the range is the generate bit of the
+// nearest earlier tile that does not propagate (0 when all do): the CTA looks
+// 256 tiles further back at a time, for random limbs once.  Earlier ranges of
+// the same scan are complete (stream order).  One ballot gives every tile of
+// the range its carry-in: lane t of warp 0 adds tile t's at its first limb,
+// where it ripples while limbs wrap to zero; a tile that propagates holds
+// ones only and becomes zeros, by the whole CTA (a difference of nearly equal
+// operands has long runs of such tiles).
+constexpr int kFixTiles = 32;
 __global__ void __launch_bounds__(256) carry_fix_kernel(const u32* flags, u64 t0, u64 t1, u64 total, u64* out,
                                                         u64 out_limit, u64* side) {
-  const u64 t = t0 + (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= t1 || !((flags[t] >> 2) & 1)) return;
-  const u64 end = min((t + 1) * kScanTile, total);
-  for (u64 k = t * kScanTile; k < end; ++k) {
-    u64* q = k < out_limit ? out + k : side + (k - out_limit);
-    const u64 v = *q + 1;
-    *q = v;
-    if (v != 0) break;
+  __shared__ u32 s_first, s_cin, s_ones;
+  const u64 c0 = t0 + (u64)blockIdx.x * kFixTiles;
+  const int tid = threadIdx.x;
+  u32 cin = 0;
+  for (u64 back = c0; back > 0;) {  // the same for every thread
+    const u32 f = (u64)tid < back ? flags[back - 1 - tid] : 0;  // before tile 0: a kill
+    __syncthreads();
+    if (tid == 0) s_first = 256;
+    __syncthreads();
+    if (!((f >> 1) & 1)) atomicMin(&s_first, (u32)tid);
+    __syncthreads();
+    const u32 first = s_first;
+    if (first < 256) {
+      if ((u32)tid == first) s_cin = f & 1;
+      __syncthreads();
+      cin = s_cin;
+      break;
+    }
+    back = back > 256 ? back - 256 : 0;
+  }
+  auto limb = [&](u64 k) { return k < out_limit ? out + k : side + (k - out_limit); };
+  if (tid < 32) {
+    const u64 t = c0 + tid;
+    const u32 f = t < t1 ? flags[t] : 0;
+    const u32 G = __ballot_sync(0xffffffffu, f & 1), GP = __ballot_sync(0xffffffffu, f & 3);
+    const u32 in = (u32)((u64)G + GP + cin) ^ G ^ GP;  // the carry into each lane's tile
+    const u32 ones = in & GP & ~G;
+    if (tid == 0) s_ones = ones;
+    if (t < t1 && (((in & ~ones) >> tid) & 1)) {
+      const u64 end = min((t + 1) * kScanTile, total);
+      for (u64 k = t * kScanTile; k < end; ++k)
+        if (++*limb(k) != 0) break;
+    }
+  }
+  __syncthreads();
+  for (u32 ones = s_ones; ones; ones &= ones - 1) {
+    const u64 t = c0 + __ffs(ones) - 1, end = min((t + 1) * kScanTile, total);
+    for (u64 k = t * kScanTile + tid; k < end; k += 256) *limb(k) = 0;
   }
 }
 
@@ -204,41 +197,21 @@ __global__ void wait_probe_kernel(const u32* flag, u32* err, int limit) {
   if (threadIdx.x == 0 && wait_flag(flag, limit) == 0) atomicExch(err, 1u);
 }
 
-// Base-case products of at most kColumnSumPositions positions go in two
-// launches: their column sums into the scan's sums, then the carry scan over
-// them.  A column sum is split over kSumLanes threads (thread j of a column
-// takes every kSumLanes-th term from its own start, so the threads of a
-// column read consecutive limbs of a and of b) and the partial three-word
-// sums meet in three shuffle steps.  The one-launch scan gives each thread
-// eight whole columns, so a product of a few hundred limbs had one CTA of
-// threads that each add eight columns in turn (measured: 383 x 383 limbs,
-// 137 us); one thread a column took 27 us.
-constexpr u64 kColumnSumPositions = 1 << 20;  // at most 24 MiB of sums
-constexpr int kSumLanes = 8;
-__global__ void __launch_bounds__(256) column_sums_kernel(ColumnProducer prod, u64 total, u64* sums) {
-  const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-  const u64 k = t / kSumLanes;
-  const u32 j = (u32)(t % kSumLanes);
-  W3 r{0, 0, 0};
-  if (k < total && k + 1 < prod.na + prod.nb) {
-    const u64 lo = k >= prod.nb ? k - prod.nb + 1 : 0;
-    const u64 hi = k < prod.na - 1 ? k : prod.na - 1;
-    for (u64 i = lo + j; i <= hi; i += kSumLanes) {
-      const u64 x = prod.a[i], y = prod.b[k - i];
-      r = add_w3(r, W3{x * y, mulhi(x, y), 0});
-    }
-  }
-#pragma unroll
-  for (int d = kSumLanes / 2; d >= 1; d >>= 1) {  // every lane of the warp takes part
-    const W3 o{__shfl_down_sync(0xffffffffu, r.w0, d, kSumLanes), __shfl_down_sync(0xffffffffu, r.w1, d, kSumLanes),
-               __shfl_down_sync(0xffffffffu, r.w2, d, kSumLanes)};
-    r = add_w3(r, o);
-  }
-  if (j == 0 && k < total) {
-    sums[k] = r.w0;
-    sums[total + k] = r.w1;
-    sums[2 * total + k] = r.w2;
-  }
+// Base-case products of at most 2^20 positions: each CTA forms
+// its tile's column sums in shared memory and takes the tile through the
+// lookback scan, one launch.  Small tiles spread a short product over the
+// GPU: the column sums are the work, up to 383 terms a position.
+constexpr u64 kSchoolShortTile = 256, kSchoolTile = 64, kSchoolLongTile = 1024;
+template <u64 TILE, bool ONE>
+__global__ void __launch_bounds__(256) school_kernel(ColumnProducer prod, u64 total, u64* out, u32* flags,
+                                                     u32* counter, u32* err, u32 tiles) {
+  __shared__ u64 sums[3 * (TILE + kScanE)];
+  const u32 tile = ONE ? 0 : next_tile(counter);
+  column_tile_sums<256, TILE>(sums, prod, tile);
+  __syncthreads();
+  scan_tile<SmemSumsProducer<TILE>, !ONE, 256, TILE>(SmemSumsProducer<TILE>{sums, tile * TILE - kScanE, total}, tile,
+                                                     total, out, total, nullptr, ONE ? nullptr : flags, err);
+  if (!ONE) finish_tile(flags, counter, tiles);
 }
 
 // One warp a job: lane i adds limb base + i of x and y; the block's carries
@@ -279,8 +252,7 @@ __global__ void __launch_bounds__(256) add_batch_kernel(const AddJob* __restrict
 
 // Tiles [tile_begin, tile_end) of the scan (all of them by default).  The
 // ranges of one scan go in order on one stream (each range's carry-in comes
-// from the range before: through the status words of the lookback, or the
-// chain word of the three steps).
+// from the words of the tiles before it).
 template <class Prod>
 cudaError_t run_scan(const Prod& prod, u64 total, u64* out, u64 out_limit, Scan& sc, cudaStream_t st,
                      const char* name, u64 tile_begin = 0, u64 tile_end = ~0ull) {
@@ -289,28 +261,37 @@ cudaError_t run_scan(const Prod& prod, u64 total, u64* out, u64 out_limit, Scan&
   cudaError_t e = scan_reserve(sc, tiles);
   if (e != cudaSuccess || tile_end <= tile_begin) return e;
   const u64 n = tile_end - tile_begin;
+  if (tiles == 1) {  // neither a tile number nor a status word: four dependent accesses of global memory less
+    launch_begin(name, st);
+    scan_kernel<Prod><<<1, kScanThreads, 0, st>>>(prod, total, out, out_limit, sc.side, nullptr, 0);
+    launch_end(st);
+    return cudaGetLastError();
+  }
   if (tiles <= kLookbackTiles) {
-    if (tile_begin == 0) {
-      e = cudaMemsetAsync(sc.flags, 0, (tiles + 1) * sizeof(u32), st);
-      if (e != cudaSuccess) return e;
-    }
-    e = cudaMemsetAsync(sc.counter, 0, sizeof(u32), st);
-    if (e != cudaSuccess) return e;
     launch_begin(name, st);
     scan_lookback_kernel<Prod><<<(unsigned)n, kScanThreads, 0, st>>>(prod, total, out, out_limit, sc.side, sc.flags,
-                                                                      sc.counter, sc.err, (u32)tile_begin);
+                                                                      sc.counter, sc.err, (u32)tiles);
     launch_end(st);
     return cudaGetLastError();
   }
   launch_begin(name, st);
-  scan_kernel<Prod><<<(unsigned)n, kScanThreads, 0, st>>>(prod, total, out, out_limit, sc.side, sc.flags, tile_begin);
-  launch_end(st);
-  launch_begin("scan_tile_carries", st);
-  tile_carry_kernel<<<1, kCarryThreads, 0, st>>>(sc.flags, tile_begin, tile_end, sc.chain);
+  scan_kernel<Prod><<<(unsigned)n, kScanThreads, 0, st>>>(prod, total, out, out_limit, sc.side, sc.wide, tile_begin);
   launch_end(st);
   launch_begin("scan_carry_fix", st);
-  carry_fix_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(sc.flags, tile_begin, tile_end, total, out, out_limit,
+  carry_fix_kernel<<<(unsigned)((n + kFixTiles - 1) / kFixTiles), 256, 0, st>>>(sc.wide, tile_begin, tile_end, total, out, out_limit,
                                                                  sc.side);
+  launch_end(st);
+  return cudaGetLastError();
+}
+
+template <u64 TILE>
+cudaError_t launch_school(const ColumnProducer& prod, u64 total, u64* out, Scan& sc, cudaStream_t st) {
+  const u32 tiles = (u32)((total + TILE - 1) / TILE);  // at most kLookbackTiles
+  launch_begin("school_tiles", st);
+  if (tiles == 1)
+    school_kernel<TILE, true><<<1, 256, 0, st>>>(prod, total, out, nullptr, nullptr, nullptr, 1);
+  else
+    school_kernel<TILE, false><<<tiles, 256, 0, st>>>(prod, total, out, sc.flags, sc.counter, sc.err, tiles);
   launch_end(st);
   return cudaGetLastError();
 }
@@ -321,31 +302,39 @@ u64 scan_tiles(u64 positions) { return positions ? (positions + kScanTile - 1) /
 
 cudaError_t scan_reserve(Scan& sc, u64 tiles) {
   if (sc.flags && sc.max_tiles >= tiles) return cudaSuccess;
-  if (sc.flags) cudaFree(sc.flags);
-  u64 cap = sc.max_tiles ? sc.max_tiles : 1024;
+  if (sc.flags) cudaFree(sc.flags);  // waits for the device: no scan is using it
+  u64 cap = sc.max_tiles ? sc.max_tiles : kLookbackTiles;
   while (cap < tiles) cap *= 2;
-  cudaError_t e = cudaMalloc((void**)&sc.flags, (cap + 1) * sizeof(u32));
+  // the lookback's status words (only scans of up to kLookbackTiles tiles use
+  // them), then the carry bits of longer scans
+  cudaError_t e = cudaMalloc((void**)&sc.flags, (kLookbackTiles + 1 + cap) * sizeof(u32));
+  if (e == cudaSuccess) e = cudaMemset(sc.flags, 0, (kLookbackTiles + 1) * sizeof(u32));
   if (e != cudaSuccess) {
-    sc.flags = nullptr;
+    if (sc.flags) cudaFree(sc.flags);
+    sc.flags = sc.wide = nullptr;
     sc.max_tiles = 0;
     return e;
   }
+  sc.wide = sc.flags + kLookbackTiles + 1;
   sc.max_tiles = cap;
   if (!sc.counter) {
     e = cudaMalloc((void**)&sc.counter, 4 * sizeof(u32) + 4 * sizeof(u64));
     if (e != cudaSuccess) return e;
-    sc.err = sc.counter + 1;
-    sc.chain = sc.counter + 2;
+    sc.err = sc.counter + 2;
     sc.side = reinterpret_cast<u64*>(sc.counter + 4);
     e = cudaMemset(sc.counter, 0, 4 * sizeof(u32) + 4 * sizeof(u64));
   }
   return e;
 }
 
+cudaError_t scan_reset(Scan& sc, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(sc.flags, 0, (kLookbackTiles + 1) * sizeof(u32), st);
+  return e == cudaSuccess ? cudaMemsetAsync(sc.counter, 0, 2 * sizeof(u32), st) : e;
+}
+
 void scan_free(Scan& sc) {
   if (sc.flags) cudaFree(sc.flags);
   if (sc.counter) cudaFree(sc.counter);
-  if (sc.sums) cudaFree(sc.sums);
   sc = Scan{};
 }
 
@@ -397,25 +386,11 @@ cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Sca
   cudaError_t e = scan_reserve(sc, 1);
   if (e != cudaSuccess) return e;
   const u64 total = na + nb;
-  if (total > kColumnSumPositions)
-    return run_scan(ColumnProducer{a, na, b, nb}, total, out, total, sc, st, "school_column_scan");
-  if (sc.sums_cap < total) {  // grow-only, by doubling from 4096 positions (96 KiB)
-    u64 cap = std::max<u64>(sc.sums_cap, 4096);
-    while (cap < total) cap *= 2;
-    if (sc.sums) cudaFree(sc.sums);
-    sc.sums = nullptr;
-    sc.sums_cap = 0;
-    e = cudaMalloc((void**)&sc.sums, 3 * cap * sizeof(u64));
-    if (e != cudaSuccess) return e;
-    sc.sums_cap = cap;
-  }
-  launch_begin("school_column_sums", st);
-  column_sums_kernel<<<(unsigned)((total * kSumLanes + 255) / 256), 256, 0, st>>>(ColumnProducer{a, na, b, nb}, total,
-                                                                                 sc.sums);
-  launch_end(st);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  return run_scan(SumsProducer{sc.sums, total}, total, out, total, sc, st, "school_column_scan");
+  const ColumnProducer prod{a, na, b, nb};
+  if (total <= kSchoolShortTile && nb <= 64) return launch_school<kSchoolShortTile>(prod, total, out, sc, st);
+  if (total <= kSchoolTile * kLookbackTiles) return launch_school<kSchoolTile>(prod, total, out, sc, st);
+  if (total <= kSchoolLongTile * kLookbackTiles) return launch_school<kSchoolLongTile>(prod, total, out, sc, st);
+  return run_scan(prod, total, out, total, sc, st, "school_column_scan");
 }
 
 cudaError_t add_shifted(const u64* x, u64 nx, const u64* y, u64 ny, u64 shift, u64* out, u64 n, Scan& sc,

@@ -103,14 +103,12 @@ SixCrt six_crt(int s);
 
 // Scratch for the carry scan.
 struct Scan {
-  u32* flags = nullptr;  // per-tile status words
-  u32* counter = nullptr;
+  u32* flags = nullptr;  // per-tile status words of a lookback, zero between scans (the last tile clears them)
+  u32* wide = nullptr;   // per-tile carry bits of the scans that do not wait
+  u32* counter = nullptr;  // the lookback's next tile and finished tiles (two words, zero between scans)
   u32* err = nullptr;    // nonzero after a lookback wait gave up
-  u32* chain = nullptr;  // carry between consecutive tile ranges of one scan
   u64* side = nullptr;   // limbs of the scan beyond the output (the carry words)
   u64 max_tiles = 0;
-  u64* sums = nullptr;   // column sums of base-case products, three words a position
-  u64 sums_cap = 0;      // positions they have room for
 };
 constexpr int kScanThreads = 256;
 constexpr int kScanE = 8;  // limbs per thread
@@ -271,6 +269,8 @@ std::string profile_report();
 
 u64 scan_tiles(u64 positions);
 cudaError_t scan_reserve(Scan& sc, u64 tiles);
+// Clears the lookback's words (after a wait gave up).
+cudaError_t scan_reset(Scan& sc, cudaStream_t st);
 void scan_free(Scan& sc);
 
 }  // namespace nn

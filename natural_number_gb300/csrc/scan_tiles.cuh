@@ -321,27 +321,99 @@ struct ColumnProducer {
   }
 };
 
-// Three-word values stored as three arrays (word i of position k at
-// s[i * total + k]): the column sums of a base-case product, computed before
-// the scan by one thread a position.
-struct SumsProducer {
+// The column sums of one scan tile's positions and of the kScanE positions
+// before them (the scan reads those too) in shared memory, as three word
+// arrays of TILE + kScanE: all NT threads at once, eight lanes a position,
+// the partial sums meeting in three shuffle steps.  (With one thread forming
+// its eight scan positions' sums in turn, a product of a few hundred limbs
+// keeps a few dozen threads busy.)
+template <u64 TILE>
+struct SmemSumsProducer {
   static constexpr bool kBulk = true;
   const u64* s;
+  u64 first;  // the position at s[0] (mod 2^64: tile 0's is -kScanE)
   u64 total;
   __device__ __forceinline__ W3 operator()(u64 k) const {
     if (k >= total) return W3{0, 0, 0};
-    return W3{s[k], s[total + k], s[2 * total + k]};
+    const u64 i = k - first;
+    return W3{s[i], s[TILE + kScanE + i], s[2 * (TILE + kScanE) + i]};
   }
   __device__ __forceinline__ void bulk(u64 k0, W3 (&x)[kScanE]) const {
 #pragma unroll
     for (int e = 0; e < kScanE; ++e) x[e] = (*this)(k0 + e);
   }
 };
+template <int NT, u64 TILE>
+__device__ __forceinline__ void column_tile_sums(u64* sm, const ColumnProducer& J, u64 tile) {
+  constexpr u32 kLanes = 8, kGroups = NT / kLanes;
+  const u64 size = J.na + J.nb;
+  const long long first = (long long)(tile * TILE) - kScanE;
+  const u64 end = min(size, (tile + 1) * TILE);
+  const u32 npos = (u32)((long long)end - first);  // at most TILE + kScanE
+  const u32 g = threadIdx.x / kLanes, j = threadIdx.x % kLanes;
+  const u32 rounds = (npos + kGroups - 1) / kGroups;  // the same for every thread
+  for (u32 r = 0; r < rounds; ++r) {
+    const u32 q = r * kGroups + g;
+    const long long p = first + q;
+    W3 acc{0, 0, 0};
+    if (q < npos && p >= 0 && (u64)p + 1 < size) {
+      const u64 k = (u64)p;
+      const u64 lo = k >= J.nb ? k - J.nb + 1 : 0;
+      const u64 hi = k < J.na - 1 ? k : J.na - 1;
+      for (u64 i = lo + j; i <= hi; i += kLanes) {
+        const u64 x = J.a[i], y = J.b[k - i];
+        acc = add_w3(acc, W3{x * y, mulhi(x, y), 0});
+      }
+    }
+#pragma unroll
+    for (u32 d = kLanes / 2; d >= 1; d >>= 1) {  // every lane of the warp takes part
+      const W3 o{__shfl_down_sync(0xffffffffu, acc.w0, d, kLanes), __shfl_down_sync(0xffffffffu, acc.w1, d, kLanes),
+                 __shfl_down_sync(0xffffffffu, acc.w2, d, kLanes)};
+      acc = add_w3(acc, o);
+    }
+    if (j == 0 && q < npos) {
+      sm[q] = acc.w0;
+      sm[TILE + kScanE + q] = acc.w1;
+      sm[2 * (TILE + kScanE) + q] = acc.w2;
+    }
+  }
+}
+
+// Limbs of x * B^shift at positions k0 .. k0 + 7 (zero outside x), a thread's
+// share of a sum: 16-byte loads from the first 16-byte boundary on.
+__device__ __forceinline__ void eight_limbs(u64 (&v)[kScanE], const u64* x, u64 n, u64 shift, u64 k0) {
+  if (k0 >= shift && k0 - shift + kScanE <= n) {
+    const u64* p = x + (k0 - shift);
+    const int odd = (int)((reinterpret_cast<uintptr_t>(p) >> 3) & 1);
+    if (odd) {
+      v[0] = p[0];
+#pragma unroll
+      for (int e = 1; e + 1 < kScanE; e += 2) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p + e);
+        v[e] = t.x;
+        v[e + 1] = t.y;
+      }
+      v[kScanE - 1] = p[kScanE - 1];
+    } else {
+#pragma unroll
+      for (int e = 0; e < kScanE; e += 2) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p + e);
+        v[e] = t.x;
+        v[e + 1] = t.y;
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int e = 0; e < kScanE; ++e) {
+    const u64 k = k0 + e;
+    v[e] = k >= shift && k - shift < n ? x[k - shift] : 0;
+  }
+}
 
 // x[k] + y[k - shift] (two words).
 struct AddProducer {
-  static constexpr bool kBulk = false;
-  __device__ __forceinline__ void bulk(u64, W3 (&)[kScanE]) const {}
+  static constexpr bool kBulk = true;
   const u64* x;
   u64 nx;
   const u64* y;
@@ -353,6 +425,16 @@ struct AddProducer {
     const u64 s = a + b;
     return W3{s, (u64)(s < a), 0};
   }
+  __device__ __forceinline__ void bulk(u64 k0, W3 (&w)[kScanE]) const {
+    u64 a[kScanE], b[kScanE];
+    eight_limbs(a, x, nx, 0, k0);
+    eight_limbs(b, y, ny, shift, k0);
+#pragma unroll
+    for (int e = 0; e < kScanE; ++e) {
+      const u64 s = a[e] + b[e];
+      w[e] = W3{s, (u64)(s < a[e]), 0};
+    }
+  }
 };
 
 // x*B^xs + y*B^ys (add) or, as x*B^xs + ~(y*B^ys) + cin over `count`
@@ -363,8 +445,7 @@ struct AddProducer {
 // thread) swaps add and subtract, so a sign known only on the device picks
 // the operation without a round trip to the host.
 struct LinProducer {
-  static constexpr bool kBulk = false;
-  __device__ __forceinline__ void bulk(u64, W3 (&)[kScanE]) const {}
+  static constexpr bool kBulk = true;
   const u64* x;
   u64 nx, xs;
   const u64* y;
@@ -386,6 +467,19 @@ struct LinProducer {
     const u64 s2 = s + c;
     const u64 c2 = s2 < s;
     return W3{s2, c1 + c2, 0};
+  }
+  __device__ __forceinline__ void bulk(u64 k0, W3 (&w)[kScanE]) const {
+    u64 a[kScanE], b[kScanE];
+    eight_limbs(a, x, nx, xs, k0);
+    eight_limbs(b, y, ny, ys, k0);
+    const bool neg = sub ^ (flip != nullptr && __ldcg(flip) != 0);
+#pragma unroll
+    for (int e = 0; e < kScanE; ++e) {
+      const u64 v = neg ? ~b[e] : b[e];
+      const u64 c = neg && k0 + e == 0 ? (u64)cin : 0;
+      const u64 s = a[e] + v, s2 = s + c;
+      w[e] = k0 + e < count ? W3{s2, (u64)(s < a[e]) + (u64)(s2 < s), 0} : W3{0, 0, 0};
+    }
   }
 };
 
@@ -413,7 +507,7 @@ __device__ __forceinline__ u32 wait_flag(const u32* f, int limit) {
 // LOOKBACK: the tile takes its carry-in from its predecessors' status words
 // (decoupled lookback); tiles of one scan must then start in increasing order
 // (their predecessors already running), which the callers guarantee.
-// Without LOOKBACK the tile takes carry-in 0 and records in flags[tile] its
+// Without LOOKBACK the tile takes carry-in 0 and records in flags[tile] (when given) its
 // carry out for carry-in 0 (bit 0, generate) and whether a carry-in would pass
 // straight through (bit 1, propagate: every limb all ones); a later step
 // resolves the one-bit carries between tiles (carry.cu).
@@ -433,12 +527,14 @@ __device__ __forceinline__ ScanShared<NT>& scan_shared() {
   return sh;
 }
 
-// NT: threads of the CTA; a tile is NT * kScanE positions.
-template <class Prod, bool LOOKBACK = true, int NT = kScanThreads>
+// NT: threads of the CTA.  TILE: positions of a tile, NT * kScanE at most;
+// with fewer, the threads beyond them pass carries on unchanged.
+template <class Prod, bool LOOKBACK = true, int NT = kScanThreads, u64 TILE = (u64)NT * kScanE>
 __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total, u64* out, u64 out_limit, u64* side,
                                           u32* flags, u32* err) {
   constexpr int E = kScanE;
-  constexpr u64 kTile = (u64)NT * E;
+  constexpr u64 kTile = TILE;
+  static_assert(TILE % E == 0 && TILE <= (u64)NT * E);
   ScanShared<NT>& sh = scan_shared<NT>();
   u64* const s_h0 = sh.h0;
   u64* const s_h1 = sh.h1;
@@ -446,16 +542,17 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
   u32* const s_wp = sh.wp;
   u32& s_cin = sh.cin;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool on = TILE == (u64)NT * E || (u64)tid * E < TILE;
   const u64 k0 = tile * kTile + (u64)tid * E;
 
   u64 y[E];
   u64 c0 = 0, c1 = 0;
   W3 xs[E];
-  if (Prod::kBulk && k0 + E <= total) {
+  if (Prod::kBulk && on && k0 + E <= total) {
     prod.bulk(k0, xs);
   } else {
 #pragma unroll
-    for (int e = 0; e < E; ++e) xs[e] = k0 + e < total ? prod(k0 + e) : W3{0, 0, 0};
+    for (int e = 0; e < E; ++e) xs[e] = on && k0 + e < total ? prod(k0 + e) : W3{0, 0, 0};
   }
 #pragma unroll
   for (int e = 0; e < E; ++e) {
@@ -490,7 +587,7 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
     hp1 = d1;
   }
   __syncthreads();
-  if (tid > 0) {
+  if (tid > 0 && on) {
     hp0 = s_h0[tid - 1];
     hp1 = s_h1[tid - 1];
   }
@@ -500,7 +597,7 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
   u64 all = y[0];
 #pragma unroll
   for (int e = 1; e < E; ++e) all &= y[e];
-  const u32 pr = (all == ~0ull) & !g;
+  const u32 pr = !on | ((all == ~0ull) & !g);
 
   const u32 G = __ballot_sync(0xffffffffu, g);
   const u32 GP = __ballot_sync(0xffffffffu, g | pr);
@@ -519,7 +616,7 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
     const u32 tg = c_if0, tp = c_if1 & !c_if0;
     u32 cin = 0;
     if (!LOOKBACK) {
-      flags[tile] = tg | (tp << 1);
+      if (flags) flags[tile] = tg | (tp << 1);
     } else if (tile > 0) {
       flag_store(&flags[tile], kFlagAggregate | (tg << 2) | (tp << 3));
       long long j = (long long)tile - 1;
@@ -558,6 +655,7 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
   const u64 sum = (u64)G + GP + wc;
   const u32 cin_bits = (u32)sum ^ G ^ GP;
   add_ripple8(y, (cin_bits >> lane) & 1, 0);  // its carry out is the next thread's carry-in, counted above
+  if (!on) return;
   if (k0 + E <= out_limit && k0 + E <= total && !(reinterpret_cast<uintptr_t>(out) & 15)) {
 #pragma unroll
     for (int e = 0; e < E; e += 2) *reinterpret_cast<ulonglong2*>(out + k0 + e) = make_ulonglong2(y[e], y[e + 1]);

@@ -117,24 +117,25 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
   col_tile<R, col_width(R), col_threads(R), INV, false>(sm6, res, s, lambda0, blockIdx.x, blockIdx.y, tab, cap, raw);
 }
 
-constexpr int fused_threads(int R, int LGM) { return std::max(32, (1 << (R + LGM)) / 32); }
-// Two tiles of 4096 words in shared memory let six CTAs of 128 threads share
-// an SM (80 registers a thread); smaller tiles keep that register budget.
-constexpr int fused_blocks(int R, int LGM) { return std::min(16, 768 / fused_threads(R, LGM)); }
-template <int R, int LGM, bool FIRST>
-__global__ void __launch_bounds__(fused_threads(R, LGM), fused_blocks(R, LGM))
+// One unit of eight rows x V columns a thread.
+constexpr int fused_threads(int R, int LGM, int V) { return std::max(32, (1 << (R + LGM)) / (8 * V)); }
+// Two tiles of 4096 words in shared memory let six CTAs share an SM: 768
+// threads (80 registers) of four columns each, more of fewer columns.
+constexpr int fused_blocks(int R, int LGM, int V) { return std::min(24, (V == 4 ? 768 : 1024) / fused_threads(R, LGM, V)); }
+template <int R, int LGM, int V, bool FIRST>
+__global__ void __launch_bounds__(fused_threads(R, LGM, V), fused_blocks(R, LGM, V))
     six_fused_kernel(SixOperands op, int s, const int2* __restrict__ tab, u64 cap, bool reduce_in) {
   extern __shared__ __align__(16) u32 sm6[];
-  constexpr int NT = fused_threads(R, LGM);
+  constexpr int NT = fused_threads(R, LGM, V);
   u32* out = op.ra + ((u64)blockIdx.z * kPrimes << s);
   const int2* itab = tab + kPrimes * cap;
   if constexpr (FIRST) {
     const u64 at0 = blockIdx.z * op.piece;
-    fused_tile<R, LGM, NT, true, false>(sm6, op.a + at0, min(op.piece, op.na - at0), op.b, op.nb, out, s, 0, blockIdx.y,
-                                        tab, itab, cap, false, op.pieces == 1);
+    fused_tile<R, LGM, NT, V, true, false>(sm6, op.a + at0, min(op.piece, op.na - at0), op.b, op.nb, out, s, 0,
+                                           blockIdx.y, tab, itab, cap, false, op.pieces == 1);
   } else {
-    fused_tile<R, LGM, NT, false, false>(sm6, out, 0, op.b ? op.rb : nullptr, 0, out, s, blockIdx.x, blockIdx.y, tab,
-                                         itab, cap, reduce_in, false);
+    fused_tile<R, LGM, NT, V, false, false>(sm6, out, 0, op.b ? op.rb : nullptr, 0, out, s, blockIdx.x, blockIdx.y,
+                                            tab, itab, cap, reduce_in, false);
   }
 }
 
@@ -168,17 +169,29 @@ cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, int s, int lambda0, const S
   launch_end(st);
   return cudaGetLastError();
 }
-template <int R, int LGM, bool FIRST>
-cudaError_t launch_fused(const SixOperands& op, int s, const SixTables& t, bool reduce_in, cudaStream_t st) {
+template <int R, int LGM, int V, bool FIRST>
+cudaError_t launch_fused_v(const SixOperands& op, int s, const SixTables& t, bool reduce_in, cudaStream_t st) {
   constexpr int tile = (int)tile_words32<1 << LGM>(R) * 4;
-  static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, FIRST>, 2 * tile);
+  static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, V, FIRST>, 2 * tile);
   if (ok != cudaSuccess) return ok;
   const int smem = (op.b ? 2 : 1) * tile;
   const dim3 grid(FIRST ? 1u : (unsigned)((1ull << s) >> (R + LGM)), kPrimes, op.pieces);
   launch_begin(FIRST ? "six_small_pass" : "six_fused_row_pass", st);
-  six_fused_kernel<R, LGM, FIRST><<<grid, fused_threads(R, LGM), smem, st>>>(op, s, t.tab, t.cap, reduce_in);
+  six_fused_kernel<R, LGM, V, FIRST><<<grid, fused_threads(R, LGM, V), smem, st>>>(op, s, t.tab, t.cap, reduce_in);
   launch_end(st);
   return cudaGetLastError();
+}
+// Columns a thread: as few as keep the grid within one wave of the GPU's
+// 152 x 768 threads, so a short product uses as many of them as it can.
+template <int R, int LGM, bool FIRST>
+cudaError_t launch_fused(const SixOperands& op, int s, const SixTables& t, bool reduce_in, cudaStream_t st) {
+  if constexpr (LGM == 3) {
+    const u64 units = ((u64)kPrimes * op.pieces << s) / 8;  // of one column
+    if (units <= 152 * 768) return launch_fused_v<R, LGM, 1, FIRST>(op, s, t, reduce_in, st);
+    if constexpr (R == 9)
+      if (units <= 2 * 152 * 768) return launch_fused_v<R, LGM, 2, FIRST>(op, s, t, reduce_in, st);
+  }
+  return launch_fused_v<R, LGM, 4, FIRST>(op, s, t, reduce_in, st);
 }
 
 cudaError_t load_pass(const SixOperands& op, int s, int R, const SixTables& t, u32 t0, u32 t1, cudaStream_t st) {

@@ -97,33 +97,72 @@ __device__ __forceinline__ i32 mont(i64 c, const Prime& P) {
   return (i32)((u32)(c >> 32) - (u32)__mulhi(m, P.p));
 }
 
-// A twiddle pair and two neighbouring ones (16-byte load).
+// V neighbouring words: one 16-, 8- or 4-byte access.
+template <int V>
+struct alignas(4 * V) Words {
+  i32 v[V];
+};
+template <bool CG, int V>
+__device__ __forceinline__ Words<V> ldv(const void* p) {
+  Words<V> w;
+  if constexpr (V == 4) {
+    const int4* q = reinterpret_cast<const int4*>(p);
+    const int4 t = CG ? __ldcg(q) : *q;
+    w.v[0] = t.x, w.v[1] = t.y, w.v[2] = t.z, w.v[3] = t.w;
+  } else if constexpr (V == 2) {
+    const int2* q = reinterpret_cast<const int2*>(p);
+    const int2 t = CG ? __ldcg(q) : *q;
+    w.v[0] = t.x, w.v[1] = t.y;
+  } else {
+    const i32* q = reinterpret_cast<const i32*>(p);
+    w.v[0] = CG ? __ldcg(q) : *q;
+  }
+  return w;
+}
+template <bool CG, int V>
+__device__ __forceinline__ void stv(void* p, const Words<V>& w) {
+  if constexpr (V == 4) {
+    const int4 t = make_int4(w.v[0], w.v[1], w.v[2], w.v[3]);
+    if (CG)
+      __stcg(reinterpret_cast<int4*>(p), t);
+    else
+      *reinterpret_cast<int4*>(p) = t;
+  } else if constexpr (V == 2) {
+    const int2 t = make_int2(w.v[0], w.v[1]);
+    if (CG)
+      __stcg(reinterpret_cast<int2*>(p), t);
+    else
+      *reinterpret_cast<int2*>(p) = t;
+  } else {
+    if (CG)
+      __stcg(reinterpret_cast<i32*>(p), w.v[0]);
+    else
+      *reinterpret_cast<i32*>(p) = w.v[0];
+  }
+}
 template <bool CG>
 __device__ __forceinline__ int4 ld4(const void* p) {
   const int4* q = reinterpret_cast<const int4*>(p);
-  if (CG) return __ldcg(q);
-  return *q;
-}
-template <bool CG>
-__device__ __forceinline__ void st4(void* p, int4 v) {
-  int4* q = reinterpret_cast<int4*>(p);
-  if (CG)
-    __stcg(q, v);
-  else
-    *q = v;
+  return CG ? __ldcg(q) : *q;
 }
 
-// A unit: 2^K rows of four neighbouring columns in registers.
-template <int K>
+// A unit: 2^K rows of V neighbouring columns in registers.  V = 4 has the
+// fewest shared-memory instructions and twiddle loads a butterfly; V = 1 and 2
+// spread a short transform over four and two times the threads, where the
+// GPU would otherwise be mostly idle.
+template <int K, int V>
 struct Unit {
-  i32 x[1 << K][4];
-  __device__ __forceinline__ void set(int m, int4 v) {
-    x[m][0] = v.x;
-    x[m][1] = v.y;
-    x[m][2] = v.z;
-    x[m][3] = v.w;
+  i32 x[1 << K][V];
+  __device__ __forceinline__ void set(int m, const Words<V>& w) {
+#pragma unroll
+    for (int c = 0; c < V; ++c) x[m][c] = w.v[c];
   }
-  __device__ __forceinline__ int4 get(int m) const { return make_int4(x[m][0], x[m][1], x[m][2], x[m][3]); }
+  __device__ __forceinline__ Words<V> get(int m) const {
+    Words<V> w;
+#pragma unroll
+    for (int c = 0; c < V; ++c) w.v[c] = x[m][c];
+    return w;
+  }
 };
 
 // The twiddle pairs of local level lv of a unit whose block index at the
@@ -143,8 +182,8 @@ __device__ __forceinline__ void twiddles(int2 (&w)[1 << LV], const int2* __restr
   }
 }
 
-template <int K, int LV>
-__device__ __forceinline__ void fwd_level(Unit<K>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+template <int K, int V, int LV>
+__device__ __forceinline__ void fwd_level(Unit<K, V>& u, const int2* __restrict__ tw, u32 b, i32 p) {
   int2 w[1 << LV];
   twiddles<LV>(w, tw, b);
   constexpr int half = (1 << K) >> (LV + 1);
@@ -153,20 +192,20 @@ __device__ __forceinline__ void fwd_level(Unit<K>& u, const int2* __restrict__ t
 #pragma unroll
     for (int m = 0; m < half; ++m)
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
+      for (int c = 0; c < V; ++c)
         fwd_bfly(u.x[g * 2 * half + m][c], u.x[g * 2 * half + m + half][c], w[g].x, w[g].y, p);
 }
 // Levels [LV0, K) of a unit.
-template <int K, int LV = 0>
-__device__ __forceinline__ void fwd_levels(Unit<K>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+template <int K, int LV = 0, int V>
+__device__ __forceinline__ void fwd_levels(Unit<K, V>& u, const int2* __restrict__ tw, u32 b, i32 p) {
   if constexpr (LV < K) {
-    fwd_level<K, LV>(u, tw, b, p);
+    fwd_level<K, V, LV>(u, tw, b, p);
     fwd_levels<K, LV + 1>(u, tw, b, p);
   }
 }
 
-template <int K, int LV>
-__device__ __forceinline__ void inv_level(Unit<K>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+template <int K, int V, int LV>
+__device__ __forceinline__ void inv_level(Unit<K, V>& u, const int2* __restrict__ tw, u32 b, i32 p) {
   int2 w[1 << LV];
   twiddles<LV>(w, tw, b);
   constexpr int half = (1 << K) >> (LV + 1);
@@ -175,23 +214,23 @@ __device__ __forceinline__ void inv_level(Unit<K>& u, const int2* __restrict__ t
 #pragma unroll
     for (int m = 0; m < half; ++m)
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
+      for (int c = 0; c < V; ++c)
         inv_bfly(u.x[g * 2 * half + m][c], u.x[g * 2 * half + m + half][c], w[g].x, w[g].y, p);
 }
-template <int K, int LV = K - 1>
-__device__ __forceinline__ void inv_levels(Unit<K>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+template <int K, int LV = K - 1, int V>
+__device__ __forceinline__ void inv_levels(Unit<K, V>& u, const int2* __restrict__ tw, u32 b, i32 p) {
   if constexpr (LV >= 0) {
-    inv_level<K, LV>(u, tw, b, p);
+    inv_level<K, V, LV>(u, tw, b, p);
     inv_levels<K, LV - 1>(u, tw, b, p);
   }
 }
 // The outputs of an inverse group above 1.5 p: row 0, and row 1 of three levels.
-template <int K>
-__device__ __forceinline__ void inv_fold(Unit<K>& u, const Prime& P) {
+template <int K, int V>
+__device__ __forceinline__ void inv_fold(Unit<K, V>& u, const Prime& P) {
 #pragma unroll
   for (int m = 0; m < (K == 3 ? 2 : 1); ++m)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) u.x[m][c] = reduce(u.x[m][c], P);
+    for (int c = 0; c < V; ++c) u.x[m][c] = reduce(u.x[m][c], P);
 }
 
 // Levels of a tile of R levels go in groups of at most three, one
@@ -233,24 +272,24 @@ constexpr int col_width(int R) { return R >= 7 ? 32 : 4096 >> R; }
 constexpr int batch_col_width(int R) { return R == 9 ? 16 : col_width(R); }
 
 // Forward levels [0, R) of one tile of C columns x 2^R rows, block index ksb
-// at its first level.  load(row, col) gives the four words at (row, col ..
-// col + 3), store puts four finished words; between groups the words go
+// at its first level.  load(row, col) gives the V words from (row, col), store
+// puts V finished words; between groups the words go
 // through sm.  HALF: the rows from 2^(R-1) are zero, so level 0 copies.
 // START: a reduction of the loaded words; LAST: one of the stored words.
-template <int R, int C, int NT, bool START, bool LAST, class Load, class Store>
+template <int R, int C, int NT, int V, bool START, bool LAST, class Load, class Store>
 __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const Store& store, bool half_zero,
                                              const int2* __restrict__ tw, u32 ksb, const Prime& P, bool start_red) {
   constexpr int G = groups_of(R);
   auto group = [&](auto gc) {
     constexpr int g = decltype(gc)::value;
     constexpr int K = group_size(R, g), l = group_start(R, g), nsub = R - l - K;
-    constexpr u32 units = (u32)(C / 4) << (R - K);
+    constexpr u32 units = (u32)(C / V) << (R - K);
     if (g > 0) __syncthreads();
 #pragma unroll 1
     for (u32 i = threadIdx.x; i < units; i += NT) {
-      const u32 col = (i % (C / 4)) * 4, v = i / (C / 4);
+      const u32 col = (i % (C / V)) * V, v = i / (C / V);
       const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
-      Unit<K> u;
+      Unit<K, V> u;
       const u32 b = (ksb << l) + rb;
       u32* sp = sm + at<C>(row0) + col;
       if constexpr (g == 0) {
@@ -269,14 +308,14 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
 #pragma unroll
               for (int m = 0; m < (1 << K); ++m)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) u.x[m][c] = reduce(u.x[m][c], P);
+                for (int c = 0; c < V; ++c) u.x[m][c] = reduce(u.x[m][c], P);
             }
           }
           fwd_levels<K>(u, tw, b, P.p);
         }
       } else {
 #pragma unroll
-        for (int m = 0; m < (1 << K); ++m) u.set(m, *reinterpret_cast<const int4*>(sp + at<C>((u32)m << nsub)));
+        for (int m = 0; m < (1 << K); ++m) u.set(m, ldv<false, V>(sp + at<C>((u32)m << nsub)));
         fwd_levels<K>(u, tw, b, P.p);
       }
       if constexpr (g + 1 == G) {
@@ -284,13 +323,13 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
         for (int m = 0; m < (1 << K); ++m) {
           if (LAST) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) u.x[m][c] = reduce(u.x[m][c], P);
+            for (int c = 0; c < V; ++c) u.x[m][c] = reduce(u.x[m][c], P);
           }
           store(row0 + ((u32)m << nsub), col, u.get(m));
         }
       } else {
 #pragma unroll
-        for (int m = 0; m < (1 << K); ++m) *reinterpret_cast<int4*>(sp + at<C>((u32)m << nsub)) = u.get(m);
+        for (int m = 0; m < (1 << K); ++m) stv<false, V>(sp + at<C>((u32)m << nsub), u.get(m));
       }
     }
   };
@@ -302,20 +341,20 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
 // Inverse levels R-1 .. 0 of one tile; the groups in the opposite order.
 // raw: the outputs of the last group go out unreduced (up to 12 p, for the
 // CRT; overlapping pieces are added there and want at most 1.5 p).
-template <int R, int C, int NT, class Load, class Store>
+template <int R, int C, int NT, int V, class Load, class Store>
 __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const Store& store,
                                              const int2* __restrict__ tw, u32 ksb, const Prime& P, bool raw) {
   constexpr int G = groups_of(R);
   auto group = [&](auto gc) {
     constexpr int g = decltype(gc)::value;
     constexpr int K = group_size(R, g), l = group_start(R, g), nsub = R - l - K;
-    constexpr u32 units = (u32)(C / 4) << (R - K);
+    constexpr u32 units = (u32)(C / V) << (R - K);
     if (g + 1 < G) __syncthreads();
 #pragma unroll 1
     for (u32 i = threadIdx.x; i < units; i += NT) {
-      const u32 col = (i % (C / 4)) * 4, v = i / (C / 4);
+      const u32 col = (i % (C / V)) * V, v = i / (C / V);
       const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
-      Unit<K> u;
+      Unit<K, V> u;
       const u32 b = (ksb << l) + rb;
       u32* sp = sm + at<C>(row0) + col;
 #pragma unroll
@@ -323,7 +362,7 @@ __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const St
         if constexpr (g + 1 == G)
           u.set(m, load(row0 + ((u32)m << nsub), col));
         else
-          u.set(m, *reinterpret_cast<const int4*>(sp + at<C>((u32)m << nsub)));
+          u.set(m, ldv<false, V>(sp + at<C>((u32)m << nsub)));
       }
       inv_levels<K>(u, tw, b, P.p);
       if (g > 0 || !raw) inv_fold<K>(u, P);
@@ -332,7 +371,7 @@ __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const St
         if constexpr (g == 0)
           store(row0 + ((u32)m << nsub), col, u.get(m));
         else
-          *reinterpret_cast<int4*>(sp + at<C>((u32)m << nsub)) = u.get(m);
+          stv<false, V>(sp + at<C>((u32)m << nsub), u.get(m));
       }
     }
   };
@@ -341,22 +380,28 @@ __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const St
   group(std::integral_constant<int, 0>{});
 }
 
-// Four limbs from position pos as residues (zero at and beyond n).
-__device__ __forceinline__ int4 limbs4(const u64* __restrict__ in, u64 n, u64 pos, bool vec, const Prime& P) {
-  u64 x[4] = {0, 0, 0, 0};
-  if (pos + 4 <= n && vec) {
-    const ulonglong2 v0 = __ldg(reinterpret_cast<const ulonglong2*>(in + pos));
-    const ulonglong2 v1 = __ldg(reinterpret_cast<const ulonglong2*>(in + pos) + 1);
-    x[0] = v0.x;
-    x[1] = v0.y;
-    x[2] = v1.x;
-    x[3] = v1.y;
+// V limbs from position pos as residues (zero at and beyond n).
+template <int V>
+__device__ __forceinline__ Words<V> limb_words(const u64* __restrict__ in, u64 n, u64 pos, bool vec, const Prime& P) {
+  u64 x[V];
+#pragma unroll
+  for (int c = 0; c < V; ++c) x[c] = 0;
+  if (V > 1 && vec && pos + V <= n) {
+#pragma unroll
+    for (int c = 0; c + 1 < V; c += 2) {
+      const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(in + pos + c));
+      x[c] = t.x;
+      x[c + 1] = t.y;
+    }
   } else {
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+    for (int c = 0; c < V; ++c)
       if (pos + c < n) x[c] = __ldg(in + pos + c);
   }
-  return make_int4(limb_residue(x[0], P), limb_residue(x[1], P), limb_residue(x[2], P), limb_residue(x[3], P));
+  Words<V> w;
+#pragma unroll
+  for (int c = 0; c < V; ++c) w.v[c] = limb_residue(x[c], P);
+  return w;
 }
 
 // The first pass of one operand: levels [0, R) from its limbs, columns
@@ -369,9 +414,9 @@ __device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u
   u32* out = res + ((u64)prime << s) + (u64)tile * C;
   const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
   const u64 col0 = (u64)tile * C;
-  forward_tile<R, C, NT, false, false>(
-      sm, [&](u32 row, u32 col) { return limbs4(in, n, ((u64)row << lg_s) + col0 + col, vec, P); },
-      [&](u32 row, u32 col, int4 v) { st4<CG>(out + ((u64)row << lg_s) + col, v); }, n <= (1ull << (s - 1)),
+  forward_tile<R, C, NT, 4, false, false>(
+      sm, [&](u32 row, u32 col) { return limb_words<4>(in, n, ((u64)row << lg_s) + col0 + col, vec, P); },
+      [&](u32 row, u32 col, const Words<4>& w) { stv<CG>(out + ((u64)row << lg_s) + col, w); }, n <= (1ull << (s - 1)),
       tab + prime * cap, 0, P, false);
 }
 
@@ -385,12 +430,12 @@ __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, 
   const u32 ksb = tile / per;
   u32* g = res + ((u64)prime << s) + ((u64)ksb << (lg_s + R)) + (u64)(tile % per) * C;
   const int2* tw = tab + prime * cap;
-  auto ld = [&](u32 row, u32 col) { return ld4<CG>(g + ((u64)row << lg_s) + col); };
-  auto st = [&](u32 row, u32 col, int4 v) { st4<CG>(g + ((u64)row << lg_s) + col, v); };
+  auto ld = [&](u32 row, u32 col) { return ldv<CG, 4>(g + ((u64)row << lg_s) + col); };
+  auto st = [&](u32 row, u32 col, const Words<4>& w) { stv<CG>(g + ((u64)row << lg_s) + col, w); };
   if constexpr (INV)
-    inverse_tile<R, C, NT>(sm, ld, st, tw, ksb, P, raw);
+    inverse_tile<R, C, NT, 4>(sm, ld, st, tw, ksb, P, raw);
   else
-    forward_tile<R, C, NT, false, false>(sm, ld, st, false, tw, ksb, P, false);
+    forward_tile<R, C, NT, 4, false, false>(sm, ld, st, false, tw, ksb, P, false);
 }
 
 // Products of the blocks of 8 coefficients of a tile: block row r of A times
@@ -489,7 +534,7 @@ __device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const int2
 // kAll everything; kForward only a's forward levels, written back to a;
 // kProduct products and inverse of operands whose forward levels are done.
 enum : int { kAll = 0, kForward = 1, kProduct = 2 };
-template <int R, int LGM, int NT, bool FIRST, bool CG>
+template <int R, int LGM, int NT, int V, bool FIRST, bool CG>
 __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const void* b, u64 nb, u32* out, int s,
                                            u32 tile, int prime, const int2* __restrict__ tab,
                                            const int2* __restrict__ itab, u64 cap, bool reduce_in, bool raw, int mode = kAll) {
@@ -501,18 +546,18 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
   const u64 off = FIRST ? 0 : ((u64)prime << s) + ((u64)tile << (R + LGM));
   u32* sa = sm;
   u32* sb = b ? sm + W : sm;
-  auto to = [&](u32* t) { return [t](u32 row, u32 col, int4 v) { *reinterpret_cast<int4*>(t + at<C>(row) + col) = v; }; };
+  auto to = [&](u32* t) { return [t](u32 row, u32 col, const Words<V>& w) { stv<false>(t + at<C>(row) + col, w); }; };
   auto forward = [&](const void* src, u64 n, u32* t) {
     if constexpr (FIRST) {
       const u64* in = static_cast<const u64*>(src);
       const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-      forward_tile<R, C, NT, false, true>(
-          t, [&](u32 row, u32 col) { return limbs4(in, n, (u64)row * C + col, vec, P); }, to(t), n <= (1ull << (s - 1)),
+      forward_tile<R, C, NT, V, false, true>(
+          t, [&](u32 row, u32 col) { return limb_words<V>(in, n, (u64)row * C + col, vec, P); }, to(t), n <= (1ull << (s - 1)),
           tw, 0, P, false);
     } else {
       const u32* in = static_cast<const u32*>(src) + off;
-      forward_tile<R, C, NT, true, true>(
-          t, [&](u32 row, u32 col) { return ld4<CG>(in + row * C + col); }, to(t), false, tw, tile, P, reduce_in);
+      forward_tile<R, C, NT, V, true, true>(
+          t, [&](u32 row, u32 col) { return ldv<CG, V>(in + row * C + col); }, to(t), false, tw, tile, P, reduce_in);
     }
   };
   auto fetch = [&](const void* src, u32* t) {  // kProduct: words whose forward levels are done
@@ -526,7 +571,7 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
       __syncthreads();
       u32* back = out + off;
       for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT)
-        st4<CG>(back + i, *reinterpret_cast<const int4*>(sa + at<C>(i / C) + i % C));
+        stv<CG>(back + i, ldv<false, 4>(sa + at<C>(i / C) + i % C));
       return;
     }
     if (b) forward(b, nb, sb);
@@ -541,9 +586,9 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
     leaf_products<R, LGM, NT>(sa, sb, tw, FIRST ? 0 : tile, P);
   u32* dst = out + ((u64)prime << s) + (FIRST ? 0 : (u64)tile << (R + LGM));
   __syncthreads();
-  inverse_tile<R, C, NT>(
-      sa, [&](u32 row, u32 col) { return *reinterpret_cast<const int4*>(sa + at<C>(row) + col); },
-      [&](u32 row, u32 col, int4 v) { st4<CG>(dst + row * C + col, v); }, itw, FIRST ? 0 : tile, P, FIRST && raw);
+  inverse_tile<R, C, NT, V>(
+      sa, [&](u32 row, u32 col) { return ldv<false, V>(sa + at<C>(row) + col); },
+      [&](u32 row, u32 col, const Words<V>& w) { stv<CG>(dst + row * C + col, w); }, itw, FIRST ? 0 : tile, P, FIRST && raw);
 }
 
 }  // namespace six
