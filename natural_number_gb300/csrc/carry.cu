@@ -359,15 +359,14 @@ cudaError_t six_save(const SixOperands& op, const SixPlan& pl, u64* out, Scan& s
                      const std::function<cudaError_t(u64, u64)>& done) {
   const u64 L = 1ull << pl.s, nb = op.b ? op.nb : op.na, size = op.na + nb;
   const u64 tiles = scan_tiles(size);
-  const SixCrt crt = six_crt(pl.s);
   cudaError_t e = scan_reserve(sc, tiles);
   for (int k = 0; k < chunks && e == cudaSuccess; ++k) {
     const u64 t0 = tiles * k / chunks, t1 = tiles * (k + 1) / chunks;
     if (t1 == t0) continue;
     if (op.pieces == 1)
-      e = run_scan(SixCrtProducer<false>{op.ra, L, size - 1, crt}, size, out, size, sc, st, "six_crt_scan", t0, t1);
+      e = run_scan(SixCrtProducer<false>{op.ra, L, size - 1}, size, out, size, sc, st, "six_crt_scan", t0, t1);
     else
-      e = run_scan(PieceCrtProducer<false>{op.ra, L, op.piece, op.pieces, nb, size - 1, crt}, size, out, size, sc, st,
+      e = run_scan(PieceCrtProducer<false>{op.ra, L, op.piece, op.pieces, nb, size - 1}, size, out, size, sc, st,
                    "six_crt_scan", t0, t1);
     if (e == cudaSuccess && done) e = done(t0 * kScanTile, std::min(size, t1 * kScanTile));
   }

@@ -6,6 +6,7 @@
 #include <dlfcn.h>
 
 #include <algorithm>
+#include <array>
 #include <bit>
 #include <cstdio>
 #include <cstdlib>
@@ -140,7 +141,7 @@ struct nn_context {
   int batch_fused = 1;        // batches: last forward levels, products and first inverse levels in one item
   int batch_merge = 1;        // kept for callers that set it: every batch tile fills its CTA
   int batch_split = 1;        // batches: unbalanced products in pieces sharing one transform
-  int batch_blocks_per_sm = 0;  // persistent CTAs per SM (0: occupancy limit)
+  int batch_blocks_per_sm = 0;  // kept for callers that set it: a CTA an item
   int batch_solo_scale = 22;    // batches: products of this scale and up run one at a time (0: never)
 };
 
@@ -148,20 +149,16 @@ struct nn_batch {
   u64 count = 0;
   std::vector<u64> na, nb;
   std::vector<nn::BatchJob> jobs;
-  std::vector<nn::BatchItem> items;
-  std::vector<nn::u32> need;
+  std::vector<nn::BatchItem> items;        // by launch
+  std::vector<nn::BatchSegment> segments;  // the launches, in order
   std::vector<u64> off_a, off_b;
   std::vector<char> swap;  // NTT job whose second operand is the longer one
   std::vector<u64> solo;   // jobs run one at a time after the batch kernel
   u64 arena_words = 0;
-  nn::u32 n_ctrs = 0, n_flags = 0;
-  size_t smem = 0;
-  int grid = 0;
+  nn::u32 n_flags = 0;
   nn::BatchJob* d_jobs = nullptr;
   nn::BatchItem* d_items = nullptr;
-  nn::u32* d_need = nullptr;
-  nn::u32* d_state = nullptr;  // done[n_ctrs], head, pad
-  nn::u32* d_flags = nullptr;
+  nn::u32* d_state = nullptr;  // a ticket counter a launch, then the scans' status words
   u64* d_arena = nullptr;
   u64 dev_words = 0;           // budget accounting of the above
   nn::BatchJob* h_jobs = nullptr;  // pinned staging of the job table
@@ -319,9 +316,12 @@ nn_status six_residues(nn_context* c, DBuf& buf, nn::SixOperands& op, const nn::
   return NN_OK;
 }
 
+// Coefficients of a transform's product: a piece's when the longer operand is split.
+u64 six_length(const nn::SixOperands& op) { return op.piece + (op.b ? op.nb : op.na) - 1; }
+
 // op's product over six primes at scale s (op.b nullptr: the square).
 nn_status six_product(nn_context* c, u64* d_out, nn::SixOperands op, int s) {
-  const nn::SixPlan pl = nn::six_plan(std::max(s, nn::kSixMinScale));
+  const nn::SixPlan pl = nn::six_plan(std::max(s, nn::kSixMinScale), six_length(op));
   DBuf buf(c);
   nn_status st = six_residues(c, buf, op, pl);
   if (st != NN_OK) return st;
@@ -343,7 +343,7 @@ constexpr int kInChunks = 8, kCopyChunks = 8;
 nn_status six_product_from_host(nn_context* c, u64* d_out, u64* da, const u64* ha, u64 na, u64* db, const u64* hb,
                                 u64 nb, int s, u64* h_out, bool* used) {
   *used = false;
-  const nn::SixPlan pl = nn::six_plan(std::max(s, nn::kSixMinScale));
+  const nn::SixPlan pl = nn::six_plan(std::max(s, nn::kSixMinScale), na + nb - 1);
   const u64 tiles = nn::six_first_pass_tiles(pl), width = nn::six_first_pass_columns(pl);
   if (pl.n < 2) return NN_OK;
   *used = true;
@@ -394,7 +394,9 @@ nn_status six_product_from_host(nn_context* c, u64* d_out, u64* da, const u64* h
 // two pieces overlap at any position.  The cost of a word is its levels plus
 // about four levels' worth of load, block products and CRT.
 int six_split(u64 nx, u64 ny, int s, u64* k, u64* P) {
-  double best = 3.0 * (double)(1ull << s) * (s + 1);
+  // one transform: the eighths of it that hold the product
+  const double part = (double)std::clamp<u64>(((nx + ny - 1) * 8 + (1ull << s) - 1) >> s, 5, 8) / 8;
+  double best = 3.0 * part * (double)(1ull << s) * (s + 1);
   int s_best = s;
   *k = nx;
   *P = 1;
@@ -483,9 +485,8 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
   B->off_a.assign(count, 0);
   B->off_b.assign(count, 0);
   B->swap.assign(count, 0);
-  std::vector<int> steps(count, 0);
+  std::vector<u64> order;  // jobs with items
   int max_s = nn::kSixMinScale;
-  size_t smem = 8;
   for (u64 j = 0; j < count; ++j) {
     if (!na[j] || !nb[j]) {
       c->err = "batch: empty operand";
@@ -497,158 +498,176 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
     J.nb = nb[j];
     J.piece = na[j];
     J.pieces = 1;
-    J.ctr_base = B->n_ctrs;
     J.flag_base = B->n_flags;
-    B->n_flags += (nn::u32)nn::batch_scan_tiles(na[j] + nb[j]);
     const u64 mn = std::min(na[j], nb[j]), mx = std::max(na[j], nb[j]);
     if (mn < c->batch_ntt_min || (mn < c->batch_school_balanced && mx <= 2 * mn)) {
-      steps[j] = 1;
-      smem = std::max(smem, nn::kColumnTileSmem);  // the item's column sums
-    } else {
-      J.square = square ? square[j] : 0;
-      if (J.square && na[j] != nb[j]) {
-        c->err = "batch: a square needs equal operand sizes";
-        return NN_ERR_INVALID;
-      }
-      // operand 0 is the longer one; it may be split into pieces
-      B->swap[j] = na[j] < nb[j];
-      J.na = std::max(na[j], nb[j]);
-      J.nb = std::min(na[j], nb[j]);
-      J.piece = J.na;
-      int s = std::max(ntt_scale(J.na, J.nb), nn::kSixMinScale);
-      if (c->batch_solo_scale > 0 && s >= c->batch_solo_scale) {
-        // From this scale on one product fills the GPU by itself and the
-        // one-product passes beat the batch kernel's: no items, no arena; the
-        // launch runs it alone.
-        B->solo.push_back(j);
-        continue;
-      }
-      if (c->batch_split && !J.square) s = six_split(J.na, J.nb, s, &J.piece, &J.pieces);
-      if (s > nn::kSixMaxScale) {
-        c->err = "batch: transform too long for one batch";
-        return NN_ERR_INVALID;
-      }
-      J.plan = nn::six_plan(s, s < 64 ? c->batch_r_last_at[s] : 0);
-      max_s = std::max(max_s, s);
-      for (int k = 0; k < J.plan.n; ++k) smem = std::max(smem, nn::batch_pass_smem(J.plan, k, J.square));
-      const int m = J.plan.n;
-      J.rows = m > 1 && !c->batch_fused;
-      // forward strided passes, (the last forward levels alone,) the fused
-      // pass, inverse strided passes, CRT
-      steps[j] = (m - 1) + J.rows + 1 + (m - 1) + 1;
-      B->off_a[j] = B->arena_words;
-      B->arena_words += J.pieces * (3ull << s);
-      if (!J.square && m > 1) {
-        B->off_b[j] = B->arena_words;
-        B->arena_words += 3ull << s;
-      }
+      B->n_flags += (nn::u32)((na[j] + nb[j] + nn::kBatchSumTile - 1) / nn::kBatchSumTile);
+      order.push_back(j);
+      continue;
     }
-    B->n_ctrs += steps[j];
+    J.square = square ? square[j] : 0;
+    if (J.square && na[j] != nb[j]) {
+      c->err = "batch: a square needs equal operand sizes";
+      return NN_ERR_INVALID;
+    }
+    // operand 0 is the longer one; it may be split into pieces
+    B->swap[j] = na[j] < nb[j];
+    J.na = mx;
+    J.nb = mn;
+    J.piece = J.na;
+    int s = std::max(ntt_scale(J.na, J.nb), nn::kSixMinScale);
+    if (c->batch_solo_scale > 0 && s >= c->batch_solo_scale) {
+      // From this scale on one product fills the GPU by itself: no items, no
+      // arena; the launch runs it alone.
+      B->solo.push_back(j);
+      continue;
+    }
+    if (c->batch_split && !J.square) s = six_split(J.na, J.nb, s, &J.piece, &J.pieces);
+    if (s > nn::kSixMaxScale) {
+      c->err = "batch: transform too long for one batch";
+      return NN_ERR_INVALID;
+    }
+    J.plan = nn::six_plan(s, J.pieces > 1 ? 1ull << s : J.na + J.nb - 1, c->batch_r_last_at[s]);
+    max_s = std::max(max_s, s);
+    J.rows = J.plan.n > 1 && !c->batch_fused;
+    B->n_flags += (nn::u32)nn::scan_tiles(na[j] + nb[j]);
+    B->off_a[j] = B->arena_words;
+    B->arena_words += J.pieces * (3ull << s);
+    if (!J.square && J.plan.n > 1) {
+      B->off_b[j] = B->arena_words;
+      B->arena_words += 3ull << s;
+    }
+    order.push_back(j);
   }
-  B->need.assign(B->n_ctrs, 0);
-  const int max_steps = *std::max_element(steps.begin(), steps.end());  // 0 when every job runs alone
-  B->items.clear();
-  // Within a step, jobs of one scale one after another, the longest first:
-  // CTAs that share an SM then mostly run the same tile's code, and the step
-  // ends with its smallest items.
-  std::vector<u64> order(count);
-  std::iota(order.begin(), order.end(), 0);
+  // The longest jobs' items first in each launch, so that it ends with its
+  // smallest; jobs of one scale one after another.
   std::stable_sort(order.begin(), order.end(), [&](u64 x, u64 y) { return B->jobs[x].plan.s > B->jobs[y].plan.s; });
-  for (int st = 0; st < max_steps; ++st) {
-    for (u64 j : order) {
-      if (st >= steps[j]) continue;
-      const nn::BatchJob& J = B->jobs[j];
-      auto push = [&](unsigned char kind, int pass, int prime, int operand, u64 tile, u64 ntile = 1) {
-        nn::BatchItem it{};
-        it.job = (nn::u32)j;
-        it.step = (unsigned short)st;
-        it.kind = kind;
-        it.pass = (unsigned char)pass;
-        it.prime = (unsigned char)prime;
-        it.operand = (unsigned char)operand;
-        it.tile = (nn::u32)tile;
-        it.ntile = (unsigned short)ntile;
-        B->items.push_back(it);
-        B->need[J.ctr_base + st] += 1;
-      };
-      const nn::SixPlan& pl = J.plan;
-      if (pl.s == 0) {
-        for (u64 t = 0; t < nn::batch_scan_tiles(J.na + J.nb); ++t) push(nn::kItemColumn, 0, 0, 0, t);
-        continue;
-      }
-      const int m = pl.n, fused_at = m - 1 + J.rows;
-      // items of pass k over operand 0's pieces (tiles numbered across them) or operand 1
-      auto pass_items = [&](unsigned char kind, int k, int operand) {
-        const u64 each = nn::batch_pass_tiles(pl, k), tiles = each * (operand == 0 ? J.pieces : 1);
-        const u64 tw = (1ull << pl.s) / each;
-        const u64 per = std::clamp<u64>(c->batch_item_words / tw, 1, 0xffff);  // BatchItem::ntile is 16-bit
-        for (int pr = 0; pr < 6; ++pr)
-          for (u64 t = 0; t < tiles; t += per) push(kind, k, pr, operand, t, std::min(per, tiles - t));
-      };
-      const int operands = J.square ? 1 : 2;
-      if (st < m - 1) {
-        for (int op = 0; op < operands; ++op) pass_items(nn::kItemFwd, st, op);
-      } else if (st < fused_at) {
-        for (int op = 0; op < operands; ++op) pass_items(nn::kItemRow, m - 1, op);
-      } else if (st == fused_at) {
-        pass_items(nn::kItemFused, m - 1, 0);
-      } else if (st < fused_at + m) {
-        pass_items(nn::kItemInv, fused_at + m - 1 - st, 0);  // inverse passes m-2 .. 0
-      } else {
-        for (u64 t = 0; t < nn::batch_scan_tiles(J.na + J.nb); ++t) push(nn::kItemCrt, 0, 0, 0, t);
-      }
+
+  // One launch a (phase, kind, pass, R, block length): its items.
+  std::map<std::array<int, 5>, std::vector<nn::BatchItem>> launches;
+  for (u64 j : order) {
+    const nn::BatchJob& J = B->jobs[j];
+    const nn::SixPlan& pl = J.plan;
+    auto item = [&](u64 tile, u64 ntile, int prime, int operand) {
+      nn::BatchItem it{};
+      it.job = (nn::u32)j;
+      it.tile = (nn::u32)tile;
+      it.ntile = (unsigned short)ntile;
+      it.prime = (unsigned char)prime;
+      it.operand = (unsigned char)operand;
+      return it;
+    };
+    if (pl.s == 0) {
+      auto& v = launches[{0, nn::kBatchColumns, 0, 0, 0}];
+      for (u64 t = 0; t * nn::kBatchSumTile < J.na + J.nb; ++t) v.push_back(item(t, 1, 0, 0));
+      continue;
     }
+    const int m = pl.n;
+    // items of pass k over operand 0's pieces (tiles numbered across them) or operand 1
+    auto pass_items = [&](int phase, int kind, int k, int operand) {
+      const bool row = k == m - 1;
+      auto& v = launches[{phase, kind, row ? J.rows : k, pl.R[k], row ? pl.lgm : 0}];
+      const u64 each = nn::batch_pass_tiles(pl, k), tiles = each * (operand == 0 ? J.pieces : 1);
+      const u64 words = std::max<u64>((1ull << pl.s) / 8 * (k > 0 ? pl.k8 : 8) / each, 1);
+      const u64 per = std::clamp<u64>(c->batch_item_words / words, 1, 0xffff);  // BatchItem::ntile is 16-bit
+      for (u64 t = 0; t < tiles; t += per)  // the six primes of a tile's limbs or words one after another
+        for (int pr = 0; pr < 6; ++pr) v.push_back(item(t, std::min(per, tiles - t), pr, operand));
+    };
+    const int operands = J.square ? 1 : 2;
+    if (m == 1) {
+      auto& v = launches[{0, nn::kBatchSmall, 0, pl.R[0], 0}];
+      for (u64 i = 0; i < J.pieces; ++i)
+        for (int pr = 0; pr < 6; ++pr) v.push_back(item(i, 1, pr, 0));
+    } else {
+      for (int op = 0; op < operands; ++op) {
+        pass_items(0, nn::kBatchLoad, 0, op);
+        for (int k = 1; k < m - 1; ++k) pass_items(k, nn::kBatchCol, k, op);
+        if (J.rows) pass_items(3, nn::kBatchRow, m - 1, op);
+      }
+      pass_items(4, nn::kBatchFused, m - 1, 0);
+      for (int k = m - 2; k >= 0; --k) pass_items(7 - k, nn::kBatchInvCol, k, 0);
+    }
+    auto& v = launches[{8, J.pieces > 1 ? nn::kBatchPieceCrt : nn::kBatchCrt, 0, 0, 0}];
+    for (u64 t = 0; t < nn::scan_tiles(J.na + J.nb); ++t) v.push_back(item(t, 1, 0, 0));
   }
-  if (B->items.size() >= 0xffffffffull) {
-    c->err = "batch: too many work items";
-    return NN_ERR_INVALID;
+  for (auto& [key, v] : launches) {
+    if (B->items.size() + v.size() >= 0xffffffffull) {
+      c->err = "batch: too many work items";
+      return NN_ERR_INVALID;
+    }
+    B->segments.push_back({key[0], key[1], key[2], key[3], key[4], (nn::u32)B->items.size(), (nn::u32)v.size()});
+    B->items.insert(B->items.end(), v.begin(), v.end());
   }
-  B->smem = smem;
   NN_CK(c, nn::six_tables_ensure(c->six, max_s, c->stream, &c->retired_tables), "twiddle tables");
-  int per_sm = 0;
-  NN_CK(c, nn::batch_configure(&per_sm, smem), "batch kernel attributes");
-  if (c->batch_blocks_per_sm > 0) per_sm = std::min(per_sm, c->batch_blocks_per_sm);
-  int sms = 0;
-  NN_CK(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device), "device attributes");
-  B->grid = std::max(1, per_sm) * sms;
-  // device tables
   // Regions in one allocation, each rounded to 256 bytes: the residues are
   // read and written with 16-byte vector accesses.
   auto words = [](u64 bytes) { return (bytes + 255) / 256 * 32; };
-  const u64 w_jobs = words(count * sizeof(nn::BatchJob)), w_items = words(B->items.size() * sizeof(nn::BatchItem));
-  const u64 w_need = words(4ull * B->n_ctrs), w_state = words(4ull * (B->n_ctrs + 4)),
-            w_flags = words(4ull * (B->n_flags + 2));
+  const u64 w_jobs = words(count * sizeof(nn::BatchJob)), w_items = words(B->items.size() * sizeof(nn::BatchItem)),
+            w_state = words(4ull * (B->segments.size() + B->n_flags + 2));
   u64* p = nullptr;
-  B->dev_words = w_jobs + w_items + w_need + w_state + w_flags + B->arena_words;
+  B->dev_words = w_jobs + w_items + w_state + B->arena_words;
   nn_status st = dev_alloc(c, &p, B->dev_words);
   if (st != NN_OK) return st;
   B->d_jobs = reinterpret_cast<nn::BatchJob*>(p);
   B->d_items = reinterpret_cast<nn::BatchItem*>(p + w_jobs);
-  B->d_need = reinterpret_cast<nn::u32*>(p + w_jobs + w_items);
-  B->d_state = reinterpret_cast<nn::u32*>(p + w_jobs + w_items + w_need);
-  B->d_flags = reinterpret_cast<nn::u32*>(p + w_jobs + w_items + w_need + w_state);
-  B->d_arena = p + w_jobs + w_items + w_need + w_state + w_flags;
+  B->d_state = reinterpret_cast<nn::u32*>(p + w_jobs + w_items);
+  B->d_arena = p + w_jobs + w_items + w_state;
   NN_CK(c, c->stage.upload(B->d_items, B->items.data(), B->items.size() * sizeof(nn::BatchItem), c->stream),
         "upload items");
-  NN_CK(c, c->stage.upload(B->d_need, B->need.data(), B->need.size() * 4, c->stream), "upload counts");
   NN_CK(c, cudaEventCreateWithFlags(&B->ran, cudaEventDisableTiming), "event");
   return NN_OK;
 }
 
-// Records the run sequence (job table upload, counter resets, persistent
-// kernel) into a CUDA graph on the context's own stream.
+// The run's launches on `st` (after the job table's upload): counters and
+// status words cleared, then phase by phase; with `side` streams, the launches
+// of one phase side by side.
+cudaError_t batch_sequence(nn_context* c, nn_batch* B, cudaStream_t st, cudaStream_t* side = nullptr, int n_side = 0,
+                           cudaEvent_t ev = nullptr) {
+  const u64 n = B->segments.size();
+  cudaError_t e = cudaMemsetAsync(B->d_state, 0, (n + B->n_flags + 2) * 4, st);
+  nn::u32* flags = B->d_state + n;
+  for (u64 i = 0; i < n && e == cudaSuccess;) {
+    u64 end = i + 1;
+    while (end < n && B->segments[end].phase == B->segments[i].phase) ++end;
+    const int used = (int)std::min<u64>(end - i - 1, n_side);  // side streams of this phase
+    if (used) e = cudaEventRecord(ev, st);
+    for (int k = 0; k < used && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(side[k], ev, 0);
+    for (u64 g = i; g < end && e == cudaSuccess; ++g) {
+      const int lane = (int)((g - i) % (used + 1));
+      const cudaStream_t s = lane ? side[lane - 1] : st;
+      if (!side) nn::launch_begin("batch_launch", s);
+      e = nn::batch_launch_segment(B->segments[g], B->d_jobs, B->d_items, B->d_state + g, flags, c->scan.err, c->six, s);
+      if (!side) nn::launch_end(s);
+    }
+    for (int k = 0; k < used && e == cudaSuccess; ++k) {
+      e = cudaEventRecord(ev, side[k]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ev, 0);
+    }
+    i = end;
+  }
+  return e;
+}
+
+// Records the run (job table upload, then batch_sequence) into a CUDA graph.
 nn_status batch_capture(nn_context* c, nn_batch* B) {
-  cudaStream_t cs = c->own;
-  NN_CK(c, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "begin capture");
-  cudaMemcpyAsync(B->d_jobs, B->h_jobs, B->count * sizeof(nn::BatchJob), cudaMemcpyHostToDevice, cs);
-  cudaMemsetAsync(B->d_state, 0, (B->n_ctrs + 4) * 4, cs);
-  cudaMemsetAsync(B->d_flags, 0, (B->n_flags + 2) * 4, cs);
-  cudaError_t le = nn::batch_launch(B->d_jobs, B->d_items, (nn::u32)B->items.size(), B->d_need, B->d_state,
-                                    B->d_state + B->n_ctrs, B->d_flags, c->scan.err, c->six, B->grid, B->smem, cs);
-  cudaError_t e = cudaStreamEndCapture(cs, &B->graph);
-  if (le != cudaSuccess) return fail(c, le, "batch launch (capture)");
-  NN_CK(c, e, "end capture");
-  NN_CK(c, cudaGraphInstantiate(&B->exec, B->graph, 0), "graph instantiate");
+  constexpr int kSide = 3;
+  cudaStream_t cs = c->own, side[kSide] = {};
+  cudaEvent_t ev = nullptr;
+  cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  for (int k = 0; k < kSide && e == cudaSuccess; ++k) e = cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    cudaError_t le =
+        cudaMemcpyAsync(B->d_jobs, B->h_jobs, B->count * sizeof(nn::BatchJob), cudaMemcpyHostToDevice, cs);
+    if (le == cudaSuccess) le = batch_sequence(c, B, cs, side, kSide, ev);
+    e = cudaStreamEndCapture(cs, &B->graph);
+    if (le != cudaSuccess) e = le;
+  }
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&B->exec, B->graph, 0);
+  for (cudaStream_t s : side)
+    if (s) cudaStreamDestroy(s);
+  if (ev) cudaEventDestroy(ev);
+  NN_CK(c, e, "batch graph");
   return NN_OK;
 }
 
@@ -1163,13 +1182,7 @@ nn_status nn_batch_launch(nn_context* c, nn_batch* B, const nn_mul_job* jobs) {
   if (st != NN_OK) return st;
   if (!B->items.empty()) {
     NN_CK(c, c->stage.upload(B->d_jobs, table.data(), B->count * sizeof(nn::BatchJob), c->stream), "upload jobs");
-    NN_CK(c, cudaMemsetAsync(B->d_state, 0, (B->n_ctrs + 4) * 4, c->stream), "reset counters");
-    NN_CK(c, cudaMemsetAsync(B->d_flags, 0, (B->n_flags + 2) * 4, c->stream), "reset flags");
-    nn::launch_begin("batch_persistent", c->stream);
-    cudaError_t le = nn::batch_launch(B->d_jobs, B->d_items, (nn::u32)B->items.size(), B->d_need, B->d_state,
-                                      B->d_state + B->n_ctrs, B->d_flags, c->scan.err, c->six, B->grid,
-                                      B->smem, c->stream);
-    nn::launch_end(c->stream);
+    const cudaError_t le = batch_sequence(c, B, c->stream);
     NN_CK(c, le, "batch launch");
   }
   st = batch_solo(c, B, jobs);
@@ -1192,7 +1205,7 @@ nn_status nn_batch_run(nn_context* c, nn_batch* B, const nn_mul_job* jobs) {
       nn_status st = batch_capture(c, B);
       if (st != NN_OK) return st;
     }
-    nn::launch_begin("batch_persistent", c->stream);
+    nn::launch_begin("batch_graph", c->stream);
     cudaError_t ge = cudaGraphLaunch(B->exec, c->stream);
     nn::launch_end(c->stream);
     NN_CK(c, ge, "graph launch");

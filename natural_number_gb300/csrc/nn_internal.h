@@ -65,15 +65,21 @@ void six_tables_free(SixTables& t);
 constexpr int kSixMinScale = 4, kSixMaxScale = 31;
 // The passes of a transform of scale s: levels R[k] from lambda0[k], the last
 // pass over contiguous tiles, down to blocks of 2^lgm coefficients.
+// k8 eighths of the transform are computed (5 to 8): the product has at most
+// k8 / 8 * 2^s coefficients.
+// The last inverse pass multiplies by scale[i] modulo prime i (with its
+// companion): the inverse of the factors that the passes leave, times that of
+// the other primes' product, as the CRT wants it.
 struct SixPlan {
-  int s, lgm, n;
+  int s, lgm, n, k8;
   int R[3], lambda0[3];
+  int2 scale[6];
   // more than 18 levels: the lazy words are reduced at the last pass's start
   constexpr bool reduce_in() const { return lambda0[n - 1] + R[n - 1] > 18; }
 };
-// row_levels: levels of the last pass of a two-pass transform, where it can
+// length: coefficients of the product.  row_levels: levels of the last pass of a two-pass transform, where it can
 // have that many (0: as even as possible).
-SixPlan six_plan(int s, int row_levels = 0);
+SixPlan six_plan(int s, u64 length, int row_levels = 0);
 
 // Operands of a product: a in `pieces` pieces of `piece` limbs (one piece of
 // na limbs: not split), residues ra [pieces][6][2^s]; b (nullptr: a square),
@@ -95,12 +101,6 @@ u32 six_first_pass_columns(const SixPlan& pl);
 cudaError_t six_load(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st, u32 tile0 = 0,
                      u32 tile1 = ~0u);
 cudaError_t six_finish(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st);
-// The multipliers of the CRT after a transform of scale s.
-struct SixCrt {
-  int w[6], wp[6];
-};
-SixCrt six_crt(int s);
-
 // Scratch for the carry scan.
 struct Scan {
   u32* flags = nullptr;  // per-tile status words of a lookback, zero between scans (the last tile clears them)
@@ -114,23 +114,12 @@ constexpr int kScanThreads = 256;
 constexpr int kScanE = 8;  // limbs per thread
 constexpr u64 kScanTile = (u64)kScanThreads * kScanE;
 
-// Batched products (batch.cu): jobs, their work items, and the launch.  CTAs
-// of 128 threads: a unit of eight rows x four columns a thread is a tile of
-// 4096 words, the contiguous passes' tile.  A pass item covers consecutive
-// tiles worth at least kBatchItemWords residues, so an item's fixed cost
-// (queue, dependency check, barriers) stays small beside its work.
-constexpr int kBatchThreads = 128;
-constexpr u64 kBatchScanTile = (u64)kBatchThreads * kScanE;
-inline u64 batch_scan_tiles(u64 positions) { return (positions + kBatchScanTile - 1) / kBatchScanTile; }
-// A base-case item's column sums in shared memory: a scan tile's positions
-// and the kScanE before them, three words each.
-constexpr u64 kColumnTileWords = kBatchScanTile + kScanE;
-constexpr size_t kColumnTileSmem = 3 * kColumnTileWords * 8;
+// Batched products (batch.cu): jobs, their work items by launch, and the run.
+// A pass item covers consecutive tiles worth about kBatchItemWords residues,
+// so a CTA's fixed cost (its item and job) stays small beside its work.
 constexpr u64 kBatchItemWords = 8192;
-// Forward (load or strided) pass, fused last pass, inverse strided pass, CRT
-// and base-case items; kItemRow: the last pass's forward levels alone, before
-// a fused item that runs only the products and inverse levels (batch_fused 0).
-enum : unsigned char { kItemFwd = 0, kItemRow = 1, kItemInv = 2, kItemCrt = 3, kItemColumn = 4, kItemFused = 5 };
+constexpr int kBatchSumThreads = 128;  // base-case items: 1024 positions
+constexpr u64 kBatchSumTile = (u64)kBatchSumThreads * kScanE;
 struct BatchJob {
   const u64* a;  // NTT jobs: the longer operand (split into pieces)
   const u64* b;
@@ -140,25 +129,31 @@ struct BatchJob {
   u32* res_b;    // [6][2^s]
   u64 piece;     // limbs of a per piece (na when not split)
   u64 pieces;
-  u32 ctr_base;  // first (job, step) completion counter
   u32 flag_base; // first carry-scan status word
   int square;    // a == b: one transform
-  int rows;      // kItemRow steps ran: the fused items start at the products
+  int rows;      // the last pass's forward levels run on their own (batch_fused 0)
   SixPlan plan;  // plan.s 0 for a schoolbook job
 };
 struct BatchItem {
-  u32 job;
-  unsigned short step;
-  unsigned char kind, pass, prime, operand;
-  unsigned short ntile;  // consecutive tiles (pass items) handled by this item
-  u32 tile;
+  u32 job, tile;
+  unsigned short ntile;  // consecutive tiles (pass items) of this item
+  unsigned char prime, operand;
 };
-// Tiles a transform has in pass k of its plan, and a CTA's shared memory for them.
+// Launches of a batch, in order: those of one phase are independent.
+enum BatchKind : int { kBatchLoad, kBatchCol, kBatchRow, kBatchFused, kBatchInvCol, kBatchSmall, kBatchCrt,
+                       kBatchPieceCrt, kBatchColumns };
+struct BatchSegment {
+  int phase, kind;
+  int pass;    // strided passes: its index in the jobs' plans
+  int R, lgm;  // levels; log2 of the block length (contiguous passes)
+  u32 first, count;  // items
+};
+// Tiles a transform has in pass k of its plan.
 u32 batch_pass_tiles(const SixPlan& pl, int k);
-size_t batch_pass_smem(const SixPlan& pl, int k, bool square);
-cudaError_t batch_configure(int* blocks_per_sm, size_t smem);
-cudaError_t batch_launch(const BatchJob* jobs, const BatchItem* items, u32 n_items, const u32* need, u32* done,
-                         u32* head, u32* flags, u32* err, const SixTables& t, int grid, size_t smem, cudaStream_t st);
+// tickets: a zeroed word a segment (the carry scans' tile order); flags: the
+// scans' zeroed status words.
+cudaError_t batch_launch_segment(const BatchSegment& seg, const BatchJob* jobs, const BatchItem* items, u32* ticket,
+                                 u32* flags, u32* err, const SixTables& t, cudaStream_t st);
 
 // Many sums at once (carry.cu): job j writes out = x + y in nout >=
 // max(nx, ny) + 1 limbs, or with `sub` out = x - y mod B^nout (x >= y: the

@@ -119,14 +119,14 @@ struct CrtProducerT {
 typedef CrtProducerT<false> CrtProducer;
 
 
-// CRT of the six-prime residues (six_tiles.cuh): with t_i = r_i * k_i mod p_i
-// (k_i = (M/p_i)^-1 and the transform's scale; any representative in (0, 2p)),
-// the coefficient is sum t_i (M/p_i) - q M for q = floor(sum t_i / p_i): it is
+// CRT of the six-prime residues (six_tiles.cuh), which the last inverse pass
+// leaves multiplied by (M/p_i)^-1: with t_i any representative in (0, 4p), the
+// coefficient is sum t_i (M/p_i) - q M for q = floor(sum t_i / p_i): it is
 // below 2^160 (two overlapping pieces, up to 2^31 limbs each), under a quarter
 // of M = 2^162.25, so a sum of 15-bit fractions tells q.  Column j of the sum
 // adds the t_i times word j of M/p_i in 64 bits without carries (six terms
-// below 2^61), then one pass propagates them; q M enters as q times 2^192 - M.
-// 42 multiply-adds, none dependent on another before the columns, where
+// below 2^61.2), then one pass propagates them; q M enters as q times 2^192 - M.
+// 36 wide multiply-adds, none dependent on another before the columns, where
 // Garner's mixed radix has fifteen dependent modular products.
 struct SixWords {
   u32 w[6];
@@ -156,26 +156,26 @@ constexpr SixWords six_negated(SixWords a) {
   return a;
 }
 template <int I>
-__device__ __forceinline__ void six_crt_term(int y, const SixCrt& k, u64 (&col)[6], u32& frac) {
+__device__ __forceinline__ void six_crt_term(int y, u64 (&col)[6], u32& frac) {
   constexpr u32 p = six::prime_of(I);
   constexpr SixWords m = six_modulus_without(I);
   constexpr u32 f = (u32)(((1ull << 39) + p / 2) / p);
-  const u32 t = (u32)six::mul_mod(y, k.w[I], k.wp[I], (int)p) + p;
-  frac += (t >> 12) * f;  // t / p in units of 2^-27, within 2^-11
+  const u32 t = (u32)y + 2 * p;  // |y| <= 1.5 p: two pieces' residues may have been added
+  frac += (t >> 12) * f;  // t / p in units of 2^-27, within 2^-10
 #pragma unroll
   for (int j = 0; j < 5; ++j) col[j] += (u64)t * m.w[j];
 }
-__device__ __forceinline__ W3 six_garner(const int (&y)[six::kPrimes], const SixCrt& k) {
+__device__ __forceinline__ W3 six_garner(const int (&y)[six::kPrimes]) {
   static_assert(six::kPrimes == 6);
   constexpr SixWords neg = six_negated(six_modulus_without(six::kPrimes));
   u64 col[6] = {0, 0, 0, 0, 0, 0};
   u32 frac = 1u << 24;  // an eighth: the coefficient's own fraction is below a quarter
-  six_crt_term<0>(y[0], k, col, frac);
-  six_crt_term<1>(y[1], k, col, frac);
-  six_crt_term<2>(y[2], k, col, frac);
-  six_crt_term<3>(y[3], k, col, frac);
-  six_crt_term<4>(y[4], k, col, frac);
-  six_crt_term<5>(y[5], k, col, frac);
+  six_crt_term<0>(y[0], col, frac);
+  six_crt_term<1>(y[1], col, frac);
+  six_crt_term<2>(y[2], col, frac);
+  six_crt_term<3>(y[3], col, frac);
+  six_crt_term<4>(y[4], col, frac);
+  six_crt_term<5>(y[5], col, frac);
   const u32 q = frac >> 27;
   u32 w[6];
   u64 c = 0;
@@ -187,20 +187,19 @@ __device__ __forceinline__ W3 six_garner(const int (&y)[six::kPrimes], const Six
   }
   return W3{(u64)w[1] << 32 | w[0], (u64)w[3] << 32 | w[2], (u64)w[5] << 32 | w[4]};
 }
-__device__ __forceinline__ void six_garner4(const int4 (&v)[six::kPrimes], const SixCrt& k, W3 (&x)[kScanE], int e0) {
+__device__ __forceinline__ void six_garner4(const int4 (&v)[six::kPrimes], W3 (&x)[kScanE], int e0) {
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     int y[six::kPrimes];
 #pragma unroll
     for (int q = 0; q < six::kPrimes; ++q) y[q] = e == 0 ? v[q].x : e == 1 ? v[q].y : e == 2 ? v[q].z : v[q].w;
-    x[e0 + e] = six_garner(y, k);
+    x[e0 + e] = six_garner(y);
   }
 }
 template <bool CG>
 struct SixCrtProducer {
   const u32* res;  // [6][L]
   u64 L, count;
-  SixCrt k;
   static constexpr bool kBulk = true;
   // One position: the ends of a product only, so a call rather than sixteen
   // inlined copies in the scan.
@@ -212,7 +211,7 @@ struct SixCrtProducer {
       const u32* r = res + q * L + i;
       y[q] = (int)(CG ? __ldcg(r) : *r);
     }
-    return six_garner(y, k);
+    return six_garner(y);
   }
   // Eight consecutive positions from k0 (a multiple of 8) with 16-byte loads.
   __device__ __forceinline__ void bulk(u64 k0, W3 (&x)[kScanE]) const {
@@ -226,7 +225,7 @@ struct SixCrtProducer {
       int4 v[six::kPrimes];
 #pragma unroll
       for (int q = 0; q < six::kPrimes; ++q) v[q] = six::ld4<CG>(res + q * L + k0 + e0);
-      six_garner4(v, k, x, e0);
+      six_garner4(v, x, e0);
     }
   }
 };
@@ -244,7 +243,6 @@ template <bool CG>
 struct PieceCrtProducer {
   const u32* res;
   u64 L, k, P, ny, count;
-  SixCrt crt;
   static constexpr bool kBulk = true;
   __device__ __forceinline__ u64 piece_of(u64 j) const {
     const u64 i = j / k;
@@ -262,7 +260,7 @@ struct PieceCrtProducer {
       y[q] = (int)(CG ? __ldcg(c + q * L) : c[q * L]);
       if (ov) y[q] += (int)(CG ? __ldcg(b + q * L) : b[q * L]);
     }
-    return six_garner(y, crt);
+    return six_garner(y);
   }
   __device__ __forceinline__ void bulk(u64 k0, W3 (&x)[kScanE]) const {
     const u64 i = piece_of(k0), r = k0 - i * k;  // one piece for the eight positions
@@ -289,7 +287,7 @@ struct PieceCrtProducer {
           v[q].w += ov > e0 + 3 ? w.w : 0;
         }
       }
-      six_garner4(v, crt, x, e0);
+      six_garner4(v, x, e0);
     }
   }
 };

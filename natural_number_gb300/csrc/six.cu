@@ -67,6 +67,26 @@ Factors make_factors() {
   return F;
 }
 
+// 2^(96 - t) / (M / p_i) modulo each prime, by t.
+struct ScaleTable {
+  int2 f[kRootLog + 2][kPrimes];
+};
+ScaleTable make_scales() {
+  ScaleTable S;
+  for (int i = 0; i < kPrimes; ++i) {
+    const u64 p = prime_of(i);
+    u64 m = 1;
+    for (int j = 0; j < kPrimes; ++j)
+      if (j != i) m = m * (prime_of(j) % p) % p;
+    const u64 inv = h_pow(m, p - 2, p);
+    for (int t = 0; t < kRootLog + 2; ++t) {
+      const i32 w = h_center(h_pow(2, 96 - t, p) * inv % p, p);
+      S.f[t][i] = make_int2(w, h_companion(w, p));
+    }
+  }
+  return S;
+}
+
 // W[b] = the product of rho_t over the bits t of b (and of the inverses in
 // the second direction), centred, with its companion.  One launch writes
 // every entry of the 12 tables; an entry is at most 21 products.
@@ -85,67 +105,55 @@ __global__ void __launch_bounds__(256) six_table_kernel(int2* tab, u64 cap, cons
   tab[blockIdx.y * cap + b] = make_int2(w, (i32)((n + (n < 0 ? -(i64)h : (i64)h)) / p));
 }
 
-// Threads of a CTA: one unit of eight rows x four columns each.
-constexpr int col_threads(int R) { return std::max(32, (col_width(R) / 4) << (R - 3)); }
-constexpr int col_smem(int R) { return groups_of(R) > 1 ? (int)tile_words32<32>(R) * (col_width(R) / 32) * 4 : 0; }
-// Registers: 64 a thread; tiles of up to 2^8 rows as many CTAs as that allows.
-constexpr int col_blocks(int R) { return std::min(16, 1024 / col_threads(R)); }
-
 // First pass of up to two operands, the first in pieces: CTA (6 tile + prime,
 // y): piece y of a, or b for y = pieces.  The CTAs of one tile's six primes
 // run together, so its limbs cross HBM about once.
 template <int R>
 __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
-    six_load_kernel(SixOperands op, int s, const int2* __restrict__ tab, u64 cap, u32 tile0) {
+    six_load_kernel(SixOperands op, int s, const int2* __restrict__ tab, u64 cap, u32 tile0, int k8) {
   extern __shared__ __align__(16) u32 sm6[];
   const int prime = (int)(blockIdx.x % kPrimes);
   const u32 tile = tile0 + blockIdx.x / kPrimes;
   if (blockIdx.y < op.pieces) {
     const u64 at0 = blockIdx.y * op.piece;
     load_tile<R, col_width(R), col_threads(R), false>(sm6, op.a + at0, min(op.piece, op.na - at0),
-                                        op.ra + ((u64)blockIdx.y * kPrimes << s), s, tile, prime, tab, cap);
+                                        op.ra + ((u64)blockIdx.y * kPrimes << s), s, tile, prime, tab, cap, k8);
   } else {
-    load_tile<R, col_width(R), col_threads(R), false>(sm6, op.b, op.nb, op.rb, s, tile, prime, tab, cap);
+    load_tile<R, col_width(R), col_threads(R), false>(sm6, op.b, op.nb, op.rb, s, tile, prime, tab, cap, k8);
   }
 }
 
 template <int R, bool INV>
 __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
-    six_col_kernel(u32* ra, u32* rb, u32 pieces, int s, int lambda0, const int2* __restrict__ tab, u64 cap, bool raw) {
+    six_col_kernel(u32* ra, u32* rb, u32 pieces, const SixPlan pl, int lambda0, const int2* __restrict__ tab, u64 cap) {
   extern __shared__ __align__(16) u32 sm6[];
-  u32* res = blockIdx.z < pieces ? ra + ((u64)blockIdx.z * kPrimes << s) : rb;
-  col_tile<R, col_width(R), col_threads(R), INV, false>(sm6, res, s, lambda0, blockIdx.x, blockIdx.y, tab, cap, raw);
+  u32* res = blockIdx.z < pieces ? ra + ((u64)blockIdx.z * kPrimes << pl.s) : rb;
+  const bool last = INV && lambda0 == 0;
+  col_tile<R, col_width(R), col_threads(R), INV, false>(sm6, res, pl.s, lambda0, blockIdx.x, blockIdx.y, tab, cap, last,
+                                                           pl.scale[blockIdx.y], last ? pl.k8 : 8);
 }
 
-// One unit of eight rows x V columns a thread.
-constexpr int fused_threads(int R, int LGM, int V) { return std::max(32, (1 << (R + LGM)) / (8 * V)); }
-// Two tiles of 4096 words in shared memory let six CTAs share an SM: 768
-// threads (80 registers) of four columns each, more of fewer columns.
-constexpr int fused_blocks(int R, int LGM, int V) { return std::min(24, (V == 4 ? 768 : 1024) / fused_threads(R, LGM, V)); }
 template <int R, int LGM, int V, bool FIRST>
 __global__ void __launch_bounds__(fused_threads(R, LGM, V), fused_blocks(R, LGM, V))
-    six_fused_kernel(SixOperands op, int s, const int2* __restrict__ tab, u64 cap, bool reduce_in) {
+    six_fused_kernel(SixOperands op, const SixPlan pl, const int2* __restrict__ tab, u64 cap) {
   extern __shared__ __align__(16) u32 sm6[];
   constexpr int NT = fused_threads(R, LGM, V);
+  const int s = pl.s;
   u32* out = op.ra + ((u64)blockIdx.z * kPrimes << s);
   const int2* itab = tab + kPrimes * cap;
   if constexpr (FIRST) {
     const u64 at0 = blockIdx.z * op.piece;
     fused_tile<R, LGM, NT, V, true, false>(sm6, op.a + at0, min(op.piece, op.na - at0), op.b, op.nb, out, s, 0,
-                                           blockIdx.y, tab, itab, cap, false, op.pieces == 1);
+                                           blockIdx.y, tab, itab, cap, false, kAll, pl.scale[blockIdx.y], pl.k8);
   } else {
     fused_tile<R, LGM, NT, V, false, false>(sm6, out, 0, op.b ? op.rb : nullptr, 0, out, s, blockIdx.x, blockIdx.y,
-                                            tab, itab, cap, reduce_in, false);
+                                            tab, itab, cap, pl.reduce_in(), kAll, make_int2(0, 0), 8);
   }
 }
 
-template <class Kernel>
-cudaError_t allow_smem(Kernel k, int bytes) {
-  return bytes > 48 * 1024 ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
-}
-
 template <int R>
-cudaError_t launch_load(const SixOperands& op, int s, const SixTables& t, u32 tile0, u32 tile1, cudaStream_t st) {
+cudaError_t launch_load(const SixOperands& op, int s, int k8, const SixTables& t, u32 tile0, u32 tile1,
+                        cudaStream_t st) {
   constexpr int smem = col_smem(R);
   static const cudaError_t ok = allow_smem(six_load_kernel<R>, smem);
   if (ok != cudaSuccess) return ok;
@@ -153,108 +161,112 @@ cudaError_t launch_load(const SixOperands& op, int s, const SixTables& t, u32 ti
   tile1 = std::min(tile1, tiles);
   const dim3 grid(kPrimes * (tile1 - tile0), op.pieces + (op.b ? 1 : 0));
   launch_begin("six_load_col_pass", st);
-  six_load_kernel<R><<<grid, col_threads(R), smem, st>>>(op, s, t.tab, t.cap, tile0);
+  six_load_kernel<R><<<grid, col_threads(R), smem, st>>>(op, s, t.tab, t.cap, tile0, k8);
   launch_end(st);
   return cudaGetLastError();
 }
 template <int R, bool INV>
-cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, int s, int lambda0, const SixTables& t, cudaStream_t st) {
+cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int lambda0, const SixTables& t,
+                       cudaStream_t st) {
   constexpr int smem = col_smem(R);
   static const cudaError_t ok = allow_smem(six_col_kernel<R, INV>, smem);
   if (ok != cudaSuccess) return ok;
-  const dim3 grid((unsigned)((1ull << s) / ((u64)col_width(R) << R)), kPrimes, pieces + (rb ? 1 : 0));
+  // past the first pass, only the blocks of the first k8 eighths
+  const u64 tiles = (1ull << pl.s) / ((u64)col_width(R) << R);
+  const dim3 grid((unsigned)(lambda0 ? tiles / 8 * pl.k8 : tiles), kPrimes, pieces + (rb ? 1 : 0));
   launch_begin(INV ? (lambda0 == 0 ? "six_inv_last_col_pass" : "six_inv_col_pass") : "six_fwd_col_pass", st);
-  six_col_kernel<R, INV><<<grid, col_threads(R), smem, st>>>(
-      ra, rb, pieces, s, lambda0, t.tab + (INV ? kPrimes * t.cap : 0), t.cap, INV && lambda0 == 0 && pieces == 1);
+  six_col_kernel<R, INV><<<grid, col_threads(R), smem, st>>>(ra, rb, pieces, pl, lambda0,
+                                                              t.tab + (INV ? kPrimes * t.cap : 0), t.cap);
   launch_end(st);
   return cudaGetLastError();
 }
 template <int R, int LGM, int V, bool FIRST>
-cudaError_t launch_fused_v(const SixOperands& op, int s, const SixTables& t, bool reduce_in, cudaStream_t st) {
+cudaError_t launch_fused_v(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
   constexpr int tile = (int)tile_words32<1 << LGM>(R) * 4;
   static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, V, FIRST>, 2 * tile);
   if (ok != cudaSuccess) return ok;
   const int smem = (op.b ? 2 : 1) * tile;
-  const dim3 grid(FIRST ? 1u : (unsigned)((1ull << s) >> (R + LGM)), kPrimes, op.pieces);
+  const dim3 grid(FIRST ? 1u : (unsigned)(((1ull << pl.s) >> (R + LGM + 3)) * pl.k8), kPrimes, op.pieces);
   launch_begin(FIRST ? "six_small_pass" : "six_fused_row_pass", st);
-  six_fused_kernel<R, LGM, V, FIRST><<<grid, fused_threads(R, LGM, V), smem, st>>>(op, s, t.tab, t.cap, reduce_in);
+  six_fused_kernel<R, LGM, V, FIRST><<<grid, fused_threads(R, LGM, V), smem, st>>>(op, pl, t.tab, t.cap);
   launch_end(st);
   return cudaGetLastError();
 }
 // Columns a thread: as few as keep the grid within one wave of the GPU's
 // 152 x 768 threads, so a short product uses as many of them as it can.
 template <int R, int LGM, bool FIRST>
-cudaError_t launch_fused(const SixOperands& op, int s, const SixTables& t, bool reduce_in, cudaStream_t st) {
+cudaError_t launch_fused(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
   if constexpr (LGM == 3) {
-    const u64 units = ((u64)kPrimes * op.pieces << s) / 8;  // of one column
-    if (units <= 152 * 768) return launch_fused_v<R, LGM, 1, FIRST>(op, s, t, reduce_in, st);
+    const u64 units = ((u64)kPrimes * op.pieces << pl.s) / 64 * pl.k8;  // of one column
+    if (units <= 152 * 768) return launch_fused_v<R, LGM, 1, FIRST>(op, pl, t, st);
     if constexpr (R == 9)
-      if (units <= 2 * 152 * 768) return launch_fused_v<R, LGM, 2, FIRST>(op, s, t, reduce_in, st);
+      if (units <= 2 * 152 * 768) return launch_fused_v<R, LGM, 2, FIRST>(op, pl, t, st);
   }
-  return launch_fused_v<R, LGM, 4, FIRST>(op, s, t, reduce_in, st);
+  return launch_fused_v<R, LGM, 4, FIRST>(op, pl, t, st);
 }
 
-cudaError_t load_pass(const SixOperands& op, int s, int R, const SixTables& t, u32 t0, u32 t1, cudaStream_t st) {
+cudaError_t load_pass(const SixOperands& op, int s, int k8, int R, const SixTables& t, u32 t0, u32 t1,
+                      cudaStream_t st) {
   switch (R) {
-    case 4: return launch_load<4>(op, s, t, t0, t1, st);
-    case 5: return launch_load<5>(op, s, t, t0, t1, st);
-    case 6: return launch_load<6>(op, s, t, t0, t1, st);
-    case 7: return launch_load<7>(op, s, t, t0, t1, st);
-    case 8: return launch_load<8>(op, s, t, t0, t1, st);
-    case 9: return launch_load<9>(op, s, t, t0, t1, st);
+    case 4: return launch_load<4>(op, s, k8, t, t0, t1, st);
+    case 5: return launch_load<5>(op, s, k8, t, t0, t1, st);
+    case 6: return launch_load<6>(op, s, k8, t, t0, t1, st);
+    case 7: return launch_load<7>(op, s, k8, t, t0, t1, st);
+    case 8: return launch_load<8>(op, s, k8, t, t0, t1, st);
+    case 9: return launch_load<9>(op, s, k8, t, t0, t1, st);
   }
   return cudaErrorInvalidValue;
 }
 template <bool INV>
-cudaError_t col_pass(u32* ra, u32* rb, u32 pieces, int s, int lambda0, int R, const SixTables& t, cudaStream_t st) {
-  switch (R) {
-    case 4: return launch_col<4, INV>(ra, rb, pieces, s, lambda0, t, st);
-    case 5: return launch_col<5, INV>(ra, rb, pieces, s, lambda0, t, st);
-    case 6: return launch_col<6, INV>(ra, rb, pieces, s, lambda0, t, st);
-    case 7: return launch_col<7, INV>(ra, rb, pieces, s, lambda0, t, st);
-    case 8: return launch_col<8, INV>(ra, rb, pieces, s, lambda0, t, st);
-    case 9: return launch_col<9, INV>(ra, rb, pieces, s, lambda0, t, st);
+cudaError_t col_pass(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int k, const SixTables& t, cudaStream_t st) {
+  const int lambda0 = pl.lambda0[k];
+  switch (pl.R[k]) {
+    case 4: return launch_col<4, INV>(ra, rb, pieces, pl, lambda0, t, st);
+    case 5: return launch_col<5, INV>(ra, rb, pieces, pl, lambda0, t, st);
+    case 6: return launch_col<6, INV>(ra, rb, pieces, pl, lambda0, t, st);
+    case 7: return launch_col<7, INV>(ra, rb, pieces, pl, lambda0, t, st);
+    case 8: return launch_col<8, INV>(ra, rb, pieces, pl, lambda0, t, st);
+    case 9: return launch_col<9, INV>(ra, rb, pieces, pl, lambda0, t, st);
   }
   return cudaErrorInvalidValue;
 }
 cudaError_t fused_pass(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
-  const int R = pl.R[pl.n - 1], s = pl.s;
-  const bool red = pl.reduce_in();
+  const int R = pl.R[pl.n - 1];
   if (pl.n == 1) {
     switch (R) {
-      case 1: return launch_fused<1, 3, true>(op, s, t, red, st);
-      case 2: return launch_fused<2, 3, true>(op, s, t, red, st);
-      case 3: return launch_fused<3, 3, true>(op, s, t, red, st);
-      case 4: return launch_fused<4, 3, true>(op, s, t, red, st);
-      case 5: return launch_fused<5, 3, true>(op, s, t, red, st);
-      case 6: return launch_fused<6, 3, true>(op, s, t, red, st);
-      case 7: return launch_fused<7, 3, true>(op, s, t, red, st);
-      case 8: return launch_fused<8, 3, true>(op, s, t, red, st);
-      case 9: return launch_fused<9, 3, true>(op, s, t, red, st);
+      case 1: return launch_fused<1, 3, true>(op, pl, t, st);
+      case 2: return launch_fused<2, 3, true>(op, pl, t, st);
+      case 3: return launch_fused<3, 3, true>(op, pl, t, st);
+      case 4: return launch_fused<4, 3, true>(op, pl, t, st);
+      case 5: return launch_fused<5, 3, true>(op, pl, t, st);
+      case 6: return launch_fused<6, 3, true>(op, pl, t, st);
+      case 7: return launch_fused<7, 3, true>(op, pl, t, st);
+      case 8: return launch_fused<8, 3, true>(op, pl, t, st);
+      case 9: return launch_fused<9, 3, true>(op, pl, t, st);
     }
     return cudaErrorInvalidValue;
   }
   switch (pl.lgm) {
-    case 4: return launch_fused<8, 4, false>(op, s, t, red, st);
-    case 5: return launch_fused<7, 5, false>(op, s, t, red, st);
-    case 6: return launch_fused<6, 6, false>(op, s, t, red, st);
-    case 7: return launch_fused<5, 7, false>(op, s, t, red, st);
-    case 8: return launch_fused<4, 8, false>(op, s, t, red, st);
-    case 9: return launch_fused<4, 9, false>(op, s, t, red, st);
+    case 4: return launch_fused<8, 4, false>(op, pl, t, st);
+    case 5: return launch_fused<7, 5, false>(op, pl, t, st);
+    case 6: return launch_fused<6, 6, false>(op, pl, t, st);
+    case 7: return launch_fused<5, 7, false>(op, pl, t, st);
+    case 8: return launch_fused<4, 8, false>(op, pl, t, st);
+    case 9: return launch_fused<4, 9, false>(op, pl, t, st);
   }
   switch (R) {
-    case 5: return launch_fused<5, 3, false>(op, s, t, red, st);
-    case 6: return launch_fused<6, 3, false>(op, s, t, red, st);
-    case 7: return launch_fused<7, 3, false>(op, s, t, red, st);
-    case 8: return launch_fused<8, 3, false>(op, s, t, red, st);
-    case 9: return launch_fused<9, 3, false>(op, s, t, red, st);
+    case 5: return launch_fused<5, 3, false>(op, pl, t, st);
+    case 6: return launch_fused<6, 3, false>(op, pl, t, st);
+    case 7: return launch_fused<7, 3, false>(op, pl, t, st);
+    case 8: return launch_fused<8, 3, false>(op, pl, t, st);
+    case 9: return launch_fused<9, 3, false>(op, pl, t, st);
   }
   return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
-SixPlan six_plan(int s, int row_levels) {
+SixPlan six_plan(int s, u64 length, int row_levels) {
   SixPlan pl{};
   pl.s = s;
   const int T = std::min(s - 3, kRootLog);
@@ -275,6 +287,13 @@ SixPlan six_plan(int s, int row_levels) {
     left -= pl.R[k];
   }
   pl.R[pl.n - 1] = row;
+  const u64 eighth = (1ull << s) / 8;
+  pl.k8 = pl.R[0] >= 3 ? (int)std::clamp<u64>((length + eighth - 1) / eighth, 5, 8) : 8;
+  // The product residues are the coefficients times 2^T (the inverse's sums;
+  // 2^(T+1) of a truncated transform) and 2^-96 (the Montgomery steps of the
+  // two operands' limbs and of the blocks' products).
+  static const ScaleTable scales = make_scales();
+  std::copy_n(scales.f[T + (pl.k8 < 8)], kPrimes, pl.scale);
   return pl;
 }
 
@@ -321,36 +340,17 @@ u32 six_first_pass_columns(const SixPlan& pl) { return (u32)col_width(pl.R[0]); 
 
 cudaError_t six_load(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st, u32 tile0,
                      u32 tile1) {
-  return pl.n == 1 ? cudaSuccess : load_pass(op, pl.s, pl.R[0], t, tile0, tile1, st);
+  return pl.n == 1 ? cudaSuccess : load_pass(op, pl.s, pl.k8, pl.R[0], t, tile0, tile1, st);
 }
 
 cudaError_t six_finish(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   for (int k = 1; k + 1 < pl.n && e == cudaSuccess; ++k)
-    e = col_pass<false>(op.ra, op.b ? op.rb : nullptr, op.pieces, pl.s, pl.lambda0[k], pl.R[k], t, st);
+    e = col_pass<false>(op.ra, op.b ? op.rb : nullptr, op.pieces, pl, k, t, st);
   if (e == cudaSuccess) e = fused_pass(op, pl, t, st);
   for (int k = pl.n - 2; k >= 0 && e == cudaSuccess; --k)
-    e = col_pass<true>(op.ra, nullptr, op.pieces, pl.s, pl.lambda0[k], pl.R[k], t, st);
+    e = col_pass<true>(op.ra, nullptr, op.pieces, pl, k, t, st);
   return e;
-}
-
-// The product residues are the coefficients times 2^T (the inverse's sums)
-// and 2^-96 (the Montgomery steps of the two operands' limbs and of the
-// blocks' products); the CRT multiplies them by the inverse of that and of
-// the other primes' product.
-SixCrt six_crt(int s) {
-  SixCrt c;
-  const int T = std::min(s - 3, kRootLog);
-  for (int i = 0; i < kPrimes; ++i) {
-    const u64 p = prime_of(i);
-    u64 m = 1;
-    for (int j = 0; j < kPrimes; ++j)
-      if (j != i) m = m * (prime_of(j) % p) % p;
-    const u64 k = h_pow(2, 96 - T, p) * h_pow(m, p - 2, p) % p;
-    c.w[i] = h_center(k, p);
-    c.wp[i] = h_companion(c.w[i], p);
-  }
-  return c;
 }
 
 }  // namespace nn

@@ -233,11 +233,67 @@ __device__ __forceinline__ void inv_fold(Unit<K, V>& u, const Prime& P) {
     for (int c = 0; c < V; ++c) u.x[m][c] = reduce(u.x[m][c], P);
 }
 
+// Truncated transforms.  A product of at most k/8 L coefficients, k = 5, 6, 7,
+// is determined by its residues in the first k of the eight blocks at depth
+// 3: the passes then leave the others out, and only the last inverse group
+// (levels 2, 1, 0 of eight rows y_b, b < k known) differs.  With X the eighth
+// of the transform, P = sum_{j<k} a_j X^j, i = W[1], w = W[2], h = W[3] = i w
+// (w^2 = i, h^2 = -i, h^3 = w), the first four rows give 4 u = 4 P mod X^4 - 1,
+// the next two 2 v = 2 P mod X^2 - i, the seventh P(h); eliminating gives
+//  k = 5: 4 (a0 - a4) = 4 y4 - w 4u1 - i 4u2 - h 4u3
+//  k = 6: 4 (a_j - a_(j+4)) = 2 2v_j - i 4u_(j+2), j = 0, 1
+//  k = 7: E = 4 (a1 - a5) = 2 2v1 - i 4u3, F = 4 y6 - h E - w 4u3,
+//         8 (a0 - a4) = 2 2v0 + F, 8 (a2 - a6) = -i (2 2v0 - F).
+// Rows 0 .. k-1 receive 16 a_j, twice what the full group's sums give: the
+// transform's scale takes that into account.
+template <int V>
+__device__ __forceinline__ void inv_truncated(Unit<3, V>& u, int k8, const int2* __restrict__ itw,
+                                              const int2* __restrict__ ftw, const Prime& P) {
+  const i32 p = P.p;
+  const int2 i1 = __ldg(ftw + 1), w1 = __ldg(ftw + 2), h1 = __ldg(ftw + 3), ii = __ldg(itw + 1), wi = __ldg(itw + 2);
+#pragma unroll
+  for (int c = 0; c < V; ++c) {
+    const i32 y0 = u.x[0][c], y1 = u.x[1][c], y2 = u.x[2][c], y3 = u.x[3][c], y4 = u.x[4][c], y5 = u.x[5][c];
+    const i32 s0 = y0 + y1, d0 = y0 - y1, s1 = y2 + y3, d1 = mul_mod(y2 - y3, ii.x, ii.y, p);
+    const i32 u0 = reduce(s0 + s1, P), u2 = reduce(s0 - s1, P), u1 = reduce(d0 + d1, P), u3 = reduce(d0 - d1, P);
+    if (k8 == 5) {
+      const i32 d = 4 * reduce(y4, P) - mul_mod(u1, w1.x, w1.y, p) - mul_mod(u2, i1.x, i1.y, p) -
+                    mul_mod(u3, h1.x, h1.y, p);
+      u.x[0][c] = 2 * (u0 + d);
+      u.x[4][c] = 2 * (u0 - d);
+      u.x[1][c] = 4 * u1;
+      u.x[2][c] = 4 * u2;
+      u.x[3][c] = 4 * u3;
+    } else {
+      const i32 v0 = reduce(y4 + y5, P), v1 = mul_mod(y4 - y5, wi.x, wi.y, p);
+      const i32 e = 2 * v1 - mul_mod(u3, i1.x, i1.y, p);
+      u.x[1][c] = 2 * (u1 + e);
+      u.x[5][c] = 2 * (u1 - e);
+      u.x[3][c] = 4 * u3;
+      if (k8 == 6) {
+        const i32 d = 2 * v0 - mul_mod(u2, i1.x, i1.y, p);
+        u.x[0][c] = 2 * (u0 + d);
+        u.x[4][c] = 2 * (u0 - d);
+        u.x[2][c] = 4 * u2;
+      } else {
+        const i32 f = 4 * reduce(u.x[6][c], P) - mul_mod(e, h1.x, h1.y, p) - mul_mod(u3, w1.x, w1.y, p);
+        const i32 g = mul_mod(2 * v0 - f, i1.x, i1.y, p);
+        u.x[0][c] = 2 * u0 + 2 * v0 + f;
+        u.x[4][c] = 2 * u0 - 2 * v0 - f;
+        u.x[2][c] = 2 * u2 - g;
+        u.x[6][c] = 2 * u2 + g;
+      }
+    }
+  }
+}
+
 // Levels of a tile of R levels go in groups of at most three, one
 // shared-memory exchange between groups: groups_of(R) of them, the longer
-// ones first (forward order).
+// ones first (forward order; the first one three levels from R = 3 on, for
+// the truncated transforms).
 constexpr int groups_of(int R) { return (R + 2) / 3; }
 constexpr int group_size(int R, int g) {
+  if (R == 4) return g == 0 ? 3 : 1;
   int left = R, k = 0;
   for (int i = 0; i <= g; ++i) {
     const int n = groups_of(R) - i;
@@ -267,26 +323,49 @@ constexpr u32 tile_words32(int R) {
 // Columns of a strided tile: 32 (128 bytes), more where few rows would leave
 // the CTA with few units.
 constexpr int col_width(int R) { return R >= 7 ? 32 : 4096 >> R; }
-// In the batch kernel: 16 (64 bytes) at 9 levels, so that every tile stays
-// within the shared memory of the two tiles of a fused item.
-constexpr int batch_col_width(int R) { return R == 9 ? 16 : col_width(R); }
+
+// ---- launch shapes ----
+
+constexpr int at_least_warp(int threads) { return threads < 32 ? 32 : threads; }
+// Threads of a strided pass's CTA: one unit of eight rows x four columns each.
+constexpr int col_threads(int R) { return at_least_warp((col_width(R) / 4) << (R - 3)); }
+constexpr int col_smem(int R) { return groups_of(R) > 1 ? (int)tile_words32<32>(R) * (col_width(R) / 32) * 4 : 0; }
+// Registers: 64 a thread; tiles of up to 2^8 rows as many CTAs as that allows.
+constexpr int col_blocks(int R) { return 1024 / col_threads(R) < 16 ? 1024 / col_threads(R) : 16; }
+
+// One unit of eight rows x V columns a thread.
+constexpr int fused_threads(int R, int LGM, int V) { return at_least_warp((1 << (R + LGM)) / (8 * V)); }
+// Two tiles of 4096 words in shared memory let six CTAs share an SM: 768
+// threads (80 registers) of four columns each, more of fewer columns.
+constexpr int fused_blocks(int R, int LGM, int V) { 
+  const int n = (V == 4 ? 768 : 1024) / fused_threads(R, LGM, V);
+  return n < 24 ? n : 24;
+}
+template <class Kernel>
+inline cudaError_t allow_smem(Kernel k, int bytes) {
+  return bytes > 48 * 1024 ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
+}
 
 // Forward levels [0, R) of one tile of C columns x 2^R rows, block index ksb
 // at its first level.  load(row, col) gives the V words from (row, col), store
 // puts V finished words; between groups the words go
 // through sm.  HALF: the rows from 2^(R-1) are zero, so level 0 copies.
 // START: a reduction of the loaded words; LAST: one of the stored words.
+// k8 < 8: only the rows of the first k8 eighths are finished and stored.
 template <int R, int C, int NT, int V, bool START, bool LAST, class Load, class Store>
 __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const Store& store, bool half_zero,
-                                             const int2* __restrict__ tw, u32 ksb, const Prime& P, bool start_red) {
+                                             const int2* __restrict__ tw, u32 ksb, const Prime& P, bool start_red,
+                                             int k8 = 8) {
   constexpr int G = groups_of(R);
   auto group = [&](auto gc) {
     constexpr int g = decltype(gc)::value;
     constexpr int K = group_size(R, g), l = group_start(R, g), nsub = R - l - K;
     constexpr u32 units = (u32)(C / V) << (R - K);
     if (g > 0) __syncthreads();
+    const u32 todo = g == 0 ? units : units / 8 * k8;
+    const int keep = g == 0 && K == 3 ? k8 : 8;
 #pragma unroll 1
-    for (u32 i = threadIdx.x; i < units; i += NT) {
+    for (u32 i = threadIdx.x; i < todo; i += NT) {
       const u32 col = (i % (C / V)) * V, v = i / (C / V);
       const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
       Unit<K, V> u;
@@ -325,11 +404,12 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
 #pragma unroll
             for (int c = 0; c < V; ++c) u.x[m][c] = reduce(u.x[m][c], P);
           }
-          store(row0 + ((u32)m << nsub), col, u.get(m));
+          if (m < 5 || m < keep) store(row0 + ((u32)m << nsub), col, u.get(m));
         }
       } else {
 #pragma unroll
-        for (int m = 0; m < (1 << K); ++m) stv<false, V>(sp + at<C>((u32)m << nsub), u.get(m));
+        for (int m = 0; m < (1 << K); ++m)
+          if (m < 5 || m < keep) stv<false, V>(sp + at<C>((u32)m << nsub), u.get(m));
       }
     }
   };
@@ -339,19 +419,23 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
 }
 
 // Inverse levels R-1 .. 0 of one tile; the groups in the opposite order.
-// raw: the outputs of the last group go out unreduced (up to 12 p, for the
-// CRT; overlapping pieces are added there and want at most 1.5 p).
+// last: the transform's last pass; its outputs are multiplied by the scale,
+// which also makes them 0.75 p at most (k8 < 8, with the forward table ftw: a
+// truncated transform's).
 template <int R, int C, int NT, int V, class Load, class Store>
 __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const Store& store,
-                                             const int2* __restrict__ tw, u32 ksb, const Prime& P, bool raw) {
+                                             const int2* __restrict__ tw, u32 ksb, const Prime& P, bool last,
+                                             int2 scale, int k8, const int2* __restrict__ ftw) {
   constexpr int G = groups_of(R);
   auto group = [&](auto gc) {
     constexpr int g = decltype(gc)::value;
     constexpr int K = group_size(R, g), l = group_start(R, g), nsub = R - l - K;
     constexpr u32 units = (u32)(C / V) << (R - K);
     if (g + 1 < G) __syncthreads();
+    const u32 todo = g == 0 ? units : units / 8 * k8;
+    const int keep = g == 0 && K == 3 ? k8 : 8;
 #pragma unroll 1
-    for (u32 i = threadIdx.x; i < units; i += NT) {
+    for (u32 i = threadIdx.x; i < todo; i += NT) {
       const u32 col = (i % (C / V)) * V, v = i / (C / V);
       const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
       Unit<K, V> u;
@@ -359,15 +443,29 @@ __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const St
       u32* sp = sm + at<C>(row0) + col;
 #pragma unroll
       for (int m = 0; m < (1 << K); ++m) {
+        if (m >= 5 && m >= keep) continue;
         if constexpr (g + 1 == G)
           u.set(m, load(row0 + ((u32)m << nsub), col));
         else
           u.set(m, ldv<false, V>(sp + at<C>((u32)m << nsub)));
       }
-      inv_levels<K>(u, tw, b, P.p);
-      if (g > 0 || !raw) inv_fold<K>(u, P);
+      if (g == 0 && K == 3 && keep < 8) {
+        if constexpr (g == 0 && K == 3) inv_truncated(u, keep, tw, ftw, P);
+      } else {
+        inv_levels<K>(u, tw, b, P.p);
+      }
+      if (g == 0 && last) {
+#pragma unroll
+        for (int m = 0; m < (1 << K); ++m)
+#pragma unroll
+          for (int c = 0; c < V; ++c)
+            if (m < 5 || m < keep) u.x[m][c] = mul_mod(u.x[m][c], scale.x, scale.y, P.p);
+      } else {
+        inv_fold<K>(u, P);
+      }
 #pragma unroll
       for (int m = 0; m < (1 << K); ++m) {
+        if (m >= 5 && m >= keep) continue;
         if constexpr (g == 0)
           store(row0 + ((u32)m << nsub), col, u.get(m));
         else
@@ -408,7 +506,7 @@ __device__ __forceinline__ Words<V> limb_words(const u64* __restrict__ in, u64 n
 // [tile * C, tile * C + C) of every row of 2^(s-R).
 template <int R, int C, int NT, bool CG>
 __device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u64 n, u32* res, int s, u32 tile,
-                                          int prime, const int2* __restrict__ tab, u64 cap) {
+                                          int prime, const int2* __restrict__ tab, u64 cap, int k8) {
   const Prime P = c_primes[prime];
   const int lg_s = s - R;
   u32* out = res + ((u64)prime << s) + (u64)tile * C;
@@ -417,13 +515,16 @@ __device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u
   forward_tile<R, C, NT, 4, false, false>(
       sm, [&](u32 row, u32 col) { return limb_words<4>(in, n, ((u64)row << lg_s) + col0 + col, vec, P); },
       [&](u32 row, u32 col, const Words<4>& w) { stv<CG>(out + ((u64)row << lg_s) + col, w); }, n <= (1ull << (s - 1)),
-      tab + prime * cap, 0, P, false);
+      tab + prime * cap, 0, P, false, k8);
 }
 
-// Levels [lambda0, lambda0 + R) of residues in place: forward or inverse.
+// Levels [lambda0, lambda0 + R) of residues in place: forward or inverse (tab:
+// the inverse table, which follows the forward one).  k8: of the whole
+// transform, for its last inverse pass only.
 template <int R, int C, int NT, bool INV, bool CG>
 __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, u32 tile, int prime,
-                                         const int2* __restrict__ tab, u64 cap, bool raw = false) {
+                                         const int2* __restrict__ tab, u64 cap, bool last = false,
+                                         int2 scale = int2{}, int k8 = 8) {
   const Prime P = c_primes[prime];
   const int lg_s = s - lambda0 - R;
   const u32 per = (u32)((1ull << lg_s) / C);  // tiles a block
@@ -433,7 +534,7 @@ __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, 
   auto ld = [&](u32 row, u32 col) { return ldv<CG, 4>(g + ((u64)row << lg_s) + col); };
   auto st = [&](u32 row, u32 col, const Words<4>& w) { stv<CG>(g + ((u64)row << lg_s) + col, w); };
   if constexpr (INV)
-    inverse_tile<R, C, NT, 4>(sm, ld, st, tw, ksb, P, raw);
+    inverse_tile<R, C, NT, 4>(sm, ld, st, tw, ksb, P, last, scale, k8, tw - kPrimes * cap);
   else
     forward_tile<R, C, NT, 4, false, false>(sm, ld, st, false, tw, ksb, P, false);
 }
@@ -443,9 +544,9 @@ __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, 
 // magnitude, so the sums of eight products stay below 2^57.
 template <int R, int NT>
 __device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const int2* __restrict__ tw, u32 ksb,
-                                               const Prime& P) {
+                                               const Prime& P, u32 rows) {
 #pragma unroll 1
-  for (u32 r = threadIdx.x; r < (1u << R); r += NT) {
+  for (u32 r = threadIdx.x; r < rows; r += NT) {
     const u32 blk = (ksb << R) + r;
     int2 c = __ldg(tw + (blk >> 1));
     if (blk & 1) c = make_int2(-c.x, -c.y);
@@ -531,13 +632,15 @@ __device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const int2
 // first inverse levels.  a and b are residues after the strided passes (b
 // nullptr: a square), or, FIRST, limbs (na, nb of them; a transform of one
 // pass).  The inverse goes to out.  Modes for a batch run step by step:
+// (scale, k8: of a one-pass transform; otherwise the caller leaves tiles out.)
 // kAll everything; kForward only a's forward levels, written back to a;
 // kProduct products and inverse of operands whose forward levels are done.
 enum : int { kAll = 0, kForward = 1, kProduct = 2 };
 template <int R, int LGM, int NT, int V, bool FIRST, bool CG>
 __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const void* b, u64 nb, u32* out, int s,
                                            u32 tile, int prime, const int2* __restrict__ tab,
-                                           const int2* __restrict__ itab, u64 cap, bool reduce_in, bool raw, int mode = kAll) {
+                                           const int2* __restrict__ itab, u64 cap, bool reduce_in, int mode, int2 scale,
+                                           int k8) {
   constexpr int C = 1 << LGM;
   constexpr u32 W = tile_words32<C>(R);
   const Prime P = c_primes[prime];
@@ -553,7 +656,7 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
       const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
       forward_tile<R, C, NT, V, false, true>(
           t, [&](u32 row, u32 col) { return limb_words<V>(in, n, (u64)row * C + col, vec, P); }, to(t), n <= (1ull << (s - 1)),
-          tw, 0, P, false);
+          tw, 0, P, false, k8);
     } else {
       const u32* in = static_cast<const u32*>(src) + off;
       forward_tile<R, C, NT, V, true, true>(
@@ -566,7 +669,10 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
       *reinterpret_cast<int4*>(t + at<C>(i / C) + i % C) = ld4<CG>(in + i);
   };
   if (FIRST || mode != kProduct) {
-    forward(a, na, sa);
+    // one copy of the code for both operands
+    const int operands = b && (FIRST || mode != kForward) ? 2 : 1;
+#pragma unroll 1
+    for (int op = 0; op < operands; ++op) forward(op ? b : a, op ? nb : na, op ? sb : sa);
     if (!FIRST && mode == kForward) {
       __syncthreads();
       u32* back = out + off;
@@ -574,21 +680,20 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
         stv<CG>(back + i, ldv<false, 4>(sa + at<C>(i / C) + i % C));
       return;
     }
-    if (b) forward(b, nb, sb);
   } else if constexpr (!FIRST) {
     fetch(a, sa);
     if (b) fetch(b, sb);
   }
   __syncthreads();
   if constexpr (LGM == 3)
-    leaf_products8<R, NT>(sa, sb, tw, FIRST ? 0 : tile, P);
+    leaf_products8<R, NT>(sa, sb, tw, FIRST ? 0 : tile, P, FIRST && R >= 3 ? (u32)k8 << (R - 3) : 1u << R);
   else
     leaf_products<R, LGM, NT>(sa, sb, tw, FIRST ? 0 : tile, P);
   u32* dst = out + ((u64)prime << s) + (FIRST ? 0 : (u64)tile << (R + LGM));
   __syncthreads();
   inverse_tile<R, C, NT, V>(
       sa, [&](u32 row, u32 col) { return ldv<false, V>(sa + at<C>(row) + col); },
-      [&](u32 row, u32 col, const Words<V>& w) { stv<CG>(dst + row * C + col, w); }, itw, FIRST ? 0 : tile, P, FIRST && raw);
+      [&](u32 row, u32 col, const Words<V>& w) { stv<CG>(dst + row * C + col, w); }, itw, FIRST ? 0 : tile, P, FIRST, scale, FIRST ? k8 : 8, tw);
 }
 
 }  // namespace six

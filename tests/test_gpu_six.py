@@ -48,6 +48,36 @@ def test_every_scale_vs_oracle(ctx, oracle, s):
         assert np.array_equal(got[: want.size], want) and not got[want.size:].any()
 
 
+@pytest.mark.parametrize("s", [6, 9, 10, 12, 13, 14, 17, 18, 19, 22])
+def test_truncated_transforms_vs_oracle(ctx, oracle, s):
+    """Products that end at, just below and just above each eighth of the
+    transform, one at a time and in a batch (which takes the short ones too)."""
+    import torch
+    L = 1 << s
+    sizes = []
+    for k in (5, 6, 7):
+        for length in (k * L // 8 - 1, k * L // 8, k * L // 8 + 1):
+            na = length // 2 + 1 + (length // 16 if k == 6 else 0)
+            sizes.append((na, length + 1 - na))
+    a_list = [limbs(s + k, na) for k, (na, _) in enumerate(sizes)]
+    b_list = [limbs(s + 50 + k, nb) for k, (_, nb) in enumerate(sizes)]
+    da, db = [to_dev(a) for a in a_list], [to_dev(b) for b in b_list]
+    outs = [torch.empty(na + nb, dtype=torch.uint64, device="cuda") for na, nb in sizes]
+    old = {k: ctx.get_tunable(k) for k in ("batch_ntt_min", "batch_school_balanced")}
+    try:
+        ctx.set_tunable("batch_ntt_min", 1)
+        ctx.set_tunable("batch_school_balanced", 0)
+        ctx.batch([x for x, _ in sizes], [y for _, y in sizes]).run(list(zip(da, db)), outs)
+        ctx.synchronize()
+    finally:
+        for k, v in old.items():
+            ctx.set_tunable(k, v)
+    for k in range(len(sizes)):
+        want = oracle.mul(a_list[k], b_list[k])
+        for got in (to_host(product(ctx, da[k], db[k])), to_host(outs[k])):
+            assert np.array_equal(got[: want.size], want) and not got[want.size:].any(), sizes[k]
+
+
 @pytest.mark.parametrize("s", [20, 21, 22, 23, 24, 25, 26, 27, 28])
 def test_long_scales_by_residues(ctx, s):
     import torch

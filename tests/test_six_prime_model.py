@@ -15,6 +15,8 @@ LIMIT = 1 << 31
 
 
 def groups(R):
+    if R == 4:
+        return [(0, 3), (3, 1)]
     n, left, out, l = (R + 2) // 3, R, [], 0
     for i in range(n):
         k = -(-left // (n - i))
@@ -107,17 +109,17 @@ def center(w, p):
     return w - p if w > p // 2 else w
 
 
-def crt(y, kappa):
+def crt(y):
     cols, frac = [0] * 6, 1 << 24
     for i, p in enumerate(P):
-        t = mul_mod(y[i], kappa[i], p) + p
-        assert 0 < t < 2 * p
+        t = y[i] + 2 * p
+        assert 0 < t < 4 * p
         frac += (t >> 12) * (((1 << 39) + p // 2) // p)
         m = M // p
         for j in range(5):
             cols[j] += t * ((m >> (32 * j)) & 0xffffffff)
         assert m >> 160 == 0
-    assert frac < 1 << 32 and max(cols) < 1 << 63
+    assert frac < 1 << 32 and max(cols) < (1 << 64) - (1 << 37)
     neg = (1 << 192) - M
     v = sum(c << (32 * j) for j, c in enumerate(cols)) + (frac >> 27) * neg
     return v % (1 << 192)
@@ -125,17 +127,54 @@ def crt(y, kappa):
 
 def test_crt_quotient_over_its_range():
     rng = random.Random(3)
-    kappa = [center(pow(M // p, -1, p), p) for p in P]
+    inv = [pow(M // p, -1, p) for p in P]
     values = [0, 1, 2, (1 << 160) - 1, 1 << 160, (1 << 128) - 1] + [rng.randrange(1 << 160) for _ in range(2000)]
     values += [rng.randrange(1 << rng.randrange(1, 161)) for _ in range(2000)]
     for v in values:
-        y = []
-        for p in P:
-            r = center(v, p)
-            y.append(max(-LIMIT + 1, min(LIMIT - 1, r + p * rng.randrange(-12, 13))) if abs(r) < p // 8 else r)
-            if (y[-1] - v) % p:
-                y[-1] = r
-        assert crt(y, kappa) == v
+        base = [center(v * k, p) for k, p in zip(inv, P)]
+        for shift in ([0] * 6, [1] * 6, [-1] * 6, [rng.choice((-1, 0, 1)) for _ in P]):  # up to 1.5 p
+            assert crt([r + d * p for r, d, p in zip(base, shift, P)]) == v
+
+
+@pytest.mark.parametrize("p", P)
+@pytest.mark.parametrize("k8", [5, 6, 7])
+def test_truncated_last_group(p, k8):
+    """Rows y_b = P(c_b) of a polynomial of k8 coefficients at the first k8 of
+    the eight points, to 16 times its coefficients; every intermediate at its
+    worst stays in 32 bits."""
+    rng = random.Random(p + k8)
+    g = root(p)
+    i, w = pow(g, 1 << 20, p), pow(g, 1 << 19, p)
+    h = i * w % p
+    points = [1, p - 1, i, p - i, w, p - w, h, p - h]
+    a = [rng.randrange(p) for _ in range(k8)]
+    y = [sum(v * pow(points[b], j, p) for j, v in enumerate(a)) for b in range(k8)] + [0] * (8 - k8)
+    ii, wi = pow(i, -1, p), pow(w, -1, p)
+    u0, u2 = y[0] + y[1] + y[2] + y[3], y[0] + y[1] - y[2] - y[3]
+    d1 = (y[2] - y[3]) * ii
+    u1, u3 = y[0] - y[1] + d1, y[0] - y[1] - d1
+    out = [0] * 8
+    if k8 == 5:
+        d = 4 * y[4] - w * u1 - i * u2 - h * u3
+        out = [2 * (u0 + d), 4 * u1, 4 * u2, 4 * u3, 2 * (u0 - d)]
+    else:
+        v0, v1 = y[4] + y[5], (y[4] - y[5]) * wi
+        e = 2 * v1 - i * u3
+        out[1], out[5], out[3] = 2 * (u1 + e), 2 * (u1 - e), 4 * u3
+        if k8 == 6:
+            d = 2 * v0 - i * u2
+            out[0], out[4], out[2] = 2 * (u0 + d), 2 * (u0 - d), 4 * u2
+        else:
+            f = 4 * y[6] - h * e - w * u3
+            q = (2 * v0 - f) * i
+            out[0], out[4] = 2 * u0 + 2 * v0 + f, 2 * u0 - 2 * v0 - f
+            out[2], out[6] = 2 * u2 - q, 2 * u2 + q
+    assert [v % p for v in out[:k8]] == [16 * v % p for v in a]
+    step = lambda x: 0.5 + x * p / 2**33  # noqa: E731  a product or a reduction, in p; rows come in below 1.5 p
+    u, v = step(6.0), step(3.0)
+    d5, d6 = 4 * step(1.5) + 3 * step(u), 2 * v + step(u)
+    f7 = 4 * step(1.5) + step(d6) + step(u)
+    assert max(2 * (u + d5), 2 * (u + d6), 2 * u + 2 * v + f7, 4 * u, 2 * v + f7) < LIMIT / p  # then scaled, to 0.75 p
 
 
 def root(p):
@@ -189,7 +228,8 @@ def test_products(s, T, na, nb):
                     u, v = o[2 * b * h + i], o[2 * b * h + h + i]
                     o[2 * b * h + i], o[2 * b * h + h + i] = (u + v) % p, (u - v) * wi % p
         res.append(o)
-    kappa = [center(pow(2, 96 - T, p) * pow(M // p, -1, p), p) for p in P]
-    total = sum(crt([center(res[i][k], P[i]) for i in range(6)], kappa) << (64 * k) for k in range(na + nb - 1))
+    scale = [pow(2, 96 - T, p) * pow(M // p, -1, p) for p in P]
+    total = sum(crt([mul_mod(center(res[i][k], P[i]), center(scale[i], P[i]), P[i]) for i in range(6)]) << (64 * k)
+                for k in range(na + nb - 1))
     val = lambda X: sum(v << (64 * i) for i, v in enumerate(X))  # noqa: E731
     assert total == val(A) * val(B)
