@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
       n = min(J.piece, J.na - pt.piece * J.piece);
       res = J.res_a + (pt.piece * kPrimes << s);
     }
-    load_tile<R, col_width(R), col_threads(R), false>(sm6, in, n, res, s, tile, it.prime, t.tab, t.cap, J.plan.k8);
+    load_tile<R, col_width(R), col_threads(R)>(sm6, in, n, res, s, tile, it.prime, t.tab, t.cap, J.plan.k8);
   }
 }
 
@@ -89,13 +89,13 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
       res = J.res_a + (pt.piece * kPrimes << s);
     }
     const bool last = INV && pass == 0;
-    col_tile<R, col_width(R), col_threads(R), INV, false>(sm6, res, s, J.plan.lambda0[pass], tile, it.prime,
+    col_tile<R, col_width(R), col_threads(R), INV>(sm6, res, s, J.plan.lambda0[pass], tile, it.prime,
                                                            t.tab + (INV ? kPrimes * t.cap : 0), t.cap, last,
                                                            J.plan.scale[it.prime], last ? J.plan.k8 : 8);
   }
 }
 
-// The contiguous last pass, tile by tile (mode: six_tiles.cuh).
+// The contiguous last pass, tile by tile (MODE: six_tiles.cuh).
 template <int R, int LGM, int MODE>
 __global__ void __launch_bounds__(fused_threads(R, LGM, 4), fused_blocks(R, LGM, 4))
     batch_fused_kernel(const BatchJob* __restrict__ jobs, const BatchItem* __restrict__ items, const SixTables t) {
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(fused_threads(R, LGM, 4), fused_blocks(R, LGM,
   const BatchJob& J = jobs[it.job];
   const int s = J.plan.s;
   const u32 per = (u32)((1ull << s) >> (R + LGM));
-  const u32* b = J.square ? nullptr : J.res_b;
+  const u32* b = !J.square ? J.res_b : MODE == kProduct ? J.res_a : nullptr;
   for (u32 q = 0; q < it.ntile; ++q) {
     if (q) __syncthreads();
     u32* res = J.res_b;
@@ -114,15 +114,17 @@ __global__ void __launch_bounds__(fused_threads(R, LGM, 4), fused_blocks(R, LGM,
       tile = pt.tile;
       res = J.res_a + (pt.piece * kPrimes << s);
     }
-    fused_tile<R, LGM, fused_threads(R, LGM, 4), 4, false, false>(sm6, res, 0, b, 0, res, s, tile, it.prime, t.tab,
-                                                                  t.tab + kPrimes * t.cap, t.cap, J.plan.reduce_in(),
-                                                                  MODE, int2{}, 8);
+    fused_tile<R, LGM, fused_threads(R, LGM, 4), 4, MODE, false>(sm6, res, 0, b, 0, res, s, tile, it.prime, t.tab,
+                                                                 t.tab + kPrimes * t.cap, t.cap, J.plan.reduce_in(),
+                                                                 false, int2{}, 8);
   }
 }
 
-// Columns a thread of a one-pass transform: a warp or more of busy threads.
+// One-pass transforms from limbs: a's pieces with b (kAll), with b's finished
+// words (kReady), or b's forward levels (kForward).
+// Columns a thread: a warp or more of busy threads.
 constexpr int small_columns(int R) { return R <= 6 ? 1 : R == 7 ? 2 : 4; }
-template <int R>
+template <int R, int MODE>
 __global__ void __launch_bounds__(fused_threads(R, 3, small_columns(R)), fused_blocks(R, 3, small_columns(R)))
     batch_small_kernel(const BatchJob* __restrict__ jobs, const BatchItem* __restrict__ items, const SixTables t) {
   extern __shared__ __align__(16) u32 sm6[];
@@ -133,10 +135,13 @@ __global__ void __launch_bounds__(fused_threads(R, 3, small_columns(R)), fused_b
   for (u32 q = 0; q < it.ntile; ++q) {  // a piece an index
     if (q) __syncthreads();
     const u64 piece = it.tile + q;
-    fused_tile<R, 3, fused_threads(R, 3, V), V, true, false>(
-        sm6, J.a + piece * J.piece, min(J.piece, J.na - piece * J.piece), J.square ? nullptr : J.b, J.nb,
-        J.res_a + (piece * kPrimes << s), s, 0, it.prime, t.tab, t.tab + kPrimes * t.cap, t.cap, false, kAll,
-        J.plan.scale[it.prime], J.plan.k8);
+    const u64* a = MODE == kForward ? J.b : J.a + piece * J.piece;
+    const u64 na = MODE == kForward ? J.nb : min(J.piece, J.na - piece * J.piece);
+    const void* b = MODE == kReady ? static_cast<const void*>(J.res_b) : J.square ? nullptr : J.b;
+    u32* out = MODE == kForward ? J.res_b : J.res_a + (piece * kPrimes << s);
+    fused_tile<R, 3, fused_threads(R, 3, V), V, MODE, true>(sm6, a, na, b, J.nb, out, s, 0, it.prime, t.tab,
+                                                            t.tab + kPrimes * t.cap, t.cap, false, true,
+                                                            J.plan.scale[it.prime], J.plan.k8);
   }
 }
 
@@ -157,10 +162,10 @@ __global__ void __launch_bounds__(kScanThreads, 3)
   const BatchJob& J = jobs[it.job];
   const u64 size = J.na + J.nb, L = 1ull << J.plan.s;
   if constexpr (PIECES) {
-    const PieceCrtProducer<false> prod{J.res_a, L, J.piece, J.pieces, J.nb, size - 1};
+    const PieceCrtProducer prod{J.res_a, L, J.piece, J.pieces, J.nb, size - 1};
     scan_tile(prod, it.tile, size, J.out, size, nullptr, flags + J.flag_base, err);
   } else {
-    const SixCrtProducer<false> prod{J.res_a, L, size - 1};
+    const SixCrtProducer prod{J.res_a, L, size - 1};
     scan_tile(prod, it.tile, size, J.out, size, nullptr, flags + J.flag_base, err);
   }
 }
@@ -201,27 +206,33 @@ struct Launch {
       batch_col_kernel<R, true><<<g.count, threads, smem, st>>>(jobs, items, t, g.pass);
     return cudaGetLastError();
   }
+  template <int R, int LGM, int MODE>
+  cudaError_t contiguous_mode() const {
+    constexpr int smem = fused_tiles(LGM, MODE) * (int)tile_words32<1 << LGM>(R) * 4;
+    static const cudaError_t ok = allow_smem(batch_fused_kernel<R, LGM, MODE>, smem);
+    if (ok != cudaSuccess) return ok;
+    batch_fused_kernel<R, LGM, MODE><<<g.count, fused_threads(R, LGM, 4), smem, st>>>(jobs, items, t);
+    return cudaGetLastError();
+  }
   template <int R, int LGM>
   cudaError_t contiguous() const {
-    constexpr int tile = (int)tile_words32<1 << LGM>(R) * 4, threads = fused_threads(R, LGM, 4);
-    static const cudaError_t ok[3] = {allow_smem(batch_fused_kernel<R, LGM, kAll>, 2 * tile),
-                                      allow_smem(batch_fused_kernel<R, LGM, kProduct>, 2 * tile),
-                                      allow_smem(batch_fused_kernel<R, LGM, kForward>, tile)};
-    for (cudaError_t e : ok)
-      if (e != cudaSuccess) return e;
-    if (g.kind == kBatchRow)
-      batch_fused_kernel<R, LGM, kForward><<<g.count, threads, tile, st>>>(jobs, items, t);
-    else if (g.pass)  // after kBatchRow
-      batch_fused_kernel<R, LGM, kProduct><<<g.count, threads, 2 * tile, st>>>(jobs, items, t);
-    else
-      batch_fused_kernel<R, LGM, kAll><<<g.count, threads, 2 * tile, st>>>(jobs, items, t);
+    if (g.kind == kBatchRow) return contiguous_mode<R, LGM, kForward>();
+    switch (g.pass) {
+      case kBatchRowsB: return contiguous_mode<R, LGM, kReady>();
+      case kBatchRowsAll: return contiguous_mode<R, LGM, kProduct>();
+    }
+    return contiguous_mode<R, LGM, kAll>();
+  }
+  template <int R, int MODE>
+  cudaError_t small_mode() const {
+    constexpr int smem = fused_tiles(3, MODE) * (int)tile_words32<8>(R) * 4;
+    batch_small_kernel<R, MODE><<<g.count, fused_threads(R, 3, small_columns(R)), smem, st>>>(jobs, items, t);
     return cudaGetLastError();
   }
   template <int R>
   cudaError_t small() const {
-    constexpr int smem = 2 * (int)tile_words32<8>(R) * 4;
-    batch_small_kernel<R><<<g.count, fused_threads(R, 3, small_columns(R)), smem, st>>>(jobs, items, t);
-    return cudaGetLastError();
+    if (g.kind == kBatchSmallRow) return small_mode<R, kForward>();
+    return g.pass == kBatchRowsB ? small_mode<R, kReady>() : small_mode<R, kAll>();
   }
 
   cudaError_t operator()(u32* ticket, u32* flags, u32* err) const {
@@ -256,6 +267,7 @@ struct Launch {
           case 9: return contiguous<9, 3>();
         }
         break;
+      case kBatchSmallRow:
       case kBatchSmall:
         switch (g.R) {
           case 1: return small<1>();

@@ -355,6 +355,60 @@ cudaError_t ntt_save(const u64* res, int s, u64* out, u64 size, Scan& sc, u64* w
   return run_scan(CrtProducer{res, L, size - 1}, size, out, size, sc, st, "crt_carry_scan");
 }
 
+namespace {
+// Coefficient k of the six-prime residues modulo each 62-bit prime: its three
+// words by Horner's rule, b[i] = 2^64 mod p_i with its Shoup companion.
+struct TwoTo64 {
+  u64 w[3], s[3];
+};
+__global__ void __launch_bounds__(256) six_to_three_kernel(const u32* res, u64 L, u64* out, const TwoTo64 b) {
+  const u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= L) return;
+  const W3 v = SixCrtProducer{res, L, L}(k);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const u64 p = g_primes.p[i], m = g_primes.m64[i];
+    const u32 ch = g_primes.c_hi[i];
+    u64 r = limb_mod(v.w2, m, p, ch);
+    r = reduce2p(shoup_mul(r, b.w[i], b.s[i], p, ch) + limb_mod(v.w1, m, p, ch), p);
+    r = reduce2p(shoup_mul(r, b.w[i], b.s[i], p, ch) + limb_mod(v.w0, m, p, ch), p);
+    out[i * L + k] = r;
+  }
+}
+}  // namespace
+
+cudaError_t six_to_three(const u32* res, int s, u64* out, cudaStream_t st) {
+  u64 p[3];
+  primes_host(p);
+  TwoTo64 b;
+  for (int i = 0; i < 3; ++i) {
+    b.w[i] = (u64)(((unsigned __int128)1 << 64) % p[i]);
+    b.s[i] = (u64)(((unsigned __int128)b.w[i] << 64) / p[i]) + 1;
+  }
+  const u64 L = 1ull << s;
+  launch_begin("six_to_three", st);
+  six_to_three_kernel<<<(unsigned)((L + 255) / 256), 256, 0, st>>>(res, L, out, b);
+  launch_end(st);
+  return cudaGetLastError();
+}
+
+cudaError_t six_save_words(const u32* res, int s, u64* out, u64 size, Scan& sc, u64* written, cudaStream_t st) {
+  const u64 L = 1ull << s;
+  cudaError_t e = scan_reserve(sc, 1);
+  if (e != cudaSuccess) return e;
+  if (size - 1 <= L) {
+    *written = size;
+    return run_scan(SixCrtProducer{res, L, size - 1}, size, out, size, sc, st, "six_crt_scan");
+  }
+  e = run_scan(SixCrtProducer{res, L, L}, L + 2, out, L, sc, st, "six_crt_scan");
+  if (e != cudaSuccess) return e;
+  launch_begin("wrap_fix", st);
+  wrap_fix_kernel<<<1, 1024, 0, st>>>(out, L, sc.side);
+  launch_end(st);
+  *written = L;
+  return cudaGetLastError();
+}
+
 cudaError_t six_save(const SixOperands& op, const SixPlan& pl, u64* out, Scan& sc, cudaStream_t st, int chunks,
                      const std::function<cudaError_t(u64, u64)>& done) {
   const u64 L = 1ull << pl.s, nb = op.b ? op.nb : op.na, size = op.na + nb;
@@ -364,9 +418,9 @@ cudaError_t six_save(const SixOperands& op, const SixPlan& pl, u64* out, Scan& s
     const u64 t0 = tiles * k / chunks, t1 = tiles * (k + 1) / chunks;
     if (t1 == t0) continue;
     if (op.pieces == 1)
-      e = run_scan(SixCrtProducer<false>{op.ra, L, size - 1}, size, out, size, sc, st, "six_crt_scan", t0, t1);
+      e = run_scan(SixCrtProducer{op.ra, L, size - 1}, size, out, size, sc, st, "six_crt_scan", t0, t1);
     else
-      e = run_scan(PieceCrtProducer<false>{op.ra, L, op.piece, op.pieces, nb, size - 1}, size, out, size, sc, st,
+      e = run_scan(PieceCrtProducer{op.ra, L, op.piece, op.pieces, nb, size - 1}, size, out, size, sc, st,
                    "six_crt_scan", t0, t1);
     if (e == cudaSuccess && done) e = done(t0 * kScanTile, std::min(size, t1 * kScanTile));
   }

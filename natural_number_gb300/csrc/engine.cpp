@@ -168,10 +168,18 @@ struct nn_batch {
   bool pending = false;
 };
 
+// A kept transform.  Its residues are six-prime words — the finished forward
+// transform, or a product's residues as the CRT takes them — or the
+// three-prime words of the reference's layout: for scales the six primes do
+// not serve, and for products of more than two factors, whose coefficients may
+// exceed what six primes hold.
 struct nn_transform {
-  u64* res = nullptr;  // [3][2^scale]
+  enum Rep { kThree, kSixForward, kSixProduct };
+  u64* res = nullptr;  // [3][2^scale], or [6][2^scale] 32-bit words
   u64 words = 0;       // allocated words (3 * 2^scale at most)
   int scale = 0;
+  Rep rep = kThree;
+  nn::u32* six() const { return reinterpret_cast<nn::u32*>(res); }
 };
 
 namespace {
@@ -233,25 +241,19 @@ nn_status xform_reserve(nn_context* c, nn_transform* t, int s) {
   return NN_OK;
 }
 
-nn_status forward(nn_context* c, nn_transform* t, const u64* d_limbs, u64 n, int s) {
-  if (s < 2 || s > 40 || n == 0 || n > (1ull << s)) {
-    c->err = "forward: need 2 <= scale <= 40 and 1 <= n <= 2^scale";
-    return NN_ERR_INVALID;
-  }
+// Three-prime transform.
+nn_status forward3(nn_context* c, nn_transform* t, const u64* d_limbs, u64 n, int s) {
   NN_CK(c, nn::tables_ensure(c->tables, s, c->stream, &c->retired_tables), "twiddle tables");
   nn_status st = xform_reserve(c, t, s);
   if (st != NN_OK) return st;
+  t->rep = nn_transform::kThree;
   const std::vector<nn::Pass> plan = c->passes(s);
   NN_CK(c, nn::ntt_forward(d_limbs, n, t->res, s, c->tables, c->stream, &plan), "forward NTT");
   return NN_OK;
 }
 
-nn_status inverse_save(nn_context* c, nn_transform* t, u64* d_out, u64 size, u64* written,
-                       bool skip_last_pass = false) {
-  if (size < 2) {
-    c->err = "save: size must be at least 2";
-    return NN_ERR_INVALID;
-  }
+nn_status inverse_save3(nn_context* c, nn_transform* t, u64* d_out, u64 size, u64* written,
+                        bool skip_last_pass = false) {
   const std::vector<nn::Pass> plan = c->passes(t->scale);
   NN_CK(c, nn::ntt_inverse(t->res, t->scale, c->tables, c->stream, &plan, skip_last_pass), "inverse NTT");
   u64 w = 0;
@@ -260,14 +262,116 @@ nn_status inverse_save(nn_context* c, nn_transform* t, u64* d_out, u64 size, u64
   return NN_OK;
 }
 
+nn_status forward_args(nn_context* c, u64 n, int s) {
+  if (s >= 2 && s <= 40 && n != 0 && n <= (1ull << s)) return NN_OK;
+  c->err = "forward: need 2 <= scale <= 40 and 1 <= n <= 2^scale";
+  return NN_ERR_INVALID;
+}
+nn_status save_args(nn_context* c, u64 size) {
+  if (size >= 2) return NN_OK;
+  c->err = "save: size must be at least 2";
+  return NN_ERR_INVALID;
+}
+
+// Kept transforms over six primes up to this scale (blocks of up to 64
+// coefficients; beyond, the three-prime passes are faster).
+constexpr int kSixTransformMaxScale = 28;
+
+nn_status forward(nn_context* c, nn_transform* t, const u64* d_limbs, u64 n, int s) {
+  nn_status st = forward_args(c, n, s);
+  if (st != NN_OK) return st;
+  if (s < nn::kSixMinScale || s > kSixTransformMaxScale) return forward3(c, t, d_limbs, n, s);
+  NN_CK(c, nn::six_tables_ensure(c->six, s, c->stream, &c->retired_tables), "twiddle tables");
+  st = xform_reserve(c, t, s);
+  if (st != NN_OK) return st;
+  t->rep = nn_transform::kSixForward;
+  NN_CK(c, nn::six_forward(d_limbs, n, t->six(), nn::six_plan(s, 1ull << s), c->six, c->stream), "forward NTT");
+  return NN_OK;
+}
+
+// A six-prime transform's product residues: its own, or for a forward
+// transform those of its product with 1 (one limb), in `tmp`.
+nn_status six_product_words(nn_context* c, const nn_transform* t, DBuf& tmp, const nn::u32** words) {
+  *words = t->six();
+  if (t->rep == nn_transform::kSixProduct) return NN_OK;
+  const u64 n = 3ull << t->scale;
+  nn_status st = tmp.alloc(n + 1);
+  if (st != NN_OK) return st;
+  const u64 one = 1;
+  NN_CK(c, c->stage.upload(tmp.p + n, &one, sizeof one, c->stream), "constant");
+  const nn::SixPlan pl = nn::six_plan(t->scale, 1ull << t->scale);
+  nn::u32* w = reinterpret_cast<nn::u32*>(tmp.p);
+  NN_CK(c, nn::six_forward(tmp.p + n, 1, w, pl, c->six, c->stream), "forward NTT");
+  NN_CK(c, nn::six_pointwise(w, t->six(), w, pl, c->six, c->stream), "inverse NTT");
+  *words = w;
+  return NN_OK;
+}
+
+// t's residues modulo the three primes, as the reference's transform has
+// them, into dst: a six-prime transform's coefficients, reduced, through the
+// three-prime forward passes.
+nn_status three_words(nn_context* c, const nn_transform* t, u64* dst) {
+  if (t->rep == nn_transform::kThree) {
+    NN_CK(c, cudaMemcpyAsync(dst, t->res, (3ull << t->scale) * sizeof(u64), cudaMemcpyDeviceToDevice, c->stream),
+          "copy residues");
+    return NN_OK;
+  }
+  DBuf tmp(c);
+  const nn::u32* w = nullptr;
+  nn_status st = six_product_words(c, t, tmp, &w);
+  if (st != NN_OK) return st;
+  NN_CK(c, nn::tables_ensure(c->tables, t->scale, c->stream, &c->retired_tables), "twiddle tables");
+  NN_CK(c, nn::six_to_three(w, t->scale, dst, c->stream), "residues");
+  NN_CK(c, nn::ntt_forward_residues(dst, t->scale, c->tables, c->stream, c->passes(t->scale)), "forward NTT");
+  return NN_OK;
+}
+
+nn_status inverse_save(nn_context* c, nn_transform* t, u64* d_out, u64 size, u64* written) {
+  nn_status st = save_args(c, size);
+  if (st != NN_OK) return st;
+  if (t->rep == nn_transform::kThree) return inverse_save3(c, t, d_out, size, written);
+  DBuf tmp(c);
+  const nn::u32* w = nullptr;
+  st = six_product_words(c, t, tmp, &w);
+  if (st != NN_OK) return st;
+  u64 n = 0;
+  NN_CK(c, nn::six_save_words(w, t->scale, d_out, size, c->scan, &n, c->stream), "CRT/carry");
+  if (written) *written = n;
+  return NN_OK;
+}
+
 nn_status pointwise(nn_context* c, nn_transform* dst, const nn_transform* a, const nn_transform* b) {
   if (a->scale != b->scale || a->scale < 2) {
     c->err = "pointwise: transforms differ in scale";
     return NN_ERR_INVALID;
   }
-  nn_status st = xform_reserve(c, dst, a->scale);
+  const int s = a->scale;
+  if (a->rep == nn_transform::kSixForward && b->rep == nn_transform::kSixForward) {
+    nn_status st = xform_reserve(c, dst, s);
+    if (st != NN_OK) return st;
+    NN_CK(c, nn::six_pointwise(dst->six(), a->six(), b->six(), nn::six_plan(s, 1ull << s), c->six, c->stream),
+          "pointwise");
+    dst->rep = nn_transform::kSixProduct;
+    return NN_OK;
+  }
+  DBuf ta(c), tb(c);
+  const u64 *pa = a->res, *pb = b->res;
+  nn_status st = NN_OK;
+  if (a->rep != nn_transform::kThree) {
+    st = ta.alloc(3ull << s);
+    if (st == NN_OK) st = three_words(c, a, ta.p);
+    pa = ta.p;
+  }
+  if (st == NN_OK && b->rep != nn_transform::kThree) {
+    st = tb.alloc(3ull << s);
+    if (st == NN_OK) st = three_words(c, b, tb.p);
+    pb = tb.p;
+  }
+  if (st == NN_OK) st = xform_reserve(c, dst, s);
   if (st != NN_OK) return st;
-  NN_CK(c, nn::ntt_pointwise(dst->res, a->res, b->res, a->scale, c->tables, c->stream), "pointwise");
+  NN_CK(c, nn::tables_ensure(c->tables, s, c->stream, &c->retired_tables), "twiddle tables");
+  NN_CK(c, nn::ntt_pointwise(dst->res, pa, pb, s, c->tables, c->stream), "pointwise");
+  dst->rep = nn_transform::kThree;
   return NN_OK;
 }
 
@@ -289,26 +393,28 @@ nn_status forward_fused(nn_context* c, nn_transform* t, const u64* d_limbs, u64 
 nn_status ntt_product(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b, u64 nb, int s, u64 size,
                       u64* written) {
   nn_transform xa, xb;
-  nn_status st = forward(c, &xa, a, na, s);
+  nn_status st = forward_args(c, na, s);
+  if (st == NN_OK) st = forward_args(c, nb, s);
+  if (st == NN_OK) st = save_args(c, size);
+  if (st == NN_OK) st = forward3(c, &xa, a, na, s);
   if (st == NN_OK && c->passes(s).size() >= 2) {
     st = forward_fused(c, &xb, b, nb, s, &xa);
-    if (st == NN_OK) st = inverse_save(c, &xb, d_out, size, written, true);
+    if (st == NN_OK) st = inverse_save3(c, &xb, d_out, size, written, true);
   } else {
-    if (st == NN_OK) st = forward(c, &xb, b, nb, s);
+    if (st == NN_OK) st = forward3(c, &xb, b, nb, s);
     if (st == NN_OK) st = pointwise(c, &xb, &xa, &xb);
-    if (st == NN_OK) st = inverse_save(c, &xb, d_out, size, written);
+    if (st == NN_OK) st = inverse_save3(c, &xb, d_out, size, written);
   }
   dev_free(c, xa.res, xa.words);
   dev_free(c, xb.res, xb.words);
   return st;
 }
 
-// Residues of a product over six primes: ra, then rb unless the transforms
-// are squared or take one pass.
+// Residues of a product over six primes: ra, then rb where it is used.
 nn_status six_residues(nn_context* c, DBuf& buf, nn::SixOperands& op, const nn::SixPlan& pl) {
   NN_CK(c, nn::six_tables_ensure(c->six, pl.s, c->stream, &c->retired_tables), "twiddle tables");
   const u64 each = 3ull << pl.s;  // 6 words of 32 bits a coefficient
-  const bool two = op.b && pl.n > 1;
+  const bool two = op.b && (pl.n > 1 || nn::six_ready(op, pl));
   nn_status st = buf.alloc((op.pieces + (two ? 1 : 0)) * each);
   if (st != NN_OK) return st;
   op.ra = reinterpret_cast<nn::u32*>(buf.p);
@@ -529,11 +635,11 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
     }
     J.plan = nn::six_plan(s, J.pieces > 1 ? 1ull << s : J.na + J.nb - 1, c->batch_r_last_at[s]);
     max_s = std::max(max_s, s);
-    J.rows = J.plan.n > 1 && !c->batch_fused;
+    J.rows = J.pieces > 1 ? nn::kBatchRowsB : J.plan.n > 1 && !c->batch_fused ? nn::kBatchRowsAll : nn::kBatchRowsNone;
     B->n_flags += (nn::u32)nn::scan_tiles(na[j] + nb[j]);
     B->off_a[j] = B->arena_words;
     B->arena_words += J.pieces * (3ull << s);
-    if (!J.square && J.plan.n > 1) {
+    if (!J.square && (J.plan.n > 1 || J.rows)) {
       B->off_b[j] = B->arena_words;
       B->arena_words += 3ull << s;
     }
@@ -575,14 +681,16 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
     };
     const int operands = J.square ? 1 : 2;
     if (m == 1) {
-      auto& v = launches[{0, nn::kBatchSmall, 0, pl.R[0], 0}];
+      if (J.rows)
+        for (int pr = 0; pr < 6; ++pr) launches[{3, nn::kBatchSmallRow, 0, pl.R[0], 0}].push_back(item(0, 1, pr, 1));
+      auto& v = launches[{4, nn::kBatchSmall, J.rows, pl.R[0], 0}];
       for (u64 i = 0; i < J.pieces; ++i)
         for (int pr = 0; pr < 6; ++pr) v.push_back(item(i, 1, pr, 0));
     } else {
       for (int op = 0; op < operands; ++op) {
         pass_items(0, nn::kBatchLoad, 0, op);
         for (int k = 1; k < m - 1; ++k) pass_items(k, nn::kBatchCol, k, op);
-        if (J.rows) pass_items(3, nn::kBatchRow, m - 1, op);
+        if (J.rows == nn::kBatchRowsAll || (J.rows && op == 1)) pass_items(3, nn::kBatchRow, m - 1, op);
       }
       pass_items(4, nn::kBatchFused, m - 1, 0);
       for (int k = m - 2; k >= 0; --k) pass_items(7 - k, nn::kBatchInvCol, k, 0);
@@ -931,9 +1039,7 @@ nn_status nn_transform_inverse_save(nn_context* c, nn_transform* t, uint64_t* d_
 
 nn_status nn_transform_residues(nn_context* c, const nn_transform* t, uint64_t* d_out) {
   if (!c || !t || !t->res || !d_out) return NN_ERR_INVALID;
-  NN_CK(c, cudaMemcpyAsync(d_out, t->res, (3ull << t->scale) * sizeof(u64), cudaMemcpyDeviceToDevice, c->stream),
-        "copy residues");
-  return NN_OK;
+  return three_words(c, t, d_out);
 }
 
 nn_status nn_mul(nn_context* c, uint64_t* d_out, const uint64_t* a, uint64_t na, const uint64_t* b, uint64_t nb) {

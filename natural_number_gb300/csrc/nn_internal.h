@@ -101,6 +101,17 @@ u32 six_first_pass_columns(const SixPlan& pl);
 cudaError_t six_load(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st, u32 tile0 = 0,
                      u32 tile1 = ~0u);
 cudaError_t six_finish(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st);
+// Whether six_finish takes b through its last levels by itself first (rb is
+// then needed for one-pass transforms too): worth its launch when several
+// pieces would repeat them.
+inline bool six_ready(const SixOperands& op, const SixPlan& pl) {
+  return op.b && op.pieces > 1 && ((u64)op.pieces << pl.s) >= (1ull << 18);
+}
+// The two halves apart, for a transform that is kept: all forward levels, and
+// the product of two such transforms (dst may be either) back to residues for
+// the CRT.
+cudaError_t six_forward(const u64* limbs, u64 n, u32* res, const SixPlan& pl, const SixTables& t, cudaStream_t st);
+cudaError_t six_pointwise(u32* dst, const u32* a, const u32* b, const SixPlan& pl, const SixTables& t, cudaStream_t st);
 // Scratch for the carry scan.
 struct Scan {
   u32* flags = nullptr;  // per-tile status words of a lookback, zero between scans (the last tile clears them)
@@ -131,7 +142,7 @@ struct BatchJob {
   u64 pieces;
   u32 flag_base; // first carry-scan status word
   int square;    // a == b: one transform
-  int rows;      // the last pass's forward levels run on their own (batch_fused 0)
+  int rows;      // whose last forward levels run on their own (BatchRows)
   SixPlan plan;  // plan.s 0 for a schoolbook job
 };
 struct BatchItem {
@@ -140,11 +151,14 @@ struct BatchItem {
   unsigned char prime, operand;
 };
 // Launches of a batch, in order: those of one phase are independent.
-enum BatchKind : int { kBatchLoad, kBatchCol, kBatchRow, kBatchFused, kBatchInvCol, kBatchSmall, kBatchCrt,
-                       kBatchPieceCrt, kBatchColumns };
+enum BatchKind : int { kBatchLoad, kBatchCol, kBatchRow, kBatchFused, kBatchInvCol, kBatchSmallRow, kBatchSmall,
+                       kBatchCrt, kBatchPieceCrt, kBatchColumns };
+// No operand's (both go through them in the fused pass), both operands'
+// (batch_fused 0), or the shorter one's, shared by the pieces of the longer.
+enum BatchRows : int { kBatchRowsNone, kBatchRowsAll, kBatchRowsB };
 struct BatchSegment {
   int phase, kind;
-  int pass;    // strided passes: its index in the jobs' plans
+  int pass;    // strided passes: its index in the jobs' plans; contiguous ones: BatchRows
   int R, lgm;  // levels; log2 of the block length (contiguous passes)
   u32 first, count;  // items
 };
@@ -176,6 +190,8 @@ cudaError_t add_batch(const AddJob* d_jobs, u64 m, cudaStream_t st);
 // [0, 4p) for p0 and p1, [0, 2p) for p2.
 cudaError_t ntt_forward(const u64* limbs, u64 n, u64* res, int s, const Tables& t, cudaStream_t st,
                         const std::vector<Pass>* plan = nullptr);
+// The forward passes over coefficients that are already residues [3][2^s] below p.
+cudaError_t ntt_forward_residues(u64* res, int s, const Tables& t, cudaStream_t st, const std::vector<Pass>& plan);
 // Pointwise product of degree-1 residues (ntt_info.h:224-231); dst may alias a or b.
 cudaError_t ntt_pointwise(u64* dst, const u64* a, const u64* b, int s, const Tables& t, cudaStream_t st);
 // Inverse transform with the final 2^-(s-1) scale (ntt_info.h:200-221); values in [0,p).
@@ -193,6 +209,12 @@ cudaError_t ntt_fused_last(u64* res, const u64* other, int s, const Tables& t, c
 // limb_end) after each range's launch (for instance to queue its copy-back).
 cudaError_t six_save(const SixOperands& op, const SixPlan& pl, u64* out, Scan& sc, cudaStream_t st, int chunks = 1,
                      const std::function<cudaError_t(u64, u64)>& done = nullptr);
+// The same of one transform's product residues at scale s, normal or wrap mode
+// as ntt_save below.
+cudaError_t six_save_words(const u32* res, int s, u64* out, u64 size, Scan& sc, u64* written, cudaStream_t st);
+// The coefficients of product residues [6][2^s] reduced modulo the three
+// 62-bit primes: [3][2^s].
+cudaError_t six_to_three(const u32* res, int s, u64* out, cudaStream_t st);
 // CRT + carry into `size` limbs (normal mode) or the wrapped product mod
 // B^L - 1 in L limbs when size-1 > L (ntt_info.h:237-248).  Returns the
 // number of limbs written through *written (host value).

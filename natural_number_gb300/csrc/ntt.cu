@@ -651,6 +651,14 @@ cudaError_t ntt_forward(const u64* limbs, u64 n, u64* res, int s, const Tables& 
   return cudaSuccess;
 }
 
+cudaError_t ntt_forward_residues(u64* res, int s, const Tables& t, cudaStream_t st, const std::vector<Pass>& plan) {
+  for (const Pass& ps : plan) {
+    cudaError_t e = dispatch_pass<false, false, false>(res, res, 0, s, ps, t, st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 cudaError_t ntt_forward_head(const u64* limbs, u64 n, u64* res, int s, const Tables& t, cudaStream_t st,
                              const std::vector<Pass>& plan) {
   if (plan.size() < 2) return cudaErrorInvalidValue;  // the fused pass would have to load limbs

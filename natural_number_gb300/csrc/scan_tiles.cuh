@@ -196,7 +196,6 @@ __device__ __forceinline__ void six_garner4(const int4 (&v)[six::kPrimes], W3 (&
     x[e0 + e] = six_garner(y);
   }
 }
-template <bool CG>
 struct SixCrtProducer {
   const u32* res;  // [6][L]
   u64 L, count;
@@ -209,7 +208,7 @@ struct SixCrtProducer {
 #pragma unroll
     for (int q = 0; q < six::kPrimes; ++q) {
       const u32* r = res + q * L + i;
-      y[q] = (int)(CG ? __ldcg(r) : *r);
+      y[q] = (int)*r;
     }
     return six_garner(y);
   }
@@ -224,7 +223,7 @@ struct SixCrtProducer {
     for (int e0 = 0; e0 < kScanE; e0 += 4) {
       int4 v[six::kPrimes];
 #pragma unroll
-      for (int q = 0; q < six::kPrimes; ++q) v[q] = six::ld4<CG>(res + q * L + k0 + e0);
+      for (int q = 0; q < six::kPrimes; ++q) v[q] = *reinterpret_cast<const int4*>(res + q * L + k0 + e0);
       six_garner4(v, x, e0);
     }
   }
@@ -238,8 +237,7 @@ struct SixCrtProducer {
 // j - (i-1)*k of piece i-1 when that is below k + ny - 1: at most two terms
 // (k >= ny - 1), each below 2^160, so the sum fits three limbs.  k is a
 // multiple of 8, so eight positions starting at a multiple of 8 lie in one
-// piece.  Batch work items read other CTAs' results: .cg loads.
-template <bool CG>
+// piece.
 struct PieceCrtProducer {
   const u32* res;
   u64 L, k, P, ny, count;
@@ -257,8 +255,8 @@ struct PieceCrtProducer {
     int y[six::kPrimes];
 #pragma unroll
     for (int q = 0; q < six::kPrimes; ++q) {
-      y[q] = (int)(CG ? __ldcg(c + q * L) : c[q * L]);
-      if (ov) y[q] += (int)(CG ? __ldcg(b + q * L) : b[q * L]);
+      y[q] = (int)c[q * L];
+      if (ov) y[q] += (int)b[q * L];
     }
     return six_garner(y);
   }
@@ -276,11 +274,11 @@ struct PieceCrtProducer {
     for (int e0 = 0; e0 < kScanE; e0 += 4) {
       int4 v[six::kPrimes];
 #pragma unroll
-      for (int q = 0; q < six::kPrimes; ++q) v[q] = six::ld4<CG>(c + q * L + e0);
+      for (int q = 0; q < six::kPrimes; ++q) v[q] = *reinterpret_cast<const int4*>(c + q * L + e0);
       if (ov > e0) {
 #pragma unroll
         for (int q = 0; q < six::kPrimes; ++q) {
-          const int4 w = six::ld4<CG>(b + q * L + e0);
+          const int4 w = *reinterpret_cast<const int4*>(b + q * L + e0);
           v[q].x += w.x;
           v[q].y += ov > e0 + 1 ? w.y : 0;
           v[q].z += ov > e0 + 2 ? w.z : 0;

@@ -116,10 +116,10 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
   const u32 tile = tile0 + blockIdx.x / kPrimes;
   if (blockIdx.y < op.pieces) {
     const u64 at0 = blockIdx.y * op.piece;
-    load_tile<R, col_width(R), col_threads(R), false>(sm6, op.a + at0, min(op.piece, op.na - at0),
+    load_tile<R, col_width(R), col_threads(R)>(sm6, op.a + at0, min(op.piece, op.na - at0),
                                         op.ra + ((u64)blockIdx.y * kPrimes << s), s, tile, prime, tab, cap, k8);
   } else {
-    load_tile<R, col_width(R), col_threads(R), false>(sm6, op.b, op.nb, op.rb, s, tile, prime, tab, cap, k8);
+    load_tile<R, col_width(R), col_threads(R)>(sm6, op.b, op.nb, op.rb, s, tile, prime, tab, cap, k8);
   }
 }
 
@@ -129,26 +129,24 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
   extern __shared__ __align__(16) u32 sm6[];
   u32* res = blockIdx.z < pieces ? ra + ((u64)blockIdx.z * kPrimes << pl.s) : rb;
   const bool last = INV && lambda0 == 0;
-  col_tile<R, col_width(R), col_threads(R), INV, false>(sm6, res, pl.s, lambda0, blockIdx.x, blockIdx.y, tab, cap, last,
+  col_tile<R, col_width(R), col_threads(R), INV>(sm6, res, pl.s, lambda0, blockIdx.x, blockIdx.y, tab, cap, last,
                                                            pl.scale[blockIdx.y], last ? pl.k8 : 8);
 }
 
-template <int R, int LGM, int V, bool FIRST>
+// op.ra's pieces (or, FIRST, the limbs op.a) with op.rb (op.b), into `out`;
+// mode kForward: op.ra alone.
+template <int R, int LGM, int V, int MODE, bool FIRST>
 __global__ void __launch_bounds__(fused_threads(R, LGM, V), fused_blocks(R, LGM, V))
-    six_fused_kernel(SixOperands op, const SixPlan pl, const int2* __restrict__ tab, u64 cap) {
+    six_fused_kernel(SixOperands op, u32* out, const SixPlan pl, const int2* __restrict__ tab, u64 cap) {
   extern __shared__ __align__(16) u32 sm6[];
   constexpr int NT = fused_threads(R, LGM, V);
-  const int s = pl.s;
-  u32* out = op.ra + ((u64)blockIdx.z * kPrimes << s);
-  const int2* itab = tab + kPrimes * cap;
-  if constexpr (FIRST) {
-    const u64 at0 = blockIdx.z * op.piece;
-    fused_tile<R, LGM, NT, V, true, false>(sm6, op.a + at0, min(op.piece, op.na - at0), op.b, op.nb, out, s, 0,
-                                           blockIdx.y, tab, itab, cap, false, kAll, pl.scale[blockIdx.y], pl.k8);
-  } else {
-    fused_tile<R, LGM, NT, V, false, false>(sm6, out, 0, op.b ? op.rb : nullptr, 0, out, s, blockIdx.x, blockIdx.y,
-                                            tab, itab, cap, pl.reduce_in(), kAll, make_int2(0, 0), 8);
-  }
+  const u64 piece = ((u64)blockIdx.z * kPrimes) << pl.s, at0 = blockIdx.z * op.piece;
+  const void* a = FIRST ? static_cast<const void*>(op.a + at0) : op.ra + piece;
+  const void* b = FIRST && MODE == kAll ? static_cast<const void*>(op.b) : op.rb;
+  const bool last = pl.n == 1;
+  fused_tile<R, LGM, NT, V, MODE, FIRST>(sm6, a, min(op.piece, op.na - at0), b, op.nb, out + piece, pl.s, blockIdx.x,
+                                         blockIdx.y, tab, tab + kPrimes * cap, cap, pl.reduce_in(), last,
+                                         pl.scale[blockIdx.y], last ? pl.k8 : 8);
 }
 
 template <int R>
@@ -180,29 +178,27 @@ cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int lamb
   launch_end(st);
   return cudaGetLastError();
 }
-template <int R, int LGM, int V, bool FIRST>
-cudaError_t launch_fused_v(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
-  constexpr int tile = (int)tile_words32<1 << LGM>(R) * 4;
-  static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, V, FIRST>, 2 * tile);
+template <int R, int LGM, int V, int MODE, bool FIRST>
+cudaError_t launch_fused_v(const SixOperands& op, u32* out, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  constexpr int tile = (int)tile_words32<1 << LGM>(R) * 4, smem = fused_tiles(LGM, MODE) * tile;
+  static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, V, MODE, FIRST>, smem);
   if (ok != cudaSuccess) return ok;
-  const int smem = (op.b ? 2 : 1) * tile;
-  const dim3 grid(FIRST ? 1u : (unsigned)(((1ull << pl.s) >> (R + LGM + 3)) * pl.k8), kPrimes, op.pieces);
-  launch_begin(FIRST ? "six_small_pass" : "six_fused_row_pass", st);
-  six_fused_kernel<R, LGM, V, FIRST><<<grid, fused_threads(R, LGM, V), smem, st>>>(op, pl, t.tab, t.cap);
+  const u32 tiles = (u32)((1ull << pl.s) >> (R + LGM));
+  const dim3 grid(pl.n == 1 ? 1u : tiles / 8 * pl.k8, kPrimes, op.pieces);
+  launch_begin(MODE == kForward ? "six_fwd_row_pass" : FIRST ? "six_small_pass" : "six_fused_row_pass", st);
+  six_fused_kernel<R, LGM, V, MODE, FIRST><<<grid, fused_threads(R, LGM, V), MODE == kAll && !op.b ? tile : smem, st>>>(
+      op, out, pl, t.tab, t.cap);
   launch_end(st);
   return cudaGetLastError();
 }
 // Columns a thread: as few as keep the grid within one wave of the GPU's
 // 152 x 768 threads, so a short product uses as many of them as it can.
-template <int R, int LGM, bool FIRST>
-cudaError_t launch_fused(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
-  if constexpr (LGM == 3) {
-    const u64 units = ((u64)kPrimes * op.pieces << pl.s) / 64 * pl.k8;  // of one column
-    if (units <= 152 * 768) return launch_fused_v<R, LGM, 1, FIRST>(op, pl, t, st);
-    if constexpr (R == 9)
-      if (units <= 2 * 152 * 768) return launch_fused_v<R, LGM, 2, FIRST>(op, pl, t, st);
-  }
-  return launch_fused_v<R, LGM, 4, FIRST>(op, pl, t, st);
+template <int R, int LGM, int MODE, bool FIRST>
+cudaError_t launch_fused(const SixOperands& op, u32* out, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  if constexpr (LGM == 3)
+    if (((u64)kPrimes * op.pieces << pl.s) / 64 * pl.k8 <= 152 * 768)
+      return launch_fused_v<R, LGM, 1, MODE, FIRST>(op, out, pl, t, st);
+  return launch_fused_v<R, LGM, 4, MODE, FIRST>(op, out, pl, t, st);
 }
 
 cudaError_t load_pass(const SixOperands& op, int s, int k8, int R, const SixTables& t, u32 t0, u32 t1,
@@ -230,36 +226,34 @@ cudaError_t col_pass(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int k, con
   }
   return cudaErrorInvalidValue;
 }
-cudaError_t fused_pass(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+// FIRST: from limbs, the plan's only pass.
+template <int MODE, bool FIRST>
+cudaError_t fused_pass(const SixOperands& op, u32* out, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
   const int R = pl.R[pl.n - 1];
-  if (pl.n == 1) {
-    switch (R) {
-      case 1: return launch_fused<1, 3, true>(op, pl, t, st);
-      case 2: return launch_fused<2, 3, true>(op, pl, t, st);
-      case 3: return launch_fused<3, 3, true>(op, pl, t, st);
-      case 4: return launch_fused<4, 3, true>(op, pl, t, st);
-      case 5: return launch_fused<5, 3, true>(op, pl, t, st);
-      case 6: return launch_fused<6, 3, true>(op, pl, t, st);
-      case 7: return launch_fused<7, 3, true>(op, pl, t, st);
-      case 8: return launch_fused<8, 3, true>(op, pl, t, st);
-      case 9: return launch_fused<9, 3, true>(op, pl, t, st);
+  if constexpr (!FIRST) {
+    switch (pl.lgm) {
+      case 4: return launch_fused<8, 4, MODE, false>(op, out, pl, t, st);
+      case 5: return launch_fused<7, 5, MODE, false>(op, out, pl, t, st);
+      case 6: return launch_fused<6, 6, MODE, false>(op, out, pl, t, st);
+      case 7: return launch_fused<5, 7, MODE, false>(op, out, pl, t, st);
+      case 8: return launch_fused<4, 8, MODE, false>(op, out, pl, t, st);
+      case 9: return launch_fused<4, 9, MODE, false>(op, out, pl, t, st);
     }
-    return cudaErrorInvalidValue;
   }
-  switch (pl.lgm) {
-    case 4: return launch_fused<8, 4, false>(op, pl, t, st);
-    case 5: return launch_fused<7, 5, false>(op, pl, t, st);
-    case 6: return launch_fused<6, 6, false>(op, pl, t, st);
-    case 7: return launch_fused<5, 7, false>(op, pl, t, st);
-    case 8: return launch_fused<4, 8, false>(op, pl, t, st);
-    case 9: return launch_fused<4, 9, false>(op, pl, t, st);
+  if constexpr (FIRST || MODE == kProduct) {
+    switch (R) {
+      case 1: return launch_fused<1, 3, MODE, FIRST>(op, out, pl, t, st);
+      case 2: return launch_fused<2, 3, MODE, FIRST>(op, out, pl, t, st);
+      case 3: return launch_fused<3, 3, MODE, FIRST>(op, out, pl, t, st);
+      case 4: return launch_fused<4, 3, MODE, FIRST>(op, out, pl, t, st);
+    }
   }
   switch (R) {
-    case 5: return launch_fused<5, 3, false>(op, pl, t, st);
-    case 6: return launch_fused<6, 3, false>(op, pl, t, st);
-    case 7: return launch_fused<7, 3, false>(op, pl, t, st);
-    case 8: return launch_fused<8, 3, false>(op, pl, t, st);
-    case 9: return launch_fused<9, 3, false>(op, pl, t, st);
+    case 5: return launch_fused<5, 3, MODE, FIRST>(op, out, pl, t, st);
+    case 6: return launch_fused<6, 3, MODE, FIRST>(op, out, pl, t, st);
+    case 7: return launch_fused<7, 3, MODE, FIRST>(op, out, pl, t, st);
+    case 8: return launch_fused<8, 3, MODE, FIRST>(op, out, pl, t, st);
+    case 9: return launch_fused<9, 3, MODE, FIRST>(op, out, pl, t, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -343,14 +337,47 @@ cudaError_t six_load(const SixOperands& op, const SixPlan& pl, const SixTables& 
   return pl.n == 1 ? cudaSuccess : load_pass(op, pl.s, pl.k8, pl.R[0], t, tile0, tile1, st);
 }
 
-cudaError_t six_finish(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+namespace {
+cudaError_t forward_cols(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   for (int k = 1; k + 1 < pl.n && e == cudaSuccess; ++k)
     e = col_pass<false>(op.ra, op.b ? op.rb : nullptr, op.pieces, pl, k, t, st);
-  if (e == cudaSuccess) e = fused_pass(op, pl, t, st);
-  for (int k = pl.n - 2; k >= 0 && e == cudaSuccess; --k)
-    e = col_pass<true>(op.ra, nullptr, op.pieces, pl, k, t, st);
   return e;
+}
+cudaError_t inverse_cols(u32* res, u32 pieces, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  for (int k = pl.n - 2; k >= 0 && e == cudaSuccess; --k) e = col_pass<true>(res, nullptr, pieces, pl, k, t, st);
+  return e;
+}
+}  // namespace
+
+cudaError_t six_finish(const SixOperands& op, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  cudaError_t e = forward_cols(op, pl, t, st);
+  if (e == cudaSuccess) {
+    if (six_ready(op, pl)) {  // the shorter operand's last levels once, not once a piece
+      const SixOperands b{op.b, op.nb, op.nb, 1, nullptr, 0, op.rb, nullptr};
+      e = pl.n == 1 ? fused_pass<kForward, true>(b, op.rb, pl, t, st) : fused_pass<kForward, false>(b, op.rb, pl, t, st);
+      if (e == cudaSuccess)
+        e = pl.n == 1 ? fused_pass<kReady, true>(op, op.ra, pl, t, st) : fused_pass<kReady, false>(op, op.ra, pl, t, st);
+    } else {
+      e = pl.n == 1 ? fused_pass<kAll, true>(op, op.ra, pl, t, st) : fused_pass<kAll, false>(op, op.ra, pl, t, st);
+    }
+  }
+  return e == cudaSuccess ? inverse_cols(op.ra, op.pieces, pl, t, st) : e;
+}
+
+cudaError_t six_forward(const u64* limbs, u64 n, u32* res, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  const SixOperands op{limbs, n, n, 1, nullptr, 0, res, nullptr};
+  cudaError_t e = six_load(op, pl, t, st);
+  if (e == cudaSuccess) e = forward_cols(op, pl, t, st);
+  if (e != cudaSuccess) return e;
+  return pl.n == 1 ? fused_pass<kForward, true>(op, res, pl, t, st) : fused_pass<kForward, false>(op, res, pl, t, st);
+}
+
+cudaError_t six_pointwise(u32* dst, const u32* a, const u32* b, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  const SixOperands op{nullptr, 0, 0, 1, nullptr, 0, const_cast<u32*>(a), const_cast<u32*>(b)};
+  const cudaError_t e = fused_pass<kProduct, false>(op, dst, pl, t, st);
+  return e == cudaSuccess ? inverse_cols(dst, 1, pl, t, st) : e;
 }
 
 }  // namespace nn

@@ -102,48 +102,28 @@ template <int V>
 struct alignas(4 * V) Words {
   i32 v[V];
 };
-template <bool CG, int V>
+template <int V>
 __device__ __forceinline__ Words<V> ldv(const void* p) {
   Words<V> w;
   if constexpr (V == 4) {
-    const int4* q = reinterpret_cast<const int4*>(p);
-    const int4 t = CG ? __ldcg(q) : *q;
+    const int4 t = *reinterpret_cast<const int4*>(p);
     w.v[0] = t.x, w.v[1] = t.y, w.v[2] = t.z, w.v[3] = t.w;
   } else if constexpr (V == 2) {
-    const int2* q = reinterpret_cast<const int2*>(p);
-    const int2 t = CG ? __ldcg(q) : *q;
+    const int2 t = *reinterpret_cast<const int2*>(p);
     w.v[0] = t.x, w.v[1] = t.y;
   } else {
-    const i32* q = reinterpret_cast<const i32*>(p);
-    w.v[0] = CG ? __ldcg(q) : *q;
+    w.v[0] = *reinterpret_cast<const i32*>(p);
   }
   return w;
 }
-template <bool CG, int V>
+template <int V>
 __device__ __forceinline__ void stv(void* p, const Words<V>& w) {
-  if constexpr (V == 4) {
-    const int4 t = make_int4(w.v[0], w.v[1], w.v[2], w.v[3]);
-    if (CG)
-      __stcg(reinterpret_cast<int4*>(p), t);
-    else
-      *reinterpret_cast<int4*>(p) = t;
-  } else if constexpr (V == 2) {
-    const int2 t = make_int2(w.v[0], w.v[1]);
-    if (CG)
-      __stcg(reinterpret_cast<int2*>(p), t);
-    else
-      *reinterpret_cast<int2*>(p) = t;
-  } else {
-    if (CG)
-      __stcg(reinterpret_cast<i32*>(p), w.v[0]);
-    else
-      *reinterpret_cast<i32*>(p) = w.v[0];
-  }
-}
-template <bool CG>
-__device__ __forceinline__ int4 ld4(const void* p) {
-  const int4* q = reinterpret_cast<const int4*>(p);
-  return CG ? __ldcg(q) : *q;
+  if constexpr (V == 4)
+    *reinterpret_cast<int4*>(p) = make_int4(w.v[0], w.v[1], w.v[2], w.v[3]);
+  else if constexpr (V == 2)
+    *reinterpret_cast<int2*>(p) = make_int2(w.v[0], w.v[1]);
+  else
+    *reinterpret_cast<i32*>(p) = w.v[0];
 }
 
 // A unit: 2^K rows of V neighbouring columns in registers.  V = 4 has the
@@ -394,7 +374,7 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
         }
       } else {
 #pragma unroll
-        for (int m = 0; m < (1 << K); ++m) u.set(m, ldv<false, V>(sp + at<C>((u32)m << nsub)));
+        for (int m = 0; m < (1 << K); ++m) u.set(m, ldv<V>(sp + at<C>((u32)m << nsub)));
         fwd_levels<K>(u, tw, b, P.p);
       }
       if constexpr (g + 1 == G) {
@@ -409,7 +389,7 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
       } else {
 #pragma unroll
         for (int m = 0; m < (1 << K); ++m)
-          if (m < 5 || m < keep) stv<false, V>(sp + at<C>((u32)m << nsub), u.get(m));
+          if (m < 5 || m < keep) stv<V>(sp + at<C>((u32)m << nsub), u.get(m));
       }
     }
   };
@@ -447,7 +427,7 @@ __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const St
         if constexpr (g + 1 == G)
           u.set(m, load(row0 + ((u32)m << nsub), col));
         else
-          u.set(m, ldv<false, V>(sp + at<C>((u32)m << nsub)));
+          u.set(m, ldv<V>(sp + at<C>((u32)m << nsub)));
       }
       if (g == 0 && K == 3 && keep < 8) {
         if constexpr (g == 0 && K == 3) inv_truncated(u, keep, tw, ftw, P);
@@ -469,7 +449,7 @@ __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const St
         if constexpr (g == 0)
           store(row0 + ((u32)m << nsub), col, u.get(m));
         else
-          stv<false, V>(sp + at<C>((u32)m << nsub), u.get(m));
+          stv<V>(sp + at<C>((u32)m << nsub), u.get(m));
       }
     }
   };
@@ -504,7 +484,7 @@ __device__ __forceinline__ Words<V> limb_words(const u64* __restrict__ in, u64 n
 
 // The first pass of one operand: levels [0, R) from its limbs, columns
 // [tile * C, tile * C + C) of every row of 2^(s-R).
-template <int R, int C, int NT, bool CG>
+template <int R, int C, int NT>
 __device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u64 n, u32* res, int s, u32 tile,
                                           int prime, const int2* __restrict__ tab, u64 cap, int k8) {
   const Prime P = c_primes[prime];
@@ -514,14 +494,14 @@ __device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u
   const u64 col0 = (u64)tile * C;
   forward_tile<R, C, NT, 4, false, false>(
       sm, [&](u32 row, u32 col) { return limb_words<4>(in, n, ((u64)row << lg_s) + col0 + col, vec, P); },
-      [&](u32 row, u32 col, const Words<4>& w) { stv<CG>(out + ((u64)row << lg_s) + col, w); }, n <= (1ull << (s - 1)),
+      [&](u32 row, u32 col, const Words<4>& w) { stv(out + ((u64)row << lg_s) + col, w); }, n <= (1ull << (s - 1)),
       tab + prime * cap, 0, P, false, k8);
 }
 
 // Levels [lambda0, lambda0 + R) of residues in place: forward or inverse (tab:
 // the inverse table, which follows the forward one).  k8: of the whole
 // transform, for its last inverse pass only.
-template <int R, int C, int NT, bool INV, bool CG>
+template <int R, int C, int NT, bool INV>
 __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, u32 tile, int prime,
                                          const int2* __restrict__ tab, u64 cap, bool last = false,
                                          int2 scale = int2{}, int k8 = 8) {
@@ -531,8 +511,8 @@ __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, 
   const u32 ksb = tile / per;
   u32* g = res + ((u64)prime << s) + ((u64)ksb << (lg_s + R)) + (u64)(tile % per) * C;
   const int2* tw = tab + prime * cap;
-  auto ld = [&](u32 row, u32 col) { return ldv<CG, 4>(g + ((u64)row << lg_s) + col); };
-  auto st = [&](u32 row, u32 col, const Words<4>& w) { stv<CG>(g + ((u64)row << lg_s) + col, w); };
+  auto ld = [&](u32 row, u32 col) { return ldv<4>(g + ((u64)row << lg_s) + col); };
+  auto st = [&](u32 row, u32 col, const Words<4>& w) { stv(g + ((u64)row << lg_s) + col, w); };
   if constexpr (INV)
     inverse_tile<R, C, NT, 4>(sm, ld, st, tw, ksb, P, last, scale, k8, tw - kPrimes * cap);
   else
@@ -540,11 +520,13 @@ __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, 
 }
 
 // Products of the blocks of 8 coefficients of a tile: block row r of A times
-// that of B modulo x^8 - c, times 2^-32, into A.  Words at most 0.75 p in
-// magnitude, so the sums of eight products stay below 2^57.
-template <int R, int NT>
-__device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const int2* __restrict__ tw, u32 ksb,
-                                               const Prime& P, u32 rows) {
+// that of B modulo x^8 - c, times 2^-32, into sa.  A and B in shared memory (ga,
+// gb nullptr), or finished words in global memory, where a thread's block is
+// one 32-byte sector.  Words at most 0.75 p in magnitude, so the sums of eight
+// products stay below 2^57.
+template <int R, int NT, bool GA, bool GB>
+__device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const u32* ga, const u32* gb,
+                                               const int2* __restrict__ tw, u32 ksb, const Prime& P, u32 rows) {
 #pragma unroll 1
   for (u32 r = threadIdx.x; r < rows; r += NT) {
     const u32 blk = (ksb << R) + r;
@@ -552,9 +534,10 @@ __device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const int
     if (blk & 1) c = make_int2(-c.x, -c.y);
     i32 a[8], b[8], bw[8];
     int4* pa = reinterpret_cast<int4*>(sa + at<8>(r));
-    const int4* pb = reinterpret_cast<const int4*>(sb + at<8>(r));
-    *reinterpret_cast<int4*>(a) = pa[0];
-    *reinterpret_cast<int4*>(a + 4) = pa[1];
+    const int4* qa = GA ? reinterpret_cast<const int4*>(ga + 8 * r) : pa;
+    const int4* pb = reinterpret_cast<const int4*>(GB ? gb + 8 * r : sb + at<8>(r));
+    *reinterpret_cast<int4*>(a) = qa[0];
+    *reinterpret_cast<int4*>(a + 4) = qa[1];
     *reinterpret_cast<int4*>(b) = pb[0];
     *reinterpret_cast<int4*>(b + 4) = pb[1];
 #pragma unroll
@@ -627,73 +610,79 @@ __device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const int2
   }
 }
 
-// The last pass: tile `tile` (block index ksb at level lambda0, 2^R blocks of
-// 2^LGM coefficients) of both operands forward, the blocks' products, and the
-// first inverse levels.  a and b are residues after the strided passes (b
-// nullptr: a square), or, FIRST, limbs (na, nb of them; a transform of one
-// pass).  The inverse goes to out.  Modes for a batch run step by step:
-// (scale, k8: of a one-pass transform; otherwise the caller leaves tiles out.)
-// kAll everything; kForward only a's forward levels, written back to a;
-// kProduct products and inverse of operands whose forward levels are done.
-enum : int { kAll = 0, kForward = 1, kProduct = 2 };
-template <int R, int LGM, int NT, int V, bool FIRST, bool CG>
+// The last pass: tile `tile` (block index at the pass's first level, 2^R blocks
+// of 2^LGM coefficients) of the operands forward, the blocks' products, and the
+// first inverse levels, to out.
+//  kAll: both operands forward (b nullptr: a square)
+//  kReady: a forward; b's forward levels are done (FinishedWords)
+//  kProduct: those of both are done
+//  kForward: a's forward levels only, to out
+// Operands are residues after the strided passes, or, FIRST (transforms of one
+// pass), limbs (na, nb of them); finished ones are words of at most 0.75 p.
+// last: no strided inverse pass follows (scale, k8 as in inverse_tile).
+enum : int { kAll = 0, kReady = 1, kProduct = 2, kForward = 3 };
+// Shared-memory tiles of a mode: finished operands are read from global memory
+// where a block is a sector (LGM = 3).
+constexpr int fused_tiles(int LGM, int mode) { return mode == kAll || (LGM > 3 && mode != kForward) ? 2 : 1; }
+template <int R, int LGM, int NT, int V, int MODE, bool FIRST>
 __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const void* b, u64 nb, u32* out, int s,
                                            u32 tile, int prime, const int2* __restrict__ tab,
-                                           const int2* __restrict__ itab, u64 cap, bool reduce_in, int mode, int2 scale,
-                                           int k8) {
+                                           const int2* __restrict__ itab, u64 cap, bool reduce_in, bool last,
+                                           int2 scale, int k8) {
   constexpr int C = 1 << LGM;
   constexpr u32 W = tile_words32<C>(R);
   const Prime P = c_primes[prime];
   const int2* tw = tab + prime * cap;
   const int2* itw = itab + prime * cap;
-  const u64 off = FIRST ? 0 : ((u64)prime << s) + ((u64)tile << (R + LGM));
+  const u64 off = ((u64)prime << s) + ((u64)tile << (R + LGM));
   u32* sa = sm;
-  u32* sb = b ? sm + W : sm;
-  auto to = [&](u32* t) { return [t](u32 row, u32 col, const Words<V>& w) { stv<false>(t + at<C>(row) + col, w); }; };
+  u32* sb = MODE == kAll && !b ? sm : sm + W;
+  auto to = [&](u32* t) { return [t](u32 row, u32 col, const Words<V>& w) { stv(t + at<C>(row) + col, w); }; };
   auto forward = [&](const void* src, u64 n, u32* t) {
     if constexpr (FIRST) {
       const u64* in = static_cast<const u64*>(src);
       const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
       forward_tile<R, C, NT, V, false, true>(
-          t, [&](u32 row, u32 col) { return limb_words<V>(in, n, (u64)row * C + col, vec, P); }, to(t), n <= (1ull << (s - 1)),
-          tw, 0, P, false, k8);
+          t, [&](u32 row, u32 col) { return limb_words<V>(in, n, (u64)row * C + col, vec, P); }, to(t),
+          n <= (1ull << (s - 1)), tw, 0, P, false, k8);
     } else {
       const u32* in = static_cast<const u32*>(src) + off;
       forward_tile<R, C, NT, V, true, true>(
-          t, [&](u32 row, u32 col) { return ldv<CG, V>(in + row * C + col); }, to(t), false, tw, tile, P, reduce_in);
+          t, [&](u32 row, u32 col) { return ldv<V>(in + row * C + col); }, to(t), false, tw, tile, P, reduce_in);
     }
   };
-  auto fetch = [&](const void* src, u32* t) {  // kProduct: words whose forward levels are done
+  auto copy_in = [&](const void* src, u32* t) {
     const u32* in = static_cast<const u32*>(src) + off;
-    for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT)
-      *reinterpret_cast<int4*>(t + at<C>(i / C) + i % C) = ld4<CG>(in + i);
+    for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT) stv(t + at<C>(i / C) + i % C, ldv<4>(in + i));
   };
-  if (FIRST || mode != kProduct) {
+  if constexpr (MODE == kAll) {
     // one copy of the code for both operands
-    const int operands = b && (FIRST || mode != kForward) ? 2 : 1;
+    const int operands = b ? 2 : 1;
 #pragma unroll 1
     for (int op = 0; op < operands; ++op) forward(op ? b : a, op ? nb : na, op ? sb : sa);
-    if (!FIRST && mode == kForward) {
-      __syncthreads();
-      u32* back = out + off;
-      for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT)
-        stv<CG>(back + i, ldv<false, 4>(sa + at<C>(i / C) + i % C));
-      return;
-    }
-  } else if constexpr (!FIRST) {
-    fetch(a, sa);
-    if (b) fetch(b, sb);
+  } else if constexpr (MODE != kProduct) {
+    forward(a, na, sa);
+  } else if constexpr (LGM > 3) {
+    copy_in(a, sa);
   }
+  if constexpr (LGM > 3 && (MODE == kReady || MODE == kProduct)) copy_in(b, sb);
   __syncthreads();
-  if constexpr (LGM == 3)
-    leaf_products8<R, NT>(sa, sb, tw, FIRST ? 0 : tile, P, FIRST && R >= 3 ? (u32)k8 << (R - 3) : 1u << R);
-  else
-    leaf_products<R, LGM, NT>(sa, sb, tw, FIRST ? 0 : tile, P);
-  u32* dst = out + ((u64)prime << s) + (FIRST ? 0 : (u64)tile << (R + LGM));
-  __syncthreads();
-  inverse_tile<R, C, NT, V>(
-      sa, [&](u32 row, u32 col) { return ldv<false, V>(sa + at<C>(row) + col); },
-      [&](u32 row, u32 col, const Words<V>& w) { stv<CG>(dst + row * C + col, w); }, itw, FIRST ? 0 : tile, P, FIRST, scale, FIRST ? k8 : 8, tw);
+  if constexpr (MODE == kForward) {
+    u32* back = out + off;
+    for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT) stv(back + i, ldv<4>(sa + at<C>(i / C) + i % C));
+  } else {
+    if constexpr (LGM == 3)
+      leaf_products8<R, NT, MODE == kProduct, MODE != kAll>(sa, sb, static_cast<const u32*>(a) + off,
+                                                            static_cast<const u32*>(b) + off, tw, tile, P,
+                                                            FIRST && R >= 3 ? (u32)k8 << (R - 3) : 1u << R);
+    else
+      leaf_products<R, LGM, NT>(sa, sb, tw, tile, P);
+    __syncthreads();
+    u32* dst = out + off;
+    inverse_tile<R, C, NT, V>(
+        sa, [&](u32 row, u32 col) { return ldv<V>(sa + at<C>(row) + col); },
+        [&](u32 row, u32 col, const Words<V>& w) { stv(dst + row * C + col, w); }, itw, tile, P, last, scale, k8, tw);
+  }
 }
 
 }  // namespace six

@@ -116,3 +116,56 @@ def test_odd_addresses_and_all_ones(ctx, n):
         got = to_host(out[oo:oo + 2 * n])  # (B^n - 1)^2 = B^2n - 2 B^n + 1
         ones = np.uint64(0xFFFFFFFFFFFFFFFF)
         assert got[0] == 1 and not got[1:n].any() and got[n] == ones - np.uint64(1) and (got[n + 1:] == ones).all()
+
+
+@pytest.mark.parametrize("s", [4, 5, 8, 12, 13, 17, 21, 22, 26])
+def test_kept_transforms(ctx, oracle, s):
+    """A transform kept and multiplied, squared and turned back alone, in normal
+    and wrap mode; residues of a product's transform, and a product of three,
+    whose factors leave the six primes for the three-prime words."""
+    from gpu_util import P, empty_dev
+    L = 1 << s
+    na, nb = max(L // 2 - 3, 2), max(L // 2 - 1, 2)
+    a, b = limbs(s + 1, na), limbs(s + 2, nb)
+    ta, tb = ctx.transform().forward(to_dev(a), s), ctx.transform().forward(to_dev(b), s)
+    out = empty_dev(L + 2)
+    prod = ctx.transform().pointwise(ta, tb)
+    for _ in range(2):  # a product's residues can be saved again
+        w = prod.inverse_save(out, na + nb)
+        ctx.synchronize()
+        if s <= 22:
+            want = oracle.mul(a, b)
+            got = to_host(out, w)
+            assert np.array_equal(got[: want.size], want) and not got[want.size:].any()
+        else:
+            check_mod(ctx, to_dev(a), to_dev(b), out[: na + nb])
+    if s > 17:
+        return
+    sq = ctx.transform().pointwise(ta, ta)
+    sq.inverse_save(out, 2 * na)
+    want = oracle.sqr(a)
+    assert np.array_equal(to_host(out, 2 * na)[: want.size], want)
+    full = limbs(s + 3, L)  # wraps modulo B^L - 1
+    tf = ctx.transform().forward(to_dev(full), s)
+    assert ctx.transform().pointwise(tf, tb).inverse_save(out, L + 2) == L
+    assert np.array_equal(to_host(out, L), oracle.ntt_mul_raw(full, b, s, L + 2))
+    alone = ctx.transform().forward(to_dev(a), s)
+    alone.inverse_save(out, na + 1)
+    got = to_host(out, na + 1)
+    assert np.array_equal(got[:na], a) and got[na] == 0
+    res3, want3 = empty_dev(3 * L), empty_dev(3 * L)
+    one = ctx.transform().forward(to_dev(np.array([1], dtype=np.uint64)), s)
+    ctx.transform().pointwise(ta, one).residues(res3)
+    ta.residues(want3)
+    r, v = to_host(res3).reshape(3, L), to_host(want3).reshape(3, L)
+    for i in range(3):
+        assert np.array_equal(r[i] % np.uint64(P[i]), v[i] % np.uint64(P[i]))
+    small = [limbs(s + 7 + k, max(L // 4 - 2, 1)) >> np.uint64(16) for k in range(3)]  # 48-bit limbs: < 2^185 in all
+    t3 = [ctx.transform().forward(to_dev(x), s) for x in small]
+    t3[2].pointwise(ctx.transform().pointwise(t3[0], t3[1]), t3[2])
+    n = 3 * small[0].size
+    t3[2].inverse_save(out, n)
+    want = oracle.mul(oracle.mul(small[0], small[1]), small[2])
+    got = to_host(out, n)
+    k = min(n, want.size)
+    assert np.array_equal(got[:k], want[:k]) and not got[k:].any() and not want[k:].any()
