@@ -208,7 +208,7 @@ struct Launch {
   }
   template <int R, int LGM, int MODE>
   cudaError_t contiguous_mode() const {
-    constexpr int smem = fused_tiles(LGM, MODE) * (int)tile_words32<1 << LGM>(R) * 4;
+    constexpr int smem = fused_tiles(LGM, MODE) * (int)tile_words32<1 << LGM, true>(R) * 4;
     static const cudaError_t ok = allow_smem(batch_fused_kernel<R, LGM, MODE>, smem);
     if (ok != cudaSuccess) return ok;
     batch_fused_kernel<R, LGM, MODE><<<g.count, fused_threads(R, LGM, 4), smem, st>>>(jobs, items, t);
@@ -225,7 +225,7 @@ struct Launch {
   }
   template <int R, int MODE>
   cudaError_t small_mode() const {
-    constexpr int smem = fused_tiles(3, MODE) * (int)tile_words32<8>(R) * 4;
+    constexpr int smem = fused_tiles(3, MODE) * (int)tile_words32<8, true>(R) * 4;
     batch_small_kernel<R, MODE><<<g.count, fused_threads(R, 3, small_columns(R)), smem, st>>>(jobs, items, t);
     return cudaGetLastError();
   }

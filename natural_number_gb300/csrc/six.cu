@@ -180,7 +180,7 @@ cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int lamb
 }
 template <int R, int LGM, int V, int MODE, bool FIRST>
 cudaError_t launch_fused_v(const SixOperands& op, u32* out, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
-  constexpr int tile = (int)tile_words32<1 << LGM>(R) * 4, smem = fused_tiles(LGM, MODE) * tile;
+  constexpr int tile = (int)tile_words32<1 << LGM, true>(R) * 4, smem = fused_tiles(LGM, MODE) * tile;
   static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, V, MODE, FIRST>, smem);
   if (ok != cudaSuccess) return ok;
   const u32 tiles = (u32)((1ull << pl.s) >> (R + LGM));

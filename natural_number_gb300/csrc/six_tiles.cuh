@@ -50,11 +50,16 @@ struct Prime {
   u32 pinv;  // p^-1 mod 2^32 = 1 - m 2^22
   i32 u;     // round(2^32 / p)
   u32 c32;   // 2^32 mod p
+  i32 r, rp; // the same centred, and its companion round(r 2^32 / p)
 };
 constexpr u32 prime_of(int i) { return kMul[i] << 22 | 1; }
 constexpr Prime make_prime(int i) {
   const u64 p = prime_of(i), two32 = 1ull << 32;
-  return Prime{(i32)p, (u32)(1u - (kMul[i] << 22)), (i32)((two32 + p / 2) / p), (u32)(two32 % p)};
+  // 2^32 mod p as a factor of products wants its companion in 32 signed bits: centred
+  const u64 c = two32 % p;
+  const i64 cc = c > p / 2 ? (i64)c - (i64)p : (i64)c, n = cc * (i64)two32, h = (i64)p / 2;
+  return Prime{(i32)p, (u32)(1u - (kMul[i] << 22)), (i32)((two32 + p / 2) / p), (u32)c, (i32)cc,
+               (i32)((n + (n < 0 ? -h : h)) / (i64)p)};
 }
 static __constant__ Prime c_primes[kPrimes] = {make_prime(0), make_prime(1), make_prime(2),
                                                make_prime(3), make_prime(4), make_prime(5)};
@@ -288,17 +293,25 @@ constexpr int group_start(int R, int g) {
   return l;
 }
 
-// Word of (row, column) in a tile of C columns: dense 128-byte rows from C =
-// 32; narrower rows are padded by one row's length every eight rows, which
-// spreads the units of the deepest group over the banks.  A unit's rows are
-// 2^nsub apart and their offsets from the first are the same for every unit.
-template <int C>
+// Word of (row, column) in a tile of C columns.  Strided tiles (32 columns or
+// more) are dense: a 128-byte row takes every bank once.  Contiguous tiles
+// (LEAF) are laid out for the units of the deepest group and for the block
+// products, where lanes read the same word of neighbouring rows: rows of 8
+// words with a row's length after every eight, longer rows with an eighth of
+// their length (at least 16 bytes) after each.  A unit's rows are 2^nsub apart
+// and their offsets from the first are the same for every unit.
+template <int C, bool LEAF>
 __device__ __forceinline__ constexpr u32 at(u32 row) {
-  return row * C + (C < 32 ? (row >> 3) * C : 0);
+  if (!LEAF) return row * C;
+  if (C == 8) return row * C + (row >> 3) * C;
+  return row * (C + (C == 16 ? 4 : C / 8));
 }
-template <int C>
+template <int C, bool LEAF>
 constexpr u32 tile_words32(int R) {
-  return ((u32)C << R) + (C < 32 ? ((((u32)1 << R) + 7) / 8) * C : 0);
+  const u32 rows = 1u << R;
+  if (!LEAF) return rows * C;
+  if (C == 8) return rows * C + (rows + 7) / 8 * C;
+  return rows * (C + (C == 16 ? 4 : C / 8));
 }
 // Columns of a strided tile: 32 (128 bytes), more where few rows would leave
 // the CTA with few units.
@@ -309,16 +322,17 @@ constexpr int col_width(int R) { return R >= 7 ? 32 : 4096 >> R; }
 constexpr int at_least_warp(int threads) { return threads < 32 ? 32 : threads; }
 // Threads of a strided pass's CTA: one unit of eight rows x four columns each.
 constexpr int col_threads(int R) { return at_least_warp((col_width(R) / 4) << (R - 3)); }
-constexpr int col_smem(int R) { return groups_of(R) > 1 ? (int)tile_words32<32>(R) * (col_width(R) / 32) * 4 : 0; }
+constexpr int col_smem(int R) { return groups_of(R) > 1 ? (int)tile_words32<32, false>(R) * (col_width(R) / 32) * 4 : 0; }
 // Registers: 64 a thread; tiles of up to 2^8 rows as many CTAs as that allows.
 constexpr int col_blocks(int R) { return 1024 / col_threads(R) < 16 ? 1024 / col_threads(R) : 16; }
 
 // One unit of eight rows x V columns a thread.
 constexpr int fused_threads(int R, int LGM, int V) { return at_least_warp((1 << (R + LGM)) / (8 * V)); }
 // Two tiles of 4096 words in shared memory let six CTAs share an SM: 768
-// threads (80 registers) of four columns each, more of fewer columns.
+// threads (80 registers) of four columns each, more of fewer columns; 640
+// with the sums of longer blocks' products (96 registers).
 constexpr int fused_blocks(int R, int LGM, int V) { 
-  const int n = (V == 4 ? 768 : 1024) / fused_threads(R, LGM, V);
+  const int n = (LGM > 3 ? 640 : V == 4 ? 768 : 1024) / fused_threads(R, LGM, V);
   return n < 24 ? n : 24;
 }
 template <class Kernel>
@@ -332,7 +346,7 @@ inline cudaError_t allow_smem(Kernel k, int bytes) {
 // through sm.  HALF: the rows from 2^(R-1) are zero, so level 0 copies.
 // START: a reduction of the loaded words; LAST: one of the stored words.
 // k8 < 8: only the rows of the first k8 eighths are finished and stored.
-template <int R, int C, int NT, int V, bool START, bool LAST, class Load, class Store>
+template <int R, int C, bool LEAF, int NT, int V, bool START, bool LAST, class Load, class Store>
 __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const Store& store, bool half_zero,
                                              const int2* __restrict__ tw, u32 ksb, const Prime& P, bool start_red,
                                              int k8 = 8) {
@@ -350,7 +364,7 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
       const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
       Unit<K, V> u;
       const u32 b = (ksb << l) + rb;
-      u32* sp = sm + at<C>(row0) + col;
+      u32* sp = sm + at<C, LEAF>(row0) + col;
       if constexpr (g == 0) {
         if (half_zero) {
 #pragma unroll
@@ -374,7 +388,7 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
         }
       } else {
 #pragma unroll
-        for (int m = 0; m < (1 << K); ++m) u.set(m, ldv<V>(sp + at<C>((u32)m << nsub)));
+        for (int m = 0; m < (1 << K); ++m) u.set(m, ldv<V>(sp + at<C, LEAF>((u32)m << nsub)));
         fwd_levels<K>(u, tw, b, P.p);
       }
       if constexpr (g + 1 == G) {
@@ -389,7 +403,7 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
       } else {
 #pragma unroll
         for (int m = 0; m < (1 << K); ++m)
-          if (m < 5 || m < keep) stv<V>(sp + at<C>((u32)m << nsub), u.get(m));
+          if (m < 5 || m < keep) stv<V>(sp + at<C, LEAF>((u32)m << nsub), u.get(m));
       }
     }
   };
@@ -402,7 +416,7 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
 // last: the transform's last pass; its outputs are multiplied by the scale,
 // which also makes them 0.75 p at most (k8 < 8, with the forward table ftw: a
 // truncated transform's).
-template <int R, int C, int NT, int V, class Load, class Store>
+template <int R, int C, bool LEAF, int NT, int V, class Load, class Store>
 __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const Store& store,
                                              const int2* __restrict__ tw, u32 ksb, const Prime& P, bool last,
                                              int2 scale, int k8, const int2* __restrict__ ftw) {
@@ -420,14 +434,14 @@ __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const St
       const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
       Unit<K, V> u;
       const u32 b = (ksb << l) + rb;
-      u32* sp = sm + at<C>(row0) + col;
+      u32* sp = sm + at<C, LEAF>(row0) + col;
 #pragma unroll
       for (int m = 0; m < (1 << K); ++m) {
         if (m >= 5 && m >= keep) continue;
         if constexpr (g + 1 == G)
           u.set(m, load(row0 + ((u32)m << nsub), col));
         else
-          u.set(m, ldv<V>(sp + at<C>((u32)m << nsub)));
+          u.set(m, ldv<V>(sp + at<C, LEAF>((u32)m << nsub)));
       }
       if (g == 0 && K == 3 && keep < 8) {
         if constexpr (g == 0 && K == 3) inv_truncated(u, keep, tw, ftw, P);
@@ -449,7 +463,7 @@ __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const St
         if constexpr (g == 0)
           store(row0 + ((u32)m << nsub), col, u.get(m));
         else
-          stv<V>(sp + at<C>((u32)m << nsub), u.get(m));
+          stv<V>(sp + at<C, LEAF>((u32)m << nsub), u.get(m));
       }
     }
   };
@@ -492,7 +506,7 @@ __device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u
   u32* out = res + ((u64)prime << s) + (u64)tile * C;
   const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
   const u64 col0 = (u64)tile * C;
-  forward_tile<R, C, NT, 4, false, false>(
+  forward_tile<R, C, false, NT, 4, false, false>(
       sm, [&](u32 row, u32 col) { return limb_words<4>(in, n, ((u64)row << lg_s) + col0 + col, vec, P); },
       [&](u32 row, u32 col, const Words<4>& w) { stv(out + ((u64)row << lg_s) + col, w); }, n <= (1ull << (s - 1)),
       tab + prime * cap, 0, P, false, k8);
@@ -514,44 +528,104 @@ __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, 
   auto ld = [&](u32 row, u32 col) { return ldv<4>(g + ((u64)row << lg_s) + col); };
   auto st = [&](u32 row, u32 col, const Words<4>& w) { stv(g + ((u64)row << lg_s) + col, w); };
   if constexpr (INV)
-    inverse_tile<R, C, NT, 4>(sm, ld, st, tw, ksb, P, last, scale, k8, tw - kPrimes * cap);
+    inverse_tile<R, C, false, NT, 4>(sm, ld, st, tw, ksb, P, last, scale, k8, tw - kPrimes * cap);
   else
-    forward_tile<R, C, NT, 4, false, false>(sm, ld, st, false, tw, ksb, P, false);
+    forward_tile<R, C, false, NT, 4, false, false>(sm, ld, st, false, tw, ksb, P, false);
+}
+
+// Products of polynomials of 8 coefficients by Karatsuba's method three levels
+// deep: 27 multiply-adds instead of 64, at four cycles of the multiply pipe
+// each.  Digit k (base 3) of a point's index takes the coefficients with bit k
+// of their index clear (0), set (1) or both, added (2).  Sums over several
+// products add up point by point and are interpolated once; 64-bit wrap-around
+// on the way is harmless, since the coefficients themselves fit.
+template <int N>
+__device__ __forceinline__ void kara_points(const i32 (&x)[N], i32* e) {
+  if constexpr (N == 1) {
+    e[0] = x[0];
+  } else {
+    i32 lo[N / 2], hi[N / 2], both[N / 2];
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      lo[i] = x[i];
+      hi[i] = x[i + N / 2];
+      both[i] = x[i] + x[i + N / 2];
+    }
+    constexpr int T = N == 8 ? 9 : N == 4 ? 3 : 1;
+    kara_points<N / 2>(lo, e);
+    kara_points<N / 2>(hi, e + T);
+    kara_points<N / 2>(both, e + 2 * T);
+  }
+}
+// The 2 N - 1 coefficients from the points' products.
+template <int N>
+__device__ __forceinline__ void kara_interpolate(const i64* u, i64 (&t)[2 * N - 1]) {
+  if constexpr (N == 1) {
+    t[0] = u[0];
+  } else {
+    constexpr int T = N == 8 ? 9 : N == 4 ? 3 : 1, H = N / 2;
+    i64 lo[N - 1], hi[N - 1], both[N - 1];
+    kara_interpolate<H>(u, lo);
+    kara_interpolate<H>(u + T, hi);
+    kara_interpolate<H>(u + 2 * T, both);
+#pragma unroll
+    for (int i = 0; i < 2 * N - 1; ++i) t[i] = (i < N - 1 ? lo[i] : 0) + (i >= N ? hi[i - N] : 0);
+#pragma unroll
+    for (int i = 0; i < N - 1; ++i) t[i + H] += both[i] - lo[i] - hi[i];
+  }
+}
+// (sum t_i z^i) 2^-32 modulo z^8 - c, cr = c 2^32 mod p: the upper seven
+// coefficients come down through a Montgomery step each and one multiply-add.
+__device__ __forceinline__ void fold8(i64 (&t)[15], i32 cr, i32 (&o)[8], const Prime& P) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (j < 7) t[j] += (i64)mont(t[j + 8], P) * cr;
+    o[j] = mont(t[j], P);
+  }
+}
+// The constant c_b of block b, times 2^32: the roots' table holds it for even
+// b, its negative for odd b.
+__device__ __forceinline__ i32 block_constant(const int2* __restrict__ tw, u32 b, const Prime& P) {
+  const i32 c = __ldg(tw + (b >> 1)).x;
+  const i32 r = mul_mod(c, P.r, P.rp, P.p);
+  return b & 1 ? -r : r;
 }
 
 // Products of the blocks of 8 coefficients of a tile: block row r of A times
 // that of B modulo x^8 - c, times 2^-32, into sa.  A and B in shared memory (ga,
 // gb nullptr), or finished words in global memory, where a thread's block is
-// one 32-byte sector.  Words at most 0.75 p in magnitude, so the sums of eight
-// products stay below 2^57.
+// one 32-byte sector.  Words at most 0.75 p in magnitude: the sums of eight
+// products, with the folded part, stay below 2^58.
 template <int R, int NT, bool GA, bool GB>
 __device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const u32* ga, const u32* gb,
                                                const int2* __restrict__ tw, u32 ksb, const Prime& P, u32 rows) {
 #pragma unroll 1
   for (u32 r = threadIdx.x; r < rows; r += NT) {
-    const u32 blk = (ksb << R) + r;
-    int2 c = __ldg(tw + (blk >> 1));
-    if (blk & 1) c = make_int2(-c.x, -c.y);
-    i32 a[8], b[8], bw[8];
-    int4* pa = reinterpret_cast<int4*>(sa + at<8>(r));
-    const int4* qa = GA ? reinterpret_cast<const int4*>(ga + 8 * r) : pa;
-    const int4* pb = reinterpret_cast<const int4*>(GB ? gb + 8 * r : sb + at<8>(r));
-    *reinterpret_cast<int4*>(a) = qa[0];
-    *reinterpret_cast<int4*>(a + 4) = qa[1];
-    *reinterpret_cast<int4*>(b) = pb[0];
-    *reinterpret_cast<int4*>(b + 4) = pb[1];
+    const i32 cr = block_constant(tw, (ksb << R) + r, P);
+    u32* pa = sa + at<8, true>(r);
+    i64 u[27], t[15];
+    {
+      i32 x[8], ea[27], eb[27];
+      auto words = [&](const u32* q) {
+        const Words<4> w0 = ldv<4>(q), w1 = ldv<4>(q + 4);
 #pragma unroll
-    for (int j = 1; j < 8; ++j) bw[j] = mul_mod(b[j], c.x, c.y, P.p);
-    i32 o[8];
+        for (int i = 0; i < 4; ++i) {
+          x[i] = w0.v[i];
+          x[i + 4] = w1.v[i];
+        }
+      };
+      words(GA ? ga + 8 * r : pa);
+      kara_points(x, ea);
+      words(GB ? gb + 8 * r : sb + at<8, true>(r));
+      kara_points(x, eb);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      i64 t = 0;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) t += (i64)a[i] * (i <= j ? b[j - i] : bw[8 + j - i]);
-      o[j] = mont(t, P);
+      for (int i = 0; i < 27; ++i) u[i] = (i64)ea[i] * eb[i];
     }
-    pa[0] = *reinterpret_cast<int4*>(o);
-    pa[1] = *reinterpret_cast<int4*>(o + 4);
+    kara_interpolate<8>(u, t);
+    i32 o[8];
+    fold8(t, cr, o, P);
+    stv(pa, Words<4>{{o[0], o[1], o[2], o[3]}});
+    stv(pa + 4, Words<4>{{o[4], o[5], o[6], o[7]}});
   }
 }
 
@@ -559,53 +633,63 @@ __device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const u32
 // polynomials of degree below G in x over Z_p[z] / (z^8 - c), z = x^G (word
 // g + G i is the z^i coefficient of x^g): a thread forms one x^g of one block
 // from G products of 8 coefficients each, with z b in the place of b where
-// the power of x wraps.  The results go out through `put` after every thread
-// of the CTA has read the block.
+// the power of x wraps.  One level of Karatsuba's method, 48 multiply-adds a
+// product: its 21 sums leave room for five CTAs an SM, where the 27 sums of
+// three levels take 114 registers (2^25 x 2^25 limbs: fused pass 3.02 ms at four
+// CTAs, 2.73 so, 3.03 with 64 multiply-adds; 2^27 x 2^27: 19.2, 17.0, 17.5).  Results are written after every thread of the CTA has read the
+// round's blocks.
 template <int R, int LGM, int NT>
 __device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const int2* __restrict__ tw, u32 ksb,
                                               const Prime& P) {
   constexpr int C = 1 << LGM, G = C / 8;
   constexpr u32 items = (u32)G << R;
   constexpr u32 rounds = (items + NT - 1) / NT;
+#pragma unroll 1
   for (u32 it = 0; it < rounds; ++it) {
     const u32 q = it * NT + threadIdx.x;  // whole blocks a round: items of a block lie in one round
     const bool on = q < items;
-    const u32 r = on ? q / G : 0, g = q % G;
-    const u32 blk = (ksb << R) + r;
+    const u32 r = on ? q / G : 0, g = q % G, blk = (ksb << R) + r;
     int2 c = __ldg(tw + (blk >> 1));
     if (blk & 1) c = make_int2(-c.x, -c.y);
-    i64 t[15];
+    i64 lo[7], hi[7], mid[7];  // products of the lower halves, the upper ones, the sums of both
 #pragma unroll
-    for (int i = 0; i < 15; ++i) t[i] = 0;
-    u32* pa = sa + at<C>(r);
-    const u32* pb = sb + at<C>(r);
+    for (int i = 0; i < 7; ++i) lo[i] = hi[i] = mid[i] = 0;
+    u32* pa = sa + at<C, true>(r);
+    const u32* pb = sb + at<C, true>(r);
 #pragma unroll 1
     for (int h = 0; h < G; ++h) {
       const u32 k = (g - h) % G;
       const bool wrap = (u32)h > g;
-      i32 a[8], b[8];
+      i32 x[8], y[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        a[i] = (i32)pa[h + G * i];
-        b[i] = (i32)pb[k + G * i];
+        x[i] = (i32)pa[h + G * i];
+        y[i] = (i32)pb[k + G * i];
       }
-      const i32 top = mul_mod(b[7], c.x, c.y, P.p);
+      const i32 top = mul_mod(y[7], c.x, c.y, P.p);
 #pragma unroll
-      for (int i = 7; i > 0; --i) b[i] = wrap ? b[i - 1] : b[i];
-      b[0] = wrap ? top : b[0];
+      for (int i = 7; i > 0; --i) y[i] = wrap ? y[i - 1] : y[i];
+      y[0] = wrap ? top : y[0];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) t[i + j] += (i64)a[i] * b[j];
+        for (int j = 0; j < 4; ++j) {
+          lo[i + j] += (i64)x[i] * y[j];
+          hi[i + j] += (i64)x[i + 4] * y[j + 4];
+          mid[i + j] += (i64)(x[i] + x[i + 4]) * (y[j] + y[j + 4]);
+        }
     }
     __syncthreads();  // the blocks of this round have been read
     if (on) {
+      i64 t[15];
+      i32 o[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        i32 o = mont(t[i], P);
-        if (i < 7) o = (i32)((u32)o + (u32)mul_mod(mont(t[i + 8 < 15 ? i + 8 : 14], P), c.x, c.y, P.p));
-        pa[g + G * i] = (u32)reduce(o, P);
-      }
+      for (int i = 0; i < 15; ++i) t[i] = (i < 7 ? lo[i] : 0) + (i >= 8 ? hi[i - 8] : 0);
+#pragma unroll
+      for (int i = 0; i < 7; ++i) t[i + 4] += mid[i] - lo[i] - hi[i];
+      fold8(t, block_constant(tw, blk, P), o, P);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) pa[g + G * i] = (u32)reduce(o[i], P);
     }
   }
 }
@@ -630,30 +714,30 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
                                            const int2* __restrict__ itab, u64 cap, bool reduce_in, bool last,
                                            int2 scale, int k8) {
   constexpr int C = 1 << LGM;
-  constexpr u32 W = tile_words32<C>(R);
+  constexpr u32 W = tile_words32<C, true>(R);
   const Prime P = c_primes[prime];
   const int2* tw = tab + prime * cap;
   const int2* itw = itab + prime * cap;
   const u64 off = ((u64)prime << s) + ((u64)tile << (R + LGM));
   u32* sa = sm;
   u32* sb = MODE == kAll && !b ? sm : sm + W;
-  auto to = [&](u32* t) { return [t](u32 row, u32 col, const Words<V>& w) { stv(t + at<C>(row) + col, w); }; };
+  auto to = [&](u32* t) { return [t](u32 row, u32 col, const Words<V>& w) { stv(t + at<C, true>(row) + col, w); }; };
   auto forward = [&](const void* src, u64 n, u32* t) {
     if constexpr (FIRST) {
       const u64* in = static_cast<const u64*>(src);
       const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-      forward_tile<R, C, NT, V, false, true>(
+      forward_tile<R, C, true, NT, V, false, true>(
           t, [&](u32 row, u32 col) { return limb_words<V>(in, n, (u64)row * C + col, vec, P); }, to(t),
           n <= (1ull << (s - 1)), tw, 0, P, false, k8);
     } else {
       const u32* in = static_cast<const u32*>(src) + off;
-      forward_tile<R, C, NT, V, true, true>(
+      forward_tile<R, C, true, NT, V, true, true>(
           t, [&](u32 row, u32 col) { return ldv<V>(in + row * C + col); }, to(t), false, tw, tile, P, reduce_in);
     }
   };
   auto copy_in = [&](const void* src, u32* t) {
     const u32* in = static_cast<const u32*>(src) + off;
-    for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT) stv(t + at<C>(i / C) + i % C, ldv<4>(in + i));
+    for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT) stv(t + at<C, true>(i / C) + i % C, ldv<4>(in + i));
   };
   if constexpr (MODE == kAll) {
     // one copy of the code for both operands
@@ -669,7 +753,7 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
   __syncthreads();
   if constexpr (MODE == kForward) {
     u32* back = out + off;
-    for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT) stv(back + i, ldv<4>(sa + at<C>(i / C) + i % C));
+    for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT) stv(back + i, ldv<4>(sa + at<C, true>(i / C) + i % C));
   } else {
     if constexpr (LGM == 3)
       leaf_products8<R, NT, MODE == kProduct, MODE != kAll>(sa, sb, static_cast<const u32*>(a) + off,
@@ -679,8 +763,8 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
       leaf_products<R, LGM, NT>(sa, sb, tw, tile, P);
     __syncthreads();
     u32* dst = out + off;
-    inverse_tile<R, C, NT, V>(
-        sa, [&](u32 row, u32 col) { return ldv<V>(sa + at<C>(row) + col); },
+    inverse_tile<R, C, true, NT, V>(
+        sa, [&](u32 row, u32 col) { return ldv<V>(sa + at<C, true>(row) + col); },
         [&](u32 row, u32 col, const Words<V>& w) { stv(dst + row * C + col, w); }, itw, tile, P, last, scale, k8, tw);
   }
 }

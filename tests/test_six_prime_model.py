@@ -26,33 +26,39 @@ def groups(R):
     return out
 
 
-def at(C, row):
-    return row * C + ((row >> 3) * C if C < 32 else 0)
+def at(C, leaf, row):
+    if not leaf:
+        return row * C
+    return row * C + (row >> 3) * C if C == 8 else row * (C + (4 if C == 16 else C // 8))
 
 
-def tile_words(C, R):
-    return (C << R) + ((((1 << R) + 7) // 8) * C if C < 32 else 0)
+def tile_words(C, leaf, R):
+    if not leaf:
+        return C << R
+    return (C << R) + (((1 << R) + 7) // 8) * C if C == 8 else (C + (4 if C == 16 else C // 8)) << R
 
 
 def col_width(R):
-    return 32 if R >= 7 else 64 if R == 6 else 128
+    return 32 if R >= 7 else 4096 >> R
 
 
-@pytest.mark.parametrize("C,R", [(8, r) for r in range(1, 10)] + [(16, 8), (32, 7), (64, 6), (128, 5), (256, 4),
-                                 (512, 4)] + [(col_width(r), r) for r in range(4, 10)])
-def test_units_cover_the_tile(C, R):
+@pytest.mark.parametrize("C,leaf,R", [(8, True, r) for r in range(1, 10)] + [
+    (16, True, 8), (32, True, 7), (64, True, 6), (128, True, 5), (256, True, 4), (512, True, 4)] + [
+    (col_width(r), False, r) for r in range(4, 10)])
+@pytest.mark.parametrize("V", [1, 2, 4])
+def test_units_cover_the_tile(C, leaf, R, V):
     for l, K in groups(R):
         nsub, seen = R - l - K, set()
-        for i in range((C // 4) << (R - K)):
-            col, v = (i % (C // 4)) * 4, i // (C // 4)
+        for i in range((C // V) << (R - K)):
+            col, v = (i % (C // V)) * V, i // (C // V)
             rb = v >> nsub
             row0 = (rb << (nsub + K)) + (v & ((1 << nsub) - 1))
             for m in range(1 << K):
                 row = row0 + (m << nsub)
-                word = at(C, row0) + col + at(C, m << nsub)
-                assert word == at(C, row) + col and word % 4 == 0 and word + 4 <= tile_words(C, R)
+                word = at(C, leaf, row0) + col + at(C, leaf, m << nsub)
+                assert word == at(C, leaf, row) + col and word % V == 0 and word + V <= tile_words(C, leaf, R)
                 seen.add((row, col))
-        assert len(seen) == (C // 4) << R
+        assert len(seen) == (C // V) << R
 
 
 def test_primes():
