@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kBatchSumThreads, 6)
   column_tile_sums<kBatchSumThreads, kBatchSumTile>(sums, ColumnProducer{J.a, J.na, J.b, J.nb}, it.tile);
   __syncthreads();
   typedef SmemSumsProducer<kBatchSumTile> Prod;
-  scan_tile<Prod, true, kBatchSumThreads>(Prod{sums, (u64)it.tile * kBatchSumTile - kScanE, size}, it.tile, size, J.out,
+  scan_tile<Prod, kScanLookback, kBatchSumThreads>(Prod{sums, (u64)it.tile * kBatchSumTile - kScanE, size}, it.tile, size, J.out,
                                           size, nullptr, flags + J.flag_base, err);
 }
 

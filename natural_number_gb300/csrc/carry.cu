@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_lookback_kernel(Prod pro
 template <class Prod>
 __global__ void __launch_bounds__(kScanThreads, 3) scan_kernel(Prod prod, u64 total, u64* out, u64 out_limit,
                                                             u64* side, u32* flags, u64 tile_base) {
-  scan_tile<Prod, false>(prod, tile_base + blockIdx.x, total, out, out_limit, side, flags, nullptr);
+  scan_tile<Prod, kScanRecord>(prod, tile_base + blockIdx.x, total, out, out_limit, side, flags, nullptr);
 }
 
 // Step 2: 32 tiles a CTA.  The carry into the range is the generate bit of the
@@ -197,21 +197,122 @@ __global__ void wait_probe_kernel(const u32* flag, u32* err, int limit) {
   if (threadIdx.x == 0 && wait_flag(flag, limit) == 0) atomicExch(err, 1u);
 }
 
-// Base-case products of at most 2^20 positions: each CTA forms
-// its tile's column sums in shared memory and takes the tile through the
-// lookback scan, one launch.  Small tiles spread a short product over the
-// GPU: the column sums are the work, up to 383 terms a position.
-constexpr u64 kSchoolShortTile = 256, kSchoolTile = 64, kSchoolLongTile = 1024;
-template <u64 TILE, bool ONE>
+// Scans of at most eight tiles: one cluster (kScanCluster).
+template <class Prod, int NT>
+__global__ void __launch_bounds__(NT) scan_cluster_kernel(Prod prod, u64 total, u64* out, u64 out_limit, u64* side) {
+  scan_tile<Prod, kScanCluster, NT>(prod, blockIdx.x, total, out, out_limit, side, nullptr, nullptr);
+  cluster_sync();
+}
+constexpr u64 kClusterTiles = 8;
+
+// One cluster of `tiles` CTAs.
+template <class... Params, class... Args>
+cudaError_t launch_cluster(void (*kernel)(Params...), unsigned tiles, unsigned threads, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = tiles;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
+// acc += x * y as one carry chain.
+__device__ __forceinline__ void mac(W3& acc, u64 x, u64 y) {
+  asm("mad.lo.cc.u64 %0, %3, %4, %0;\n\t"
+      "madc.hi.cc.u64 %1, %3, %4, %1;\n\t"
+      "addc.u64 %2, %2, 0;"
+      : "+l"(acc.w0), "+l"(acc.w1), "+l"(acc.w2)
+      : "l"(x), "l"(y));
+}
+
+// Base-case products of up to sixteen tiles of 64 positions: one cluster.  The
+// shorter operand and the window of the longer one that a tile needs come
+// into shared memory, padded with zeros; sixteen lanes share four columns,
+// each a run of the longer operand's limbs (of odd length, so that the lanes
+// hit different banks): a step reads one limb of either operand and feeds
+// four independent sums.  383 x 383 limbs: 14.4 us with one term a step and
+// the status words of the lookback in global memory.
+constexpr int kSchoolClusterCtas = 16;
+constexpr u64 kSchoolClusterTile = 64, kSchoolShorter = 384;
+__global__ void __launch_bounds__(256) school_cluster_kernel(ColumnProducer prod, u64 total, u64* out) {
+  constexpr u64 TILE = kSchoolClusterTile;
+  constexpr int kLanes = 16;
+  __shared__ u64 sums[3 * (TILE + kScanE)];
+  __shared__ u64 window[TILE + kSchoolShorter], shorter[kSchoolShorter + 8];
+  const int tid = threadIdx.x, nb = (int)prod.nb;
+  const long long k0 = (long long)blockIdx.x * TILE, a0 = max(0ll, k0 - nb + 1);
+  const long long end = min((long long)prod.na, k0 + (long long)TILE);
+  for (long long i = a0 + tid; i < end; i += 256) window[i - a0] = prod.a[i];
+  for (int i = tid; i < nb + 8; i += 256) shorter[i] = i >= 4 && i < nb + 4 ? prod.b[i - 4] : 0;
+  __syncthreads();
+  const int g = tid / kLanes, lane = tid % kLanes;
+  const long long k = k0 + 4 * g, lo = max(0ll, k - nb + 1), hi = min((long long)prod.na - 1, k + 3);
+  const int len = hi >= lo ? (int)(hi - lo + 1) : 0, run = ((len + kLanes - 1) / kLanes) | 1;
+  const int from = min(lane * run, len), to = min(from + run, len);
+  W3 acc[4] = {};
+  const u64* wa = window + (lo - a0);
+  const u64* sb = shorter + 4 + (k - lo);  // term t: a[lo + t] with b[k + q - lo - t], q < 4
+  u64 b0 = 0, b1 = 0, b2 = 0, b3 = 0;
+  if (from < to) {
+    b0 = sb[-from];
+    b1 = sb[1 - from];
+    b2 = sb[2 - from];
+    b3 = sb[3 - from];
+  }
+  for (int t = from; t < to; ++t) {
+    const u64 x = wa[t];
+    mac(acc[0], x, b0);
+    mac(acc[1], x, b1);
+    mac(acc[2], x, b2);
+    mac(acc[3], x, b3);
+    b3 = b2;
+    b2 = b1;
+    b1 = b0;
+    b0 = sb[-t - 1];
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+#pragma unroll
+    for (int d = kLanes / 2; d >= 1; d >>= 1) {
+      const W3 o{__shfl_down_sync(0xffffffffu, acc[q].w0, d, kLanes), __shfl_down_sync(0xffffffffu, acc[q].w1, d, kLanes),
+                 __shfl_down_sync(0xffffffffu, acc[q].w2, d, kLanes)};
+      acc[q] = add_w3(acc[q], o);
+    }
+    if (lane == 0) {
+      const u64 i = kScanE + 4 * g + q;
+      sums[i] = acc[q].w0;
+      sums[TILE + kScanE + i] = acc[q].w1;
+      sums[2 * (TILE + kScanE) + i] = acc[q].w2;
+    }
+  }
+  __syncthreads();
+  typedef SmemSumsProducer<TILE> Sums;
+  scan_tile<Sums, kScanCluster, 256, TILE>(Sums{sums, (u64)k0 - kScanE, total}, blockIdx.x, total, out, total, nullptr,
+                                           nullptr, nullptr);
+  cluster_sync();
+}
+
+// Longer base-case products of at most 2^20 positions: each CTA forms its
+// tile's column sums in shared memory and takes the tile through the lookback
+// scan, one launch.  Small tiles spread a short product over the GPU: the
+// column sums are the work, up to 383 terms a position.
+constexpr u64 kSchoolTile = 64, kSchoolLongTile = 1024;
+template <u64 TILE>
 __global__ void __launch_bounds__(256) school_kernel(ColumnProducer prod, u64 total, u64* out, u32* flags,
                                                      u32* counter, u32* err, u32 tiles) {
   __shared__ u64 sums[3 * (TILE + kScanE)];
-  const u32 tile = ONE ? 0 : next_tile(counter);
+  const u32 tile = next_tile(counter);
   column_tile_sums<256, TILE>(sums, prod, tile);
   __syncthreads();
-  scan_tile<SmemSumsProducer<TILE>, !ONE, 256, TILE>(SmemSumsProducer<TILE>{sums, tile * TILE - kScanE, total}, tile,
-                                                     total, out, total, nullptr, ONE ? nullptr : flags, err);
-  if (!ONE) finish_tile(flags, counter, tiles);
+  typedef SmemSumsProducer<TILE> Sums;
+  scan_tile<Sums, kScanLookback, 256, TILE>(Sums{sums, tile * TILE - kScanE, total}, tile, total, out, total, nullptr,
+                                            flags, err);
+  finish_tile(flags, counter, tiles);
 }
 
 // One warp a job: lane i adds limb base + i of x and y; the block's carries
@@ -261,11 +362,19 @@ cudaError_t run_scan(const Prod& prod, u64 total, u64* out, u64 out_limit, Scan&
   cudaError_t e = scan_reserve(sc, tiles);
   if (e != cudaSuccess || tile_end <= tile_begin) return e;
   const u64 n = tile_end - tile_begin;
-  if (tiles == 1) {  // neither a tile number nor a status word: four dependent accesses of global memory less
+  // A whole scan of at most eight tiles: one cluster, of smaller tiles while
+  // they do (a thread's eight values are a serial chain; more CTAs share them).
+  if (tile_begin == 0 && tile_end == tiles && tiles <= kClusterTiles) {
+    constexpr int kSmall = 64;
     launch_begin(name, st);
-    scan_kernel<Prod><<<1, kScanThreads, 0, st>>>(prod, total, out, out_limit, sc.side, nullptr, 0);
+    if (total <= kClusterTiles * kSmall * kScanE)
+      e = launch_cluster(scan_cluster_kernel<Prod, kSmall>, (unsigned)((total + kSmall * kScanE - 1) / (kSmall * kScanE)),
+                         kSmall, st, prod, total, out, out_limit, sc.side);
+    else
+      e = launch_cluster(scan_cluster_kernel<Prod, kScanThreads>, (unsigned)tiles, kScanThreads, st, prod, total, out,
+                         out_limit, sc.side);
     launch_end(st);
-    return cudaGetLastError();
+    return e;
   }
   if (tiles <= kLookbackTiles) {
     launch_begin(name, st);
@@ -288,10 +397,7 @@ template <u64 TILE>
 cudaError_t launch_school(const ColumnProducer& prod, u64 total, u64* out, Scan& sc, cudaStream_t st) {
   const u32 tiles = (u32)((total + TILE - 1) / TILE);  // at most kLookbackTiles
   launch_begin("school_tiles", st);
-  if (tiles == 1)
-    school_kernel<TILE, true><<<1, 256, 0, st>>>(prod, total, out, nullptr, nullptr, nullptr, 1);
-  else
-    school_kernel<TILE, false><<<tiles, 256, 0, st>>>(prod, total, out, sc.flags, sc.counter, sc.err, tiles);
+  school_kernel<TILE><<<tiles, 256, 0, st>>>(prod, total, out, sc.flags, sc.counter, sc.err, tiles);
   launch_end(st);
   return cudaGetLastError();
 }
@@ -439,8 +545,17 @@ cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Sca
   cudaError_t e = scan_reserve(sc, 1);
   if (e != cudaSuccess) return e;
   const u64 total = na + nb;
-  const ColumnProducer prod{a, na, b, nb};
-  if (total <= kSchoolShortTile && nb <= 64) return launch_school<kSchoolShortTile>(prod, total, out, sc, st);
+  const ColumnProducer prod = na >= nb ? ColumnProducer{a, na, b, nb} : ColumnProducer{b, nb, a, na};
+  if (total <= kSchoolClusterTile * kSchoolClusterCtas && prod.nb <= kSchoolShorter) {
+    static const cudaError_t ok =  // clusters of more than eight CTAs want asking
+        cudaFuncSetAttribute(school_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (ok != cudaSuccess) return ok;
+    launch_begin("school_tiles", st);
+    e = launch_cluster(school_cluster_kernel, (unsigned)((total + kSchoolClusterTile - 1) / kSchoolClusterTile), 256, st,
+                       prod, total, out);
+    launch_end(st);
+    return e;
+  }
   if (total <= kSchoolTile * kLookbackTiles) return launch_school<kSchoolTile>(prod, total, out, sc, st);
   if (total <= kSchoolLongTile * kLookbackTiles) return launch_school<kSchoolLongTile>(prod, total, out, sc, st);
   return run_scan(prod, total, out, total, sc, st, "school_column_scan");

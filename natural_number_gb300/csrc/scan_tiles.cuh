@@ -196,27 +196,39 @@ __device__ __forceinline__ void six_garner4(const int4 (&v)[six::kPrimes], W3 (&
     x[e0 + e] = six_garner(y);
   }
 }
+// Zero at and beyond position count.
+__device__ __forceinline__ void six_mask(W3 (&x)[kScanE], u64 k0, u64 count) {
+  if (k0 + kScanE <= count) return;
+#pragma unroll
+  for (int e = 0; e < kScanE; ++e)
+    if (k0 + e >= count) x[e] = W3{0, 0, 0};
+}
+// A position's six words, as loaded (fetch) and combined (finish) apart: the
+// scan has the values before its tile in flight while it forms the tile's.
+struct SixWordsAt {
+  int y[six::kPrimes];
+  bool in;
+};
 struct SixCrtProducer {
   const u32* res;  // [6][L]
   u64 L, count;
   static constexpr bool kBulk = true;
-  // One position: the ends of a product only, so a call rather than sixteen
-  // inlined copies in the scan.
-  __device__ __noinline__ W3 operator()(u64 i) const {
-    if (i >= count) return W3{0, 0, 0};
-    int y[six::kPrimes];
+  typedef SixWordsAt Raw;
+  __device__ __forceinline__ Raw fetch(u64 i) const {
+    Raw r;
+    r.in = i < count;
 #pragma unroll
-    for (int q = 0; q < six::kPrimes; ++q) {
-      const u32* r = res + q * L + i;
-      y[q] = (int)*r;
-    }
-    return six_garner(y);
+    for (int q = 0; q < six::kPrimes; ++q) r.y[q] = r.in ? (int)res[q * L + i] : 0;
+    return r;
   }
-  // Eight consecutive positions from k0 (a multiple of 8) with 16-byte loads.
+  __device__ __forceinline__ W3 finish(const Raw& r) const { return r.in ? six_garner(r.y) : W3{0, 0, 0}; }
+  __device__ __forceinline__ W3 operator()(u64 i) const { return finish(fetch(i)); }
+  // Eight consecutive positions from k0 (a multiple of 8, at least one below
+  // count: then all eight lie in the transform) with 16-byte loads.
   __device__ __forceinline__ void bulk(u64 k0, W3 (&x)[kScanE]) const {
-    if (k0 + kScanE > count) {
+    if (k0 >= count) {
 #pragma unroll
-      for (int e = 0; e < kScanE; ++e) x[e] = (*this)(k0 + e);
+      for (int e = 0; e < kScanE; ++e) x[e] = W3{0, 0, 0};
       return;
     }
 #pragma unroll
@@ -226,6 +238,7 @@ struct SixCrtProducer {
       for (int q = 0; q < six::kPrimes; ++q) v[q] = *reinterpret_cast<const int4*>(res + q * L + k0 + e0);
       six_garner4(v, x, e0);
     }
+    six_mask(x, k0, count);
   }
 };
 
@@ -242,31 +255,34 @@ struct PieceCrtProducer {
   const u32* res;
   u64 L, k, P, ny, count;
   static constexpr bool kBulk = true;
+  typedef SixWordsAt Raw;
   __device__ __forceinline__ u64 piece_of(u64 j) const {
     const u64 i = j / k;
     return i < P ? i : P - 1;
   }
-  __device__ __noinline__ W3 operator()(u64 j) const {
-    if (j >= count) return W3{0, 0, 0};
-    const u64 i = piece_of(j), r = j - i * k;
+  __device__ __forceinline__ Raw fetch(u64 j) const {
+    Raw w;
+    w.in = j < count;
+    const u64 i = w.in ? piece_of(j) : 0, r = w.in ? j - i * k : 0;
     const u32* c = res + i * six::kPrimes * L + r;
     const u32* b = c - six::kPrimes * L + k;  // the piece before, at r + k
     const bool ov = i > 0 && r + 1 < ny;
-    int y[six::kPrimes];
 #pragma unroll
     for (int q = 0; q < six::kPrimes; ++q) {
-      y[q] = (int)c[q * L];
-      if (ov) y[q] += (int)b[q * L];
+      w.y[q] = (int)c[q * L];
+      if (ov) w.y[q] += (int)b[q * L];
     }
-    return six_garner(y);
+    return w;
   }
+  __device__ __forceinline__ W3 finish(const Raw& r) const { return r.in ? six_garner(r.y) : W3{0, 0, 0}; }
+  __device__ __forceinline__ W3 operator()(u64 j) const { return finish(fetch(j)); }
   __device__ __forceinline__ void bulk(u64 k0, W3 (&x)[kScanE]) const {
-    const u64 i = piece_of(k0), r = k0 - i * k;  // one piece for the eight positions
-    if (k0 + kScanE > count) {
+    if (k0 >= count) {
 #pragma unroll
-      for (int e = 0; e < kScanE; ++e) x[e] = (*this)(k0 + e);
+      for (int e = 0; e < kScanE; ++e) x[e] = W3{0, 0, 0};
       return;
     }
+    const u64 i = piece_of(k0), r = k0 - i * k;  // one piece for the eight positions
     const u32* c = res + i * six::kPrimes * L + r;
     const u32* b = c - six::kPrimes * L + k;
     const u64 ov = i > 0 && r + 1 < ny ? ny - 1 - r : 0;  // so many of them overlap
@@ -287,6 +303,7 @@ struct PieceCrtProducer {
       }
       six_garner4(v, x, e0);
     }
+    six_mask(x, k0, count);
   }
 };
 
@@ -500,10 +517,10 @@ __device__ __forceinline__ u32 wait_flag(const u32* f, int limit) {
 
 // One tile of the scan over positions [0, total): limbs below out_limit go to
 // out, the rest to side.
-// LOOKBACK: the tile takes its carry-in from its predecessors' status words
+// kScanLookback: the tile takes its carry-in from its predecessors' status words
 // (decoupled lookback); tiles of one scan must then start in increasing order
 // (their predecessors already running), which the callers guarantee.
-// Without LOOKBACK the tile takes carry-in 0 and records in flags[tile] (when given) its
+// kScanRecord: the tile takes carry-in 0 and records in flags[tile] (when given) its
 // carry out for carry-in 0 (bit 0, generate) and whether a carry-in would pass
 // straight through (bit 1, propagate: every limb all ones); a later step
 // resolves the one-bit carries between tiles (carry.cu).
@@ -514,7 +531,7 @@ template <int NT>
 struct ScanShared {
   u64 h0[NT], h1[NT];
   u32 wg[NT / 32], wp[NT / 32];
-  u32 cin;
+  u32 cin, bits;
   u64 x[kScanE][3];
 };
 template <int NT>
@@ -523,9 +540,44 @@ __device__ __forceinline__ ScanShared<NT>& scan_shared() {
   return sh;
 }
 
+// How a tile learns its carry-in: later (record), by the lookback, or from the
+// other tiles of its cluster.
+enum : int { kScanRecord = 0, kScanLookback = 1, kScanCluster = 2 };
+
+// All threads of all CTAs of the cluster arrive; what they wrote to shared
+// memory before is visible to the others after.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// The value at `local` in the shared memory of the cluster's CTA `rank`.
+__device__ __forceinline__ u64 cluster_load64(const u64* local, u32 rank) {
+  u64 v;
+  asm volatile(
+      "{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.u64 %0, [a];\n\t}"
+      : "=l"(v)
+      : "r"((u32)__cvta_generic_to_shared(local)), "r"(rank)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ u32 cluster_load32(const u32* local, u32 rank) {
+  u32 v;
+  asm volatile(
+      "{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.u32 %0, [a];\n\t}"
+      : "=r"(v)
+      : "r"((u32)__cvta_generic_to_shared(local)), "r"(rank)
+      : "memory");
+  return v;
+}
+
+// kScanCluster: the scan's tiles are the CTAs of one cluster, tile = rank (at
+// most 16).  A tile takes the overflow into its first position from the last
+// thread of the tile before, and its carry-in from all earlier tiles' bits,
+// both through distributed shared memory: no status words, no polling, and no
+// values formed twice.  The caller ends with cluster_sync(), so that no CTA
+// leaves while another reads its shared memory.
 // NT: threads of the CTA.  TILE: positions of a tile, NT * kScanE at most;
 // with fewer, the threads beyond them pass carries on unchanged.
-template <class Prod, bool LOOKBACK = true, int NT = kScanThreads, u64 TILE = (u64)NT * kScanE>
+template <class Prod, int MODE = kScanLookback, int NT = kScanThreads, u64 TILE = (u64)NT * kScanE>
 __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total, u64* out, u64 out_limit, u64* side,
                                           u32* flags, u32* err) {
   constexpr int E = kScanE;
@@ -544,7 +596,19 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
   u64 y[E];
   u64 c0 = 0, c1 = 0;
   W3 xs[E];
-  if (Prod::kBulk && on && k0 + E <= total) {
+  // The E positions before this tile (below): their loads go out first.
+  constexpr bool kSplit = requires { typename Prod::Raw; };
+  typedef decltype([] {
+    if constexpr (kSplit)
+      return typename Prod::Raw{};
+    else
+      return W3{};
+  }()) Before;
+  Before before{};
+  const bool preceding = MODE != kScanCluster && warp == 0 && lane < E && tile != 0;
+  if constexpr (kSplit)
+    if (preceding) before = prod.fetch(tile * kTile - E + lane);
+  if (Prod::kBulk && on && k0 < total) {
     prod.bulk(k0, xs);
   } else {
 #pragma unroll
@@ -562,9 +626,13 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
   // Overflow of the E positions before this tile: lanes 0..E-1 of warp 0
   // produce one value each, thread 0 chains them.
   u64(&s_x)[E][3] = sh.x;
-  if (warp == 0) {
-    if (lane < E && tile != 0) {
-      const W3 x = prod(tile * kTile - E + lane);
+  if (MODE != kScanCluster && warp == 0) {
+    if (preceding) {
+      W3 x;
+      if constexpr (kSplit)
+        x = prod.finish(before);
+      else
+        x = prod(tile * kTile - E + lane);
       s_x[lane][0] = x.w0;
       s_x[lane][1] = x.w1;
       s_x[lane][2] = x.w2;
@@ -572,7 +640,7 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
     __syncwarp();
   }
   u64 hp0 = 0, hp1 = 0;
-  if (tid == 0 && tile != 0) {
+  if (MODE != kScanCluster && tid == 0 && tile != 0) {
     u64 d0 = 0, d1 = 0;
     for (int e = 0; e < E; ++e) {
       const W3 t = add_w3(W3{s_x[e][0], s_x[e][1], s_x[e][2]}, W3{d0, d1, 0});
@@ -582,7 +650,15 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
     hp0 = d0;
     hp1 = d1;
   }
-  __syncthreads();
+  if constexpr (MODE == kScanCluster) {
+    cluster_sync();
+    if (tid == 0 && tile != 0) {
+      hp0 = cluster_load64(s_h0 + TILE / E - 1, (u32)tile - 1);
+      hp1 = cluster_load64(s_h1 + TILE / E - 1, (u32)tile - 1);
+    }
+  } else {
+    __syncthreads();
+  }
   if (tid > 0 && on) {
     hp0 = s_h0[tid - 1];
     hp1 = s_h1[tid - 1];
@@ -611,7 +687,9 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
     }
     const u32 tg = c_if0, tp = c_if1 & !c_if0;
     u32 cin = 0;
-    if (!LOOKBACK) {
+    if (MODE == kScanCluster) {
+      sh.bits = tg | (tp << 1);
+    } else if (MODE == kScanRecord) {
       if (flags) flags[tile] = tg | (tp << 1);
     } else if (tile > 0) {
       flag_store(&flags[tile], kFlagAggregate | (tg << 2) | (tp << 3));
@@ -642,8 +720,16 @@ __device__ __forceinline__ void scan_tile(const Prod& prod, u64 tile, u64 total,
         --j;  // predecessor propagates: look further back
       }
     }
-    if (LOOKBACK) flag_store(&flags[tile], kFlagInclusive | ((tg | (tp & cin)) << 2));
+    if (MODE == kScanLookback) flag_store(&flags[tile], kFlagInclusive | ((tg | (tp & cin)) << 2));
     s_cin = cin;
+  }
+  if constexpr (MODE == kScanCluster) {
+    cluster_sync();
+    if (warp == 0) {
+      const u32 f = (u64)lane < tile ? cluster_load32(&sh.bits, lane) : 0;
+      const u32 g1 = __ballot_sync(0xffffffffu, f & 1), gp = __ballot_sync(0xffffffffu, f & 3);
+      if (lane == 0) s_cin = ((g1 + gp) ^ g1 ^ gp) >> tile & 1;
+    }
   }
   __syncthreads();
   u32 wc = s_cin;

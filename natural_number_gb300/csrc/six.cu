@@ -135,8 +135,8 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
 
 // op.ra's pieces (or, FIRST, the limbs op.a) with op.rb (op.b), into `out`;
 // mode kForward: op.ra alone.
-template <int R, int LGM, int V, int MODE, bool FIRST>
-__global__ void __launch_bounds__(fused_threads(R, LGM, V), fused_blocks(R, LGM, V))
+template <int R, int LGM, int V, int MODE, bool FIRST, bool PAIR>
+__global__ void __launch_bounds__(fused_threads(R, LGM, V) * (PAIR ? 2 : 1), PAIR ? 1 : fused_blocks(R, LGM, V))
     six_fused_kernel(SixOperands op, u32* out, const SixPlan pl, const int2* __restrict__ tab, u64 cap) {
   extern __shared__ __align__(16) u32 sm6[];
   constexpr int NT = fused_threads(R, LGM, V);
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(fused_threads(R, LGM, V), fused_blocks(R, LGM,
   const void* a = FIRST ? static_cast<const void*>(op.a + at0) : op.ra + piece;
   const void* b = FIRST && MODE == kAll ? static_cast<const void*>(op.b) : op.rb;
   const bool last = pl.n == 1;
-  fused_tile<R, LGM, NT, V, MODE, FIRST>(sm6, a, min(op.piece, op.na - at0), b, op.nb, out + piece, pl.s, blockIdx.x,
+  fused_tile<R, LGM, NT, V, MODE, FIRST, PAIR>(sm6, a, min(op.piece, op.na - at0), b, op.nb, out + piece, pl.s, blockIdx.x,
                                          blockIdx.y, tab, tab + kPrimes * cap, cap, pl.reduce_in(), last,
                                          pl.scale[blockIdx.y], last ? pl.k8 : 8);
 }
@@ -178,23 +178,29 @@ cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int lamb
   launch_end(st);
   return cudaGetLastError();
 }
-template <int R, int LGM, int V, int MODE, bool FIRST>
+template <int R, int LGM, int V, int MODE, bool FIRST, bool PAIR = false>
 cudaError_t launch_fused_v(const SixOperands& op, u32* out, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
-  constexpr int tile = (int)tile_words32<1 << LGM, true>(R) * 4, smem = fused_tiles(LGM, MODE) * tile;
-  static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, V, MODE, FIRST>, smem);
+  constexpr int tile = (int)tile_words32<1 << LGM, true>(R) * 4, smem = fused_tiles(LGM, MODE) * tile + (PAIR ? (16 << (R - 1)) : 0);
+  static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, V, MODE, FIRST, PAIR>, smem);
   if (ok != cudaSuccess) return ok;
   const u32 tiles = (u32)((1ull << pl.s) >> (R + LGM));
   const dim3 grid(pl.n == 1 ? 1u : tiles / 8 * pl.k8, kPrimes, op.pieces);
   launch_begin(MODE == kForward ? "six_fwd_row_pass" : FIRST ? "six_small_pass" : "six_fused_row_pass", st);
-  six_fused_kernel<R, LGM, V, MODE, FIRST><<<grid, fused_threads(R, LGM, V), MODE == kAll && !op.b ? tile : smem, st>>>(
-      op, out, pl, t.tab, t.cap);
+  six_fused_kernel<R, LGM, V, MODE, FIRST, PAIR>
+      <<<grid, fused_threads(R, LGM, V) * (PAIR ? 2 : 1), MODE == kAll && !op.b ? tile : smem, st>>>(op, out, pl, t.tab,
+                                                                                                     t.cap);
   launch_end(st);
   return cudaGetLastError();
 }
-// Columns a thread: as few as keep the grid within one wave of the GPU's
-// 152 x 768 threads, so a short product uses as many of them as it can.
+// A few one-pass products: an operand a half of the CTA (six CTAs a piece:
+// up to 96 fill under one wave).  Columns a thread: as few as keep the grid
+// within one wave of the GPU's 152 x 768 threads, so a short product uses as
+// many of them as it can (a limit of 1024 threads: 18.7 instead of 17.7 us for
+// the pass at scale 18).
 template <int R, int LGM, int MODE, bool FIRST>
 cudaError_t launch_fused(const SixOperands& op, u32* out, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  if constexpr (FIRST && MODE == kAll && R >= 5)
+    if (op.b && op.pieces <= 16) return launch_fused_v<R, LGM, 1, MODE, FIRST, true>(op, out, pl, t, st);
   if constexpr (LGM == 3)
     if (((u64)kPrimes * op.pieces << pl.s) / 64 * pl.k8 <= 152 * 768)
       return launch_fused_v<R, LGM, 1, MODE, FIRST>(op, out, pl, t, st);

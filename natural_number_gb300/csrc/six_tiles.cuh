@@ -150,25 +150,37 @@ struct Unit {
   }
 };
 
+// A table of roots in global memory (read-only cache), or the part of it that
+// a tile needs, copied to shared memory.
+struct GlobalRoots {
+  const int2* p;
+  __device__ __forceinline__ int2 one(u32 b) const { return __ldg(p + b); }
+  __device__ __forceinline__ int4 pair(u64 b) const { return __ldg(reinterpret_cast<const int4*>(p + b)); }
+};
+struct SharedRoots {
+  const int2* p;
+  __device__ __forceinline__ int2 one(u32 b) const { return p[b]; }
+  __device__ __forceinline__ int4 pair(u64 b) const { return *reinterpret_cast<const int4*>(p + b); }
+};
+
 // The twiddle pairs of local level lv of a unit whose block index at the
 // unit's first level is b: W[b 2^lv + g], g < 2^lv.
-template <int LV>
-__device__ __forceinline__ void twiddles(int2 (&w)[1 << LV], const int2* __restrict__ tw, u32 b) {
+template <int LV, class Roots>
+__device__ __forceinline__ void twiddles(int2 (&w)[1 << LV], const Roots& tw, u32 b) {
   if constexpr (LV == 0) {
-    w[0] = __ldg(tw + b);
+    w[0] = tw.one(b);
   } else {
-    const int4* t = reinterpret_cast<const int4*>(tw + ((u64)b << LV));
 #pragma unroll
     for (int g = 0; g < (1 << LV); g += 2) {
-      const int4 v = __ldg(t + g / 2);
+      const int4 v = tw.pair(((u64)b << LV) + g);
       w[g] = make_int2(v.x, v.y);
       w[g + 1] = make_int2(v.z, v.w);
     }
   }
 }
 
-template <int K, int V, int LV>
-__device__ __forceinline__ void fwd_level(Unit<K, V>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+template <int K, int V, int LV, class Roots>
+__device__ __forceinline__ void fwd_level(Unit<K, V>& u, const Roots& tw, u32 b, i32 p) {
   int2 w[1 << LV];
   twiddles<LV>(w, tw, b);
   constexpr int half = (1 << K) >> (LV + 1);
@@ -181,16 +193,16 @@ __device__ __forceinline__ void fwd_level(Unit<K, V>& u, const int2* __restrict_
         fwd_bfly(u.x[g * 2 * half + m][c], u.x[g * 2 * half + m + half][c], w[g].x, w[g].y, p);
 }
 // Levels [LV0, K) of a unit.
-template <int K, int LV = 0, int V>
-__device__ __forceinline__ void fwd_levels(Unit<K, V>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+template <int K, int LV = 0, int V, class Roots>
+__device__ __forceinline__ void fwd_levels(Unit<K, V>& u, const Roots& tw, u32 b, i32 p) {
   if constexpr (LV < K) {
     fwd_level<K, V, LV>(u, tw, b, p);
     fwd_levels<K, LV + 1>(u, tw, b, p);
   }
 }
 
-template <int K, int V, int LV>
-__device__ __forceinline__ void inv_level(Unit<K, V>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+template <int K, int V, int LV, class Roots>
+__device__ __forceinline__ void inv_level(Unit<K, V>& u, const Roots& tw, u32 b, i32 p) {
   int2 w[1 << LV];
   twiddles<LV>(w, tw, b);
   constexpr int half = (1 << K) >> (LV + 1);
@@ -202,8 +214,8 @@ __device__ __forceinline__ void inv_level(Unit<K, V>& u, const int2* __restrict_
       for (int c = 0; c < V; ++c)
         inv_bfly(u.x[g * 2 * half + m][c], u.x[g * 2 * half + m + half][c], w[g].x, w[g].y, p);
 }
-template <int K, int LV = K - 1, int V>
-__device__ __forceinline__ void inv_levels(Unit<K, V>& u, const int2* __restrict__ tw, u32 b, i32 p) {
+template <int K, int LV = K - 1, int V, class Roots>
+__device__ __forceinline__ void inv_levels(Unit<K, V>& u, const Roots& tw, u32 b, i32 p) {
   if constexpr (LV >= 0) {
     inv_level<K, V, LV>(u, tw, b, p);
     inv_levels<K, LV - 1>(u, tw, b, p);
@@ -231,11 +243,11 @@ __device__ __forceinline__ void inv_fold(Unit<K, V>& u, const Prime& P) {
 //         8 (a0 - a4) = 2 2v0 + F, 8 (a2 - a6) = -i (2 2v0 - F).
 // Rows 0 .. k-1 receive 16 a_j, twice what the full group's sums give: the
 // transform's scale takes that into account.
-template <int V>
-__device__ __forceinline__ void inv_truncated(Unit<3, V>& u, int k8, const int2* __restrict__ itw,
-                                              const int2* __restrict__ ftw, const Prime& P) {
+template <int V, class Roots>
+__device__ __forceinline__ void inv_truncated(Unit<3, V>& u, int k8, const Roots& itw, const Roots& ftw,
+                                              const Prime& P) {
   const i32 p = P.p;
-  const int2 i1 = __ldg(ftw + 1), w1 = __ldg(ftw + 2), h1 = __ldg(ftw + 3), ii = __ldg(itw + 1), wi = __ldg(itw + 2);
+  const int2 i1 = ftw.one(1), w1 = ftw.one(2), h1 = ftw.one(3), ii = itw.one(1), wi = itw.one(2);
 #pragma unroll
   for (int c = 0; c < V; ++c) {
     const i32 y0 = u.x[0][c], y1 = u.x[1][c], y2 = u.x[2][c], y3 = u.x[3][c], y4 = u.x[4][c], y5 = u.x[5][c];
@@ -343,12 +355,12 @@ inline cudaError_t allow_smem(Kernel k, int bytes) {
 // Forward levels [0, R) of one tile of C columns x 2^R rows, block index ksb
 // at its first level.  load(row, col) gives the V words from (row, col), store
 // puts V finished words; between groups the words go
-// through sm.  HALF: the rows from 2^(R-1) are zero, so level 0 copies.
+// through sm; thread tid of NT.  HALF: the rows from 2^(R-1) are zero, so level 0 copies.
 // START: a reduction of the loaded words; LAST: one of the stored words.
 // k8 < 8: only the rows of the first k8 eighths are finished and stored.
-template <int R, int C, bool LEAF, int NT, int V, bool START, bool LAST, class Load, class Store>
-__device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const Store& store, bool half_zero,
-                                             const int2* __restrict__ tw, u32 ksb, const Prime& P, bool start_red,
+template <int R, int C, bool LEAF, int NT, int V, bool START, bool LAST, class Load, class Store, class Roots>
+__device__ __forceinline__ void forward_tile(u32 tid, u32* sm, const Load& load, const Store& store, bool half_zero,
+                                             const Roots& tw, u32 ksb, const Prime& P, bool start_red,
                                              int k8 = 8) {
   constexpr int G = groups_of(R);
   auto group = [&](auto gc) {
@@ -359,7 +371,7 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
     const u32 todo = g == 0 ? units : units / 8 * k8;
     const int keep = g == 0 && K == 3 ? k8 : 8;
 #pragma unroll 1
-    for (u32 i = threadIdx.x; i < todo; i += NT) {
+    for (u32 i = tid; i < todo; i += NT) {
       const u32 col = (i % (C / V)) * V, v = i / (C / V);
       const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
       Unit<K, V> u;
@@ -416,10 +428,10 @@ __device__ __forceinline__ void forward_tile(u32* sm, const Load& load, const St
 // last: the transform's last pass; its outputs are multiplied by the scale,
 // which also makes them 0.75 p at most (k8 < 8, with the forward table ftw: a
 // truncated transform's).
-template <int R, int C, bool LEAF, int NT, int V, class Load, class Store>
-__device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const Store& store,
-                                             const int2* __restrict__ tw, u32 ksb, const Prime& P, bool last,
-                                             int2 scale, int k8, const int2* __restrict__ ftw) {
+template <int R, int C, bool LEAF, int NT, int V, class Load, class Store, class Roots>
+__device__ __forceinline__ void inverse_tile(u32 tid, u32* sm, const Load& load, const Store& store,
+                                             const Roots& tw, u32 ksb, const Prime& P, bool last,
+                                             int2 scale, int k8, const Roots& ftw) {
   constexpr int G = groups_of(R);
   auto group = [&](auto gc) {
     constexpr int g = decltype(gc)::value;
@@ -429,7 +441,7 @@ __device__ __forceinline__ void inverse_tile(u32* sm, const Load& load, const St
     const u32 todo = g == 0 ? units : units / 8 * k8;
     const int keep = g == 0 && K == 3 ? k8 : 8;
 #pragma unroll 1
-    for (u32 i = threadIdx.x; i < todo; i += NT) {
+    for (u32 i = tid; i < todo; i += NT) {
       const u32 col = (i % (C / V)) * V, v = i / (C / V);
       const u32 rb = v >> nsub, row0 = (rb << (nsub + K)) + (v & ((1u << nsub) - 1));
       Unit<K, V> u;
@@ -507,9 +519,9 @@ __device__ __forceinline__ void load_tile(u32* sm, const u64* __restrict__ in, u
   const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
   const u64 col0 = (u64)tile * C;
   forward_tile<R, C, false, NT, 4, false, false>(
-      sm, [&](u32 row, u32 col) { return limb_words<4>(in, n, ((u64)row << lg_s) + col0 + col, vec, P); },
+      threadIdx.x, sm, [&](u32 row, u32 col) { return limb_words<4>(in, n, ((u64)row << lg_s) + col0 + col, vec, P); },
       [&](u32 row, u32 col, const Words<4>& w) { stv(out + ((u64)row << lg_s) + col, w); }, n <= (1ull << (s - 1)),
-      tab + prime * cap, 0, P, false, k8);
+      GlobalRoots{tab + prime * cap}, 0, P, false, k8);
 }
 
 // Levels [lambda0, lambda0 + R) of residues in place: forward or inverse (tab:
@@ -524,13 +536,14 @@ __device__ __forceinline__ void col_tile(u32* sm, u32* res, int s, int lambda0, 
   const u32 per = (u32)((1ull << lg_s) / C);  // tiles a block
   const u32 ksb = tile / per;
   u32* g = res + ((u64)prime << s) + ((u64)ksb << (lg_s + R)) + (u64)(tile % per) * C;
-  const int2* tw = tab + prime * cap;
+  const GlobalRoots tw{tab + prime * cap};
   auto ld = [&](u32 row, u32 col) { return ldv<4>(g + ((u64)row << lg_s) + col); };
   auto st = [&](u32 row, u32 col, const Words<4>& w) { stv(g + ((u64)row << lg_s) + col, w); };
   if constexpr (INV)
-    inverse_tile<R, C, false, NT, 4>(sm, ld, st, tw, ksb, P, last, scale, k8, tw - kPrimes * cap);
+    inverse_tile<R, C, false, NT, 4>(threadIdx.x, sm, ld, st, tw, ksb, P, last, scale, k8,
+                                     GlobalRoots{tw.p - kPrimes * cap});
   else
-    forward_tile<R, C, false, NT, 4, false, false>(sm, ld, st, false, tw, ksb, P, false);
+    forward_tile<R, C, false, NT, 4, false, false>(threadIdx.x, sm, ld, st, false, tw, ksb, P, false);
 }
 
 // Products of polynomials of 8 coefficients by Karatsuba's method three levels
@@ -585,8 +598,9 @@ __device__ __forceinline__ void fold8(i64 (&t)[15], i32 cr, i32 (&o)[8], const P
 }
 // The constant c_b of block b, times 2^32: the roots' table holds it for even
 // b, its negative for odd b.
-__device__ __forceinline__ i32 block_constant(const int2* __restrict__ tw, u32 b, const Prime& P) {
-  const i32 c = __ldg(tw + (b >> 1)).x;
+template <class Roots>
+__device__ __forceinline__ i32 block_constant(const Roots& tw, u32 b, const Prime& P) {
+  const i32 c = tw.one(b >> 1).x;
   const i32 r = mul_mod(c, P.r, P.rp, P.p);
   return b & 1 ? -r : r;
 }
@@ -596,9 +610,9 @@ __device__ __forceinline__ i32 block_constant(const int2* __restrict__ tw, u32 b
 // gb nullptr), or finished words in global memory, where a thread's block is
 // one 32-byte sector.  Words at most 0.75 p in magnitude: the sums of eight
 // products, with the folded part, stay below 2^58.
-template <int R, int NT, bool GA, bool GB>
-__device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const u32* ga, const u32* gb,
-                                               const int2* __restrict__ tw, u32 ksb, const Prime& P, u32 rows) {
+template <int R, int NT, bool GA, bool GB, class Roots>
+__device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const u32* ga, const u32* gb, const Roots& tw,
+                                               u32 ksb, const Prime& P, u32 rows) {
 #pragma unroll 1
   for (u32 r = threadIdx.x; r < rows; r += NT) {
     const i32 cr = block_constant(tw, (ksb << R) + r, P);
@@ -638,8 +652,8 @@ __device__ __forceinline__ void leaf_products8(u32* sa, const u32* sb, const u32
 // three levels take 114 registers (2^25 x 2^25 limbs: fused pass 3.02 ms at four
 // CTAs, 2.73 so, 3.03 with 64 multiply-adds; 2^27 x 2^27: 19.2, 17.0, 17.5).  Results are written after every thread of the CTA has read the
 // round's blocks.
-template <int R, int LGM, int NT>
-__device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const int2* __restrict__ tw, u32 ksb,
+template <int R, int LGM, int NT, class Roots>
+__device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const Roots& tw, u32 ksb,
                                               const Prime& P) {
   constexpr int C = 1 << LGM, G = C / 8;
   constexpr u32 items = (u32)G << R;
@@ -649,7 +663,7 @@ __device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const int2
     const u32 q = it * NT + threadIdx.x;  // whole blocks a round: items of a block lie in one round
     const bool on = q < items;
     const u32 r = on ? q / G : 0, g = q % G, blk = (ksb << R) + r;
-    int2 c = __ldg(tw + (blk >> 1));
+    int2 c = tw.one(blk >> 1);
     if (blk & 1) c = make_int2(-c.x, -c.y);
     i64 lo[7], hi[7], mid[7];  // products of the lower halves, the upper ones, the sums of both
 #pragma unroll
@@ -704,11 +718,15 @@ __device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const int2
 // Operands are residues after the strided passes, or, FIRST (transforms of one
 // pass), limbs (na, nb of them); finished ones are words of at most 0.75 p.
 // last: no strided inverse pass follows (scale, k8 as in inverse_tile).
+// PAIR (FIRST, kAll): twice the threads, half of them an operand, and the
+// 2^(R-1) roots of either direction that a one-pass transform needs copied to
+// shared memory while the limbs are on their way: a lone short product waits
+// on memory a third as often.
 enum : int { kAll = 0, kReady = 1, kProduct = 2, kForward = 3 };
 // Shared-memory tiles of a mode: finished operands are read from global memory
 // where a block is a sector (LGM = 3).
 constexpr int fused_tiles(int LGM, int mode) { return mode == kAll || (LGM > 3 && mode != kForward) ? 2 : 1; }
-template <int R, int LGM, int NT, int V, int MODE, bool FIRST>
+template <int R, int LGM, int NT, int V, int MODE, bool FIRST, bool PAIR = false>
 __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const void* b, u64 nb, u32* out, int s,
                                            u32 tile, int prime, const int2* __restrict__ tab,
                                            const int2* __restrict__ itab, u64 cap, bool reduce_in, bool last,
@@ -716,30 +734,43 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
   constexpr int C = 1 << LGM;
   constexpr u32 W = tile_words32<C, true>(R);
   const Prime P = c_primes[prime];
-  const int2* tw = tab + prime * cap;
-  const int2* itw = itab + prime * cap;
+  const int2* const tw0 = tab + prime * cap;
+  const int2* const itw0 = itab + prime * cap;
   const u64 off = ((u64)prime << s) + ((u64)tile << (R + LGM));
   u32* sa = sm;
   u32* sb = MODE == kAll && !b ? sm : sm + W;
+  constexpr u32 kRoots = 1u << (R - 1);
+  int2* const sroots = reinterpret_cast<int2*>(sm + 2 * W);
+  typedef std::conditional_t<PAIR, SharedRoots, GlobalRoots> Roots;
+  const Roots tw{PAIR ? sroots : tw0}, itw{PAIR ? sroots + kRoots : itw0};
+  const u32 tid = PAIR ? threadIdx.x % NT : threadIdx.x;
+  if constexpr (PAIR) {
+    for (u32 i = threadIdx.x; i < 2 * kRoots; i += 2 * NT)
+      sroots[i] = __ldg(i < kRoots ? tw0 + i : itw0 + (i - kRoots));
+    __syncthreads();
+  }
   auto to = [&](u32* t) { return [t](u32 row, u32 col, const Words<V>& w) { stv(t + at<C, true>(row) + col, w); }; };
   auto forward = [&](const void* src, u64 n, u32* t) {
     if constexpr (FIRST) {
       const u64* in = static_cast<const u64*>(src);
       const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
       forward_tile<R, C, true, NT, V, false, true>(
-          t, [&](u32 row, u32 col) { return limb_words<V>(in, n, (u64)row * C + col, vec, P); }, to(t),
+          tid, t, [&](u32 row, u32 col) { return limb_words<V>(in, n, (u64)row * C + col, vec, P); }, to(t),
           n <= (1ull << (s - 1)), tw, 0, P, false, k8);
     } else {
       const u32* in = static_cast<const u32*>(src) + off;
       forward_tile<R, C, true, NT, V, true, true>(
-          t, [&](u32 row, u32 col) { return ldv<V>(in + row * C + col); }, to(t), false, tw, tile, P, reduce_in);
+          tid, t, [&](u32 row, u32 col) { return ldv<V>(in + row * C + col); }, to(t), false, tw, tile, P, reduce_in);
     }
   };
   auto copy_in = [&](const void* src, u32* t) {
     const u32* in = static_cast<const u32*>(src) + off;
     for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT) stv(t + at<C, true>(i / C) + i % C, ldv<4>(in + i));
   };
-  if constexpr (MODE == kAll) {
+  if constexpr (PAIR) {
+    const bool second = threadIdx.x >= NT;
+    forward(second ? b : a, second ? nb : na, second ? sb : sa);
+  } else if constexpr (MODE == kAll) {
     // one copy of the code for both operands
     const int operands = b ? 2 : 1;
 #pragma unroll 1
@@ -756,15 +787,15 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
     for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT) stv(back + i, ldv<4>(sa + at<C, true>(i / C) + i % C));
   } else {
     if constexpr (LGM == 3)
-      leaf_products8<R, NT, MODE == kProduct, MODE != kAll>(sa, sb, static_cast<const u32*>(a) + off,
+      leaf_products8<R, PAIR ? 2 * NT : NT, MODE == kProduct, MODE != kAll>(sa, sb, static_cast<const u32*>(a) + off,
                                                             static_cast<const u32*>(b) + off, tw, tile, P,
                                                             FIRST && R >= 3 ? (u32)k8 << (R - 3) : 1u << R);
     else
       leaf_products<R, LGM, NT>(sa, sb, tw, tile, P);
     __syncthreads();
     u32* dst = out + off;
-    inverse_tile<R, C, true, NT, V>(
-        sa, [&](u32 row, u32 col) { return ldv<V>(sa + at<C, true>(row) + col); },
+    inverse_tile<R, C, true, PAIR ? 2 * NT : NT, V>(
+        threadIdx.x, sa, [&](u32 row, u32 col) { return ldv<V>(sa + at<C, true>(row) + col); },
         [&](u32 row, u32 col, const Words<V>& w) { stv(dst + row * C + col, w); }, itw, tile, P, last, scale, k8, tw);
   }
 }
