@@ -74,6 +74,7 @@ template <class Prod>
 __global__ void __launch_bounds__(kScanThreads, 3) scan_lookback_kernel(Prod prod, u64 total, u64* out, u64 out_limit,
                                                                      u64* side, u32* flags, u32* counter, u32* err,
                                                                      u32 tiles) {
+  grid_begin();
   scan_tile(prod, next_tile(counter), total, out, out_limit, side, flags, err);
   finish_tile(flags, counter, tiles);
 }
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_lookback_kernel(Prod pro
 template <class Prod>
 __global__ void __launch_bounds__(kScanThreads, 3) scan_kernel(Prod prod, u64 total, u64* out, u64 out_limit,
                                                             u64* side, u32* flags, u64 tile_base) {
+  grid_begin();
   scan_tile<Prod, kScanRecord>(prod, tile_base + blockIdx.x, total, out, out_limit, side, flags, nullptr);
 }
 
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(kScanThreads, 3) scan_kernel(Prod prod, u64 to
 constexpr int kFixTiles = 32;
 __global__ void __launch_bounds__(256) carry_fix_kernel(const u32* flags, u64 t0, u64 t1, u64 total, u64* out,
                                                         u64 out_limit, u64* side) {
+  grid_begin();
   __shared__ u32 s_first, s_cin, s_ones;
   const u64 c0 = t0 + (u64)blockIdx.x * kFixTiles;
   const int tid = threadIdx.x;
@@ -141,6 +144,7 @@ __global__ void __launch_bounds__(256) carry_fix_kernel(const u32* flags, u64 t0
 // Adds side[0] + side[1]*B into out[0..L) and wraps the final carry around to
 // limb 0 (ntt_info.h:238-242): the result is the product mod B^L - 1.
 __global__ void __launch_bounds__(1024) wrap_fix_kernel(u64* out, u64 L, const u64* side) {
+  grid_begin();
   __shared__ int s_carry;
   __shared__ unsigned long long s_first;
   const int tid = threadIdx.x;
@@ -183,10 +187,12 @@ __global__ void __launch_bounds__(1024) wrap_fix_kernel(u64* out, u64 L, const u
 // out[0..n] = in[0..n) << cl and out[0..n) = in[0..n) >> cl, 1 <= cl <= 63
 // (asmShl / asmShr, asm.h:31-33); out does not overlap in.
 __global__ void shl_bits_kernel(u64* out, const u64* in, u64 n, unsigned cl) {
+  grid_begin();
   for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += (u64)gridDim.x * blockDim.x)
     out[i] = (i < n ? in[i] << cl : 0) | (i > 0 ? in[i - 1] >> (64 - cl) : 0);
 }
 __global__ void shr_bits_kernel(u64* out, const u64* in, u64 n, unsigned cl) {
+  grid_begin();
   for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x)
     out[i] = (in[i] >> cl) | (i + 1 < n ? in[i + 1] << (64 - cl) : 0);
 }
@@ -200,26 +206,11 @@ __global__ void wait_probe_kernel(const u32* flag, u32* err, int limit) {
 // Scans of at most eight tiles: one cluster (kScanCluster).
 template <class Prod, int NT>
 __global__ void __launch_bounds__(NT) scan_cluster_kernel(Prod prod, u64 total, u64* out, u64 out_limit, u64* side) {
+  grid_begin();
   scan_tile<Prod, kScanCluster, NT>(prod, blockIdx.x, total, out, out_limit, side, nullptr, nullptr);
   cluster_sync();
 }
 constexpr u64 kClusterTiles = 8;
-
-// One cluster of `tiles` CTAs.
-template <class... Params, class... Args>
-cudaError_t launch_cluster(void (*kernel)(Params...), unsigned tiles, unsigned threads, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles);
-  cfg.blockDim = dim3(threads);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = tiles;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
-}
 
 // acc += x * y as one carry chain.
 __device__ __forceinline__ void mac(W3& acc, u64 x, u64 y) {
@@ -240,6 +231,7 @@ __device__ __forceinline__ void mac(W3& acc, u64 x, u64 y) {
 constexpr int kSchoolClusterCtas = 16;
 constexpr u64 kSchoolClusterTile = 64, kSchoolShorter = 384;
 __global__ void __launch_bounds__(256) school_cluster_kernel(ColumnProducer prod, u64 total, u64* out) {
+  grid_begin();
   constexpr u64 TILE = kSchoolClusterTile;
   constexpr int kLanes = 16;
   __shared__ u64 sums[3 * (TILE + kScanE)];
@@ -305,6 +297,7 @@ constexpr u64 kSchoolTile = 64, kSchoolLongTile = 1024;
 template <u64 TILE>
 __global__ void __launch_bounds__(256) school_kernel(ColumnProducer prod, u64 total, u64* out, u32* flags,
                                                      u32* counter, u32* err, u32 tiles) {
+  grid_begin();
   __shared__ u64 sums[3 * (TILE + kScanE)];
   const u32 tile = next_tile(counter);
   column_tile_sums<256, TILE>(sums, prod, tile);
@@ -320,6 +313,7 @@ __global__ void __launch_bounds__(256) school_kernel(ColumnProducer prod, u64 to
 // and propagate bits (the same identity as the scan's warp step).  A
 // difference adds the complement of y with a carry-in of 1.
 __global__ void __launch_bounds__(256) add_batch_kernel(const AddJob* __restrict__ jobs, u64 m) {
+  grid_begin();
   const u64 j = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const u32 lane = threadIdx.x & 31;
   if (j >= m) return;  // whole warps leave together
@@ -366,40 +360,44 @@ cudaError_t run_scan(const Prod& prod, u64 total, u64* out, u64 out_limit, Scan&
   // they do (a thread's eight values are a serial chain; more CTAs share them).
   if (tile_begin == 0 && tile_end == tiles && tiles <= kClusterTiles) {
     constexpr int kSmall = 64;
+    const unsigned small = (unsigned)((total + kSmall * kScanE - 1) / (kSmall * kScanE));
     launch_begin(name, st);
     if (total <= kClusterTiles * kSmall * kScanE)
-      e = launch_cluster(scan_cluster_kernel<Prod, kSmall>, (unsigned)((total + kSmall * kScanE - 1) / (kSmall * kScanE)),
-                         kSmall, st, prod, total, out, out_limit, sc.side);
+      e = launch_next(scan_cluster_kernel<Prod, kSmall>, small, kSmall, 0, small, st, prod, total, out, out_limit,
+                      sc.side);
     else
-      e = launch_cluster(scan_cluster_kernel<Prod, kScanThreads>, (unsigned)tiles, kScanThreads, st, prod, total, out,
-                         out_limit, sc.side);
+      e = launch_next(scan_cluster_kernel<Prod, kScanThreads>, (unsigned)tiles, kScanThreads, 0, (unsigned)tiles, st,
+                      prod, total, out, out_limit, sc.side);
     launch_end(st);
     return e;
   }
   if (tiles <= kLookbackTiles) {
     launch_begin(name, st);
-    scan_lookback_kernel<Prod><<<(unsigned)n, kScanThreads, 0, st>>>(prod, total, out, out_limit, sc.side, sc.flags,
-                                                                      sc.counter, sc.err, (u32)tiles);
+    e = launch_next(scan_lookback_kernel<Prod>, (unsigned)n, kScanThreads, 0, 0, st, prod, total, out, out_limit,
+                    sc.side, sc.flags, sc.counter, sc.err, (u32)tiles);
     launch_end(st);
-    return cudaGetLastError();
+    return e;
   }
   launch_begin(name, st);
-  scan_kernel<Prod><<<(unsigned)n, kScanThreads, 0, st>>>(prod, total, out, out_limit, sc.side, sc.wide, tile_begin);
+  e = launch_next(scan_kernel<Prod>, (unsigned)n, kScanThreads, 0, 0, st, prod, total, out, out_limit, sc.side, sc.wide,
+                  tile_begin);
   launch_end(st);
+  if (e != cudaSuccess) return e;
   launch_begin("scan_carry_fix", st);
-  carry_fix_kernel<<<(unsigned)((n + kFixTiles - 1) / kFixTiles), 256, 0, st>>>(sc.wide, tile_begin, tile_end, total, out, out_limit,
-                                                                 sc.side);
+  e = launch_next(carry_fix_kernel, (unsigned)((n + kFixTiles - 1) / kFixTiles), 256, 0, 0, st, sc.wide, tile_begin,
+                  tile_end, total, out, out_limit, sc.side);
   launch_end(st);
-  return cudaGetLastError();
+  return e;
 }
 
 template <u64 TILE>
 cudaError_t launch_school(const ColumnProducer& prod, u64 total, u64* out, Scan& sc, cudaStream_t st) {
   const u32 tiles = (u32)((total + TILE - 1) / TILE);  // at most kLookbackTiles
   launch_begin("school_tiles", st);
-  school_kernel<TILE><<<tiles, 256, 0, st>>>(prod, total, out, sc.flags, sc.counter, sc.err, tiles);
+  const cudaError_t e = launch_next(school_kernel<TILE>, tiles, 256, 0, 0, st, prod, total, out, sc.flags, sc.counter,
+                                    sc.err, tiles);
   launch_end(st);
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace
@@ -452,10 +450,10 @@ cudaError_t ntt_save(const u64* res, int s, u64* out, u64 size, Scan& sc, u64* w
     e = run_scan(CrtProducer{res, L, L}, L + 2, out, L, sc, st, "crt_carry_scan");
     if (e != cudaSuccess) return e;
     launch_begin("wrap_fix", st);
-    wrap_fix_kernel<<<1, 1024, 0, st>>>(out, L, sc.side);
+    e = launch_next(wrap_fix_kernel, 1, 1024, 0, 0, st, out, L, sc.side);
     launch_end(st);
     *written = L;
-    return cudaGetLastError();
+    return e;
   }
   *written = size;
   return run_scan(CrtProducer{res, L, size - 1}, size, out, size, sc, st, "crt_carry_scan");
@@ -468,6 +466,7 @@ struct TwoTo64 {
   u64 w[3], s[3];
 };
 __global__ void __launch_bounds__(256) six_to_three_kernel(const u32* res, u64 L, u64* out, const TwoTo64 b) {
+  grid_begin();
   const u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= L) return;
   const W3 v = SixCrtProducer{res, L, L}(k);
@@ -493,9 +492,9 @@ cudaError_t six_to_three(const u32* res, int s, u64* out, cudaStream_t st) {
   }
   const u64 L = 1ull << s;
   launch_begin("six_to_three", st);
-  six_to_three_kernel<<<(unsigned)((L + 255) / 256), 256, 0, st>>>(res, L, out, b);
+  const cudaError_t e = launch_next(six_to_three_kernel, (unsigned)((L + 255) / 256), 256, 0, 0, st, res, L, out, b);
   launch_end(st);
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t six_save_words(const u32* res, int s, u64* out, u64 size, Scan& sc, u64* written, cudaStream_t st) {
@@ -509,10 +508,10 @@ cudaError_t six_save_words(const u32* res, int s, u64* out, u64 size, Scan& sc, 
   e = run_scan(SixCrtProducer{res, L, L}, L + 2, out, L, sc, st, "six_crt_scan");
   if (e != cudaSuccess) return e;
   launch_begin("wrap_fix", st);
-  wrap_fix_kernel<<<1, 1024, 0, st>>>(out, L, sc.side);
+  e = launch_next(wrap_fix_kernel, 1, 1024, 0, 0, st, out, L, sc.side);
   launch_end(st);
   *written = L;
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t six_save(const SixOperands& op, const SixPlan& pl, u64* out, Scan& sc, cudaStream_t st, int chunks,
@@ -536,9 +535,9 @@ cudaError_t six_save(const SixOperands& op, const SixPlan& pl, u64* out, Scan& s
 cudaError_t add_batch(const AddJob* d_jobs, u64 m, cudaStream_t st) {
   if (m == 0) return cudaSuccess;
   launch_begin("add_batch", st);
-  add_batch_kernel<<<(unsigned)((m * 32 + 255) / 256), 256, 0, st>>>(d_jobs, m);
+  const cudaError_t e = launch_next(add_batch_kernel, (unsigned)((m * 32 + 255) / 256), 256, 0, 0, st, d_jobs, m);
   launch_end(st);
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Scan& sc, cudaStream_t st) {
@@ -550,9 +549,9 @@ cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Sca
     static const cudaError_t ok =  // clusters of more than eight CTAs want asking
         cudaFuncSetAttribute(school_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (ok != cudaSuccess) return ok;
+    const unsigned tiles = (unsigned)((total + kSchoolClusterTile - 1) / kSchoolClusterTile);
     launch_begin("school_tiles", st);
-    e = launch_cluster(school_cluster_kernel, (unsigned)((total + kSchoolClusterTile - 1) / kSchoolClusterTile), 256, st,
-                       prod, total, out);
+    e = launch_next(school_cluster_kernel, tiles, 256, 0, tiles, st, prod, total, out);
     launch_end(st);
     return e;
   }
@@ -583,18 +582,18 @@ cudaError_t shl_bits(u64* out, const u64* in, u64 n, unsigned cl, cudaStream_t s
   }
   const unsigned blocks = (unsigned)std::min<u64>((n + 1 + 255) / 256, 152 * 16);
   launch_begin("shift_bits", st);
-  shl_bits_kernel<<<blocks, 256, 0, st>>>(out, in, n, cl);
+  const cudaError_t e = launch_next(shl_bits_kernel, blocks, 256, 0, 0, st, out, in, n, cl);
   launch_end(st);
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t shr_bits(u64* out, const u64* in, u64 n, unsigned cl, cudaStream_t st) {
   if (cl == 0) return cudaMemcpyAsync(out, in, n * 8, cudaMemcpyDeviceToDevice, st);
   const unsigned blocks = (unsigned)std::min<u64>((n + 255) / 256, 152 * 16);
   launch_begin("shift_bits", st);
-  shr_bits_kernel<<<blocks, 256, 0, st>>>(out, in, n, cl);
+  const cudaError_t e = launch_next(shr_bits_kernel, blocks, 256, 0, 0, st, out, in, n, cl);
   launch_end(st);
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t wait_probe(Scan& sc, int limit, cudaStream_t st) {

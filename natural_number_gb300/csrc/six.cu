@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(256) six_table_kernel(int2* tab, u64 cap, cons
 template <int R>
 __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
     six_load_kernel(SixOperands op, int s, const int2* __restrict__ tab, u64 cap, u32 tile0, int k8) {
+  grid_begin();
   extern __shared__ __align__(16) u32 sm6[];
   const int prime = (int)(blockIdx.x % kPrimes);
   const u32 tile = tile0 + blockIdx.x / kPrimes;
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
 template <int R, bool INV>
 __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
     six_col_kernel(u32* ra, u32* rb, u32 pieces, const SixPlan pl, int lambda0, const int2* __restrict__ tab, u64 cap) {
+  grid_begin();
   extern __shared__ __align__(16) u32 sm6[];
   u32* res = blockIdx.z < pieces ? ra + ((u64)blockIdx.z * kPrimes << pl.s) : rb;
   const bool last = INV && lambda0 == 0;
@@ -138,6 +140,7 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
 template <int R, int LGM, int V, int MODE, bool FIRST, bool PAIR>
 __global__ void __launch_bounds__(fused_threads(R, LGM, V) * (PAIR ? 2 : 1), PAIR ? 1 : fused_blocks(R, LGM, V))
     six_fused_kernel(SixOperands op, u32* out, const SixPlan pl, const int2* __restrict__ tab, u64 cap) {
+  grid_begin();
   extern __shared__ __align__(16) u32 sm6[];
   constexpr int NT = fused_threads(R, LGM, V);
   const u64 piece = ((u64)blockIdx.z * kPrimes) << pl.s, at0 = blockIdx.z * op.piece;
@@ -159,9 +162,9 @@ cudaError_t launch_load(const SixOperands& op, int s, int k8, const SixTables& t
   tile1 = std::min(tile1, tiles);
   const dim3 grid(kPrimes * (tile1 - tile0), op.pieces + (op.b ? 1 : 0));
   launch_begin("six_load_col_pass", st);
-  six_load_kernel<R><<<grid, col_threads(R), smem, st>>>(op, s, t.tab, t.cap, tile0, k8);
+  const cudaError_t e = launch_next(six_load_kernel<R>, grid, col_threads(R), smem, 0, st, op, s, t.tab, t.cap, tile0, k8);
   launch_end(st);
-  return cudaGetLastError();
+  return e;
 }
 template <int R, bool INV>
 cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int lambda0, const SixTables& t,
@@ -173,10 +176,10 @@ cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int lamb
   const u64 tiles = (1ull << pl.s) / ((u64)col_width(R) << R);
   const dim3 grid((unsigned)(lambda0 ? tiles / 8 * pl.k8 : tiles), kPrimes, pieces + (rb ? 1 : 0));
   launch_begin(INV ? (lambda0 == 0 ? "six_inv_last_col_pass" : "six_inv_col_pass") : "six_fwd_col_pass", st);
-  six_col_kernel<R, INV><<<grid, col_threads(R), smem, st>>>(ra, rb, pieces, pl, lambda0,
-                                                              t.tab + (INV ? kPrimes * t.cap : 0), t.cap);
+  const cudaError_t e = launch_next(six_col_kernel<R, INV>, grid, col_threads(R), smem, 0, st, ra, rb, pieces, pl,
+                                    lambda0, t.tab + (INV ? kPrimes * t.cap : 0), t.cap);
   launch_end(st);
-  return cudaGetLastError();
+  return e;
 }
 template <int R, int LGM, int V, int MODE, bool FIRST, bool PAIR = false>
 cudaError_t launch_fused_v(const SixOperands& op, u32* out, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
@@ -186,11 +189,11 @@ cudaError_t launch_fused_v(const SixOperands& op, u32* out, const SixPlan& pl, c
   const u32 tiles = (u32)((1ull << pl.s) >> (R + LGM));
   const dim3 grid(pl.n == 1 ? 1u : tiles / 8 * pl.k8, kPrimes, op.pieces);
   launch_begin(MODE == kForward ? "six_fwd_row_pass" : FIRST ? "six_small_pass" : "six_fused_row_pass", st);
-  six_fused_kernel<R, LGM, V, MODE, FIRST, PAIR>
-      <<<grid, fused_threads(R, LGM, V) * (PAIR ? 2 : 1), MODE == kAll && !op.b ? tile : smem, st>>>(op, out, pl, t.tab,
-                                                                                                     t.cap);
+  const cudaError_t e =
+      launch_next(six_fused_kernel<R, LGM, V, MODE, FIRST, PAIR>, grid, fused_threads(R, LGM, V) * (PAIR ? 2 : 1),
+                  MODE == kAll && !op.b ? tile : smem, 0, st, op, out, pl, t.tab, t.cap);
   launch_end(st);
-  return cudaGetLastError();
+  return e;
 }
 // A few one-pass products: an operand a half of the CTA (six CTAs a piece:
 // up to 96 fill under one wave).  Columns a thread: as few as keep the grid
