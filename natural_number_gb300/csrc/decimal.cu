@@ -5,29 +5,26 @@
 // natural.h:953-967; the last split is div_base by 10^18, natural.h:566-573)
 // and prints each leaf as 18 zero-padded digits (the first one unpadded).
 // The decimal digits of a value are unique, so a node of the tree at any
-// level has exactly one digit string of its width; here one warp takes one
+// level has exactly one digit string of its width; here one CTA takes one
 // node and peels off its 18-digit groups from the low end by repeated exact
 // division by 10^18, which is div_base's step applied 2^(i+1) times.
 //
 // A division's remainder chain runs from the top limb down, one limb after
-// the other.  The warp splits it: lane l takes a segment of the node's limbs
-// and reduces it to the map r -> (r * 2^(64 len) + segment) mod 10^18 (the
-// remainder its segment leaves for a remainder r coming in from above); a
-// scan over the lanes composes these maps from the top, so every lane knows
-// the remainder entering its segment, and the lanes then form their
-// quotient limbs at once.  A division costs two passes over a segment plus
-// five compositions instead of one pass over the whole node.
+// the other, and the next division's chain may follow one limb behind it.  So
+// the CTA's lanes hold the node in segments, the top one in lane 0, and work
+// as a pipeline: at step t lane L takes the remainder of division t - L from
+// the lane above, divides its segment by 10^18 with it and hands its own
+// remainder down.  Each division so costs its limbs' two-by-one divisions and
+// nothing else (dec_groups_kernel).
 //
-// Layout: node k's len[k] limbs at nodes[k], copied into `stride` limbs of
-// shared memory and divided there; its digits go to out[k * width, (k + 1) *
-// width), width = 18 * groups, most significant group first.
+// Layout: node k's len[k] limbs at nodes[k]; its digits go to out[k * width,
+// (k + 1) * width), width = 18 * groups, most significant group first.
 #include <cuda_runtime.h>
 
 #include "nn_device.cuh"
 #include "nn_internal.h"
 
 #include <algorithm>
-#include <atomic>
 
 namespace nn {
 
@@ -77,73 +74,68 @@ __device__ __forceinline__ void put18(char* o, u64 x) {
   for (int t = 0; t < 9; ++t) o2[t] = (unsigned short)(d[2 * t] | (d[2 * t + 1] << 8));
 }
 
-// (a * b) mod 10^18 for a, b < 10^18: the product's high word is below the
-// divisor, as the two-by-one division wants after the shift by kNorm.
-__device__ __forceinline__ u64 mulmod_group(u64 a, u64 b, u64 v) {
-  const u64 lo = a * b, hi = __umul64hi(a, b);
-  u64 r;
-  div_2by1((hi << kNorm) | (lo >> (64 - kNorm)), lo << kNorm, kGroupNorm, v, r);
-  return r >> kNorm;
-}
-
-// 2^(64 j) mod 10^18 for the segment lengths j <= kMaxSegment.
-constexpr int kMaxSegment = 256;
-constexpr int kMaxDevices = 64;
-__constant__ u64 c_limb_pow[kMaxSegment + 1];
-
-// One warp a node; `per_cta` warps a CTA, each with `stride` limbs of shared
-// memory.  A division pass over the current m limbs: segments of
-// ceil(m / 32) limbs, lane l holding limbs [l * seg, (l + 1) * seg).
-__global__ void __launch_bounds__(128) dec_groups_kernel(const u64* const* __restrict__ nodes, u64 stride,
-                                                         const u32* __restrict__ len, u64 n, u32 groups, u64 v,
-                                                         char* out) {
+// One CTA a node, `blockDim.x` lanes; lane L's segment of at most `seg` limbs
+// stands in shared memory from limb L * (seg | 1) on (an odd stride: lanes in
+// different banks).  From lane to lane remainders go by shuffle, from warp to
+// warp through a ring in shared memory that a barrier every kDecStep steps
+// covers: warp w runs 32 + kDecStep steps behind the warp above, so that it
+// reads a remainder at least one barrier after it was written.  The last lane
+// leaves its remainders, the groups, in a ring too; once a barrier the last
+// warp writes kDecStep of them as digits, a lane each.
+//
+// The quotients get shorter from the top: a warp whose limbs and remainders
+// are all zero, and the warp above it for two barriers, leaves its divisions
+// out.
+//
+// What bounds it: the 64-bit multiplies of the two-by-one divisions, and for
+// few nodes their latency (about 70 cycles a limb).
+constexpr int kDecStep = 16, kDecRing = 64, kDecMaxWarps = 16;
+__global__ void __launch_bounds__(32 * kDecMaxWarps) dec_groups_kernel(const u64* const* __restrict__ nodes,
+                                                                       const u32* __restrict__ len, u32 groups, u64 v,
+                                                                       char* out) {
   extern __shared__ u64 node_sm[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const u64 k = (u64)blockIdx.x * (blockDim.x >> 5) + warp;
-  if (k >= n) return;  // a whole warp leaves together
-  u64* a = node_sm + (u64)warp * stride;
-  u32 m = len[k];
-  const u64* w = nodes[k];
-  for (u32 j = lane; j < m; j += 32) a[j] = w[j];
-  __syncwarp();
-  char* o = out + k * (u64)groups * 18;
-  for (u32 g = groups; g-- > 0;) {
-    const u32 seg = (m + 31) / 32;  // at most kMaxSegment: m is below 32 * kMaxSegment
-    const u32 lo = min(lane * seg, m), hi = min(lo + seg, m);
-    // this lane's map r -> A r + B: B = its segment mod 10^18, A = 2^(64 len) mod 10^18
-    u64 rn = 0;
-    for (u32 j = hi; j-- > lo;) {
-      const u64 x = a[j];
-      div_2by1(rn | (x >> (64 - kNorm)), x << kNorm, kGroupNorm, v, rn);
-    }
-    u64 A = c_limb_pow[hi - lo], B = rn >> kNorm;
-    // compose from the top: lane l ends with the map of segments l .. 31
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const u64 A2 = __shfl_down_sync(0xffffffffu, A, d), B2 = __shfl_down_sync(0xffffffffu, B, d);
-      if (lane + d < 32) {
-        B = mulmod_group(A, B2, v) + B;
-        if (B >= kGroup) B -= kGroup;
-        A = mulmod_group(A, A2, v);
+  __shared__ u64 ring[kDecMaxWarps][kDecRing];
+  __shared__ u32 idle[2][kDecMaxWarps];
+  const int L = threadIdx.x, lane = L & 31, w = L >> 5, warps = (int)(blockDim.x >> 5);
+  const u32 m = len[blockIdx.x], lanes = blockDim.x, seg = (m + lanes - 1) / lanes;
+  const u32 hi = m - min(m, L * seg), n = min(hi, seg);  // limbs [hi - n, hi)
+  u64* a = node_sm + (u64)L * (seg | 1);
+  u64 any = 0;
+  for (u32 j = 0; j < n; ++j) {
+    a[j] = nodes[blockIdx.x][hi - 1 - j];  // top limb first
+    any |= a[j];
+  }
+  char* o = out + (u64)blockIdx.x * groups * 18;
+  const int lag = w * (32 + kDecStep) + lane, steps = (int)groups + (warps - 1) * (32 + kDecStep) + 31;
+  u64 rn = 0;            // this lane's last remainder, times 2^kNorm
+  u32 dead = 0;          // barriers since which this warp holds only zeros
+  for (int t0 = 0; t0 < steps; t0 += kDecStep) {
+    for (int t = t0; t < t0 + kDecStep; ++t) {
+      const int g = t - lag;
+      const bool on = g >= 0 && g < (int)groups;
+      u64 r = __shfl_up_sync(0xffffffffu, rn, 1);
+      if (lane == 0) r = w > 0 && on ? ring[w - 1][g % kDecRing] : 0;
+      if (dead == 0 && on) {
+        any = 0;
+        for (u32 j = 0; j < n; ++j) {
+          const u64 x = a[j];
+          const u64 q = div_2by1(r | (x >> (64 - kNorm)), x << kNorm, kGroupNorm, v, r);
+          a[j] = q;
+          any |= q;
+        }
+        rn = r;
       }
+      if (lane == 31 && on) ring[w][g % kDecRing] = rn;
     }
-    const u64 group = __shfl_sync(0xffffffffu, B, 0);  // the remainder of the whole node
-    u64 rin = __shfl_down_sync(0xffffffffu, B, 1);
-    if (lane == 31) rin = 0;
-    // the quotient limbs, every segment at once
-    rn = rin << kNorm;
-    u64 top_q = 1;
-    for (u32 j = hi; j-- > lo;) {
-      const u64 x = a[j];
-      const u64 q = div_2by1(rn | (x >> (64 - kNorm)), x << kNorm, kGroupNorm, v, rn);
-      a[j] = q;
-      if (j == m - 1) top_q = q;
+    const bool zero = __all_sync(0xffffffffu, any == 0 && rn == 0);
+    const int parity = t0 / kDecStep & 1;
+    if (lane == 0) idle[parity][w] = dead;
+    __syncthreads();
+    if (zero && (w == 0 || idle[parity][w - 1] >= 2)) ++dead;
+    if (w == warps - 1 && lane < kDecStep) {
+      const int g = t0 + lane - (warps - 1) * (32 + kDecStep) - 31;
+      if (g >= 0 && g < (int)groups) put18(o + (u64)(groups - 1 - g) * 18, ring[w][g % kDecRing] >> kNorm);
     }
-    // the value loses at most one limb a division (10^18 < 2^64)
-    const bool lost = __any_sync(0xffffffffu, m > 0 && hi == m && hi > lo && top_q == 0);
-    __syncwarp();
-    if (lost) --m;
-    if (lane == 0) put18(o + (u64)g * 18, group);
   }
 }
 
@@ -248,34 +240,19 @@ __global__ void __launch_bounds__(256) dec_inc_kernel(const DecFixJob* __restric
 cudaError_t dec_groups(const u64* const* nodes, u64 stride, const u32* len, u64 n, u32 groups, char* out,
                        cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  if (stride > (u64)32 * kMaxSegment || stride % 2) return cudaErrorInvalidValue;
-  // 2^(64 j) mod 10^18 into the constant bank, once per device (each device
-  // has its own copy of c_limb_pow)
-  static std::atomic<bool> powers[kMaxDevices];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-  if (!powers[dev].load()) {
-    u64 t[kMaxSegment + 1];
-    unsigned __int128 x = 1;
-    for (int j = 0; j <= kMaxSegment; ++j, x = (x << 64) % kGroup) t[j] = (u64)x;
-    e = cudaMemcpyToSymbol(c_limb_pow, t, sizeof t);
-    if (e != cudaSuccess) return e;
-    powers[dev].store(true);
-  }
+  if (stride > 8192 || stride % 2) return cudaErrorInvalidValue;
   const unsigned __int128 all = ~(unsigned __int128)0;
   const u64 v = (u64)(all / kGroupNorm);  // floor((2^128-1)/d) - 2^64: the 2^64 bit drops in the cast
-  // warps a CTA: as many nodes as 48 KiB of shared memory holds, at most four
-  const unsigned per_cta = (unsigned)std::max<u64>(1, std::min<u64>(4, (48 * 1024) / (8 * stride)));
-  const size_t smem = (size_t)per_cta * stride * 8;
-  if (smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(dec_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // four limbs a lane, up to the most warps
+  const u64 warps = std::max<u64>(1, std::min<u64>(kDecMaxWarps, (stride + 127) / 128));
+  const u64 seg = (stride + 32 * warps - 1) / (32 * warps);  // the longest node's; shorter ones take less
+  const int smem = (int)(32 * warps * (seg | 1) * 8);
+  if (smem > 32 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(dec_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
   launch_begin("dec_groups", st);
-  dec_groups_kernel<<<(unsigned)((n + per_cta - 1) / per_cta), 32 * per_cta, smem, st>>>(nodes, stride, len, n, groups,
-                                                                                          v, out);
+  dec_groups_kernel<<<(unsigned)n, (unsigned)(32 * warps), smem, st>>>(nodes, len, groups, v, out);
   launch_end(st);
   return cudaGetLastError();
 }
