@@ -11,21 +11,19 @@
 // carries are one bit each (propagate p_t = u_t is all ones; g_t and p_t are
 // exclusive), resolved by warp ballots inside a tile.
 //
-// Between tiles the per-call scans of more than kLookbackTiles tiles take two
-// launches and never wait:
+// Between tiles the per-call scans take two launches and never wait:
 //  1. every tile runs with carry-in 0, writes its limbs and records its
 //     one-bit generate and propagate (no tile waits for another);
 //  2. each CTA takes the carry into its range of tiles from the nearest tile
 //     before it that does not propagate, resolves the carries inside its range
 //     with ballots, and adds a tile's carry-in of 1 at its first limb, where
 //     it ripples only while limbs wrap to zero.
-// Smaller per-call scans, the persistent batch kernel and the
-// allocation-free entry point take the decoupled lookback instead (scan_tile
-// with LOOKBACK: one launch, each tile's carry-in from its predecessors'
-// status words), whose waits are bounded and record an error instead of
-// hanging.  A per-call lookback leaves its status words and counters zero for
-// the next scan: the CTA that finishes last clears them, so a scan is one
-// launch with nothing to reset before it.
+// The shortest are one cluster, whose CTAs exchange their bits.  Base-case
+// products and the allocation-free entry point take the decoupled lookback
+// instead (scan_tile with kScanLookback: one launch, each tile's carry-in from
+// its predecessors' status words), whose waits are bounded and record an error
+// instead of hanging.  A per-call lookback leaves its status words and counters
+// zero for the next: the CTA that finishes last clears them.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -41,11 +39,9 @@ NN_DEFINE_PRIME_UPLOADER(upload_primes_carry)
 
 namespace {
 
-// Scans of at most kLookbackTiles tiles take one launch: tile ids come from
-// an atomic counter, so every predecessor of a tile has started before it,
-// and each tile takes its carry-in by the decoupled lookback.  Their tiles fit
-// in one or two waves, so a lookback waits about one tile's work; larger
-// scans never wait.
+// Base-case products of at most kLookbackTiles tiles take one launch: tile ids
+// come from an atomic counter, so every predecessor of a tile has started
+// before it, and each tile takes its carry-in by the decoupled lookback.
 constexpr u64 kLookbackTiles = 1024;
 
 // The next tile of the scan, for every thread.
@@ -70,37 +66,31 @@ __device__ __forceinline__ void finish_tile(u32* flags, u32* counter, u32 tiles)
   if (threadIdx.x < 2) counter[threadIdx.x] = 0;
 }
 
-template <class Prod>
-__global__ void __launch_bounds__(kScanThreads, 3) scan_lookback_kernel(Prod prod, u64 total, u64* out, u64 out_limit,
-                                                                     u64* side, u32* flags, u32* counter, u32* err,
-                                                                     u32 tiles) {
-  grid_begin();
-  scan_tile(prod, next_tile(counter), total, out, out_limit, side, flags, err);
-  finish_tile(flags, counter, tiles);
-}
-
 // Step 1: tile tile_base + blockIdx.x with carry-in 0; flags[tile] receives
 // its generate (bit 0) and propagate (bit 1) bits.
-template <class Prod>
-__global__ void __launch_bounds__(kScanThreads, 3) scan_kernel(Prod prod, u64 total, u64* out, u64 out_limit,
-                                                            u64* side, u32* flags, u64 tile_base) {
+template <class Prod, int NT>
+__global__ void __launch_bounds__(NT, 768 / NT) scan_kernel(Prod prod, u64 total, u64* out, u64 out_limit, u64* side,
+                                                            u32* flags, u64 tile_base) {
   grid_begin();
-  scan_tile<Prod, kScanRecord>(prod, tile_base + blockIdx.x, total, out, out_limit, side, flags, nullptr);
+  scan_tile<Prod, kScanRecord, NT>(prod, tile_base + blockIdx.x, total, out, out_limit, side, flags, nullptr);
 }
 
 // Step 2: 32 tiles a CTA.  The carry into the range is the generate bit of the
 // nearest earlier tile that does not propagate (0 when all do): the CTA looks
 // 256 tiles further back at a time, for random limbs once.  Earlier ranges of
 // the same scan are complete (stream order).  One ballot gives every tile of
-// the range its carry-in: lane t of warp 0 adds tile t's at its first limb,
-// where it ripples while limbs wrap to zero; a tile that propagates holds
-// ones only and becomes zeros, by the whole CTA (a difference of nearly equal
-// operands has long runs of such tiles).
+// the range its carry-in: lane t of warp 0 adds tile t's at its first limb.
+// Where that limb wraps to zero, a warp carries on, 32 limbs a step (a product
+// next to a power of 2^64, as a reciprocal's with its operand, starts tiles
+// with up to 2047 limbs of all ones: one lane's walk took 14 us a launch); a tile that
+// propagates holds ones only and becomes zeros, by the whole CTA (a difference
+// of nearly equal operands has long runs of such tiles).
 constexpr int kFixTiles = 32;
+template <u64 TILE>
 __global__ void __launch_bounds__(256) carry_fix_kernel(const u32* flags, u64 t0, u64 t1, u64 total, u64* out,
                                                         u64 out_limit, u64* side) {
   grid_begin();
-  __shared__ u32 s_first, s_cin, s_ones;
+  __shared__ u32 s_first, s_cin, s_ones, s_wrapped;
   const u64 c0 = t0 + (u64)blockIdx.x * kFixTiles;
   const int tid = threadIdx.x;
   u32 cin = 0;
@@ -127,17 +117,29 @@ __global__ void __launch_bounds__(256) carry_fix_kernel(const u32* flags, u64 t0
     const u32 G = __ballot_sync(0xffffffffu, f & 1), GP = __ballot_sync(0xffffffffu, f & 3);
     const u32 in = (u32)((u64)G + GP + cin) ^ G ^ GP;  // the carry into each lane's tile
     const u32 ones = in & GP & ~G;
-    if (tid == 0) s_ones = ones;
-    if (t < t1 && (((in & ~ones) >> tid) & 1)) {
-      const u64 end = min((t + 1) * kScanTile, total);
-      for (u64 k = t * kScanTile; k < end; ++k)
-        if (++*limb(k) != 0) break;
+    const bool add = t < t1 && (((in & ~ones) >> tid) & 1);
+    const u32 wrapped = __ballot_sync(0xffffffffu, add && ++*limb(t * TILE) == 0);
+    if (tid == 0) {
+      s_ones = ones;
+      s_wrapped = wrapped;
     }
   }
   __syncthreads();
+  const u32 lane = tid & 31;
+  for (u32 left = s_wrapped, i = 0; left; left &= left - 1, ++i) {  // a warp a tile
+    if (i % 8 != (u32)tid / 32) continue;
+    const u64 t = c0 + __ffs(left) - 1, end = min((t + 1) * TILE, total);
+    for (u64 k = t * TILE + 1; k < end; k += 32) {
+      const u64 x = k + lane < end ? *limb(k + lane) : 0;
+      const u32 below = __ballot_sync(0xffffffffu, x != ~0ull);
+      const u32 first = below ? __ffs(below) - 1 : 32;
+      if (lane <= first && k + lane < end) *limb(k + lane) = lane < first ? 0 : x + 1;
+      if (first < 32) break;
+    }
+  }
   for (u32 ones = s_ones; ones; ones &= ones - 1) {
-    const u64 t = c0 + __ffs(ones) - 1, end = min((t + 1) * kScanTile, total);
-    for (u64 k = t * kScanTile + tid; k < end; k += 256) *limb(k) = 0;
+    const u64 t = c0 + __ffs(ones) - 1, end = min((t + 1) * TILE, total);
+    for (u64 k = t * TILE + tid; k < end; k += 256) *limb(k) = 0;
   }
 }
 
@@ -203,14 +205,23 @@ __global__ void wait_probe_kernel(const u32* flag, u32* err, int limit) {
   if (threadIdx.x == 0 && wait_flag(flag, limit) == 0) atomicExch(err, 1u);
 }
 
-// Scans of at most eight tiles: one cluster (kScanCluster).
-template <class Prod, int NT>
-__global__ void __launch_bounds__(NT) scan_cluster_kernel(Prod prod, u64 total, u64* out, u64 out_limit, u64* side) {
+// Scans of up to 2^17 positions run in tiles of 512, so that more SMs share
+// them (a thread's eight values are a serial chain): products of 2^16
+// coefficients 18.9 us, 19.3 in tiles of 2048, of 2^17 24.4 and 24.7, of 2^18
+// 29.9 and 29.3.  Up to eight such tiles are one cluster (kScanCluster): 9.6 us
+// for 1500 x 1201 limbs, 10.2 in two launches; sixteen, 15.9 and 15.4 us.  In one launch
+// with the lookback, 2^16 coefficients took 21.0 us, 2^18 33.3, 2^21 178
+// instead of 167.5 (sums alike: a division
+// of 2800007 by 1400003 limbs 2.50 ms with its sums so, 2.40 without).
+constexpr int kScanSmall = 64;  // threads
+constexpr u64 kClusterTiles = 8, kSmallTiles = 256;
+template <class Prod>
+__global__ void __launch_bounds__(kScanSmall) scan_cluster_kernel(Prod prod, u64 total, u64* out, u64 out_limit,
+                                                                  u64* side) {
   grid_begin();
-  scan_tile<Prod, kScanCluster, NT>(prod, blockIdx.x, total, out, out_limit, side, nullptr, nullptr);
+  scan_tile<Prod, kScanCluster, kScanSmall>(prod, blockIdx.x, total, out, out_limit, side, nullptr, nullptr);
   cluster_sync();
 }
-constexpr u64 kClusterTiles = 8;
 
 // acc += x * y as one carry chain.
 __device__ __forceinline__ void mac(W3& acc, u64 x, u64 y) {
@@ -344,7 +355,6 @@ __global__ void __launch_bounds__(256) add_batch_kernel(const AddJob* __restrict
     }
   }
 }
-
 // Tiles [tile_begin, tile_end) of the scan (all of them by default).  The
 // ranges of one scan go in order on one stream (each range's carry-in comes
 // from the words of the tiles before it).
@@ -355,37 +365,34 @@ cudaError_t run_scan(const Prod& prod, u64 total, u64* out, u64 out_limit, Scan&
   tile_end = std::min(tile_end, tiles);
   cudaError_t e = scan_reserve(sc, tiles);
   if (e != cudaSuccess || tile_end <= tile_begin) return e;
-  const u64 n = tile_end - tile_begin;
-  // A whole scan of at most eight tiles: one cluster, of smaller tiles while
-  // they do (a thread's eight values are a serial chain; more CTAs share them).
-  if (tile_begin == 0 && tile_end == tiles && tiles <= kClusterTiles) {
-    constexpr int kSmall = 64;
-    const unsigned small = (unsigned)((total + kSmall * kScanE - 1) / (kSmall * kScanE));
+  const bool whole = tile_begin == 0 && tile_end == tiles;
+  constexpr u64 kSmallTile = kScanSmall * kScanE;
+  const u64 small = (total + kSmallTile - 1) / kSmallTile;
+  if (whole && small <= kClusterTiles) {
     launch_begin(name, st);
-    if (total <= kClusterTiles * kSmall * kScanE)
-      e = launch_next(scan_cluster_kernel<Prod, kSmall>, small, kSmall, 0, small, st, prod, total, out, out_limit,
-                      sc.side);
-    else
-      e = launch_next(scan_cluster_kernel<Prod, kScanThreads>, (unsigned)tiles, kScanThreads, 0, (unsigned)tiles, st,
-                      prod, total, out, out_limit, sc.side);
+    e = launch_next(scan_cluster_kernel<Prod>, (unsigned)small, kScanSmall, 0, (unsigned)small, st, prod, total, out,
+                    out_limit, sc.side);
     launch_end(st);
     return e;
   }
-  if (tiles <= kLookbackTiles) {
-    launch_begin(name, st);
-    e = launch_next(scan_lookback_kernel<Prod>, (unsigned)n, kScanThreads, 0, 0, st, prod, total, out, out_limit,
-                    sc.side, sc.flags, sc.counter, sc.err, (u32)tiles);
-    launch_end(st);
-    return e;
-  }
+  const bool short_tiles = whole && small <= kSmallTiles;
+  const u64 n = short_tiles ? small : tile_end - tile_begin;
   launch_begin(name, st);
-  e = launch_next(scan_kernel<Prod>, (unsigned)n, kScanThreads, 0, 0, st, prod, total, out, out_limit, sc.side, sc.wide,
-                  tile_begin);
+  if (short_tiles)
+    e = launch_next(scan_kernel<Prod, kScanSmall>, (unsigned)n, kScanSmall, 0, 0, st, prod, total, out, out_limit,
+                    sc.side, sc.wide, 0);
+  else
+    e = launch_next(scan_kernel<Prod, kScanThreads>, (unsigned)n, kScanThreads, 0, 0, st, prod, total, out, out_limit,
+                    sc.side, sc.wide, tile_begin);
   launch_end(st);
   if (e != cudaSuccess) return e;
   launch_begin("scan_carry_fix", st);
-  e = launch_next(carry_fix_kernel, (unsigned)((n + kFixTiles - 1) / kFixTiles), 256, 0, 0, st, sc.wide, tile_begin,
-                  tile_end, total, out, out_limit, sc.side);
+  const unsigned ranges = (unsigned)((n + kFixTiles - 1) / kFixTiles);
+  if (short_tiles)
+    e = launch_next(carry_fix_kernel<kSmallTile>, ranges, 256, 0, 0, st, sc.wide, 0, n, total, out, out_limit, sc.side);
+  else
+    e = launch_next(carry_fix_kernel<kScanTile>, ranges, 256, 0, 0, st, sc.wide, tile_begin, tile_end, total, out,
+                    out_limit, sc.side);
   launch_end(st);
   return e;
 }
@@ -409,8 +416,7 @@ cudaError_t scan_reserve(Scan& sc, u64 tiles) {
   if (sc.flags) cudaFree(sc.flags);  // waits for the device: no scan is using it
   u64 cap = sc.max_tiles ? sc.max_tiles : kLookbackTiles;
   while (cap < tiles) cap *= 2;
-  // the lookback's status words (only scans of up to kLookbackTiles tiles use
-  // them), then the carry bits of longer scans
+  // the lookback's status words, then the carry bits of the other scans
   cudaError_t e = cudaMalloc((void**)&sc.flags, (kLookbackTiles + 1 + cap) * sizeof(u32));
   if (e == cudaSuccess) e = cudaMemset(sc.flags, 0, (kLookbackTiles + 1) * sizeof(u32));
   if (e != cudaSuccess) {
