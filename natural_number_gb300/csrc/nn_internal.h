@@ -183,7 +183,7 @@ struct AddJob {
   u64 nout;
   u64 sub = 0;
 };
-cudaError_t add_batch(const AddJob* d_jobs, u64 m, cudaStream_t st);
+cudaError_t add_batch(const AddJob* d_jobs, u64 m, u64 longest, cudaStream_t st);
 
 // Forward transform: limbs (n <= 2^s) -> residues [3][2^s] equal to
 // NTT_info::load + NTT (ntt_info.h:147-198) modulo each prime; lazy values in

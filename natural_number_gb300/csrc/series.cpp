@@ -331,8 +331,10 @@ constexpr u64 kWarpAddLimbs = 1 << 15;
 void device_adds(nn_context* c, const std::vector<nn::AddJob>& jobs) {
   cudaStream_t st = (cudaStream_t)nn_context_stream(c);
   std::vector<nn::AddJob> small;
+  u64 longest = 0;
   for (const nn::AddJob& j : jobs) {
     if (j.nout <= kWarpAddLimbs) {
+      longest = std::max(longest, j.nout);
       small.push_back(j);
       continue;
     }
@@ -347,7 +349,7 @@ void device_adds(nn_context* c, const std::vector<nn::AddJob>& jobs) {
   const u64 w = (small.size() * sizeof(nn::AddJob) + 7) / 8;
   tab.reserve(w);
   check_cuda(nn::ctx_upload(c, tab.p, small.data(), small.size() * sizeof(nn::AddJob)), "sum table");
-  check_cuda(nn::add_batch(reinterpret_cast<const nn::AddJob*>(tab.p), small.size(), st), "tree sums");
+  check_cuda(nn::add_batch(reinterpret_cast<const nn::AddJob*>(tab.p), small.size(), longest, st), "tree sums");
 }
 
 // One level's products as one batch on device pointers; the plan is released
