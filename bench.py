@@ -1,5 +1,5 @@
 #!/usr/bin/env python3
-"""Benchmark: bit-exact 2^27 x 2^27-limb three-prime NTT multiply on GB300.
+"""Benchmark: bit-exact 2^27 x 2^27-limb NTT multiply on GB300.
 
 One step = one full product of two 2^27-limb operands (1 GiB each, uniform u64
 limbs from SplitMix64 seeds, top limb nonzero) through the library's nn_mul:
@@ -43,13 +43,13 @@ SEED_A, SEED_B = 1000 + (1 << N_EXP), 7777 + (1 << N_EXP)
 FALLBACK_HBM_GBS = 6800.0
 
 # Algorithmic bytes per launch of each kernel for a product of na x nb limbs
-# at transform length L (three primes, 8-byte residues):
-#   load+first pass reads the limbs once per prime and writes residues,
+# at transform length L (six primes, 4-byte residues):
+#   load+first pass reads the limbs once and writes residues,
 #   a strided/contiguous pass reads and writes every residue once,
-#   pointwise reads two transforms and writes one, the CRT scan reads the
+#   the fused pass reads two transforms and writes one, the CRT scan reads the
 #   residues and writes the product limbs.
 def kernel_bytes(name: str, na: int, nb: int, L: int) -> float:
-    """Bytes a launch must move once (six 4-byte residues a coefficient; the
+    """Bytes a launch must move once (24 bytes of residues a coefficient; the
     forward passes of both operands share a launch)."""
     if name == "six_load_col_pass":
         return 8.0 * (na + nb) + 48.0 * L
@@ -65,9 +65,10 @@ def kernel_bytes(name: str, na: int, nb: int, L: int) -> float:
 
 
 def mul_algorithmic_bytes(na: int, nb: int, L: int) -> float:
-    """16(na+nb) + 192 L: two load+column passes, two row passes (one fused
-    with the pointwise product and the inverse row pass), the inverse column
-    pass fused with CRT and carry."""
+    """16(na+nb) + 192 L, the yardstick of a product at 24 bytes a residue in
+    two passes: two load+column passes, two row passes (one fused with the
+    pointwise product and the inverse row pass), the inverse column pass fused
+    with CRT and carry."""
     return 16.0 * (na + nb) + 192.0 * L
 
 
@@ -164,7 +165,7 @@ def measure_batched(ctx, steps: int, warmup: int, count: int = 4096) -> dict:
     """Uneven-size batch: `count` products with operand lengths drawn
     independently log-uniform in [2^6, 2^18] limbs, once one nn_mul per
     product (the unbatched path, run from a C loop) and once as one planned
-    batch (persistent work-queue launch replayed from a CUDA graph); both on
+    batch (launches by step and tile shape, replayed from a CUDA graph); both on
     the same device-resident operands, timed with CUDA events, results compared."""
     import torch
 
@@ -646,7 +647,7 @@ def main() -> None:
         iach = inst / (d_avg / 1e3)
         line["issue_roofline"] = {"bound": "int_issue", "kernel": dname, "achieved": iach, "peak": ipeak,
                                   "unit": "warp inst/s", "frac": iach / ipeak, "inst_per_launch": inst,
-                                  "source": "profiles/instructions.txt (ncu on a smaller transform, scaled by L); "
+                                  "source": "profiles/instructions.txt (ncu, scaled by L); "
                                             "peak 4 per SM per cycle"}
 
     def e2e():

@@ -112,7 +112,7 @@ nn_status nn_divmod_host(nn_context* ctx, uint64_t* q, uint64_t* r, const uint64
 nn_status nn_mul_base(nn_context* ctx, uint64_t* d_out, const uint64_t* d_a, uint64_t n_a, const uint64_t* d_b,
                       uint64_t n_b);
 
-/* ---- batches: many products in one persistent launch -------------------- */
+/* ---- batches: many products in a handful of launches --------------------- */
 /* One product of a batch (device pointers; d_out holds n_a + n_b limbs, not
  * normalised).  d_a == d_b with n_a == n_b is a square (one transform). */
 typedef struct {
@@ -126,12 +126,12 @@ typedef struct nn_batch nn_batch;
 /* Plans a batch for these operand sizes (the reference has no batch API;
  * each job is natural::_mul, natural.h:444-450): jobs whose shorter operand
  * is below the "batch_ntt_min" tunable run as schoolbook column scans, the
- * others (but balanced ones below "batch_school_balanced") as three-prime
- * NTT products at scale ceil(log2(n_a+n_b-1)).  All
- * pipelines go into one work queue drained by one persistent launch; the
- * launch sequence is captured in a CUDA graph on first run and replayed.
+ * others (but balanced ones below "batch_school_balanced") as NTT products
+ * at scale ceil(log2(n_a+n_b-1)), unbalanced ones in pieces where that is
+ * estimated faster.  A launch takes one step of all jobs at one tile shape;
+ * the launch sequence is captured in a CUDA graph on first run and replayed.
  * Products at the "batch_solo_scale" tunable's scale and up run one at a
- * time after that launch, as nn_mul (nn_sqr for squares) would.
+ * time after those launches, as nn_mul (nn_sqr for squares) would.
  * square[j] (optional) marks squares. */
 nn_status nn_batch_create(nn_context* ctx, const uint64_t* n_a, const uint64_t* n_b, const int* square,
                           uint64_t count, nn_batch** out);
@@ -156,7 +156,8 @@ nn_status nn_batch_mul(nn_context* ctx, const nn_mul_job* jobs, uint64_t count);
  * "batch_ntt_min" (default 384), "batch_school_balanced" (default 256: a
  * product whose longer operand is at most twice its shorter also takes the
  * schoolbook route while the shorter is below this; 0 = off),
- * "batch_blocks_per_sm" (0 = occupancy limit),
+ * "batch_blocks_per_sm" (0..32; kept for callers that set it, a CTA takes one
+ * item),
  * "batch_item_words" (residues per prime a batch pass item covers at least,
  * in consecutive tiles; default 8192), "batch_fused" (1, the default: a
  * batched transform of two passes or more runs both operands' last forward
@@ -167,8 +168,8 @@ nn_status nn_batch_mul(nn_context* ctx, const nn_mul_job* jobs, uint64_t count);
  * transform sharing the shorter operand's, when that is estimated faster;
  * 0: one transform per product), "batch_solo_scale" (default 22: a batched
  * product whose transform has this scale or more runs on its own through the
- * one-product passes, after the batch kernel and before the run's completion;
- * 0: every product in the batch kernel; runs that overlap on different
+ * one-product passes, after the batch's launches and before the run's completion;
+ * 0: every product in the batch's launches; runs that overlap on different
  * streams of one context need 0, since those passes share the context's
  * carry-scan scratch, as nn_mul calls on two streams do). */
 nn_status nn_context_set_tunable(nn_context* ctx, const char* name, int64_t value);

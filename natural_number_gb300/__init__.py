@@ -378,8 +378,8 @@ class Context:
 
 
 class Batch:
-    """nn_batch: a planned batch of products (one persistent launch per run,
-    replayed from a CUDA graph)."""
+    """nn_batch: a planned batch of products (a launch a step and tile
+    shape, replayed from a CUDA graph)."""
 
     def __init__(self, ctx: Context, sizes_a, sizes_b, square=None):
         self.ctx = ctx

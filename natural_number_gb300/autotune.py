@@ -3,11 +3,11 @@
 Sweeps, on the GPU it runs on:
   - the NTT pass split: levels of the contiguous pass ("r_last") and the most
     levels of a strided column pass ("r_col"), timed on one product per
-    scale (these passes serve nn_ntt_mul and the cached transforms); and the
+    scale (the three-prime passes, which serve nn_ntt_mul); and the
     levels of the contiguous pass of batched products ("batch_r_last@s");
-  - the batch shapes: persistent CTAs per SM ("batch_blocks_per_sm") and the
-    shortest operand sent down the NTT route in a batch ("batch_ntt_min"),
-    timed on the uneven-size workload.
+  - the batch shapes: the shortest operand sent down the NTT route in a batch
+    ("batch_ntt_min") and the residues a pass item covers
+    ("batch_item_words"), timed on the uneven-size workload.
 Every candidate's product is checked against the first candidate's (all
 choices compute the same exact product).  Writes the best values to
 tuning.json beside this file; Context() applies that file at creation
@@ -124,8 +124,8 @@ def tune_batch_scales(ctx, scales) -> tuple[dict, dict]:
 
 
 def tune_batch(ctx, jobs: int) -> tuple[dict, dict]:
-    """CTAs per SM, the shortest operand sent down the NTT route, and the
-    residues per pass item, on an uneven workload of `jobs` products; every
+    """The shortest operand sent down the NTT route and the residues per pass
+    item, on an uneven workload of `jobs` products; every
     setting must give the same products."""
     import torch
 
@@ -133,27 +133,24 @@ def tune_batch(ctx, jobs: int) -> tuple[dict, dict]:
     W = UnevenProducts(jobs, seed=5)
     results = {}
     ref = None
-    for per_sm in (5, 6):
-        for ntt_min in (48, 64, 96, 128):
-            for item in (8192, 16384, 32768):
-                ctx.set_tunable("batch_blocks_per_sm", per_sm)
-                ctx.set_tunable("batch_ntt_min", ntt_min)
-                ctx.set_tunable("batch_item_words", item)
-                plan = ctx.batch(W.sa, W.sb)
-                ms = _time(lambda: plan.run_jobs(W.jobs_batch), 3)
-                ctx.synchronize()
-                if ref is None:
-                    ref = W.out_batch.clone()
-                elif not torch.equal(ref, W.out_batch):
-                    raise RuntimeError(f"per_sm={per_sm} ntt_min={ntt_min} item={item} changed a product")
-                plan.close()
-                results[f"{per_sm},{ntt_min},{item}"] = ms
+    for ntt_min in (48, 64, 96, 128):
+        for item in (8192, 16384, 32768):
+            ctx.set_tunable("batch_ntt_min", ntt_min)
+            ctx.set_tunable("batch_item_words", item)
+            plan = ctx.batch(W.sa, W.sb)
+            ms = _time(lambda: plan.run_jobs(W.jobs_batch), 3)
+            ctx.synchronize()
+            if ref is None:
+                ref = W.out_batch.clone()
+            elif not torch.equal(ref, W.out_batch):
+                raise RuntimeError(f"ntt_min={ntt_min} item={item} changed a product")
+            plan.close()
+            results[f"{ntt_min},{item}"] = ms
     best = min(results, key=results.get)
-    per_sm, ntt_min, item = map(int, best.split(","))
-    ctx.set_tunable("batch_blocks_per_sm", per_sm)
+    ntt_min, item = map(int, best.split(","))
     ctx.set_tunable("batch_ntt_min", ntt_min)
     ctx.set_tunable("batch_item_words", item)
-    return ({"batch_blocks_per_sm": per_sm, "batch_ntt_min": ntt_min, "batch_item_words": item},
+    return ({"batch_ntt_min": ntt_min, "batch_item_words": item},
             {"batch_%d_ms" % jobs: results})
 
 

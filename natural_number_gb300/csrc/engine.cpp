@@ -13,7 +13,6 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <numeric>
 #include <string>
 #include <unordered_map>
 #include <unordered_set>

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(256, 4) ntt_pass_kernel(const u64* in, u64* ou
   extern __shared__ u64 sm[];
   const int prime = FIRST ? (int)(blockIdx.x % 3) : (int)blockIdx.y;
   const u64 tile = FIRST ? blockIdx.x / 3 : blockIdx.x;
-  pass_tile<C, FIRST, INV, SCALE, false>(sm, in, out, n_in, s, lambda0, R, tab, tab_stride, prime, tile);
+  pass_tile<C, FIRST, INV, SCALE>(sm, in, out, n_in, s, lambda0, R, tab, tab_stride, prime, tile);
 }
 
 // Contiguous last pass: forward levels, pointwise by `other` (nullptr
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(256, BLOCKS) ntt_fused_kernel(u64* res, const 
                                                              const u64* __restrict__ itab, u64 tab_stride) {
   extern __shared__ u64 sm[];
   // three CTAs an SM leave 80 registers a thread: room for radix-16 groups
-  pass_tile<2, false, false, false, false, true, BLOCKS == 3 ? 4 : 3>(sm, res, res, 0, s, lambda0, R, tab, tab_stride,
+  pass_tile<2, false, false, false, true, BLOCKS == 3 ? 4 : 3>(sm, res, res, 0, s, lambda0, R, tab, tab_stride,
                                                                      blockIdx.y, blockIdx.x, itab, other);
 }
 
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256) pointwise_kernel(u64* dst, const u64* a, 
                                                         const u64* __restrict__ tab, u64 tab_stride) {
   const u64 g = (u64)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= L / 4) return;
-  pointwise_group<false>(dst, a, b, L, tab, tab_stride, blockIdx.y, g);
+  pointwise_group(dst, a, b, L, tab, tab_stride, blockIdx.y, g);
 }
 
 // Strided pass over residues with TMA: one CTA's tile (16 columns x 2^R
@@ -169,15 +169,15 @@ __device__ __forceinline__ void col_tile_tma(u64* sm, u64* bar, const CUtensorMa
   mbar_wait(bar, 0);  // completed phase: this thread sees the copied tile
   bool scaled = false;  // the compile-time schedules scale in their last register group
   if (!INV)
-    tile_forward_any<C, PR, true, MAXK, false>(sm, R, ksb, tw, nullptr, 0);
+    tile_forward_any<C, PR, MAXK, false>(sm, R, ksb, tw, nullptr, 0);
   else
-    scaled = tile_inverse_any<C, PR, true, MAXK, false, SCALE>(sm, R, ksb, tw, nullptr, 0, (u32)(s - 1));
+    scaled = tile_inverse_any<C, PR, MAXK, false, SCALE>(sm, R, ksb, tw, nullptr, 0, (u32)(s - 1));
   if (SCALE && !scaled) {
     for (u32 idx = 2 * threadIdx.x; idx < nel; idx += 2 * blockDim.x) {
-      ulonglong2 v = ld2<false>(sm + idx);
+      ulonglong2 v = ld2(sm + idx);
       v.x = div_pow2(canon_c<PR>(v.x), (u32)(s - 1), p);
       v.y = div_pow2(canon_c<PR>(v.y), (u32)(s - 1), p);
-      st2<false>(sm + idx, v);
+      st2(sm + idx, v);
     }
   }
   fence_async_smem();
@@ -220,7 +220,7 @@ __device__ __forceinline__ void load_tile_tma(u64* sm, const CUtensorMap* tm, co
   const bool half = n_in <= (1ull << (s - 1));
   load_limbs_tile<C, PR, false>(sm, in, n_in, base, lg_s, half ? nel / 2 : nel, half);
   __syncthreads();
-  tile_forward_any<C, PR, true, 3, false>(sm, R, 0, tw, nullptr, half ? 1 : 0);
+  tile_forward_any<C, PR, 3, false>(sm, R, 0, tw, nullptr, half ? 1 : 0);
   fence_async_smem();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -302,7 +302,7 @@ __device__ __forceinline__ void row_tile_bulk(u64* sm, u64* bar, u64* res, const
     bulk_load(tws + 2 * ((1u << j) - 1), tw + 2 * (ksb << j), 16u << j, bar);
   if (!tile_arrived(bar, 0, err, &s_ok)) return;
   if (!INV) {
-    tile_forward_any<C, PR, true, MAXK>(sm, R, ksb, tw, tws, 0);
+    tile_forward_any<C, PR, MAXK>(sm, R, ksb, tw, tws, 0);
     if (FUSED) {
       const ulonglong2* twsv = reinterpret_cast<const ulonglong2*>(tws);
       const u64* oth = other ? other + ((u64)PR << s) + (ksb << (R + 1)) : nullptr;
@@ -314,8 +314,8 @@ __device__ __forceinline__ void row_tile_bulk(u64* sm, u64* bar, u64* res, const
         if (g4 < nel) {
           pw[k] = twsv[deep + (g4 >> 2)];
           if (oth) {
-            A01[k] = ld2<false>(oth + g4);
-            A23[k] = ld2<false>(oth + g4 + 2);
+            A01[k] = ld2(oth + g4);
+            A23[k] = ld2(oth + g4 + 2);
           }
         }
       }
@@ -339,10 +339,10 @@ __device__ __forceinline__ void row_tile_bulk(u64* sm, u64* bar, u64* res, const
         }
       }
       if (!tile_arrived(bar, 1, err, &s_ok)) return;  // its barrier also orders the products before the levels
-      tile_inverse_any<C, PR, true, MAXK>(sm, R, ksb, itw, tws, 0);
+      tile_inverse_any<C, PR, MAXK>(sm, R, ksb, itw, tws, 0);
     }
   } else {
-    tile_inverse_any<C, PR, true, MAXK>(sm, R, ksb, tw, tws, 0);
+    tile_inverse_any<C, PR, MAXK>(sm, R, ksb, tw, tws, 0);
   }
   fence_async_smem();
   __syncthreads();

@@ -1,6 +1,5 @@
-// ntt_tiles.cuh — tile-level device code of the NTT passes and the pointwise
-// product, shared by the per-call kernels (ntt.cu) and the persistent batch
-// kernel (batch.cu).  See ntt.cu for the level/pass decomposition.
+// ntt_tiles.cuh — tile-level device code of the three-prime NTT passes and the
+// pointwise product (ntt.cu, which has the level/pass decomposition).
 //
 // Every routine is specialised per prime (template PR), so the modulus and
 // its reduction constants are immediates.  In-tile indices are 32-bit.  The
@@ -76,20 +75,8 @@ __device__ __forceinline__ u64 canon_c(u64 x) {
 // spread over the banks.
 __device__ __forceinline__ u32 pad16(u32 x) { return x + ((x >> 5) << 1); }
 
-template <bool CG>
-__device__ __forceinline__ ulonglong2 ld2(const u64* p) {
-  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p);
-  if (CG) return __ldcg(q);
-  return *q;
-}
-template <bool CG>
-__device__ __forceinline__ void st2(u64* p, ulonglong2 v) {
-  ulonglong2* q = reinterpret_cast<ulonglong2*>(p);
-  if (CG)
-    __stcg(q, v);
-  else
-    *q = v;
-}
+__device__ __forceinline__ ulonglong2 ld2(const u64* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+__device__ __forceinline__ void st2(u64* p, ulonglong2 v) { *reinterpret_cast<ulonglong2*>(p) = v; }
 
 // 16-byte asynchronous global -> shared copies (L2 only, as .cg loads), so a
 // thread's loads of a tile are all in flight before any of them is waited on.
@@ -275,14 +262,13 @@ __device__ __forceinline__ void tile_inverse_ct(u64* sm, u64 ksb, const u64* tw,
 // Forward levels [l0, R) / inverse levels R-1 .. l_stop: the compile-time
 // schedules for the tile shapes of the large transforms' pass plans (strided
 // passes of 7-9 levels, contiguous passes of 10-11), the runtime loop
-// otherwise.  Only the per-call kernels take them (CT); the batch kernel
-// keeps one code path per width.
-template <int C, int PR, bool CT, int MAXK = 3, bool PAD = true>
+// otherwise.
+template <int C, int PR, int MAXK = 3, bool PAD = true>
 __device__ __forceinline__ void tile_forward_any(u64* sm, int R, u64 ksb, const u64* tw, const u64* tws, int l0) {
-  if constexpr (CT && C == 2) {
+  if constexpr (C == 2) {
     if (R == 11 && l0 == 0) return tile_forward_ct<C, PR, 11, 0, MAXK, PAD>(sm, ksb, tw, tws);
     if (R == 10 && l0 == 0) return tile_forward_ct<C, PR, 10, 0, 3, PAD>(sm, ksb, tw, tws);
-  } else if constexpr (CT && C == 16) {
+  } else if constexpr (C == 16) {
     if (R == 8 && l0 == 0) return tile_forward_ct<C, PR, 8, 0, MAXK, PAD>(sm, ksb, tw, tws);
     if (R == 8 && l0 == 1) return tile_forward_ct<C, PR, 8, 1, 3, PAD>(sm, ksb, tw, tws);
     if (R == 9 && l0 == 0) return tile_forward_ct<C, PR, 9, 0, 3, PAD>(sm, ksb, tw, tws);
@@ -295,13 +281,13 @@ __device__ __forceinline__ void tile_forward_any(u64* sm, int R, u64 ksb, const 
 // SC: a compile-time schedule also applies the scale 2^-sc_sh in its last
 // group; returns whether it did (the runtime loop leaves the scale to the
 // caller).
-template <int C, int PR, bool CT, int MAXK = 3, bool PAD = true, bool SC = false>
+template <int C, int PR, int MAXK = 3, bool PAD = true, bool SC = false>
 __device__ __forceinline__ bool tile_inverse_any(u64* sm, int R, u64 ksb, const u64* tw, const u64* tws, int l_stop,
                                                  u32 sc_sh = 0) {
-  if constexpr (CT && C == 2) {
+  if constexpr (C == 2) {
     if (R == 11 && l_stop == 0) return tile_inverse_ct<C, PR, 11, 0, MAXK, PAD, SC>(sm, ksb, tw, tws, sc_sh), SC;
     if (R == 10 && l_stop == 0) return tile_inverse_ct<C, PR, 10, 0, 3, PAD, SC>(sm, ksb, tw, tws, sc_sh), SC;
-  } else if constexpr (CT && C == 16) {
+  } else if constexpr (C == 16) {
     if (R == 8 && l_stop == 0) return tile_inverse_ct<C, PR, 8, 0, MAXK, PAD, SC>(sm, ksb, tw, tws, sc_sh), SC;
     if (R == 9 && l_stop == 0) return tile_inverse_ct<C, PR, 9, 0, 3, PAD, SC>(sm, ksb, tw, tws, sc_sh), SC;
     if (R == 7 && l_stop == 0) return tile_inverse_ct<C, PR, 7, 0, 3, PAD, SC>(sm, ksb, tw, tws, sc_sh), SC;
@@ -387,13 +373,10 @@ __device__ __forceinline__ void load_limbs_tile(u64* sm, const u64* in, u64 n_in
 // FUSED (contiguous passes only): after the forward levels, multiply
 // pointwise by the other operand's residues `other` and run the inverse
 // levels before writing back.
-// skip: the first `skip` local levels are not run (already done by the pass
-// before).  A contiguous tile of R levels with skip = w is 2^w consecutive
-// tiles of R - w levels, so small tiles can be worked on together.
-template <int C, bool FIRST, bool INV, bool SCALE, bool CG, bool FUSED, int PR, int MAXK = 3>
+template <int C, bool FIRST, bool INV, bool SCALE, bool FUSED, int PR, int MAXK = 3>
 __device__ __forceinline__ void pass_tile_p(u64* sm, const u64* in, u64* out, u64 n_in, int s, int lambda0, int R,
                                             const u64* __restrict__ tab, const u64* __restrict__ itab, u64 tab_stride,
-                                            u64 tile, const u64* other, int skip) {
+                                            u64 tile, const u64* other) {
   constexpr u64 p = PrimeC<PR>::p;
   const u64 L = 1ull << s;
   const u64* tw = tab + (u64)PR * tab_stride;
@@ -402,8 +385,8 @@ __device__ __forceinline__ void pass_tile_p(u64* sm, const u64* in, u64* out, u6
   const u64 ksb = tile / tiles_per_sb;
   const u64 base = (ksb << (lg_s + R)) + (tile % tiles_per_sb) * C;
   const u32 nel = (u32)C << R;
-  static_assert(C == 2 || C == 16 || C == 32 || C == 64 || C == 128, "tile widths");
-  constexpr int LGC = C == 2 ? 1 : C == 16 ? 4 : C == 32 ? 5 : C == 64 ? 6 : 7;
+  static_assert(C == 2 || C == 16, "tile widths");
+  constexpr int LGC = C == 2 ? 1 : 4;
 
   // With every limb in the lower half of the transform (n_in <= L/2), level 0
   // pairs each limb with a zero: both outputs are the limb's residue, written
@@ -424,7 +407,7 @@ __device__ __forceinline__ void pass_tile_p(u64* sm, const u64* in, u64* out, u6
   __syncthreads();
 
   if (!INV) {
-    tile_forward_any<C, PR, !CG, MAXK>(sm, R, ksb, tw, tws, half ? 1 : skip);
+    tile_forward_any<C, PR, MAXK>(sm, R, ksb, tw, tws, half ? 1 : 0);
     if (FUSED) {  // contiguous tile: smem index == position - base; other == nullptr squares
       const u64* oth = other ? other + (u64)PR * L : nullptr;
       const ulonglong2* twsv = reinterpret_cast<const ulonglong2*>(tws);
@@ -433,7 +416,7 @@ __device__ __forceinline__ void pass_tile_p(u64* sm, const u64* in, u64* out, u6
         const u64 Bv[4] = {sm[pad16(g4)], sm[pad16(g4 + 1)], sm[pad16(g4 + 2)], sm[pad16(g4 + 3)]};
         u64 A[4] = {Bv[0], Bv[1], Bv[2], Bv[3]};
         if (oth) {
-          const ulonglong2 A0 = ld2<CG>(oth + base + g4), A1 = ld2<CG>(oth + base + g4 + 2);
+          const ulonglong2 A0 = ld2(oth + base + g4), A1 = ld2(oth + base + g4 + 2);
           A[0] = A0.x;
           A[1] = A0.y;
           A[2] = A1.x;
@@ -449,10 +432,10 @@ __device__ __forceinline__ void pass_tile_p(u64* sm, const u64* in, u64* out, u6
       stage_twiddles(tws, itw, ksb, R);
       cp_async_wait_all();
       __syncthreads();
-      tile_inverse_any<C, PR, !CG, MAXK>(sm, R, ksb, itw, tws, skip);
+      tile_inverse_any<C, PR, MAXK>(sm, R, ksb, itw, tws, 0);
     }
   } else {
-    tile_inverse_any<C, PR, !CG>(sm, R, ksb, tw, tws, skip);
+    tile_inverse_any<C, PR>(sm, R, ksb, tw, tws, 0);
   }
 
   u64* dst = out + (u64)PR * L;
@@ -463,36 +446,34 @@ __device__ __forceinline__ void pass_tile_p(u64* sm, const u64* in, u64* out, u6
       v.x = div_pow2(canon_c<PR>(v.x), (u32)(s - 1), p);
       v.y = div_pow2(canon_c<PR>(v.y), (u32)(s - 1), p);
     }
-    st2<CG>(dst + pos, v);
+    st2(dst + pos, v);
   }
 }
 
 // MAXK: the largest register group (levels) the compile-time schedules may
 // use; 4 only where the kernel has the registers for 16 residues a thread.
-template <int C, bool FIRST, bool INV, bool SCALE, bool CG, bool FUSED = false, int MAXK = 3>
+template <int C, bool FIRST, bool INV, bool SCALE, bool FUSED = false, int MAXK = 3>
 __device__ __forceinline__ void pass_tile(u64* sm, const u64* in, u64* out, u64 n_in, int s, int lambda0, int R,
                                           const u64* __restrict__ tab, u64 tab_stride, int prime, u64 tile,
-                                          const u64* __restrict__ itab = nullptr, const u64* other = nullptr,
-                                          int skip = 0) {
+                                          const u64* __restrict__ itab = nullptr, const u64* other = nullptr) {
   if (prime == 0)
-    pass_tile_p<C, FIRST, INV, SCALE, CG, FUSED, 0, MAXK>(sm, in, out, n_in, s, lambda0, R, tab, itab, tab_stride,
-                                                         tile, other, skip);
+    pass_tile_p<C, FIRST, INV, SCALE, FUSED, 0, MAXK>(sm, in, out, n_in, s, lambda0, R, tab, itab, tab_stride,
+                                                         tile, other);
   else if (prime == 1)
-    pass_tile_p<C, FIRST, INV, SCALE, CG, FUSED, 1, MAXK>(sm, in, out, n_in, s, lambda0, R, tab, itab, tab_stride,
-                                                         tile, other, skip);
+    pass_tile_p<C, FIRST, INV, SCALE, FUSED, 1, MAXK>(sm, in, out, n_in, s, lambda0, R, tab, itab, tab_stride,
+                                                         tile, other);
   else
-    pass_tile_p<C, FIRST, INV, SCALE, CG, FUSED, 2, MAXK>(sm, in, out, n_in, s, lambda0, R, tab, itab, tab_stride,
-                                                         tile, other, skip);
+    pass_tile_p<C, FIRST, INV, SCALE, FUSED, 2, MAXK>(sm, in, out, n_in, s, lambda0, R, tab, itab, tab_stride,
+                                                         tile, other);
 }
 
 // Pointwise product of one group g (4 residues) of prime i.
-template <bool CG>
 __device__ __forceinline__ void pointwise_group(u64* dst, const u64* a, const u64* b, u64 L,
                                                 const u64* __restrict__ tab, u64 tab_stride, int i, u64 g) {
   const ulonglong2 wv = __ldg(reinterpret_cast<const ulonglong2*>(tab + (u64)i * tab_stride) + g);
   const u64 off = (u64)i * L + 4 * g;
-  const ulonglong2 A0 = ld2<CG>(a + off), A1 = ld2<CG>(a + off + 2);
-  const ulonglong2 B0 = ld2<CG>(b + off), B1 = ld2<CG>(b + off + 2);
+  const ulonglong2 A0 = ld2(a + off), A1 = ld2(a + off + 2);
+  const ulonglong2 B0 = ld2(b + off), B1 = ld2(b + off + 2);
   const u64 A[4] = {A0.x, A0.y, A1.x, A1.y}, Bv[4] = {B0.x, B0.y, B1.x, B1.y};
   u64 o[4];
   if (i == 0)
@@ -501,8 +482,8 @@ __device__ __forceinline__ void pointwise_group(u64* dst, const u64* a, const u6
     pointwise4<1>(o, A, Bv, wv);
   else
     pointwise4<2>(o, A, Bv, wv);
-  st2<CG>(dst + off, make_ulonglong2(o[0], o[1]));
-  st2<CG>(dst + off + 2, make_ulonglong2(o[2], o[3]));
+  st2(dst + off, make_ulonglong2(o[0], o[1]));
+  st2(dst + off + 2, make_ulonglong2(o[2], o[3]));
 }
 
 }  // namespace nn

@@ -1,7 +1,6 @@
-// scan_tiles.cuh — tile-level device code of the multiword carry scan
-// (decoupled lookback) and its value producers, shared by the per-call kernels
-// (carry.cu) and the persistent batch kernel (batch.cu).  See carry.cu for the
-// scheme.
+// scan_tiles.cuh — tile-level device code of the multiword carry scan and its
+// value producers, shared by the per-call kernels (carry.cu) and the batches'
+// (batch.cu).  See carry.cu for the scheme.
 #pragma once
 
 #include "nn_device.cuh"
@@ -52,25 +51,14 @@ __device__ __forceinline__ u64 add_ripple8(u64 (&y)[8], u64 a0, u64 a1) {
 
 // Garner: x = r0 + p0*u + p0*p1*v with u = (r1-r0)/p0 mod p1 and
 // v = ((r2-r0)/p0 - u)/p1 mod p2; residues in [0,p) after the inverse.
-template <bool CG>
-struct CrtProducerT {
+struct CrtProducer {
   const u64* res;
   u64 L;
   u64 count;
   static constexpr bool kBulk = true;
   __device__ __forceinline__ W3 operator()(u64 k) const {
     if (k >= count) return W3{0, 0, 0};
-    u64 x0, x1, x2;
-    if (CG) {
-      x0 = __ldcg(res + k);
-      x1 = __ldcg(res + L + k);
-      x2 = __ldcg(res + 2 * L + k);
-    } else {
-      x0 = res[k];
-      x1 = res[L + k];
-      x2 = res[2 * L + k];
-    }
-    return garner(x0, x1, x2);
+    return garner(res[k], res[L + k], res[2 * L + k]);
   }
   // Eight consecutive positions from k0 (a multiple of 8) with 16-byte loads.
   __device__ __forceinline__ void bulk(u64 k0, W3 (&x)[kScanE]) const {
@@ -84,8 +72,7 @@ struct CrtProducerT {
     for (int i = 0; i < 3; ++i)
 #pragma unroll
       for (int e = 0; e < kScanE; e += 2) {
-        const ulonglong2* q = reinterpret_cast<const ulonglong2*>(res + (u64)i * L + k0 + e);
-        const ulonglong2 v = CG ? __ldcg(q) : *q;
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(res + (u64)i * L + k0 + e);
         r[i][e] = v.x;
         r[i][e + 1] = v.y;
       }
@@ -115,9 +102,6 @@ struct CrtProducerT {
     return r;
   }
 };
-
-typedef CrtProducerT<false> CrtProducer;
-
 
 // CRT of the six-prime residues (six_tiles.cuh), which the last inverse pass
 // leaves multiplied by (M/p_i)^-1: with t_i any representative in (0, 4p), the

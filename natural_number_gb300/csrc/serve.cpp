@@ -3,8 +3,8 @@
 // Clients submit multiply and divide requests on host memory.  A scheduler
 // thread admits requests in arrival order while their estimated device
 // footprint fits the HBM budget; every pass of its loop uploads the newly
-// admitted products' operands and launches them as one batch (nn_batch_launch,
-// the persistent work-queue kernel) on the next of several streams, so a batch
+// admitted products' operands and launches them as one batch (nn_batch_launch)
+// on the next of several streams, so a batch
 // formed from later arrivals runs while earlier batches are still on the
 // device.  Completed batches are found through events; their results are
 // copied back, their memory and budget released, and more requests admitted.

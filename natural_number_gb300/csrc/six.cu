@@ -279,7 +279,7 @@ SixPlan six_plan(int s, u64 length, int row_levels) {
   // The contiguous tile as long as the strided passes keep four levels (two
   // passes: batched products of 2^14 limbs 0.084 ns a limb with 9 levels there,
   // 0.126 with 6) or six (three passes: 2^24 x 2^24 limbs 2.80 ms with 6 + 7 +
-  // 9 levels, 2.86 with 7 + 7 + 8; at 2^21 7 levels and 9 read 378 and 394 us).
+  // 9 levels, 2.86 with 7 + 7 + 8; at 2^21 7 levels and 9 read 348 and 355 us).
   int row = T;
   if (pl.n == 2) row = std::min(9, T - 4);
   if (pl.n == 3) row = pl.lgm > 3 ? row_max : std::min(9, T - 12);

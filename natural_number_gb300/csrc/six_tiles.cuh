@@ -1,5 +1,5 @@
 // six_tiles.cuh — tile-level device code of the six-prime 32-bit NTT, shared
-// by the per-call kernels (six.cu) and the persistent batch kernel (batch.cu).
+// by the per-call kernels (six.cu) and the batches' (batch.cu).
 //
 // A product of limbs is a convolution of 64-bit digits whose coefficients
 // stay below min(n_a, n_b) * 2^128.  It is computed modulo six primes
