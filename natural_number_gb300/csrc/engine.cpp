@@ -523,6 +523,35 @@ int six_split(u64 nx, u64 ny, int s, u64* k, u64* P) {
   return s_best;
 }
 
+// Whether na x nb limbs (na >= nb) run as the base case.  Both ways give the
+// same limbs; with a product's launches 1.3 us apart the transforms win well
+// below the reference's 384 limbs.  Measured, transforms / base case, us: 224 x
+// 224 6.1 / 5.6, 256 x 256 6.4 / 6.8, 383 x 383 6.5 / 8.1; beyond the one
+// cluster of 1024 positions 1024 x 96 7.0 / 7.1, 2048 x 192 7.4 / 9.5, 2048 x 64
+// 6.8 / 6.7; long operands 16384 x 32 9.0 / 10.6, 2^20 x 32 58.8 / 81.1, 2^20 x
+// 300 70 / 743, but 2^20 x 16 74.3 / 44.7.
+bool base_case(u64 na, u64 nb) {
+  return !(nb >= 256 || (nb >= 96 && na + nb > 1024) || (nb >= 32 && na >= 16384));
+}
+
+// A product of fewer than kNttMulThreshold limbs needs no memory as the base
+// case: it takes that where the transforms' would not fit the budget or, while
+// the stream is captured, their tables are not there yet.
+nn_status short_product(nn_context* c, u64* d_out, const nn::SixOperands& op, int s) {
+  bool base = false;
+  if (!nn::six_tables_cover(c->six, s)) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    base = cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
+  }
+  if (!base) {
+    const nn_status st = six_product(c, d_out, op, s);
+    if (st != NN_ERR_BUDGET && st != NN_ERR_OOM) return st;
+  }
+  const u64* b = op.b ? op.b : op.a;
+  NN_CK(c, nn::school_mul(op.a, op.na, b, op.nb, d_out, c->scan, c->stream), "base-case product");
+  return NN_OK;
+}
+
 nn_status mul_impl(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b, u64 nb) {
   if (!d_out || !a || !b || na == 0 || nb == 0) {
     c->err = "mul: null pointer or empty operand";
@@ -532,7 +561,7 @@ nn_status mul_impl(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b
     std::swap(a, b);
     std::swap(na, nb);
   }
-  if (nb < kNttMulThreshold) {  // natural.h:445-446 -> _mul_base
+  if (base_case(na, nb)) {  // natural.h:445-446 -> _mul_base
     NN_CK(c, nn::school_mul(a, na, b, nb, d_out, c->scan, c->stream), "base-case product");
     return NN_OK;
   }
@@ -541,7 +570,8 @@ nn_status mul_impl(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b
   u64 piece, pieces;
   const int s = six_split(na, nb, ntt_scale(na, nb), &piece, &pieces);
   if (s > nn::kSixMaxScale) return ntt_product(c, d_out, a, na, b, nb, s, na + nb, nullptr);
-  return six_product(c, d_out, nn::SixOperands{a, na, piece, (nn::u32)pieces, b, nb, nullptr, nullptr}, s);
+  const nn::SixOperands op{a, na, piece, (nn::u32)pieces, b, nb, nullptr, nullptr};
+  return nb < kNttMulThreshold ? short_product(c, d_out, op, s) : six_product(c, d_out, op, s);
 }
 
 nn_status sqr_impl(nn_context* c, u64* d_out, const u64* a, u64 n) {
@@ -549,14 +579,15 @@ nn_status sqr_impl(nn_context* c, u64* d_out, const u64* a, u64 n) {
     c->err = "sqr: null pointer or empty operand";
     return NN_ERR_INVALID;
   }
-  if (n < kNttMulThreshold) {  // natural.h:530-531 -> _sqr_base
+  if (base_case(n, n)) {  // natural.h:530-531 -> _sqr_base
     NN_CK(c, nn::school_mul(a, n, a, n, d_out, c->scan, c->stream), "base-case square");
     return NN_OK;
   }
   // natural::_sqr_NTT (natural.h:433-442): one transform.
   const int s = ntt_scale(n, n);
   if (s > nn::kSixMaxScale) return ntt_product(c, d_out, a, n, a, n, s, 2 * n, nullptr);
-  return six_product(c, d_out, nn::SixOperands{a, n, n, 1, nullptr, n, nullptr, nullptr}, s);
+  const nn::SixOperands op{a, n, n, 1, nullptr, n, nullptr, nullptr};
+  return n < kNttMulThreshold ? short_product(c, d_out, op, s) : six_product(c, d_out, op, s);
 }
 
 // Grow-only device staging buffer `slot` of at least `words` limbs.
