@@ -86,7 +86,7 @@ nn_status nn_transform_inverse_save(nn_context* ctx, nn_transform* t, uint64_t* 
 nn_status nn_transform_residues(nn_context* ctx, const nn_transform* t, uint64_t* d_out);
 
 /* ---- products on device pointers ---------------------------------------- */
-/* natural::_mul (natural.h:444-450): base case below 384 limbs, NTT above,
+/* natural::_mul (natural.h:444-450): base case for short operands, NTT else,
  * with the unbalanced split of natural.h:391-419.  d_out: n_a + n_b limbs. */
 nn_status nn_mul(nn_context* ctx, uint64_t* d_out, const uint64_t* d_a, uint64_t n_a, const uint64_t* d_b,
                  uint64_t n_b);

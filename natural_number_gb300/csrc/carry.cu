@@ -82,9 +82,9 @@ __global__ void __launch_bounds__(NT, 768 / NT) scan_kernel(Prod prod, u64 total
 // the range its carry-in: lane t of warp 0 adds tile t's at its first limb.
 // Where that limb wraps to zero, a warp carries on, 32 limbs a step (a product
 // next to a power of 2^64, as a reciprocal's with its operand, starts tiles
-// with up to 2047 limbs of all ones: one lane's walk took 14 us a launch); a tile that
-// propagates holds ones only and becomes zeros, by the whole CTA (a difference
-// of nearly equal operands has long runs of such tiles).
+// with up to 2047 limbs of all ones: one lane's walk took 14 us a launch, 8 so);
+// a tile that propagates holds ones only and becomes zeros, by the whole CTA (a
+// difference of nearly equal operands has long runs of such tiles).
 constexpr int kFixTiles = 32;
 template <u64 TILE>
 __global__ void __launch_bounds__(256) carry_fix_kernel(const u32* flags, u64 t0, u64 t1, u64 total, u64* out,
@@ -209,10 +209,10 @@ __global__ void wait_probe_kernel(const u32* flag, u32* err, int limit) {
 // them (a thread's eight values are a serial chain): products of 2^16
 // coefficients 18.9 us, 19.3 in tiles of 2048, of 2^17 24.4 and 24.7, of 2^18
 // 29.9 and 29.3.  Up to eight such tiles are one cluster (kScanCluster): 9.6 us
-// for 1500 x 1201 limbs, 10.2 in two launches; sixteen, 15.9 and 15.4 us.  In one launch
-// with the lookback, 2^16 coefficients took 21.0 us, 2^18 33.3, 2^21 178
-// instead of 167.5 (sums alike: a division
-// of 2800007 by 1400003 limbs 2.50 ms with its sums so, 2.40 without).
+// for 1500 x 1201 limbs, 10.2 in two launches; sixteen, 15.9 and 15.4 us.  In
+// one launch with the lookback, 2^16 coefficients took 21.0 us, 2^18 33.3, 2^21
+// 178 instead of 167.5 (sums alike: a division of 2800007 by 1400003 limbs 2.50
+// ms with its sums so, 2.40 without).
 constexpr int kScanSmall = 64;  // threads
 constexpr u64 kClusterTiles = 8, kSmallTiles = 256;
 template <class Prod>

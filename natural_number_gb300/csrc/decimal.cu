@@ -87,8 +87,10 @@ __device__ __forceinline__ void put18(char* o, u64 x) {
 // are all zero, and the warp above it for two barriers, leaves its divisions
 // out.
 //
-// What bounds it: the 64-bit multiplies of the two-by-one divisions, and for
-// few nodes their latency (about 70 cycles a limb).
+// What bounds it: the 64-bit multiplies of the two-by-one divisions, about 300
+// cycles a limb and step with three warps a scheduler.  420 nodes of 480 limbs
+// (512 groups each): 0.45 ms; with one warp a node, every division split over
+// its lanes by a scan of remainder maps, 1.2 ms.
 constexpr int kDecStep = 16, kDecRing = 64, kDecMaxWarps = 16;
 __global__ void __launch_bounds__(32 * kDecMaxWarps) dec_groups_kernel(const u64* const* __restrict__ nodes,
                                                                        const u32* __restrict__ len, u32 groups, u64 v,

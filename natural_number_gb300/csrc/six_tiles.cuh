@@ -693,7 +693,7 @@ __device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const Root
           mid[i + j] += (i64)(x[i] + x[i + 4]) * (y[j] + y[j + 4]);
         }
     }
-    __syncthreads();  // the blocks of this round have been read
+    __syncthreads();  // these blocks have been read
     if (on) {
       i64 t[15];
       i32 o[8];
