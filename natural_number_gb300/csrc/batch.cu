@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(256) batch_carry_kernel(const BatchJob* __rest
   }
 }
 
-__global__ void __launch_bounds__(kBatchSumThreads, 6)
+__global__ void __launch_bounds__(kBatchSumThreads, 3)
     batch_columns_kernel(const BatchJob* __restrict__ jobs, const BatchItem* __restrict__ items, u32* ticket,
                          u32* flags, u32* err) {
   __shared__ u64 sums[3 * (kBatchSumTile + kScanE)];
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kBatchSumThreads, 6)
   column_tile_sums<kBatchSumThreads, kBatchSumTile>(sums, ColumnProducer{J.a, J.na, J.b, J.nb}, it.tile);
   __syncthreads();
   typedef SmemSumsProducer<kBatchSumTile> Prod;
-  scan_tile<Prod, kScanLookback, kBatchSumThreads>(Prod{sums, (u64)it.tile * kBatchSumTile - kScanE, size}, it.tile, size, J.out,
+  scan_tile<Prod, kScanLookback, kBatchSumThreads, kBatchSumTile>(Prod{sums, (u64)it.tile * kBatchSumTile - kScanE, size}, it.tile, size, J.out,
                                           size, nullptr, flags + J.flag_base, err);
 }
 

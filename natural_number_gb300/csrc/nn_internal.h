@@ -130,8 +130,11 @@ constexpr u64 kScanTile = (u64)kScanThreads * kScanE;
 // A pass item covers consecutive tiles worth about kBatchItemWords residues,
 // so a CTA's fixed cost (its item and job) stays small beside its work.
 constexpr u64 kBatchItemWords = 8192;
-constexpr int kBatchSumThreads = 128;  // base-case items: 1024 positions
-constexpr u64 kBatchSumTile = (u64)kBatchSumThreads * kScanE;
+// Base-case items: 256 positions by 256 threads.  With 1024 positions by 128
+// threads one item's column sums took 40 us, the whole of a small batch's time:
+// 64 jobs of 8 to 1024 limbs 62 us, 37 so.
+constexpr int kBatchSumThreads = 256;
+constexpr u64 kBatchSumTile = 256;
 struct BatchJob {
   const u64* a;  // NTT jobs: the longer operand (split into pieces)
   const u64* b;
