@@ -288,24 +288,6 @@ nn_status forward(nn_context* c, nn_transform* t, const u64* d_limbs, u64 n, int
   return NN_OK;
 }
 
-// A six-prime transform's product residues: its own, or for a forward
-// transform those of its product with 1 (one limb), in `tmp`.
-nn_status six_product_words(nn_context* c, const nn_transform* t, DBuf& tmp, const nn::u32** words) {
-  *words = t->six();
-  if (t->rep == nn_transform::kSixProduct) return NN_OK;
-  const u64 n = 3ull << t->scale;
-  nn_status st = tmp.alloc(n + 1);
-  if (st != NN_OK) return st;
-  const u64 one = 1;
-  NN_CK(c, c->stage.upload(tmp.p + n, &one, sizeof one, c->stream), "constant");
-  const nn::SixPlan pl = nn::six_plan(t->scale, 1ull << t->scale);
-  nn::u32* w = reinterpret_cast<nn::u32*>(tmp.p);
-  NN_CK(c, nn::six_forward(tmp.p + n, 1, w, pl, c->six, c->stream), "forward NTT");
-  NN_CK(c, nn::six_pointwise(w, t->six(), w, pl, c->six, c->stream), "inverse NTT");
-  *words = w;
-  return NN_OK;
-}
-
 // t's residues modulo the three primes, as the reference's transform has
 // them, into dst: a six-prime transform's coefficients, reduced, through the
 // three-prime forward passes.
@@ -316,25 +298,32 @@ nn_status three_words(nn_context* c, const nn_transform* t, u64* dst) {
     return NN_OK;
   }
   DBuf tmp(c);
-  const nn::u32* w = nullptr;
-  nn_status st = six_product_words(c, t, tmp, &w);
-  if (st != NN_OK) return st;
+  const nn::u32* w = t->six();
+  if (t->rep == nn_transform::kSixForward) {
+    nn_status st = tmp.alloc(3ull << t->scale);
+    if (st != NN_OK) return st;
+    nn::u32* back = reinterpret_cast<nn::u32*>(tmp.p);
+    NN_CK(c, nn::six_inverse(back, w, nn::six_inverse_plan(t->scale), c->six, c->stream), "inverse NTT");
+    w = back;
+  }
   NN_CK(c, nn::tables_ensure(c->tables, t->scale, c->stream, &c->retired_tables), "twiddle tables");
   NN_CK(c, nn::six_to_three(w, t->scale, dst, c->stream), "residues");
   NN_CK(c, nn::ntt_forward_residues(dst, t->scale, c->tables, c->stream, c->passes(t->scale)), "forward NTT");
   return NN_OK;
 }
 
+// A forward transform goes back in place: only kernels on the stream, as a
+// captured graph wants them, and no memory beyond the transform's own.
 nn_status inverse_save(nn_context* c, nn_transform* t, u64* d_out, u64 size, u64* written) {
   nn_status st = save_args(c, size);
   if (st != NN_OK) return st;
   if (t->rep == nn_transform::kThree) return inverse_save3(c, t, d_out, size, written);
-  DBuf tmp(c);
-  const nn::u32* w = nullptr;
-  st = six_product_words(c, t, tmp, &w);
-  if (st != NN_OK) return st;
+  if (t->rep == nn_transform::kSixForward) {
+    NN_CK(c, nn::six_inverse(t->six(), t->six(), nn::six_inverse_plan(t->scale), c->six, c->stream), "inverse NTT");
+    t->rep = nn_transform::kSixProduct;
+  }
   u64 n = 0;
-  NN_CK(c, nn::six_save_words(w, t->scale, d_out, size, c->scan, &n, c->stream), "CRT/carry");
+  NN_CK(c, nn::six_save_words(t->six(), t->scale, d_out, size, c->scan, &n, c->stream), "CRT/carry");
   if (written) *written = n;
   return NN_OK;
 }

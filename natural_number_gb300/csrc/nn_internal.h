@@ -81,6 +81,8 @@ struct SixPlan {
 // length: coefficients of the product.  row_levels: levels of the last pass of a two-pass transform, where it can
 // have that many (0: as even as possible).
 SixPlan six_plan(int s, u64 length, int row_levels = 0);
+// The plan that takes one operand's finished transform back by itself.
+SixPlan six_inverse_plan(int s);
 
 // Operands of a product: a in `pieces` pieces of `piece` limbs (one piece of
 // na limbs: not split), residues ra [pieces][6][2^s]; b (nullptr: a square),
@@ -113,6 +115,8 @@ inline bool six_ready(const SixOperands& op, const SixPlan& pl) {
 // the CRT.
 cudaError_t six_forward(const u64* limbs, u64 n, u32* res, const SixPlan& pl, const SixTables& t, cudaStream_t st);
 cudaError_t six_pointwise(u32* dst, const u32* a, const u32* b, const SixPlan& pl, const SixTables& t, cudaStream_t st);
+// A finished transform (dst may be it) back to the residues of its operand for the CRT; pl: six_inverse_plan's.
+cudaError_t six_inverse(u32* dst, const u32* a, const SixPlan& pl, const SixTables& t, cudaStream_t st);
 // Scratch for the carry scan.
 struct Scan {
   u32* flags = nullptr;  // per-tile status words of a lookback, zero between scans (the last tile clears them)

@@ -67,11 +67,11 @@ Factors make_factors() {
   return F;
 }
 
-// 2^(96 - t) / (M / p_i) modulo each prime, by t.
+// 2^(32 steps - t) / (M / p_i) modulo each prime, by t.
 struct ScaleTable {
   int2 f[kRootLog + 2][kPrimes];
 };
-ScaleTable make_scales() {
+ScaleTable make_scales(int steps) {
   ScaleTable S;
   for (int i = 0; i < kPrimes; ++i) {
     const u64 p = prime_of(i);
@@ -80,7 +80,7 @@ ScaleTable make_scales() {
       if (j != i) m = m * (prime_of(j) % p) % p;
     const u64 inv = h_pow(m, p - 2, p);
     for (int t = 0; t < kRootLog + 2; ++t) {
-      const i32 w = h_center(h_pow(2, 96 - t, p) * inv % p, p);
+      const i32 w = h_center(h_pow(2, 32 * steps - t, p) * inv % p, p);
       S.f[t][i] = make_int2(w, h_companion(w, p));
     }
   }
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(col_threads(R), col_blocks(R))
 }
 
 // op.ra's pieces (or, FIRST, the limbs op.a) with op.rb (op.b), into `out`;
-// mode kForward: op.ra alone.
+// modes kForward and kInverse: op.ra alone.
 template <int R, int LGM, int V, int MODE, bool FIRST, bool PAIR>
 __global__ void __launch_bounds__(fused_threads(R, LGM, V) * (PAIR ? 2 : 1), PAIR ? 1 : fused_blocks(R, LGM, V))
     six_fused_kernel(SixOperands op, u32* out, const SixPlan pl, const int2* __restrict__ tab, u64 cap) {
@@ -188,7 +188,7 @@ cudaError_t launch_fused_v(const SixOperands& op, u32* out, const SixPlan& pl, c
   if (ok != cudaSuccess) return ok;
   const u32 tiles = (u32)((1ull << pl.s) >> (R + LGM));
   const dim3 grid(pl.n == 1 ? 1u : tiles / 8 * pl.k8, kPrimes, op.pieces);
-  launch_begin(MODE == kForward ? "six_fwd_row_pass" : FIRST ? "six_small_pass" : "six_fused_row_pass", st);
+  launch_begin(MODE == kForward ? "six_fwd_row_pass" : MODE == kInverse ? "six_inv_row_pass" : FIRST ? "six_small_pass" : "six_fused_row_pass", st);
   const cudaError_t e =
       launch_next(six_fused_kernel<R, LGM, V, MODE, FIRST, PAIR>, grid, fused_threads(R, LGM, V) * (PAIR ? 2 : 1),
                   MODE == kAll && !op.b ? tile : smem, 0, st, op, out, pl, t.tab, t.cap);
@@ -249,7 +249,7 @@ cudaError_t fused_pass(const SixOperands& op, u32* out, const SixPlan& pl, const
       case 9: return launch_fused<4, 9, MODE, false>(op, out, pl, t, st);
     }
   }
-  if constexpr (FIRST || MODE == kProduct) {
+  if constexpr (FIRST || MODE == kProduct || MODE == kInverse) {
     switch (R) {
       case 1: return launch_fused<1, 3, MODE, FIRST>(op, out, pl, t, st);
       case 2: return launch_fused<2, 3, MODE, FIRST>(op, out, pl, t, st);
@@ -295,8 +295,16 @@ SixPlan six_plan(int s, u64 length, int row_levels) {
   // The product residues are the coefficients times 2^T (the inverse's sums;
   // 2^(T+1) of a truncated transform) and 2^-96 (the Montgomery steps of the
   // two operands' limbs and of the blocks' products).
-  static const ScaleTable scales = make_scales();
+  static const ScaleTable scales = make_scales(3);
   std::copy_n(scales.f[T + (pl.k8 < 8)], kPrimes, pl.scale);
+  return pl;
+}
+
+SixPlan six_inverse_plan(int s) {
+  SixPlan pl = six_plan(s, 1ull << s);
+  // the inverse's sums, and the one Montgomery step of the operand's limbs
+  static const ScaleTable scales = make_scales(1);
+  std::copy_n(scales.f[std::min(s - 3, kRootLog)], kPrimes, pl.scale);
   return pl;
 }
 
@@ -391,6 +399,12 @@ cudaError_t six_forward(const u64* limbs, u64 n, u32* res, const SixPlan& pl, co
 cudaError_t six_pointwise(u32* dst, const u32* a, const u32* b, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
   const SixOperands op{nullptr, 0, 0, 1, nullptr, 0, const_cast<u32*>(a), const_cast<u32*>(b)};
   const cudaError_t e = fused_pass<kProduct, false>(op, dst, pl, t, st);
+  return e == cudaSuccess ? inverse_cols(dst, 1, pl, t, st) : e;
+}
+
+cudaError_t six_inverse(u32* dst, const u32* a, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
+  const SixOperands op{nullptr, 0, 0, 1, nullptr, 0, const_cast<u32*>(a), nullptr};
+  const cudaError_t e = fused_pass<kInverse, false>(op, dst, pl, t, st);
   return e == cudaSuccess ? inverse_cols(dst, 1, pl, t, st) : e;
 }
 

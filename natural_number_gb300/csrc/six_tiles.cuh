@@ -715,6 +715,7 @@ __device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const Root
 //  kReady: a forward; b's forward levels are done (FinishedWords)
 //  kProduct: those of both are done
 //  kForward: a's forward levels only, to out
+//  kInverse: a's are done, and it is taken back alone, without a product
 // Operands are residues after the strided passes, or, FIRST (transforms of one
 // pass), limbs (na, nb of them); finished ones are words of at most 0.75 p.
 // last: no strided inverse pass follows (scale, k8 as in inverse_tile).
@@ -722,10 +723,12 @@ __device__ __forceinline__ void leaf_products(u32* sa, const u32* sb, const Root
 // 2^(R-1) roots of either direction that a one-pass transform needs copied to
 // shared memory while the limbs are on their way: a lone short product waits
 // on memory a third as often.
-enum : int { kAll = 0, kReady = 1, kProduct = 2, kForward = 3 };
+enum : int { kAll = 0, kReady = 1, kProduct = 2, kForward = 3, kInverse = 4 };
 // Shared-memory tiles of a mode: finished operands are read from global memory
 // where a block is a sector (LGM = 3).
-constexpr int fused_tiles(int LGM, int mode) { return mode == kAll || (LGM > 3 && mode != kForward) ? 2 : 1; }
+constexpr int fused_tiles(int LGM, int mode) {
+  return mode == kAll || (LGM > 3 && mode != kForward && mode != kInverse) ? 2 : 1;
+}
 template <int R, int LGM, int NT, int V, int MODE, bool FIRST, bool PAIR = false>
 __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const void* b, u64 nb, u32* out, int s,
                                            u32 tile, int prime, const int2* __restrict__ tab,
@@ -775,9 +778,9 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
     const int operands = b ? 2 : 1;
 #pragma unroll 1
     for (int op = 0; op < operands; ++op) forward(op ? b : a, op ? nb : na, op ? sb : sa);
-  } else if constexpr (MODE != kProduct) {
+  } else if constexpr (MODE != kProduct && MODE != kInverse) {
     forward(a, na, sa);
-  } else if constexpr (LGM > 3) {
+  } else if constexpr (LGM > 3 || MODE == kInverse) {
     copy_in(a, sa);
   }
   if constexpr (LGM > 3 && (MODE == kReady || MODE == kProduct)) copy_in(b, sb);
@@ -786,7 +789,9 @@ __device__ __forceinline__ void fused_tile(u32* sm, const void* a, u64 na, const
     u32* back = out + off;
     for (u32 i = 4 * threadIdx.x; i < ((u32)C << R); i += 4 * NT) stv(back + i, ldv<4>(sa + at<C, true>(i / C) + i % C));
   } else {
-    if constexpr (LGM == 3)
+    if constexpr (MODE == kInverse) {
+      // the words as they are
+    } else if constexpr (LGM == 3)
       leaf_products8<R, PAIR ? 2 * NT : NT, MODE == kProduct, MODE != kAll>(sa, sb, static_cast<const u32*>(a) + off,
                                                             static_cast<const u32*>(b) + off, tw, tile, P,
                                                             FIRST && R >= 3 ? (u32)k8 << (R - 3) : 1u << R);
