@@ -18,12 +18,12 @@
 //     before it that does not propagate, resolves the carries inside its range
 //     with ballots, and adds a tile's carry-in of 1 at its first limb, where
 //     it ripples only while limbs wrap to zero.
-// The shortest are one cluster, whose CTAs exchange their bits.  Base-case
-// products and the allocation-free entry point take the decoupled lookback
-// instead (scan_tile with kScanLookback: one launch, each tile's carry-in from
-// its predecessors' status words), whose waits are bounded and record an error
-// instead of hanging.  A per-call lookback leaves its status words and counters
-// zero for the next: the CTA that finishes last clears them.
+// The shortest are one cluster, whose CTAs exchange their bits.  No scan leaves
+// anything behind for the next one.  The batches' base case and the
+// allocation-free entry point take the decoupled lookback instead (scan_tile
+// with kScanLookback: one launch, each tile's carry-in from its predecessors'
+// status words, cleared before the launch), whose waits are bounded and record
+// an error instead of hanging.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,33 +38,6 @@ namespace nn {
 NN_DEFINE_PRIME_UPLOADER(upload_primes_carry)
 
 namespace {
-
-// Base-case products of at most kLookbackTiles tiles take one launch: tile ids
-// come from an atomic counter, so every predecessor of a tile has started
-// before it, and each tile takes its carry-in by the decoupled lookback.
-constexpr u64 kLookbackTiles = 1024;
-
-// The next tile of the scan, for every thread.
-__device__ __forceinline__ u32 next_tile(u32* counter) {
-  __shared__ u32 s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
-  __syncthreads();
-  return s_tile;
-}
-// The last tile of a scan to finish (of all its launches) clears the status
-// words and counters: every other tile's lookback is over by then.
-__device__ __forceinline__ void finish_tile(u32* flags, u32* counter, u32 tiles) {
-  __shared__ u32 s_last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(counter + 1, 1u) + 1 == tiles;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  for (u32 i = threadIdx.x; i < tiles; i += blockDim.x) flags[i] = 0;
-  if (threadIdx.x < 2) counter[threadIdx.x] = 0;
-}
 
 // Step 1: tile tile_base + blockIdx.x with carry-in 0; flags[tile] receives
 // its generate (bit 0) and propagate (bit 1) bits.
@@ -300,23 +273,28 @@ __global__ void __launch_bounds__(256) school_cluster_kernel(ColumnProducer prod
   cluster_sync();
 }
 
-// Longer base-case products of at most 2^20 positions: each CTA forms its
-// tile's column sums in shared memory and takes the tile through the lookback
-// scan, one launch.  Small tiles spread a short product over the GPU: the
-// column sums are the work, up to 383 terms a position.
-constexpr u64 kSchoolTile = 64, kSchoolLongTile = 1024;
+// Longer base-case products: each CTA forms its tile's column sums in shared
+// memory, eight lanes a position, and runs the scan's first step on them.
+// Small tiles spread a short product over the GPU: the column sums are the
+// work, up to 383 terms a position.  Longer operands here have few terms a
+// position, and beyond kSchoolLong a thread forms those of eight positions by
+// itself (run_scan).  Measured, us, tiles of 64 / 256 / 1024 positions / run_scan:
+// 1500 x 40 limbs 4.9 / 8.5 / 23.0, 32768 x 16 7.6 / 8.1 / 20.2, 65000 x 31 13.8 /
+// 12.4 / 26.7 / 18.2, 131072 x 16 18.5 / 14.9 / 20.4 / 15.7, 262144 x 31 42.1 /
+// 32.2 / 35.8 / 26.5.  With the lookback in one launch, its tiles from a
+// counter, 1500 x 40 took 6.1, 131072 x 16 24.6.
+constexpr u64 kSchoolTile = 64, kSchoolWideTile = 256;
+constexpr u64 kSchoolShort = 3 << 14, kSchoolLong = 3 << 16;
 template <u64 TILE>
-__global__ void __launch_bounds__(256) school_kernel(ColumnProducer prod, u64 total, u64* out, u32* flags,
-                                                     u32* counter, u32* err, u32 tiles) {
+__global__ void __launch_bounds__(256) school_kernel(ColumnProducer prod, u64 total, u64* out, u32* flags) {
   grid_begin();
   __shared__ u64 sums[3 * (TILE + kScanE)];
-  const u32 tile = next_tile(counter);
+  const u64 tile = blockIdx.x;
   column_tile_sums<256, TILE>(sums, prod, tile);
   __syncthreads();
   typedef SmemSumsProducer<TILE> Sums;
-  scan_tile<Sums, kScanLookback, 256, TILE>(Sums{sums, tile * TILE - kScanE, total}, tile, total, out, total, nullptr,
-                                            flags, err);
-  finish_tile(flags, counter, tiles);
+  scan_tile<Sums, kScanRecord, 256, TILE>(Sums{sums, tile * TILE - kScanE, total}, tile, total, out, total, nullptr,
+                                          flags, nullptr);
 }
 
 // One warp a job: lane i adds limb base + i of x and y; the block's carries
@@ -400,6 +378,16 @@ __global__ void __launch_bounds__(256) add_batch_long_kernel(const AddJob* __res
   }
 }
 
+// Step 2 over tiles [t0, t1) of TILE positions.
+template <u64 TILE>
+cudaError_t carry_fix(u64 t0, u64 t1, u64 total, u64* out, u64 out_limit, Scan& sc, cudaStream_t st) {
+  launch_begin("scan_carry_fix", st);
+  const cudaError_t e = launch_next(carry_fix_kernel<TILE>, (unsigned)((t1 - t0 + kFixTiles - 1) / kFixTiles), 256, 0, 0,
+                                    st, sc.flags, t0, t1, total, out, out_limit, sc.side);
+  launch_end(st);
+  return e;
+}
+
 // Tiles [tile_begin, tile_end) of the scan (all of them by default).  The
 // ranges of one scan go in order on one stream (each range's carry-in comes
 // from the words of the tiles before it).
@@ -425,71 +413,63 @@ cudaError_t run_scan(const Prod& prod, u64 total, u64* out, u64 out_limit, Scan&
   launch_begin(name, st);
   if (short_tiles)
     e = launch_next(scan_kernel<Prod, kScanSmall>, (unsigned)n, kScanSmall, 0, 0, st, prod, total, out, out_limit,
-                    sc.side, sc.wide, 0);
+                    sc.side, sc.flags, 0);
   else
     e = launch_next(scan_kernel<Prod, kScanThreads>, (unsigned)n, kScanThreads, 0, 0, st, prod, total, out, out_limit,
-                    sc.side, sc.wide, tile_begin);
+                    sc.side, sc.flags, tile_begin);
   launch_end(st);
   if (e != cudaSuccess) return e;
-  launch_begin("scan_carry_fix", st);
-  const unsigned ranges = (unsigned)((n + kFixTiles - 1) / kFixTiles);
-  if (short_tiles)
-    e = launch_next(carry_fix_kernel<kSmallTile>, ranges, 256, 0, 0, st, sc.wide, 0, n, total, out, out_limit, sc.side);
-  else
-    e = launch_next(carry_fix_kernel<kScanTile>, ranges, 256, 0, 0, st, sc.wide, tile_begin, tile_end, total, out,
-                    out_limit, sc.side);
-  launch_end(st);
-  return e;
+  return short_tiles ? carry_fix<kSmallTile>(0, n, total, out, out_limit, sc, st)
+                     : carry_fix<kScanTile>(tile_begin, tile_end, total, out, out_limit, sc, st);
 }
 
 template <u64 TILE>
 cudaError_t launch_school(const ColumnProducer& prod, u64 total, u64* out, Scan& sc, cudaStream_t st) {
-  const u32 tiles = (u32)((total + TILE - 1) / TILE);  // at most kLookbackTiles
+  const u64 tiles = (total + TILE - 1) / TILE;
+  cudaError_t e = scan_reserve(sc, tiles);
+  if (e != cudaSuccess) return e;
   launch_begin("school_tiles", st);
-  const cudaError_t e = launch_next(school_kernel<TILE>, tiles, 256, 0, 0, st, prod, total, out, sc.flags, sc.counter,
-                                    sc.err, tiles);
+  e = launch_next(school_kernel<TILE>, (unsigned)tiles, 256, 0, 0, st, prod, total, out, sc.flags);
   launch_end(st);
-  return e;
+  return e == cudaSuccess ? carry_fix<TILE>(0, tiles, total, out, total, sc, st) : e;
 }
 
 }  // namespace
 
 u64 scan_tiles(u64 positions) { return positions ? (positions + kScanTile - 1) / kScanTile : 1; }
 
+// Carry bits for that many tiles.
 cudaError_t scan_reserve(Scan& sc, u64 tiles) {
-  if (sc.flags && sc.max_tiles >= tiles) return cudaSuccess;
-  if (sc.flags) cudaFree(sc.flags);  // waits for the device: no scan is using it
-  u64 cap = sc.max_tiles ? sc.max_tiles : kLookbackTiles;
-  while (cap < tiles) cap *= 2;
-  // the lookback's status words, then the carry bits of the other scans
-  cudaError_t e = cudaMalloc((void**)&sc.flags, (kLookbackTiles + 1 + cap) * sizeof(u32));
-  if (e == cudaSuccess) e = cudaMemset(sc.flags, 0, (kLookbackTiles + 1) * sizeof(u32));
-  if (e != cudaSuccess) {
-    if (sc.flags) cudaFree(sc.flags);
-    sc.flags = sc.wide = nullptr;
-    sc.max_tiles = 0;
-    return e;
-  }
-  sc.wide = sc.flags + kLookbackTiles + 1;
-  sc.max_tiles = cap;
-  if (!sc.counter) {
-    e = cudaMalloc((void**)&sc.counter, 4 * sizeof(u32) + 4 * sizeof(u64));
+  if (!sc.err) {
+    u32* words = nullptr;
+    cudaError_t e = cudaMalloc((void**)&words, 2 * sizeof(u32) + 4 * sizeof(u64));
     if (e != cudaSuccess) return e;
-    sc.err = sc.counter + 2;
-    sc.side = reinterpret_cast<u64*>(sc.counter + 4);
-    e = cudaMemset(sc.counter, 0, 4 * sizeof(u32) + 4 * sizeof(u64));
+    e = cudaMemset(words, 0, 2 * sizeof(u32) + 4 * sizeof(u64));
+    // the context's streams do not wait for the legacy one
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e != cudaSuccess) {
+      cudaFree(words);
+      return e;
+    }
+    sc.err = words;
+    sc.probe = words + 1;
+    sc.side = reinterpret_cast<u64*>(words + 2);
   }
-  return e;
-}
-
-cudaError_t scan_reset(Scan& sc, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(sc.flags, 0, (kLookbackTiles + 1) * sizeof(u32), st);
-  return e == cudaSuccess ? cudaMemsetAsync(sc.counter, 0, 2 * sizeof(u32), st) : e;
+  if (sc.max_tiles >= tiles) return cudaSuccess;
+  u64 cap = sc.max_tiles ? sc.max_tiles : 1024;
+  while (cap < tiles) cap *= 2;
+  if (sc.flags) cudaFree(sc.flags);  // waits for the device: no scan is using it
+  sc.flags = nullptr;
+  sc.max_tiles = 0;
+  const cudaError_t e = cudaMalloc((void**)&sc.flags, cap * sizeof(u32));
+  if (e != cudaSuccess) return e;
+  sc.max_tiles = cap;
+  return cudaSuccess;
 }
 
 void scan_free(Scan& sc) {
   if (sc.flags) cudaFree(sc.flags);
-  if (sc.counter) cudaFree(sc.counter);
+  if (sc.err) cudaFree(sc.err);
   sc = Scan{};
 }
 
@@ -597,8 +577,6 @@ cudaError_t add_batch(const AddJob* d_jobs, u64 m, u64 longest, cudaStream_t st)
 }
 
 cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Scan& sc, cudaStream_t st) {
-  cudaError_t e = scan_reserve(sc, 1);
-  if (e != cudaSuccess) return e;
   const u64 total = na + nb;
   const ColumnProducer prod = na >= nb ? ColumnProducer{a, na, b, nb} : ColumnProducer{b, nb, a, na};
   if (total <= kSchoolClusterTile * kSchoolClusterCtas && prod.nb <= kSchoolShorter) {
@@ -607,12 +585,12 @@ cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Sca
     if (ok != cudaSuccess) return ok;
     const unsigned tiles = (unsigned)((total + kSchoolClusterTile - 1) / kSchoolClusterTile);
     launch_begin("school_tiles", st);
-    e = launch_next(school_cluster_kernel, tiles, 256, 0, tiles, st, prod, total, out);
+    const cudaError_t e = launch_next(school_cluster_kernel, tiles, 256, 0, tiles, st, prod, total, out);
     launch_end(st);
     return e;
   }
-  if (total <= kSchoolTile * kLookbackTiles) return launch_school<kSchoolTile>(prod, total, out, sc, st);
-  if (total <= kSchoolLongTile * kLookbackTiles) return launch_school<kSchoolLongTile>(prod, total, out, sc, st);
+  if (total <= kSchoolShort) return launch_school<kSchoolTile>(prod, total, out, sc, st);
+  if (total <= kSchoolLong) return launch_school<kSchoolWideTile>(prod, total, out, sc, st);
   return run_scan(prod, total, out, total, sc, st, "school_column_scan");
 }
 
@@ -655,10 +633,8 @@ cudaError_t shr_bits(u64* out, const u64* in, u64 n, unsigned cl, cudaStream_t s
 cudaError_t wait_probe(Scan& sc, int limit, cudaStream_t st) {
   cudaError_t e = scan_reserve(sc, 1);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(sc.flags, 0, sizeof(u32), st);
-  if (e != cudaSuccess) return e;
   launch_begin("wait_probe", st);
-  wait_probe_kernel<<<1, 32, 0, st>>>(sc.flags, sc.err, limit);
+  wait_probe_kernel<<<1, 32, 0, st>>>(sc.probe, sc.err, limit);
   launch_end(st);
   return cudaGetLastError();
 }

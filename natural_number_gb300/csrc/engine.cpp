@@ -1016,7 +1016,6 @@ nn_status nn_context_synchronize(nn_context* c) {
   NN_CK(c, cudaMemcpy(&err, c->scan.err, sizeof err, cudaMemcpyDeviceToHost), "read error flag");
   if (err) {
     cudaMemset(c->scan.err, 0, sizeof err);
-    nn::scan_reset(c->scan, c->stream);
     c->err = "carry lookback wait exceeded its bound";
     return NN_ERR_TIMEOUT;
   }
@@ -1034,7 +1033,7 @@ const char* nn_last_error(const nn_context* c) { return c ? c->err.c_str() : "no
 uint64_t nn_context_device_bytes(const nn_context* c) {
   if (!c) return 0;
   return c->held + 2 * 3 * c->tables.cap * sizeof(u64) + 2 * 6 * c->six.cap * sizeof(int2) +
-         (c->scan.max_tiles + 1026) * 4;
+         c->scan.max_tiles * 4;
 }
 
 nn_status nn_transform_create(nn_context* c, nn_transform** out) {

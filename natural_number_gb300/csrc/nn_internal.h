@@ -117,14 +117,13 @@ cudaError_t six_forward(const u64* limbs, u64 n, u32* res, const SixPlan& pl, co
 cudaError_t six_pointwise(u32* dst, const u32* a, const u32* b, const SixPlan& pl, const SixTables& t, cudaStream_t st);
 // A finished transform (dst may be it) back to the residues of its operand for the CRT; pl: six_inverse_plan's.
 cudaError_t six_inverse(u32* dst, const u32* a, const SixPlan& pl, const SixTables& t, cudaStream_t st);
-// Scratch for the carry scan.
+// Scratch for the carry scan.  Nothing in it outlives a scan but the error word.
 struct Scan {
-  u32* flags = nullptr;  // per-tile status words of a lookback, zero between scans (the last tile clears them)
-  u32* wide = nullptr;   // per-tile carry bits of the scans that do not wait
-  u32* counter = nullptr;  // the lookback's next tile and finished tiles (two words, zero between scans)
+  u32* flags = nullptr;  // per-tile carry bits
   u32* err = nullptr;    // nonzero after a lookback wait gave up
+  u32* probe = nullptr;  // a status word that nothing sets
   u64* side = nullptr;   // limbs of the scan beyond the output (the carry words)
-  u64 max_tiles = 0;
+  u64 max_tiles = 0;     // tiles that flags holds
 };
 constexpr int kScanThreads = 256;
 constexpr int kScanE = 8;  // limbs per thread
@@ -294,8 +293,6 @@ std::string profile_report();
 
 u64 scan_tiles(u64 positions);
 cudaError_t scan_reserve(Scan& sc, u64 tiles);
-// Clears the lookback's words (after a wait gave up).
-cudaError_t scan_reset(Scan& sc, cudaStream_t st);
 void scan_free(Scan& sc);
 
 }  // namespace nn
