@@ -438,7 +438,9 @@ cudaError_t launch_school(const ColumnProducer& prod, u64 total, u64* out, Scan&
 
 u64 scan_tiles(u64 positions) { return positions ? (positions + kScanTile - 1) / kScanTile : 1; }
 
-// Carry bits for that many tiles.
+// Carry bits for that many tiles.  A replaced buffer stays until the context
+// goes: a captured graph, or work on another stream, may still use it; the
+// replaced ones together are smaller than the live one.
 cudaError_t scan_reserve(Scan& sc, u64 tiles) {
   if (!sc.err) {
     u32* words = nullptr;
@@ -458,16 +460,18 @@ cudaError_t scan_reserve(Scan& sc, u64 tiles) {
   if (sc.max_tiles >= tiles) return cudaSuccess;
   u64 cap = sc.max_tiles ? sc.max_tiles : 1024;
   while (cap < tiles) cap *= 2;
-  if (sc.flags) cudaFree(sc.flags);  // waits for the device: no scan is using it
-  sc.flags = nullptr;
-  sc.max_tiles = 0;
-  const cudaError_t e = cudaMalloc((void**)&sc.flags, cap * sizeof(u32));
+  u32* flags = nullptr;
+  const cudaError_t e = cudaMalloc((void**)&flags, cap * sizeof(u32));
   if (e != cudaSuccess) return e;
+  if (sc.flags) sc.replaced.push_back(sc.flags);
+  sc.flags = flags;
   sc.max_tiles = cap;
+  sc.held_tiles += cap;
   return cudaSuccess;
 }
 
 void scan_free(Scan& sc) {
+  for (u32* p : sc.replaced) cudaFree(p);
   if (sc.flags) cudaFree(sc.flags);
   if (sc.err) cudaFree(sc.err);
   sc = Scan{};

@@ -1033,7 +1033,7 @@ const char* nn_last_error(const nn_context* c) { return c ? c->err.c_str() : "no
 uint64_t nn_context_device_bytes(const nn_context* c) {
   if (!c) return 0;
   return c->held + 2 * 3 * c->tables.cap * sizeof(u64) + 2 * 6 * c->six.cap * sizeof(int2) +
-         c->scan.max_tiles * 4;
+         c->scan.held_tiles * 4;
 }
 
 nn_status nn_transform_create(nn_context* c, nn_transform** out) {

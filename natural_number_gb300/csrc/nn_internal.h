@@ -124,6 +124,8 @@ struct Scan {
   u32* probe = nullptr;  // a status word that nothing sets
   u64* side = nullptr;   // limbs of the scan beyond the output (the carry words)
   u64 max_tiles = 0;     // tiles that flags holds
+  u64 held_tiles = 0;    // ... and the replaced ones with it
+  std::vector<u32*> replaced;  // carry bits of smaller scans
 };
 constexpr int kScanThreads = 256;
 constexpr int kScanE = 8;  // limbs per thread

@@ -1,4 +1,6 @@
-"""The carry scans' scratch: what one scan leaves there never matters to the next."""
+"""The carry scans' scratch: what a scan finds there never matters to the next
+one, and a captured graph keeps the words it was captured with when a longer
+scan of the same context wants more."""
 import numpy as np
 import pytest
 
@@ -56,3 +58,31 @@ def test_products_after_overlapping_ones(oracle):
         assert np.array_equal(to_host(outs[2])[: want.size], want)
     ctx.set_stream(None)
     ctx.close()
+
+
+@pytest.mark.parametrize("na,nb", [(20000, 20), (3000, 2500), (400000, 300000)])
+def test_replay_after_the_scratch_grew(oracle, na, nb):
+    import torch
+    import natural_number_gb300 as nn
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ctx = nn.Context(0)
+        x, y, out = empty(na), empty(nb), empty(na + nb)
+        x.copy_(to_dev(limbs(1, na)))
+        y.copy_(to_dev(limbs(2, nb)))
+        ctx.mul_device(out, x, y)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            ctx.mul_device(out, x, y)
+        long = torch.randint(-(2**63), 2**63 - 1, (1 << 22,), dtype=torch.int64, device="cuda").view(torch.uint64)
+        t = empty(1 << 23)
+        ctx.mul_device(t, long, long)  # 4096 tiles: more than the scratch held
+        for seed in (3, 5):
+            a, b = limbs(seed, na), limbs(seed + 1, nb)
+            x.copy_(to_dev(a))
+            y.copy_(to_dev(b))
+            graph.replay()
+            stream.synchronize()
+            want = oracle.mul(a, b)
+            assert np.array_equal(to_host(out)[: want.size], want)
+        ctx.close()
