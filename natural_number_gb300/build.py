@@ -25,7 +25,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 CU_SOURCES = ["batch.cu", "six.cu", "ntt.cu", "carry.cu", "noalloc.cu", "decimal.cu"]
 CPP_SOURCES = ["engine.cpp", "profile.cpp", "natural_ops.cpp", "serve.cpp", "series.cpp", "host_glue.cpp", "divide.cpp",
                "host_pool.cpp"]
-HEADERS = ["nn_device.cuh", "nn_internal.h", "ntt_tiles.cuh", "six_tiles.cuh", "scan_tiles.cuh", "tma.cuh", "context_access.h",
+HEADERS = ["device_once.h", "stage_ring.h", "nn_device.cuh", "nn_internal.h", "ntt_tiles.cuh", "six_tiles.cuh", "scan_tiles.cuh", "tma.cuh", "context_access.h",
            "../../include/natural_gb300.hpp"]
 
 

@@ -227,10 +227,11 @@ struct Launch {
   template <int R>
   cudaError_t strided() const {
     constexpr int smem = col_smem(R), threads = col_threads(R);
-    static const cudaError_t ok[3] = {allow_smem(batch_load_kernel<R>, smem), allow_smem(batch_col_kernel<R, false>, smem),
-                                      allow_smem(batch_col_kernel<R, true>, smem)};
-    for (cudaError_t e : ok)
-      if (e != cudaSuccess) return e;
+    static DeviceOnce once[3];
+    const cudaError_t e = g.kind == kBatchLoad  ? allow_smem<smem>(once[0], batch_load_kernel<R>)
+                          : g.kind == kBatchCol ? allow_smem<smem>(once[1], batch_col_kernel<R, false>)
+                                                : allow_smem<smem>(once[2], batch_col_kernel<R, true>);
+    if (e != cudaSuccess) return e;
     if (g.kind == kBatchLoad)
       batch_load_kernel<R><<<g.count, threads, smem, st>>>(jobs, items, t);
     else if (g.kind == kBatchCol)
@@ -242,8 +243,8 @@ struct Launch {
   template <int R, int LGM, int MODE>
   cudaError_t contiguous_mode() const {
     constexpr int smem = fused_tiles(LGM, MODE) * (int)tile_words32<1 << LGM, true>(R) * 4;
-    static const cudaError_t ok = allow_smem(batch_fused_kernel<R, LGM, MODE>, smem);
-    if (ok != cudaSuccess) return ok;
+    static DeviceOnce once;
+    if (const cudaError_t e = allow_smem<smem>(once, batch_fused_kernel<R, LGM, MODE>); e != cudaSuccess) return e;
     batch_fused_kernel<R, LGM, MODE><<<g.count, fused_threads(R, LGM, 4), smem, st>>>(jobs, items, t);
     return cudaGetLastError();
   }
@@ -259,6 +260,7 @@ struct Launch {
   template <int R, int MODE>
   cudaError_t small_mode() const {
     constexpr int smem = fused_tiles(3, MODE) * (int)tile_words32<8, true>(R) * 4;
+    static_assert(smem <= 48 * 1024);
     batch_small_kernel<R, MODE><<<g.count, fused_threads(R, 3, small_columns(R)), smem, st>>>(jobs, items, t);
     return cudaGetLastError();
   }

@@ -584,12 +584,12 @@ cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Sca
   const u64 total = na + nb;
   const ColumnProducer prod = na >= nb ? ColumnProducer{a, na, b, nb} : ColumnProducer{b, nb, a, na};
   if (total <= kSchoolClusterTile * kSchoolClusterCtas && prod.nb <= kSchoolShorter) {
-    static const cudaError_t ok =  // clusters of more than eight CTAs want asking
-        cudaFuncSetAttribute(school_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (ok != cudaSuccess) return ok;
+    static DeviceOnce once;  // clusters of more than eight CTAs want asking
+    cudaError_t e = kernel_attribute(once, school_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
     const unsigned tiles = (unsigned)((total + kSchoolClusterTile - 1) / kSchoolClusterTile);
     launch_begin("school_tiles", st);
-    const cudaError_t e = launch_next(school_cluster_kernel, tiles, 256, 0, tiles, st, prod, total, out);
+    e = launch_next(school_cluster_kernel, tiles, 256, 0, tiles, st, prod, total, out);
     launch_end(st);
     return e;
   }

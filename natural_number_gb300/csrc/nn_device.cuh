@@ -10,6 +10,8 @@
 
 #include <cuda_runtime.h>
 
+#include "device_once.h"
+
 namespace nn {
 
 typedef std::uint64_t u64;
@@ -48,6 +50,23 @@ cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, unsigned threads, 
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
   if (e != cudaSuccess) cudaGetLastError();  // reported here, once
   return e;
+}
+
+// Sets a kernel's attribute on the current device, once (attributes belong to a
+// device); `once` is the kernel's own.
+template <class Kernel>
+cudaError_t kernel_attribute(DeviceOnce& once, Kernel kernel, cudaFuncAttribute attribute, int value) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return once(device, cudaSuccess, [&] { return cudaFuncSetAttribute(kernel, attribute, value); });
+}
+// Lets a kernel have BYTES of dynamic shared memory on the current device.
+template <int BYTES, class Kernel>
+cudaError_t allow_smem(DeviceOnce& once, Kernel kernel) {
+  if constexpr (BYTES > 48 * 1024)
+    return kernel_attribute(once, kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+  return cudaSuccess;
 }
 
 struct PrimeSet {

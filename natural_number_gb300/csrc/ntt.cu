@@ -426,13 +426,9 @@ bool col_tensor_map(CUtensorMap* m, const u64* res, int s, int lambda0, int R) {
 template <bool INV, bool SCALE, int BLOCKS, int THREADS = 256>
 cudaError_t launch_col_tma_b(const CUtensorMap& tm, int s, const Pass& ps, const Tables& t, cudaStream_t st) {
   const size_t smem = ((size_t)16 << ps.R) * 8;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(ntt_col_tma_kernel<INV, SCALE, BLOCKS, THREADS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static DeviceOnce once;
+  const cudaError_t e = allow_smem<200 * 1024>(once, ntt_col_tma_kernel<INV, SCALE, BLOCKS, THREADS>);
+  if (e != cudaSuccess) return e;
   const u64 tiles = (1ull << s) / ((u64)16 << ps.R);
   launch_begin(INV ? (SCALE ? "ntt_inv_last_col_pass" : "ntt_inv_col_pass") : "ntt_fwd_col_pass", st);
   ntt_col_tma_kernel<INV, SCALE, BLOCKS, THREADS><<<dim3((unsigned)tiles, 3), THREADS, smem, st>>>(
@@ -456,13 +452,9 @@ cudaError_t launch_col_tma(const CUtensorMap& tm, int s, const Pass& ps, const T
 template <bool INV, int BLOCKS>
 cudaError_t launch_row_bulk(u64* out, int s, const Pass& ps, const Tables& t, cudaStream_t st) {
   const size_t smem = tile_smem_bytes(2, ps.R);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(ntt_row_bulk_kernel<INV, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         200 * 1024);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static DeviceOnce once;
+  const cudaError_t e = allow_smem<200 * 1024>(once, ntt_row_bulk_kernel<INV, BLOCKS>);
+  if (e != cudaSuccess) return e;
   const u64 tiles = (1ull << s) / ((u64)2 << ps.R);
   launch_begin(INV ? "ntt_inv_row_pass" : "ntt_fwd_row_pass", st);
   ntt_row_bulk_kernel<INV, BLOCKS><<<dim3((unsigned)tiles, 3), 256, smem, st>>>(out, s, ps.R, INV ? t.iroot : t.root,
@@ -475,13 +467,9 @@ template <int BLOCKS, int THREADS>
 cudaError_t launch_load_tma(const CUtensorMap& tm, const u64* in, u64 n_in, int s, const Pass& ps, const Tables& t,
                             cudaStream_t st) {
   const size_t smem = ((size_t)16 << ps.R) * 8;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(ntt_load_tma_kernel<BLOCKS, THREADS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static DeviceOnce once;
+  const cudaError_t e = allow_smem<200 * 1024>(once, ntt_load_tma_kernel<BLOCKS, THREADS>);
+  if (e != cudaSuccess) return e;
   const u64 tiles = (1ull << s) / ((u64)16 << ps.R);
   launch_begin("ntt_fwd_load_col_pass", st);
   ntt_load_tma_kernel<BLOCKS, THREADS><<<(unsigned)(3 * tiles), THREADS, smem, st>>>(tm, in, n_in, s, ps.R, t.root,
@@ -512,13 +500,9 @@ cudaError_t launch_pass(const u64* in, u64* out, u64 n_in, int s, const Pass& ps
     }
   }
   const size_t smem = tile_smem_bytes(ps.C, ps.R);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(ntt_pass_kernel<C, FIRST, INV, SCALE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static DeviceOnce once;
+  const cudaError_t e = allow_smem<200 * 1024>(once, ntt_pass_kernel<C, FIRST, INV, SCALE>);
+  if (e != cudaSuccess) return e;
   const u64 tiles = (1ull << s) / ((u64)ps.C << ps.R);
   const dim3 grid = FIRST ? dim3((unsigned)(3 * tiles), 1) : dim3((unsigned)tiles, 3);
   const char* name = C == 2 ? (INV ? "ntt_inv_row_pass" : "ntt_fwd_row_pass")
@@ -675,38 +659,31 @@ cudaError_t ntt_fused_last(u64* res, const u64* other, int s, const Tables& t, c
   const Pass& ps = plan.back();
   if (ps.C != 2) return cudaErrorInvalidValue;
   const size_t smem = tile_smem_bytes(ps.C, ps.R);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(ntt_fused_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(ntt_fused_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
   const u64 tiles = (1ull << s) / ((u64)ps.C << ps.R);
   dim3 grid((unsigned)tiles, 3);
   const u64 nel = (u64)2 << ps.R;
   if (aligned16(res) && (!other || aligned16(other)) && ps.lambda0 + ps.R == s - 1 &&
       nel <= (u64)4 * kPointwiseGroups * 256) {
-    static bool bulk_configured = false;
-    if (!bulk_configured) {
-      cudaError_t e = cudaFuncSetAttribute(ntt_fused_bulk_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           200 * 1024);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(ntt_fused_bulk_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      if (e != cudaSuccess) return e;
-      bulk_configured = true;
-    }
+    static DeviceOnce once[2];
+    const bool four = 4 * smem <= 227 * 1024 && nel <= (u64)2 * kPointwiseGroups * 256;
+    const cudaError_t e = four ? allow_smem<200 * 1024>(once[0], ntt_fused_bulk_kernel<4>)
+                               : allow_smem<200 * 1024>(once[1], ntt_fused_bulk_kernel<3>);
+    if (e != cudaSuccess) return e;
     launch_begin("ntt_fused_row_pass", st);
-    if (4 * smem <= 227 * 1024 && nel <= (u64)2 * kPointwiseGroups * 256)
+    if (four)
       ntt_fused_bulk_kernel<4><<<grid, 256, smem, st>>>(res, other, s, ps.R, t.root, t.iroot, t.cap, t.err);
     else
       ntt_fused_bulk_kernel<3><<<grid, 256, smem, st>>>(res, other, s, ps.R, t.root, t.iroot, t.cap, t.err);
     launch_end(st);
     return cudaGetLastError();
   }
+  static DeviceOnce once[2];
+  const bool four = 4 * smem <= 227 * 1024;
+  const cudaError_t e = four ? allow_smem<200 * 1024>(once[0], ntt_fused_kernel<4>)
+                             : allow_smem<200 * 1024>(once[1], ntt_fused_kernel<3>);
+  if (e != cudaSuccess) return e;
   launch_begin("ntt_fused_row_pass", st);
-  if (4 * smem <= 227 * 1024)
+  if (four)
     ntt_fused_kernel<4><<<grid, 256, smem, st>>>(res, other, s, ps.lambda0, ps.R, t.root, t.iroot, t.cap);
   else
     ntt_fused_kernel<3><<<grid, 256, smem, st>>>(res, other, s, ps.lambda0, ps.R, t.root, t.iroot, t.cap);

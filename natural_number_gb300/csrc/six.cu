@@ -156,8 +156,8 @@ template <int R>
 cudaError_t launch_load(const SixOperands& op, int s, int k8, const SixTables& t, u32 tile0, u32 tile1,
                         cudaStream_t st) {
   constexpr int smem = col_smem(R);
-  static const cudaError_t ok = allow_smem(six_load_kernel<R>, smem);
-  if (ok != cudaSuccess) return ok;
+  static DeviceOnce once;
+  if (const cudaError_t e = allow_smem<smem>(once, six_load_kernel<R>); e != cudaSuccess) return e;
   const u32 tiles = (u32)((1ull << s) / ((u64)col_width(R) << R));
   tile1 = std::min(tile1, tiles);
   const dim3 grid(kPrimes * (tile1 - tile0), op.pieces + (op.b ? 1 : 0));
@@ -170,8 +170,8 @@ template <int R, bool INV>
 cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int lambda0, const SixTables& t,
                        cudaStream_t st) {
   constexpr int smem = col_smem(R);
-  static const cudaError_t ok = allow_smem(six_col_kernel<R, INV>, smem);
-  if (ok != cudaSuccess) return ok;
+  static DeviceOnce once;
+  if (const cudaError_t e = allow_smem<smem>(once, six_col_kernel<R, INV>); e != cudaSuccess) return e;
   // past the first pass, only the blocks of the first k8 eighths
   const u64 tiles = (1ull << pl.s) / ((u64)col_width(R) << R);
   const dim3 grid((unsigned)(lambda0 ? tiles / 8 * pl.k8 : tiles), kPrimes, pieces + (rb ? 1 : 0));
@@ -184,8 +184,9 @@ cudaError_t launch_col(u32* ra, u32* rb, u32 pieces, const SixPlan& pl, int lamb
 template <int R, int LGM, int V, int MODE, bool FIRST, bool PAIR = false>
 cudaError_t launch_fused_v(const SixOperands& op, u32* out, const SixPlan& pl, const SixTables& t, cudaStream_t st) {
   constexpr int tile = (int)tile_words32<1 << LGM, true>(R) * 4, smem = fused_tiles(LGM, MODE) * tile + (PAIR ? (16 << (R - 1)) : 0);
-  static const cudaError_t ok = allow_smem(six_fused_kernel<R, LGM, V, MODE, FIRST, PAIR>, smem);
-  if (ok != cudaSuccess) return ok;
+  static DeviceOnce once;
+  if (const cudaError_t e = allow_smem<smem>(once, six_fused_kernel<R, LGM, V, MODE, FIRST, PAIR>); e != cudaSuccess)
+    return e;
   const u32 tiles = (u32)((1ull << pl.s) >> (R + LGM));
   const dim3 grid(pl.n == 1 ? 1u : tiles / 8 * pl.k8, kPrimes, op.pieces);
   launch_begin(MODE == kForward ? "six_fwd_row_pass" : MODE == kInverse ? "six_inv_row_pass" : FIRST ? "six_small_pass" : "six_fused_row_pass", st);

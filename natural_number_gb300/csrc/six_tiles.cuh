@@ -347,10 +347,6 @@ constexpr int fused_blocks(int R, int LGM, int V) {
   const int n = (LGM > 3 ? 640 : V == 4 ? 768 : 1024) / fused_threads(R, LGM, V);
   return n < 24 ? n : 24;
 }
-template <class Kernel>
-inline cudaError_t allow_smem(Kernel k, int bytes) {
-  return bytes > 48 * 1024 ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
-}
 
 // Forward levels [0, R) of one tile of C columns x 2^R rows, block index ksb
 // at its first level.  load(row, col) gives the V words from (row, col), store
