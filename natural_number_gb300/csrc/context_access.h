@@ -18,4 +18,7 @@ nn_status ctx_fail(nn_context* c, cudaError_t e, const char* what);
 cudaError_t ctx_upload(nn_context* c, void* d_dst, const void* h_src, u64 bytes);
 void ctx_error(nn_context* c, const char* msg);
 nn_status ctx_scratch(nn_context* c, int slot, u64 words, u64** p);  // grow-only staging, slots 0-2
+// Device bytes that a batch without the "batch_few" rule takes for this product
+// beside its operands and its share of the job table.
+u64 ctx_batch_job_bytes(const nn_context* c, u64 na, u64 nb);
 }  // namespace nn

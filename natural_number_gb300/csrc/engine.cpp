@@ -142,6 +142,7 @@ struct nn_context {
   int batch_split = 1;        // batches: unbalanced products in pieces sharing one transform
   int batch_blocks_per_sm = 0;  // kept for callers that set it: a CTA an item
   int batch_solo_scale = 22;    // batches: products of this scale and up run one at a time (0: never)
+  int batch_few = 1;            // batches of a few short products: one scale for all of them
 };
 
 struct nn_batch {
@@ -598,6 +599,37 @@ nn_status scratch(nn_context* c, int slot, u64 words, u64** p) {
 // Batches: a work queue over all jobs' pipeline steps (batch.cu).
 // ---------------------------------------------------------------------------
 
+// How a product of a batch runs: as column sums (plan.s 0), through transforms,
+// by itself after the batch's launches, or not at all.
+enum class BatchRoute { kColumns, kTransforms, kSolo, kTooLong };
+
+bool batch_columns(const nn_context* c, u64 na, u64 nb) {
+  const u64 mn = std::min(na, nb), mx = std::max(na, nb);
+  return mn < c->batch_ntt_min || (mn < c->batch_school_balanced && mx <= 2 * mn);
+}
+
+// J's pieces, plan and rows from its sizes (na >= nb) and `square`.  few: one of
+// a few products; those of a scale up to few_s take that.
+BatchRoute batch_route(const nn_context* c, nn::BatchJob& J, bool few, int few_s) {
+  constexpr int kFewUnsplit = 14;
+  J.piece = J.na;
+  J.pieces = 1;
+  if (batch_columns(c, J.na, J.nb)) return BatchRoute::kColumns;
+  int s = std::max(ntt_scale(J.na, J.nb), nn::kSixMinScale);
+  // From this scale on one product fills the GPU by itself: no items, no
+  // arena; the launch runs it alone.
+  if (c->batch_solo_scale > 0 && s >= c->batch_solo_scale) return BatchRoute::kSolo;
+  if (s <= few_s) s = few_s;
+  if (c->batch_split && !J.square && !(few && s <= kFewUnsplit)) s = six_split(J.na, J.nb, s, &J.piece, &J.pieces);
+  if (s > nn::kSixMaxScale) return BatchRoute::kTooLong;
+  J.plan = nn::six_plan(s, J.pieces > 1 ? 1ull << s : J.na + J.nb - 1, c->batch_r_last_at[s]);
+  J.rows = J.pieces > 1 ? nn::kBatchRowsB : J.plan.n > 1 && !c->batch_fused ? nn::kBatchRowsAll : nn::kBatchRowsNone;
+  return BatchRoute::kTransforms;
+}
+// Words of a transforms job's residues: operand 0's, and operand 1's where they are used.
+u64 batch_words_a(const nn::BatchJob& J) { return J.pieces * (3ull << J.plan.s); }
+u64 batch_words_b(const nn::BatchJob& J) { return !J.square && (J.plan.n > 1 || J.rows) ? 3ull << J.plan.s : 0; }
+
 nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, const int* square, u64 count) {
   if (count >= 0xffffffffull) {  // BatchItem::job is 32-bit
     c->err = "batch: too many products";
@@ -616,10 +648,11 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
   // work: up to 152 jobs whose operands fit one pass take one scale, the
   // largest such one of the batch, so that their passes are one launch (six
   // CTAs a job, under a wave), and products of up to 2^14 limbs are not split.
-  // (Budgeted contexts keep the smaller arenas.)  64 jobs of 8 to 1024 limbs:
-  // 68 us before, 62 us so; 111 of 44 to 6439 limbs 194 and 190 us.
-  constexpr int kOnePass = 12, kFewUnsplit = 14;
-  const bool few = count <= 152 && !c->budget;
+  // (Contexts with a budget, or "batch_few" 0, keep the smaller arenas.)  64
+  // jobs of 8 to 1024 limbs: 68 us before, 62 us so; 111 of 44 to 6439 limbs 194
+  // and 190 us.
+  constexpr int kOnePass = 12;
+  const bool few = c->batch_few && count <= 152 && !c->budget;
   int few_s = 0;
   for (u64 j = 0; few && j < count; ++j) {
     if (!na[j] || !nb[j]) continue;
@@ -638,8 +671,7 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
     J.piece = na[j];
     J.pieces = 1;
     J.flag_base = B->n_flags;
-    const u64 mn = std::min(na[j], nb[j]), mx = std::max(na[j], nb[j]);
-    if (mn < c->batch_ntt_min || (mn < c->batch_school_balanced && mx <= 2 * mn)) {
+    if (batch_columns(c, na[j], nb[j])) {
       B->n_flags += (nn::u32)((na[j] + nb[j] + nn::kBatchSumTile - 1) / nn::kBatchSumTile);
       order.push_back(j);
       continue;
@@ -651,31 +683,24 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
     }
     // operand 0 is the longer one; it may be split into pieces
     B->swap[j] = na[j] < nb[j];
-    J.na = mx;
-    J.nb = mn;
-    J.piece = J.na;
-    int s = std::max(ntt_scale(J.na, J.nb), nn::kSixMinScale);
-    if (c->batch_solo_scale > 0 && s >= c->batch_solo_scale) {
-      // From this scale on one product fills the GPU by itself: no items, no
-      // arena; the launch runs it alone.
+    J.na = std::max(na[j], nb[j]);
+    J.nb = std::min(na[j], nb[j]);
+    const BatchRoute route = batch_route(c, J, few, few_s);
+    if (route == BatchRoute::kSolo) {
       B->solo.push_back(j);
       continue;
     }
-    if (s <= few_s) s = few_s;
-    if (c->batch_split && !J.square && !(few && s <= kFewUnsplit)) s = six_split(J.na, J.nb, s, &J.piece, &J.pieces);
-    if (s > nn::kSixMaxScale) {
+    if (route == BatchRoute::kTooLong) {
       c->err = "batch: transform too long for one batch";
       return NN_ERR_INVALID;
     }
-    J.plan = nn::six_plan(s, J.pieces > 1 ? 1ull << s : J.na + J.nb - 1, c->batch_r_last_at[s]);
-    max_s = std::max(max_s, s);
-    J.rows = J.pieces > 1 ? nn::kBatchRowsB : J.plan.n > 1 && !c->batch_fused ? nn::kBatchRowsAll : nn::kBatchRowsNone;
+    max_s = std::max(max_s, J.plan.s);
     B->n_flags += (nn::u32)nn::scan_tiles(na[j] + nb[j]);
     B->off_a[j] = B->arena_words;
-    B->arena_words += J.pieces * (3ull << s);
-    if (!J.square && (J.plan.n > 1 || J.rows)) {
+    B->arena_words += batch_words_a(J);
+    if (const u64 words = batch_words_b(J)) {
       B->off_b[j] = B->arena_words;
-      B->arena_words += 3ull << s;
+      B->arena_words += words;
     }
     order.push_back(j);
   }
@@ -845,6 +870,14 @@ cudaError_t ctx_upload(nn_context* c, void* d_dst, const void* h_src, u64 bytes)
 }
 void ctx_error(nn_context* c, const char* msg) { c->err = msg; }
 nn_status ctx_scratch(nn_context* c, int slot, u64 words, u64** p) { return scratch(c, slot, words, p); }
+u64 ctx_batch_job_bytes(const nn_context* c, u64 na, u64 nb) {
+  BatchJob J{};
+  J.na = std::max(na, nb);
+  J.nb = std::min(na, nb);
+  if (batch_route(c, J, false, 0) != BatchRoute::kTransforms) return (na + nb) / 16;  // an item and a flag a tile
+  const u64 bytes = 8 * (batch_words_a(J) + batch_words_b(J));
+  return bytes + bytes / 512;  // its items: 12 bytes for 8192 words of a prime, a pass
+}
 }  // namespace nn
 
 extern "C" {
@@ -1225,6 +1258,8 @@ nn_status nn_context_set_tunable(nn_context* c, const char* name, int64_t v) {
     c->batch_blocks_per_sm = (int)v;
   else if (k == "batch_solo_scale" && (v == 0 || (v >= 2 && v < 64)))
     c->batch_solo_scale = (int)v;
+  else if (k == "batch_few" && (v == 0 || v == 1))
+    c->batch_few = (int)v;
   else if (k == "batch_school_balanced" && v >= 0)
     c->batch_school_balanced = (u64)v;
   else {
@@ -1255,6 +1290,7 @@ int64_t nn_context_get_tunable(const nn_context* c, const char* name) {
   if (k == "batch_split") return (int64_t)c->batch_split;
   if (k == "batch_blocks_per_sm") return c->batch_blocks_per_sm;
   if (k == "batch_solo_scale") return c->batch_solo_scale;
+  if (k == "batch_few") return c->batch_few;
   if (k == "batch_school_balanced") return (int64_t)c->batch_school_balanced;
   return -1;
 }

@@ -28,6 +28,7 @@
 
 #include "../../include/natural_gb300.h"
 #include "../../include/natural_gb300.hpp"
+#include "context_access.h"
 
 namespace {
 
@@ -72,7 +73,10 @@ struct InFlight {
 
 int scale_of(uint64_t n1, uint64_t n2) { return 64 - __builtin_clzll(n1 + n2 - 2 ? n1 + n2 - 2 : 1); }
 
-// Estimated device bytes while a request is in flight.
+// Estimated device bytes while a request is in flight: what a request is
+// refused by when it is above the budget.  A product is charged at least what its
+// batch allocates for it (ctx_batch_job_bytes): short products with a transform
+// take more than their part here, and are then admitted one by one.
 uint64_t footprint(int kind, uint64_t na, uint64_t nb) {
   const uint64_t L = 1ull << scale_of(na, nb);
   if (kind == 0) return 16 * (na + nb) + (std::min(na, nb) >= 256 ? 48 * L : 0) + 4096;
@@ -329,6 +333,8 @@ nn_status submit(nn_server* S, Request* R, uint64_t* ticket) {
     delete R;
     return NN_ERR_BUDGET;
   }
+  if (R->kind == 0)
+    R->bytes = std::max(R->bytes, 16 * (R->na + R->nb) + 4096 + nn::ctx_batch_job_bytes(S->ctx, R->na, R->nb));
   {
     std::lock_guard<std::mutex> lk(S->mu);
     if (S->stop) {
@@ -364,6 +370,10 @@ nn_status nn_server_create(int device, uint64_t hbm_budget, int streams, int div
   // streams at once, and a product run on its own (the batch_solo_scale
   // route) would use the context's one carry-scan scratch from each of them.
   nn_context_set_tunable(S->ctx, "batch_solo_scale", 0);
+  // A product's memory is what it was charged, whatever runs beside it: 152
+  // products of 64 x 200 limbs beside one of 2000 x 2000 would take 14.9 MB of
+  // residues at that one's scale, 1.9 MB at their own.
+  nn_context_set_tunable(S->ctx, "batch_few", 0);
   // Product batches run on high-priority streams and divisions (long chains
   // of dependent kernels on the worker contexts) on low-priority ones, so a
   // batch that arrives while a division runs gets the SMs as they free up.
