@@ -1105,7 +1105,15 @@ nn_status nn_transform_inverse_save(nn_context* c, nn_transform* t, uint64_t* d_
 
 nn_status nn_transform_residues(nn_context* c, const nn_transform* t, uint64_t* d_out) {
   if (!c || !t || !t->res || !d_out) return NN_ERR_INVALID;
-  return three_words(c, t, d_out);
+  if (t->rep == nn_transform::kThree || !(reinterpret_cast<std::uintptr_t>(d_out) & 15)) return three_words(c, t, d_out);
+  // the passes read and write 16 bytes at a time
+  DBuf words(c);
+  nn_status st = words.alloc(3ull << t->scale);
+  if (st == NN_OK) st = three_words(c, t, words.p);
+  if (st != NN_OK) return st;
+  NN_CK(c, cudaMemcpyAsync(d_out, words.p, (3ull << t->scale) * sizeof(u64), cudaMemcpyDeviceToDevice, c->stream),
+        "copy residues");
+  return NN_OK;
 }
 
 nn_status nn_mul(nn_context* c, uint64_t* d_out, const uint64_t* a, uint64_t na, const uint64_t* b, uint64_t nb) {
