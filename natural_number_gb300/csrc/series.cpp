@@ -216,8 +216,15 @@ struct Stats {
   u64 gpu_products = 0, host_products = 0, batches = 0;
 };
 
+// An allocation of device memory (or the budget's share of it) that failed.
+struct DeviceMemory : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
 void check_cuda(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) throw std::runtime_error(std::string("natural_gb300: ") + what + ": " + cudaGetErrorString(e));
+  if (e == cudaSuccess) return;
+  cudaGetLastError();  // reported here, once
+  if (e == cudaErrorMemoryAllocation) throw DeviceMemory(std::string("natural_gb300: ") + what);
+  throw std::runtime_error(std::string("natural_gb300: ") + what + ": " + cudaGetErrorString(e));
 }
 
 // Grow-only pinned host buffer.
@@ -365,6 +372,7 @@ nn_batch* device_products(nn_context* c, const std::vector<nn_mul_job>& jobs) {
   if (s == NN_OK) s = nn_batch_launch(c, B, jobs.data());
   if (s != NN_OK) {
     if (B) nn_batch_destroy(c, B);
+    if (s == NN_ERR_OOM || s == NN_ERR_BUDGET) throw DeviceMemory("natural_gb300: tree products");
     nn_gb300::check(s, "tree products");
   }
   return B;
@@ -864,9 +872,9 @@ u64 decimal_digits(const natural& x) {
   return std::abs(l - std::round(l)) < 1e-5 ? 0 : (u64)l + 1;
 }
 
-char* to_dec_levels(nn_context* c, const natural& x, u64 host_below, Staging& stg, Stats& S, u64* len) {
+// lean: nothing is held beyond its level, for conversions that need the memory.
+char* dec_levels(nn_context* c, const natural& x, u64 host_below, Stats& S, u64* len, bool lean) {
   using namespace nn_gb300;
-  (void)stg;
   const int top = dec_init(x);
   if (top < 0) return export_str(std::to_string(x[0]), len);
   DecCache& C = dec_cache();
@@ -895,9 +903,10 @@ char* to_dec_levels(nn_context* c, const natural& x, u64 host_below, Staging& st
   DLevel powers(st);
   std::vector<DNum> dbases(top + 1), dbases_r(top + 1);
   u64 power_words = 0;
-  for (int k = top; split(k); --k) power_words += DLevel::words(C.base[k].size) + DLevel::words(C.base_r[k].size);
-  powers.reserve(power_words);
-  for (int k = top; split(k); --k)
+  for (int k = top; !lean && split(k); --k)
+    power_words += DLevel::words(C.base[k].size) + DLevel::words(C.base_r[k].size);
+  if (power_words) powers.reserve(power_words);
+  for (int k = top; !lean && split(k); --k)
     for (const bool r : {false, true}) {
       const natural& b = r ? C.base_r[k] : C.base[k];
       DNum& d = (r ? dbases_r : dbases)[k] = powers.take(b.size);
@@ -922,7 +931,7 @@ char* to_dec_levels(nn_context* c, const natural& x, u64 host_below, Staging& st
         try {
           plans.push_back(device_products(c, jobs));
           return;
-        } catch (const std::exception&) {
+        } catch (const DeviceMemory&) {
           release_plans(c, before);
         }
       }
@@ -933,7 +942,9 @@ char* to_dec_levels(nn_context* c, const natural& x, u64 host_below, Staging& st
     const u64 nb = base.size, nr = base_r.size;
     const unsigned n_shl = (unsigned)(std::countl_zero(base[nb - 1]) + 1) & 63;
     const u64 shift = ((nb + 2) << 6) - n_shl;  // natural.h:958-960
-    const DNum dbase = dbases[i], dbase_r = dbases_r[i];
+    DLevel own_base(st), own_base_r(st);
+    const DNum dbase = lean ? to_device(own_base, base) : dbases[i],
+               dbase_r = lean ? to_device(own_base_r, base_r) : dbases_r[i];
     const u64 n = nodes.size();
     std::vector<DNum> y(n), hp(n), hi(n), p(n), lo(n);
     u64 w = 0;
@@ -998,6 +1009,7 @@ char* to_dec_levels(nn_context* c, const natural& x, u64 host_below, Staging& st
     S.gpu_products += 2 * n;
     nodes.swap(next);
     cur = std::move(nxt);
+    if (lean) release_plans(c, plans);
   }
   // The nodes left, each below base[i]^2 = 10^(18 * 2^(i+1)): 2^(i+1) groups
   // of 18 digits a node written in place of the tree's leaves
@@ -1043,6 +1055,20 @@ char* to_dec_levels(nn_context* c, const natural& x, u64 host_below, Staging& st
   return out;
 }
 
+char* to_dec_levels(nn_context* c, const natural& x, u64 host_below, Stats& S, u64* len) {
+  for (const bool lean : {false, true}) {
+    Stats attempt = S;
+    try {
+      char* digits = dec_levels(c, x, host_below, attempt, len, lean);
+      S = attempt;
+      return digits;
+    } catch (const DeviceMemory&) {
+      if (lean) throw;
+    }
+  }
+  return nullptr;  // not reached
+}
+
 void fill_timing(double* t, const double* v, int k) {
   if (t)
     for (int i = 0; i < k; ++i) t[i] = v[i];
@@ -1069,7 +1095,7 @@ nn_status nn_pi_dec_levels(nn_context* c, uint64_t terms, uint64_t acc, uint64_t
     num *= denc;
     den = div_on_device(c, den, num);
     const double t_div = since(t0) - t_tree;
-    char* digits_out = to_dec_levels(c, den, host_below, stg, S, len);
+    char* digits_out = to_dec_levels(c, den, host_below, S, len);
     const double t_all = since(t0);
     const double tv[8] = {t_all, t_tree, t_div, t_all - t_tree - t_div, S.gpu_s, S.host_s, (double)S.gpu_products,
                           (double)S.host_products};
@@ -1097,7 +1123,7 @@ nn_status nn_e_dec_levels(nn_context* c, uint64_t terms, uint64_t digits, uint64
     num *= pow(natural(10), digits);
     num = div_on_device(c, num, den);
     const double t_div = since(t0) - t_tree;
-    char* digits_out = to_dec_levels(c, num, host_below, stg, S, len);
+    char* digits_out = to_dec_levels(c, num, host_below, S, len);
     const double t_all = since(t0);
     const double tv[8] = {t_all, t_tree, t_div, t_all - t_tree - t_div, S.gpu_s, S.host_s, (double)S.gpu_products,
                           (double)S.host_products};
@@ -1118,8 +1144,7 @@ nn_status nn_to_dec_levels(nn_context* c, const uint64_t* a, uint64_t na, uint64
   try {
     const natural x = to_natural(a, na);
     Stats S;
-    Staging stg;
-    *out = to_dec_levels(c, x, host_below, stg, S, len);
+    *out = to_dec_levels(c, x, host_below, S, len);
     return *out ? NN_OK : NN_ERR_OOM;
   } catch (const std::bad_alloc&) {
     return NN_ERR_OOM;
