@@ -525,18 +525,16 @@ bool base_case(u64 na, u64 nb) {
 }
 
 // A product of fewer than kNttMulThreshold limbs needs no memory as the base
-// case: it takes that where the transforms' would not fit the budget or, while
-// the stream is captured, their tables are not there yet.
+// case: it takes that where the transforms' would not fit the budget, and while
+// the stream is captured, where their memory would be a part of the graph (which
+// then has one instance at a time and cannot be part of another graph).
 nn_status short_product(nn_context* c, u64* d_out, const nn::SixOperands& op, int s) {
-  bool base = false;
-  if (!nn::six_tables_cover(c->six, s)) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    base = cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
-  }
-  if (!base) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
     const nn_status st = six_product(c, d_out, op, s);
     if (st != NN_ERR_BUDGET && st != NN_ERR_OOM) return st;
   }
+  cudaGetLastError();  // the question's own failure
   const u64* b = op.b ? op.b : op.a;
   NN_CK(c, nn::school_mul(op.a, op.na, b, op.nb, d_out, c->scan, c->stream), "base-case product");
   return NN_OK;

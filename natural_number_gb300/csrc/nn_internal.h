@@ -59,7 +59,6 @@ struct SixTables {
   int2* tab = nullptr;
   u64 cap = 0;
 };
-bool six_tables_cover(const SixTables& t, int s);  // whether they serve scale s already
 cudaError_t six_tables_ensure(SixTables& t, int s, cudaStream_t st, std::vector<u64*>* retired = nullptr);
 void six_tables_free(SixTables& t);
 

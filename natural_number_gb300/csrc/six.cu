@@ -309,14 +309,9 @@ SixPlan six_inverse_plan(int s) {
   return pl;
 }
 
-static u64 tables_need(int s) {
-  return std::max<u64>(8, 1ull << (std::min(std::max(s, kSixMinScale) - 3, kRootLog) - 1));
-}
-bool six_tables_cover(const SixTables& t, int s) { return t.cap >= tables_need(s); }
-
 cudaError_t six_tables_ensure(SixTables& t, int s, cudaStream_t st, std::vector<u64*>* retired) {
-  if (six_tables_cover(t, s)) return cudaSuccess;
-  const u64 need = tables_need(s);
+  const u64 need = std::max<u64>(8, 1ull << (std::min(std::max(s, kSixMinScale) - 3, kRootLog) - 1));
+  if (t.cap >= need) return cudaSuccess;
   // from the size of one-pass transforms at once, then doubling: a handful of
   // growths in a context's life
   const u64 cap = std::max<u64>(need, 1 << 12);
