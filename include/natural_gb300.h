@@ -173,9 +173,9 @@ nn_status nn_batch_mul(nn_context* ctx, const nn_mul_job* jobs, uint64_t count);
  * streams of one context need 0, since those passes share the context's
  * carry-scan scratch, as nn_mul calls on two streams do), "batch_few" (1, the
  * default: in a batch of up to 152 products, those whose operands fit a one-pass
- * transform take the largest such one of the batch, and those of up to 2^14 limbs
- * are not split, for fewer launches and more memory; 0: each as it would in a
- * larger batch, or in a context with a budget). */
+ * transform take the largest such one of the batch, and beside a longer transform
+ * those of up to 2^14 limbs are not split, for fewer launches and more memory; 0:
+ * each as it would in a larger batch, or in a context with a budget). */
 nn_status nn_context_set_tunable(nn_context* ctx, const char* name, int64_t value);
 int64_t nn_context_get_tunable(const nn_context* ctx, const char* name);
 

@@ -606,10 +606,10 @@ bool batch_columns(const nn_context* c, u64 na, u64 nb) {
   return mn < c->batch_ntt_min || (mn < c->batch_school_balanced && mx <= 2 * mn);
 }
 
-// J's pieces, plan and rows from its sizes (na >= nb) and `square`.  few: one of
-// a few products; those of a scale up to few_s take that.
-BatchRoute batch_route(const nn_context* c, nn::BatchJob& J, bool few, int few_s) {
-  constexpr int kFewUnsplit = 14;
+// J's pieces, plan and rows from its sizes (na >= nb) and `square`; one of a
+// scale up to few_s takes that, and one of a scale up to `whole` its own, unsplit
+// (0: none).
+BatchRoute batch_route(const nn_context* c, nn::BatchJob& J, int few_s, int whole) {
   J.piece = J.na;
   J.pieces = 1;
   if (batch_columns(c, J.na, J.nb)) return BatchRoute::kColumns;
@@ -617,8 +617,10 @@ BatchRoute batch_route(const nn_context* c, nn::BatchJob& J, bool few, int few_s
   // From this scale on one product fills the GPU by itself: no items, no
   // arena; the launch runs it alone.
   if (c->batch_solo_scale > 0 && s >= c->batch_solo_scale) return BatchRoute::kSolo;
-  if (s <= few_s) s = few_s;
-  if (c->batch_split && !J.square && !(few && s <= kFewUnsplit)) s = six_split(J.na, J.nb, s, &J.piece, &J.pieces);
+  if (s <= few_s)
+    s = few_s;
+  else if (c->batch_split && !J.square && s > whole)
+    s = six_split(J.na, J.nb, s, &J.piece, &J.pieces);
   if (s > nn::kSixMaxScale) return BatchRoute::kTooLong;
   J.plan = nn::six_plan(s, J.pieces > 1 ? 1ull << s : J.na + J.nb - 1, c->batch_r_last_at[s]);
   J.rows = J.pieces > 1 ? nn::kBatchRowsB : J.plan.n > 1 && !c->batch_fused ? nn::kBatchRowsAll : nn::kBatchRowsNone;
@@ -645,17 +647,26 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
   // A few short products are bound by the number of launches, not by their
   // work: up to 152 jobs whose operands fit one pass take one scale, the
   // largest such one of the batch, so that their passes are one launch (six
-  // CTAs a job, under a wave), and products of up to 2^14 limbs are not split.
-  // (Contexts with a budget, or "batch_few" 0, keep the smaller arenas.)  64
-  // jobs of 8 to 1024 limbs: 68 us before, 62 us so; 111 of 44 to 6439 limbs 194
-  // and 190 us.
-  constexpr int kOnePass = 12;
+  // CTAs a job, under a wave), and where the batch has launches of two passes
+  // anyhow, products of up to 2^14 limbs are not split.  (Contexts with a budget,
+  // or "batch_few" 0, keep the smaller arenas.)  With and without, us: 64 jobs of
+  // 8 to 1024 limbs 38 and 45, one of 2000 x 2000 limbs beside 150 of 64 x 200 43
+  // and 50, beside 150 of 120 x 120 42 and 48, 111 of 44 to 6439 limbs 120 and 144.
+  // Unsplit by themselves five products of 16000 x 300 limbs take 137, split 31.
+  constexpr int kOnePass = 12, kFewWhole = 14;
   const bool few = c->batch_few && count <= 152 && !c->budget;
-  int few_s = 0;
+  int few_s = 0, whole = 0;
   for (u64 j = 0; few && j < count; ++j) {
-    if (!na[j] || !nb[j]) continue;
-    const int s = ntt_scale(na[j], nb[j]);
-    if (s <= kOnePass && std::min(na[j], nb[j]) >= c->batch_ntt_min) few_s = std::max(few_s, s);
+    const u64 mx = std::max(na[j], nb[j]), mn = std::min(na[j], nb[j]);
+    if (!mn || mn < c->batch_ntt_min) continue;
+    const int s = ntt_scale(mx, mn);
+    if (s <= kOnePass) {
+      few_s = std::max(few_s, s);
+    } else if (!whole && (c->batch_solo_scale == 0 || s < c->batch_solo_scale)) {
+      u64 piece, pieces = 1;
+      if (c->batch_split && !(square && square[j])) six_split(mx, mn, s, &piece, &pieces);
+      if (pieces == 1) whole = kFewWhole;
+    }
   }
   for (u64 j = 0; j < count; ++j) {
     if (!na[j] || !nb[j]) {
@@ -683,7 +694,7 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
     B->swap[j] = na[j] < nb[j];
     J.na = std::max(na[j], nb[j]);
     J.nb = std::min(na[j], nb[j]);
-    const BatchRoute route = batch_route(c, J, few, few_s);
+    const BatchRoute route = batch_route(c, J, few_s, whole);
     if (route == BatchRoute::kSolo) {
       B->solo.push_back(j);
       continue;
@@ -872,7 +883,7 @@ u64 ctx_batch_job_bytes(const nn_context* c, u64 na, u64 nb) {
   BatchJob J{};
   J.na = std::max(na, nb);
   J.nb = std::min(na, nb);
-  if (batch_route(c, J, false, 0) != BatchRoute::kTransforms) return (na + nb) / 16;  // an item and a flag a tile
+  if (batch_route(c, J, 0, 0) != BatchRoute::kTransforms) return (na + nb) / 16;  // an item and a flag a tile
   const u64 bytes = 8 * (batch_words_a(J) + batch_words_b(J));
   return bytes + bytes / 512;  // its items: 12 bytes for 8192 words of a prime, a pass
 }
