@@ -500,6 +500,9 @@ namespace {
 struct TwoTo64 {
   u64 w[3], s[3];
 };
+// HALVES: out is res itself; a word's halves go where two of its coefficient's
+// residues were.
+template <bool HALVES>
 __global__ void __launch_bounds__(256) six_to_three_kernel(const u32* res, u64 L, u64* out, const TwoTo64 b) {
   grid_begin();
   const u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -512,8 +515,29 @@ __global__ void __launch_bounds__(256) six_to_three_kernel(const u32* res, u64 L
     u64 r = limb_mod(v.w2, m, p, ch);
     r = reduce2p(shoup_mul(r, b.w[i], b.s[i], p, ch) + limb_mod(v.w1, m, p, ch), p);
     r = reduce2p(shoup_mul(r, b.w[i], b.s[i], p, ch) + limb_mod(v.w0, m, p, ch), p);
-    out[i * L + k] = r;
+    if (HALVES) {
+      u32* half = reinterpret_cast<u32*>(out) + 2 * i * L + k;
+      half[0] = (u32)r;
+      half[L] = (u32)(r >> 32);
+    } else {
+      out[i * L + k] = r;
+    }
   }
+}
+// One of the two steps that bring the halves together, a plane of 2^bits of them
+// (all low ones, then all high ones) a blockIdx.y: half j belongs at j rotated
+// left by one bit, which is the reversal of its bits and then that of all but the
+// lowest.  Either is its own inverse, so it goes by swaps, in place.
+__global__ void __launch_bounds__(256) swap_halves_kernel(u32* x, int bits, bool all) {
+  grid_begin();
+  const u32 j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >> bits) return;
+  const u32 q = all ? __brev(j) >> (32 - bits) : (j & 1) | (__brev(j >> 1) >> (33 - bits)) << 1;
+  if (j >= q) return;
+  x += (u64)blockIdx.y << bits;
+  const u32 t = x[j];
+  x[j] = x[q];
+  x[q] = t;
 }
 }  // namespace
 
@@ -526,9 +550,17 @@ cudaError_t six_to_three(const u32* res, int s, u64* out, cudaStream_t st) {
     b.s[i] = (u64)(((unsigned __int128)b.w[i] << 64) / p[i]) + 1;
   }
   const u64 L = 1ull << s;
+  const bool in_place = static_cast<const void*>(res) == out;
   launch_begin("six_to_three", st);
-  const cudaError_t e = launch_next(six_to_three_kernel, (unsigned)((L + 255) / 256), 256, 0, 0, st, res, L, out, b);
+  cudaError_t e = launch_next(in_place ? six_to_three_kernel<true> : six_to_three_kernel<false>,
+                              (unsigned)((L + 255) / 256), 256, 0, 0, st, res, L, out, b);
   launch_end(st);
+  for (int step = 0; in_place && step < 2 && e == cudaSuccess; ++step) {
+    launch_begin("swap_halves", st);
+    e = launch_next(swap_halves_kernel, dim3((unsigned)((2 * L + 255) / 256), 3), 256, 0, 0, st,
+                    reinterpret_cast<u32*>(out), s + 1, step == 0);
+    launch_end(st);
+  }
   return e;
 }
 

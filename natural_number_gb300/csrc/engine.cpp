@@ -227,6 +227,16 @@ struct DBuf {
   ~DBuf() { dev_free(c, p, words); }
 };
 
+bool short_of_memory(nn_status st) { return st == NN_ERR_BUDGET || st == NN_ERR_OOM; }
+
+// Whether the context's stream is captured (or cannot tell).
+bool capturing(const nn_context* c) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess) return capture != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 nn_status xform_reserve(nn_context* c, nn_transform* t, int s) {
   const u64 need = 3ull << s;
   if (t->words < need) {
@@ -290,27 +300,57 @@ nn_status forward(nn_context* c, nn_transform* t, const u64* d_limbs, u64 n, int
 }
 
 // t's residues modulo the three primes, as the reference's transform has
-// them, into dst: a six-prime transform's coefficients, reduced, through the
-// three-prime forward passes.
+// them, into dst (on a 16-byte boundary): a six-prime transform's coefficients,
+// reduced, through the three-prime forward passes.
 nn_status three_words(nn_context* c, const nn_transform* t, u64* dst) {
   if (t->rep == nn_transform::kThree) {
     NN_CK(c, cudaMemcpyAsync(dst, t->res, (3ull << t->scale) * sizeof(u64), cudaMemcpyDeviceToDevice, c->stream),
           "copy residues");
     return NN_OK;
   }
+  NN_CK(c, nn::tables_ensure(c->tables, t->scale, c->stream, &c->retired_tables), "twiddle tables");
   DBuf tmp(c);
   const nn::u32* w = t->six();
   if (t->rep == nn_transform::kSixForward) {
-    nn_status st = tmp.alloc(3ull << t->scale);
-    if (st != NN_OK) return st;
-    nn::u32* back = reinterpret_cast<nn::u32*>(tmp.p);
+    const nn_status st = tmp.alloc(3ull << t->scale);
+    if (st != NN_OK && !short_of_memory(st)) return st;
+    nn::u32* back = reinterpret_cast<nn::u32*>(st == NN_OK ? tmp.p : dst);
     NN_CK(c, nn::six_inverse(back, w, nn::six_inverse_plan(t->scale), c->six, c->stream), "inverse NTT");
     w = back;
   }
-  NN_CK(c, nn::tables_ensure(c->tables, t->scale, c->stream, &c->retired_tables), "twiddle tables");
   NN_CK(c, nn::six_to_three(w, t->scale, dst, c->stream), "residues");
   NN_CK(c, nn::ntt_forward_residues(dst, t->scale, c->tables, c->stream, c->passes(t->scale)), "forward NTT");
   return NN_OK;
+}
+
+// The same in t's own memory: the transform is still the same one.  Not while
+// the stream is captured, where t changes with every replay.
+nn_status become_three(nn_context* c, nn_transform* t) {
+  NN_CK(c, nn::tables_ensure(c->tables, t->scale, c->stream, &c->retired_tables), "twiddle tables");
+  if (t->rep == nn_transform::kSixForward) {
+    NN_CK(c, nn::six_inverse(t->six(), t->six(), nn::six_inverse_plan(t->scale), c->six, c->stream), "inverse NTT");
+    t->rep = nn_transform::kSixProduct;
+  }
+  NN_CK(c, nn::six_to_three(t->six(), t->scale, t->res, c->stream), "residues");
+  t->rep = nn_transform::kThree;
+  NN_CK(c, nn::ntt_forward_residues(t->res, t->scale, c->tables, c->stream, c->passes(t->scale)), "forward NTT");
+  NN_CK(c, nn::ntt_canonical(t->res, t->scale, c->stream), "forward NTT");  // it may be taken back alone
+  return NN_OK;
+}
+
+// t's three-prime words: its own, or a copy in tmp, or, where there is no memory
+// for one (a product of three factors took none when every transform had three
+// primes), t's own from now on.
+nn_status three_operand(nn_context* c, const nn_transform* t, DBuf& tmp, const u64** words) {
+  *words = t->res;
+  if (t->rep == nn_transform::kThree) return NN_OK;
+  nn_status st = tmp.alloc(3ull << t->scale);
+  if (st == NN_OK) {
+    *words = tmp.p;
+    return three_words(c, t, tmp.p);
+  }
+  if (!short_of_memory(st) || capturing(c)) return st;
+  return become_three(c, const_cast<nn_transform*>(t));
 }
 
 // A forward transform goes back in place: only kernels on the stream, as a
@@ -344,18 +384,10 @@ nn_status pointwise(nn_context* c, nn_transform* dst, const nn_transform* a, con
     return NN_OK;
   }
   DBuf ta(c), tb(c);
-  const u64 *pa = a->res, *pb = b->res;
-  nn_status st = NN_OK;
-  if (a->rep != nn_transform::kThree) {
-    st = ta.alloc(3ull << s);
-    if (st == NN_OK) st = three_words(c, a, ta.p);
-    pa = ta.p;
-  }
-  if (st == NN_OK && b->rep != nn_transform::kThree) {
-    st = tb.alloc(3ull << s);
-    if (st == NN_OK) st = three_words(c, b, tb.p);
-    pb = tb.p;
-  }
+  const u64 *pa = nullptr, *pb = nullptr;
+  nn_status st = three_operand(c, a, ta, &pa);
+  if (st == NN_OK && b != a) st = three_operand(c, b, tb, &pb);
+  if (b == a) pb = pa;
   if (st == NN_OK) st = xform_reserve(c, dst, s);
   if (st != NN_OK) return st;
   NN_CK(c, nn::tables_ensure(c->tables, s, c->stream, &c->retired_tables), "twiddle tables");
@@ -529,12 +561,10 @@ bool base_case(u64 na, u64 nb) {
 // the stream is captured, where their memory would be a part of the graph (which
 // then has one instance at a time and cannot be part of another graph).
 nn_status short_product(nn_context* c, u64* d_out, const nn::SixOperands& op, int s) {
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+  if (!capturing(c)) {
     const nn_status st = six_product(c, d_out, op, s);
-    if (st != NN_ERR_BUDGET && st != NN_ERR_OOM) return st;
+    if (!short_of_memory(st)) return st;
   }
-  cudaGetLastError();  // the question's own failure
   const u64* b = op.b ? op.b : op.a;
   NN_CK(c, nn::school_mul(op.a, op.na, b, op.nb, d_out, c->scan, c->stream), "base-case product");
   return NN_OK;
@@ -1116,11 +1146,11 @@ nn_status nn_transform_residues(nn_context* c, const nn_transform* t, uint64_t* 
   if (!c || !t || !t->res || !d_out) return NN_ERR_INVALID;
   if (t->rep == nn_transform::kThree || !(reinterpret_cast<std::uintptr_t>(d_out) & 15)) return three_words(c, t, d_out);
   // the passes read and write 16 bytes at a time
-  DBuf words(c);
-  nn_status st = words.alloc(3ull << t->scale);
-  if (st == NN_OK) st = three_words(c, t, words.p);
+  DBuf tmp(c);
+  const u64* words = nullptr;
+  const nn_status st = three_operand(c, t, tmp, &words);
   if (st != NN_OK) return st;
-  NN_CK(c, cudaMemcpyAsync(d_out, words.p, (3ull << t->scale) * sizeof(u64), cudaMemcpyDeviceToDevice, c->stream),
+  NN_CK(c, cudaMemcpyAsync(d_out, words, (3ull << t->scale) * sizeof(u64), cudaMemcpyDeviceToDevice, c->stream),
         "copy residues");
   return NN_OK;
 }

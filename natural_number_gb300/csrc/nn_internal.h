@@ -200,6 +200,8 @@ cudaError_t ntt_forward(const u64* limbs, u64 n, u64* res, int s, const Tables& 
                         const std::vector<Pass>* plan = nullptr);
 // The forward passes over coefficients that are already residues [3][2^s] below p.
 cudaError_t ntt_forward_residues(u64* res, int s, const Tables& t, cudaStream_t st, const std::vector<Pass>& plan);
+// A forward transform's lazy values to [0, p), as ntt_inverse takes them.
+cudaError_t ntt_canonical(u64* res, int s, cudaStream_t st);
 // Pointwise product of degree-1 residues (ntt_info.h:224-231); dst may alias a or b.
 cudaError_t ntt_pointwise(u64* dst, const u64* a, const u64* b, int s, const Tables& t, cudaStream_t st);
 // Inverse transform with the final 2^-(s-1) scale (ntt_info.h:200-221); values in [0,p).
@@ -221,7 +223,7 @@ cudaError_t six_save(const SixOperands& op, const SixPlan& pl, u64* out, Scan& s
 // as ntt_save below.
 cudaError_t six_save_words(const u32* res, int s, u64* out, u64 size, Scan& sc, u64* written, cudaStream_t st);
 // The coefficients of product residues [6][2^s] reduced modulo the three
-// 62-bit primes: [3][2^s].
+// 62-bit primes: [3][2^s], s < 31; out may be res, apart from it otherwise.
 cudaError_t six_to_three(const u32* res, int s, u64* out, cudaStream_t st);
 // CRT + carry into `size` limbs (normal mode) or the wrapped product mod
 // B^L - 1 in L limbs when size-1 > L (ntt_info.h:237-248).  Returns the

@@ -132,6 +132,14 @@ __global__ void __launch_bounds__(256) pointwise_kernel(u64* dst, const u64* a, 
   pointwise_group(dst, a, b, L, tab, tab_stride, blockIdx.y, g);
 }
 
+// The forward passes' lazy values to [0, p), as the inverse passes take them.
+__global__ void __launch_bounds__(256) canonical_kernel(u64* res, u64 L) {
+  const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= L) return;
+  u64& x = res[blockIdx.y * L + i];
+  x = blockIdx.y == 0 ? canon_c<0>(x) : blockIdx.y == 1 ? canon_c<1>(x) : canon_c<2>(x);
+}
+
 // Strided pass over residues with TMA: one CTA's tile (16 columns x 2^R
 // rows of one prime, R <= 9) is one or two boxes of the 3-D view
 // [3 * 2^lambda0 super-blocks][2^R rows][2^lg_s columns] of the residues,
@@ -707,6 +715,14 @@ cudaError_t ntt_pointwise(u64* dst, const u64* a, const u64* b, int s, const Tab
   dim3 grid((unsigned)((groups + 255) / 256), 3);
   launch_begin("ntt_pointwise", st);
   pointwise_kernel<<<grid, 256, 0, st>>>(dst, a, b, 1ull << s, t.root, t.cap);
+  launch_end(st);
+  return cudaGetLastError();
+}
+
+cudaError_t ntt_canonical(u64* res, int s, cudaStream_t st) {
+  const u64 L = 1ull << s;
+  launch_begin("ntt_canonical", st);
+  canonical_kernel<<<dim3((unsigned)((L + 255) / 256), 3), 256, 0, st>>>(res, L);
   launch_end(st);
   return cudaGetLastError();
 }
