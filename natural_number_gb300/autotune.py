@@ -6,8 +6,8 @@ Sweeps, on the GPU it runs on:
     scale (the three-prime passes, which serve nn_ntt_mul); and the
     levels of the contiguous pass of batched products ("batch_r_last@s");
   - the batch shapes: the shortest operand sent down the NTT route in a batch
-    ("batch_ntt_min") and the residues a pass item covers
-    ("batch_item_words"), timed on the uneven-size workload.
+    ("batch_ntt_min", "batch_school_balanced") and the residues a pass item
+    covers ("batch_item_words"), timed on the uneven-size workload.
 Every candidate's product is checked against the first candidate's (all
 choices compute the same exact product).  Writes the best values to
 tuning.json beside this file; Context() applies that file at creation
@@ -125,33 +125,37 @@ def tune_batch_scales(ctx, scales) -> tuple[dict, dict]:
 
 def tune_batch(ctx, jobs: int) -> tuple[dict, dict]:
     """The shortest operand sent down the NTT route and the residues per pass
-    item, on an uneven workload of `jobs` products; every
-    setting must give the same products."""
+    item, then the base case of balanced products, on an uneven workload of
+    `jobs` products; every setting must give the same products."""
     import torch
 
     from .workloads import UnevenProducts
     W = UnevenProducts(jobs, seed=5)
-    results = {}
     ref = None
-    for ntt_min in (48, 64, 96, 128):
-        for item in (8192, 16384, 32768):
-            ctx.set_tunable("batch_ntt_min", ntt_min)
-            ctx.set_tunable("batch_item_words", item)
-            plan = ctx.batch(W.sa, W.sb)
-            ms = _time(lambda: plan.run_jobs(W.jobs_batch), 3)
-            ctx.synchronize()
-            if ref is None:
-                ref = W.out_batch.clone()
-            elif not torch.equal(ref, W.out_batch):
-                raise RuntimeError(f"ntt_min={ntt_min} item={item} changed a product")
-            plan.close()
-            results[f"{ntt_min},{item}"] = ms
-    best = min(results, key=results.get)
-    ntt_min, item = map(int, best.split(","))
-    ctx.set_tunable("batch_ntt_min", ntt_min)
-    ctx.set_tunable("batch_item_words", item)
-    return ({"batch_ntt_min": ntt_min, "batch_item_words": item},
-            {"batch_%d_ms" % jobs: results})
+
+    def ms(settings: dict) -> float:
+        nonlocal ref
+        for name, value in settings.items():
+            ctx.set_tunable(name, value)
+        plan = ctx.batch(W.sa, W.sb)
+        t = _time(lambda: plan.run_jobs(W.jobs_batch), 3)
+        ctx.synchronize()
+        plan.close()
+        if ref is None:
+            ref = W.out_batch.clone()
+        elif not torch.equal(ref, W.out_batch):
+            raise RuntimeError(f"{settings} changed a product")
+        return t
+
+    shapes = {f"{ntt_min},{item}": ms({"batch_ntt_min": ntt_min, "batch_item_words": item})
+              for ntt_min in (48, 64, 96, 128) for item in (1024, 2048, 4096, 8192, 16384, 32768)}
+    ntt_min, item = map(int, min(shapes, key=shapes.get).split(","))
+    best = {"batch_ntt_min": ntt_min, "batch_item_words": item}
+    balanced = {str(v): ms({**best, "batch_school_balanced": v}) for v in (0, 96, 112, 128, 192, 256, 384)}
+    best["batch_school_balanced"] = int(min(balanced, key=balanced.get))
+    for name, value in best.items():
+        ctx.set_tunable(name, value)
+    return best, {"batch_%d_ms" % jobs: shapes, "batch_%d_balanced_ms" % jobs: balanced}
 
 
 def main() -> None:
@@ -171,10 +175,10 @@ def main() -> None:
     b, l = tune_passes(ctx, [int(x) for x in args.n_exps.split(",")])
     best.update(b)
     log.update(l)
-    b, l = tune_batch_scales(ctx, [int(x) for x in args.batch_scales.split(",")])
+    b, l = tune_batch(ctx, args.jobs)
     best.update(b)
     log.update(l)
-    b, l = tune_batch(ctx, args.jobs)
+    b, l = tune_batch_scales(ctx, [int(x) for x in args.batch_scales.split(",")])
     best.update(b)
     log.update(l)
     doc = {"tunables": best, "device": torch.cuda.get_device_name(0), "seconds": round(time.time() - t0, 1),

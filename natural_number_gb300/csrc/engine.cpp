@@ -796,6 +796,9 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
     auto& v = launches[{8, J.pieces > 1 ? nn::kBatchPieceCrt : nn::kBatchCrt, 0, 0, 0}];
     for (u64 t = 0; t < nn::scan_tiles(J.na + J.nb); ++t) v.push_back(item(t, 1, 0, 0));
   }
+  u64 total = 0;
+  for (const auto& [key, v] : launches) total += v.size();
+  B->items.reserve(total);
   for (auto& [key, v] : launches) {
     if (B->items.size() + v.size() >= 0xffffffffull) {
       c->err = "batch: too many work items";
