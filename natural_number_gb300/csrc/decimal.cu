@@ -92,6 +92,11 @@ __device__ __forceinline__ void put18(char* o, u64 x) {
 // (512 groups each): 0.45 ms; with one warp a node, every division split over
 // its lanes by a scan of remainder maps, 1.2 ms.
 constexpr int kDecStep = 16, kDecRing = 64, kDecMaxWarps = 16;
+constexpr u64 kDecMaxLimbs = 8192;
+// Shared memory of a node of `limbs` in the lanes of `warps`.
+constexpr int dec_smem(u64 warps, u64 limbs) {
+  return (int)(32 * warps * ((limbs + 32 * warps - 1) / (32 * warps) | 1) * 8);
+}
 __global__ void __launch_bounds__(32 * kDecMaxWarps) dec_groups_kernel(const u64* const* __restrict__ nodes,
                                                                        const u32* __restrict__ len, u32 groups, u64 v,
                                                                        char* out) {
@@ -242,17 +247,16 @@ __global__ void __launch_bounds__(256) dec_inc_kernel(const DecFixJob* __restric
 cudaError_t dec_groups(const u64* const* nodes, u64 stride, const u32* len, u64 n, u32 groups, char* out,
                        cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  if (stride > 8192 || stride % 2) return cudaErrorInvalidValue;
+  if (stride > kDecMaxLimbs || stride % 2) return cudaErrorInvalidValue;
   const unsigned __int128 all = ~(unsigned __int128)0;
   const u64 v = (u64)(all / kGroupNorm);  // floor((2^128-1)/d) - 2^64: the 2^64 bit drops in the cast
   // four limbs a lane, up to the most warps
   const u64 warps = std::max<u64>(1, std::min<u64>(kDecMaxWarps, (stride + 127) / 128));
-  const u64 seg = (stride + 32 * warps - 1) / (32 * warps);  // the longest node's; shorter ones take less
-  const int smem = (int)(32 * warps * (seg | 1) * 8);
-  if (smem > 32 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(dec_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
+  const int smem = dec_smem(warps, stride);  // the longest node's; shorter ones take less
+  // the most that any call wants, so that no other thread's call takes it back before this one's launch
+  static DeviceOnce once;
+  if (const cudaError_t e = allow_smem<dec_smem(kDecMaxWarps, kDecMaxLimbs)>(once, dec_groups_kernel); e != cudaSuccess)
+    return e;
   launch_begin("dec_groups", st);
   dec_groups_kernel<<<(unsigned)n, (unsigned)(32 * warps), smem, st>>>(nodes, len, groups, v, out);
   launch_end(st);
