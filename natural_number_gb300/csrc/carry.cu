@@ -398,29 +398,31 @@ cudaError_t run_scan(const Prod& prod, u64 total, u64* out, u64 out_limit, Scan&
   tile_end = std::min(tile_end, tiles);
   cudaError_t e = scan_reserve(sc, tiles);
   if (e != cudaSuccess || tile_end <= tile_begin) return e;
-  const bool whole = tile_begin == 0 && tile_end == tiles;
-  constexpr u64 kSmallTile = kScanSmall * kScanE;
-  const u64 small = (total + kSmallTile - 1) / kSmallTile;
-  if (whole && small <= kClusterTiles) {
-    launch_begin(name, st);
-    e = launch_next(scan_cluster_kernel<Prod>, (unsigned)small, kScanSmall, 0, (unsigned)small, st, prod, total, out,
-                    out_limit, sc.side);
-    launch_end(st);
-    return e;
+  // the short ones, whole: column sums come here only beyond them (school_mul)
+  if constexpr (Prod::kBulk) {
+    const bool whole = tile_begin == 0 && tile_end == tiles;
+    constexpr u64 kSmallTile = kScanSmall * kScanE;
+    const u64 small = (total + kSmallTile - 1) / kSmallTile;
+    if (whole && small <= kClusterTiles) {
+      launch_begin(name, st);
+      e = launch_next(scan_cluster_kernel<Prod>, (unsigned)small, kScanSmall, 0, (unsigned)small, st, prod, total, out,
+                      out_limit, sc.side);
+      launch_end(st);
+      return e;
+    }
+    if (whole && small <= kSmallTiles) {
+      launch_begin(name, st);
+      e = launch_next(scan_kernel<Prod, kScanSmall>, (unsigned)small, kScanSmall, 0, 0, st, prod, total, out, out_limit,
+                      sc.side, sc.flags, 0);
+      launch_end(st);
+      return e == cudaSuccess ? carry_fix<kSmallTile>(0, small, total, out, out_limit, sc, st) : e;
+    }
   }
-  const bool short_tiles = whole && small <= kSmallTiles;
-  const u64 n = short_tiles ? small : tile_end - tile_begin;
   launch_begin(name, st);
-  if (short_tiles)
-    e = launch_next(scan_kernel<Prod, kScanSmall>, (unsigned)n, kScanSmall, 0, 0, st, prod, total, out, out_limit,
-                    sc.side, sc.flags, 0);
-  else
-    e = launch_next(scan_kernel<Prod, kScanThreads>, (unsigned)n, kScanThreads, 0, 0, st, prod, total, out, out_limit,
-                    sc.side, sc.flags, tile_begin);
+  e = launch_next(scan_kernel<Prod, kScanThreads>, (unsigned)(tile_end - tile_begin), kScanThreads, 0, 0, st, prod, total,
+                  out, out_limit, sc.side, sc.flags, tile_begin);
   launch_end(st);
-  if (e != cudaSuccess) return e;
-  return short_tiles ? carry_fix<kSmallTile>(0, n, total, out, out_limit, sc, st)
-                     : carry_fix<kScanTile>(tile_begin, tile_end, total, out, out_limit, sc, st);
+  return e == cudaSuccess ? carry_fix<kScanTile>(tile_begin, tile_end, total, out, out_limit, sc, st) : e;
 }
 
 template <u64 TILE>
