@@ -72,7 +72,11 @@ void nn_transform_set_scale(nn_transform* t, int scale);
  * (ntt_info.h:180-198): residues of n <= 2^scale limbs under the three primes,
  * transformed.  Grows the twiddle tables as NTT_info::init does (ntt_info.h:22-41). */
 nn_status nn_transform_forward(nn_context* ctx, nn_transform* t, const uint64_t* d_limbs, uint64_t n, int scale);
-/* NTT_info::mul (ntt_info.h:224-231): dst = a (.) b; dst may be a or b. */
+/* NTT_info::mul (ntt_info.h:224-231): dst = a (.) b; dst may be a or b.  Where
+ * one of them is a product already, copies of up to 3 * 2^scale words an operand
+ * are taken from the budget; an operand whose copy has no room changes its words
+ * in place (the transform stays the same: calls that use it on other streams must
+ * then be ordered with this one). */
 nn_status nn_transform_pointwise(nn_context* ctx, nn_transform* dst, const nn_transform* a, const nn_transform* b);
 /* NTT_info::INTT (ntt_info.h:200-221) followed by NTT_info::save
  * (ntt_info.h:237-248): writes `size` limbs, or, when size-1 > 2^scale (wrap
@@ -313,7 +317,7 @@ nn_status nn_e_dec_host(nn_context* ctx, uint64_t terms, uint64_t digits, char**
  * limbs (on a GB300 with 16 host cores: 128 for pi, 256 for e), run whole on
  * host threads.  The decimal split
  * runs its levels while the split powers have at least host_below limbs;
- * the nodes left become digits on the device (one thread a node peels off
+ * the nodes left become digits on the device (one CTA a node peels off
  * 18-digit groups, natural.h:566-573 and 994-1011) and come back in one copy.
  * terms must be a power of two (the trees are then perfect).  timing (8
  * doubles, may be NULL): total s, tree s, division s, decimal s, GPU-batch s,

@@ -153,7 +153,7 @@ struct nn_batch {
   std::vector<nn::BatchSegment> segments;  // the launches, in order
   std::vector<u64> off_a, off_b;
   std::vector<char> swap;  // NTT job whose second operand is the longer one
-  std::vector<u64> solo;   // jobs run one at a time after the batch kernel
+  std::vector<u64> solo;   // jobs run one at a time after the launches
   u64 arena_words = 0;
   nn::u32 n_flags = 0;
   nn::BatchJob* d_jobs = nullptr;
@@ -624,7 +624,7 @@ nn_status scratch(nn_context* c, int slot, u64 words, u64** p) {
 }
 
 // ---------------------------------------------------------------------------
-// Batches: a work queue over all jobs' pipeline steps (batch.cu).
+// Batches: launches of one step and tile shape over all jobs (batch.cu).
 // ---------------------------------------------------------------------------
 
 // How a product of a batch runs: as column sums (plan.s 0), through transforms,

@@ -812,16 +812,6 @@ const T* table(nn_context* c, DLevel& L, const std::vector<T>& v) {
   return reinterpret_cast<const T*>(L.p);
 }
 
-// Decimal digits (std::formatter<natural>, natural.h:1089-1091) into a
-// malloc'd, NUL-terminated buffer of *len digits: the split tree of
-// _format_dec, level by level while the split powers have at least
-// host_below limbs, all in device memory: a level's products (hi = base_r *
-// (v >> ..) >> shift, then base * hi) run as two batches, the shift as one
-// launch, lo = v - base * hi as one batched difference and the correction
-// loop (natural.h:962-965) as one launch, one warp a node; the nodes left
-// become digits on the device, one warp a node (decimal.cu), and the string
-// comes back in one copy.  Only node 0, the first, can end with hi = 0 and
-// then splits into its lo alone: one flag a level comes back for it.
 // The split's correction for a level of a few long nodes: dec_fix walks each
 // node with one warp, which for nodes of hundreds of thousands of limbs is a
 // long serial walk; here the test runs one warp a node, every subtraction
@@ -872,6 +862,17 @@ u64 decimal_digits(const natural& x) {
   return std::abs(l - std::round(l)) < 1e-5 ? 0 : (u64)l + 1;
 }
 
+// Decimal digits (std::formatter<natural>, natural.h:1089-1091) into a
+// malloc'd, NUL-terminated buffer of *len digits: the split tree of
+// _format_dec, level by level while the split powers have at least
+// host_below limbs, all in device memory: a level's products (hi = base_r *
+// (v >> ..) >> shift, then base * hi) run as two batches, the shift as one
+// launch, lo = v - base * hi as one batched difference and the correction
+// loop (natural.h:962-965) as one launch, one warp a node; the nodes left
+// become digits on the device, one CTA a node (decimal.cu), and the string
+// comes back in one copy.  Only node 0, the first, can end with hi = 0 and
+// then splits into its lo alone: x's number of digits tells, or, where that is
+// not known, one flag that comes back.
 // lean: nothing is held beyond its level, for conversions that need the memory.
 char* dec_levels(nn_context* c, const natural& x, u64 host_below, Stats& S, u64* len, bool lean) {
   using namespace nn_gb300;
