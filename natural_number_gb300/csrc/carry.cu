@@ -196,15 +196,6 @@ __global__ void __launch_bounds__(kScanSmall) scan_cluster_kernel(Prod prod, u64
   cluster_sync();
 }
 
-// acc += x * y as one carry chain.
-__device__ __forceinline__ void mac(W3& acc, u64 x, u64 y) {
-  asm("mad.lo.cc.u64 %0, %3, %4, %0;\n\t"
-      "madc.hi.cc.u64 %1, %3, %4, %1;\n\t"
-      "addc.u64 %2, %2, 0;"
-      : "+l"(acc.w0), "+l"(acc.w1), "+l"(acc.w2)
-      : "l"(x), "l"(y));
-}
-
 // Base-case products of up to sixteen tiles of 64 positions: one cluster.  The
 // shorter operand and the window of the longer one that a tile needs come
 // into shared memory, padded with zeros; sixteen lanes share four columns,
@@ -275,16 +266,20 @@ __global__ void __launch_bounds__(256) school_cluster_kernel(ColumnProducer prod
 
 // Longer base-case products: each CTA forms its tile's column sums in shared
 // memory, eight lanes a position, and runs the scan's first step on them.
-// Small tiles spread a short product over the GPU: the column sums are the
-// work, up to 383 terms a position.  Longer operands here have few terms a
-// position, and beyond kSchoolLong a thread forms those of eight positions by
-// itself (run_scan).  Measured, us, tiles of 64 / 256 / 1024 positions / run_scan:
-// 1500 x 40 limbs 4.9 / 8.5 / 23.0, 32768 x 16 7.6 / 8.1 / 20.2, 65000 x 31 13.8 /
-// 12.4 / 26.7 / 18.2, 131072 x 16 18.5 / 14.9 / 20.4 / 15.7, 262144 x 31 42.1 /
-// 32.2 / 35.8 / 26.5.  With the lookback in one launch, its tiles from a
-// counter, 1500 x 40 took 6.1, 131072 x 16 24.6.
-constexpr u64 kSchoolTile = 64, kSchoolWideTile = 256;
-constexpr u64 kSchoolShort = 3 << 14, kSchoolLong = 3 << 16;
+// A tile forms the sums of the eight positions before it too, so that its CTA's
+// 32 groups of lanes have no part of a round idle at 56 and 248 positions (64 and
+// 256: three rounds for 72, nine for 264; 4000 x 4000 limbs 77 us, 60 so).  Small
+// tiles spread a short product over the GPU: the column sums are the work.  Of a
+// long operand times a short one, up to kSchoolFew limbs beyond kSchoolLong, a
+// thread forms the sums of eight positions by itself (run_scan).  Measured, us,
+// tiles of 56 / 248 positions / run_scan: 8000 x 383 limbs 14 / 26 / 269, 40000 x
+// 383 26 / 38 / 271, 65000 x 383 39 / 39 / 271, 131072 x 1 19 / 15 / 15, x 31 24 /
+// 21 / 28, 196000 x 1 - / 20 / 15, 262144 x 31 - / 33 / 28, x 40 - / 28 / 34, x 383
+// - / 115 / 272, 2^20 x 31 - / 110 / 81, x 40 - / 94 / 101, x 383 - / 433 / 890.
+// run_scan takes an eighth of the tiles' words, too: what is captured keeps to it
+// where more would have to be allocated.
+constexpr u64 kSchoolTile = 56, kSchoolWideTile = 248;
+constexpr u64 kSchoolShort = kSchoolTile << 10, kSchoolLong = 3 << 16, kSchoolFew = 39;
 template <u64 TILE>
 __global__ void __launch_bounds__(256) school_kernel(ColumnProducer prod, u64 total, u64* out, u32* flags) {
   grid_begin();
@@ -628,7 +623,13 @@ cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Sca
     return e;
   }
   if (total <= kSchoolShort) return launch_school<kSchoolTile>(prod, total, out, sc, st);
-  if (total <= kSchoolLong) return launch_school<kSchoolWideTile>(prod, total, out, sc, st);
+  const u64 tiles = (total + kSchoolWideTile - 1) / kSchoolWideTile;
+  if (total <= kSchoolLong || (prod.nb > kSchoolFew && tiles <= 0x7fffffff)) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (tiles <= sc.max_tiles ||
+        (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone))
+      return launch_school<kSchoolWideTile>(prod, total, out, sc, st);
+  }
   return run_scan(prod, total, out, total, sc, st, "school_column_scan");
 }
 

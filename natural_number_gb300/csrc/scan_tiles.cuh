@@ -31,6 +31,15 @@ __device__ __forceinline__ W3 add_w3(W3 a, W3 b) {
   return r;
 }
 
+// acc += x * y as one carry chain.
+__device__ __forceinline__ void mac(W3& acc, u64 x, u64 y) {
+  asm("mad.lo.cc.u64 %0, %3, %4, %0;\n\t"
+      "madc.hi.cc.u64 %1, %3, %4, %1;\n\t"
+      "addc.u64 %2, %2, 0;"
+      : "+l"(acc.w0), "+l"(acc.w1), "+l"(acc.w2)
+      : "l"(x), "l"(y));
+}
+
 // y[0..8) += a0 + a1 * 2^64 (a carry rippling through all eight words);
 // returns the carry out of the top word.
 __device__ __forceinline__ u64 add_ripple8(u64 (&y)[8], u64 a0, u64 a1) {
@@ -359,7 +368,7 @@ __device__ __forceinline__ void column_tile_sums(u64* sm, const ColumnProducer& 
       const u64 hi = k < J.na - 1 ? k : J.na - 1;
       for (u64 i = lo + j; i <= hi; i += kLanes) {
         const u64 x = J.a[i], y = J.b[k - i];
-        acc = add_w3(acc, W3{x * y, mulhi(x, y), 0});
+        mac(acc, x, y);
       }
     }
 #pragma unroll
