@@ -1036,7 +1036,7 @@ char* dec_levels(nn_context* c, const natural& x, u64 host_below, Stats& S, u64*
   std::string head(width, '0');
   u32 failed = 0;
   check_cuda(cudaMemcpyAsync(head.data(), dout, width, cudaMemcpyDeviceToHost, st), "download");
-  check_cuda(cudaMemcpyAsync(&failed, err, 4, cudaMemcpyDeviceToHost, st), "flag");
+  if (i < top) check_cuda(cudaMemcpyAsync(&failed, err, 4, cudaMemcpyDeviceToHost, st), "flag");  // set by splits
   check_cuda(cudaStreamSynchronize(st), "decimal digits");
   if (failed) throw std::runtime_error("natural_gb300: decimal split correction did not converge");
   u64 off = 0;
