@@ -133,7 +133,7 @@ typedef struct nn_batch nn_batch;
  * others (but balanced ones below "batch_school_balanced") as NTT products
  * at scale ceil(log2(n_a+n_b-1)), unbalanced ones in pieces where that is
  * estimated faster.  A launch takes one step of all jobs at one tile shape;
- * the launch sequence is captured in a CUDA graph on first run and replayed.
+ * the launch sequence is captured in a CUDA graph on the second run and replayed.
  * Products at the "batch_solo_scale" tunable's scale and up run one at a
  * time after those launches, as nn_mul (nn_sqr for squares) would.
  * square[j] (optional) marks squares. */
@@ -142,7 +142,8 @@ nn_status nn_batch_create(nn_context* ctx, const uint64_t* n_a, const uint64_t* 
 /* Runs the planned batch on these operands (sizes must match the plan). */
 nn_status nn_batch_run(nn_context* ctx, nn_batch* batch, const nn_mul_job* jobs);
 /* As nn_batch_run, but launched directly rather than from the CUDA graph
- * (for plans that run once). */
+ * (for plans that run once).  Not while the stream is captured: the job table
+ * goes up from memory that is used again. */
 nn_status nn_batch_launch(nn_context* ctx, nn_batch* batch, const nn_mul_job* jobs);
 /* Releases a plan; waits for its last run to finish first. */
 nn_status nn_batch_destroy(nn_context* ctx, nn_batch* batch);

@@ -379,7 +379,7 @@ class Context:
 
 class Batch:
     """nn_batch: a planned batch of products (a launch a step and tile
-    shape, replayed from a CUDA graph)."""
+    shape, from the second run on replayed from a CUDA graph)."""
 
     def __init__(self, ctx: Context, sizes_a, sizes_b, square=None):
         self.ctx = ctx
