@@ -188,7 +188,7 @@ def measure_batched(ctx, steps: int, warmup: int, count: int = 4096) -> dict:
     t0 = time.perf_counter()
     plan = ctx.batch(W.sa, W.sb)
     plan_s = time.perf_counter() - t0
-    for _ in range(max(warmup, 1)):
+    for _ in range(max(warmup, 2)):  # the second run makes the graph
         plan.run_jobs(W.jobs_batch)
     batch_ms = timed(lambda: plan.run_jobs(W.jobs_batch), steps)
     ctx.synchronize()

@@ -32,7 +32,8 @@ def _time(fn, reps: int) -> float:
     import torch
     s = torch.cuda.current_stream()
     a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    fn()
+    for _ in range(2):  # a batch's second run makes its graph
+        fn()
     torch.cuda.synchronize()
     a.record(s)
     for _ in range(reps):
