@@ -91,7 +91,8 @@ nn_status nn_transform_residues(nn_context* ctx, const nn_transform* t, uint64_t
 
 /* ---- products on device pointers ---------------------------------------- */
 /* natural::_mul (natural.h:444-450): base case for short operands, NTT else,
- * with the unbalanced split of natural.h:391-419.  d_out: n_a + n_b limbs. */
+ * with the unbalanced split of natural.h:391-419.  d_out: n_a + n_b limbs,
+ * which an operand may lie in. */
 nn_status nn_mul(nn_context* ctx, uint64_t* d_out, const uint64_t* d_a, uint64_t n_a, const uint64_t* d_b,
                  uint64_t n_b);
 /* natural::_sqr (natural.h:529-535).  d_out: 2 n limbs. */

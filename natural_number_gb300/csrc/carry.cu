@@ -609,10 +609,13 @@ cudaError_t add_batch(const AddJob* d_jobs, u64 m, u64 longest, cudaStream_t st)
   return e;
 }
 
+bool school_whole(u64 na, u64 nb) {
+  return na + nb <= kSchoolClusterTile * kSchoolClusterCtas && std::min(na, nb) <= kSchoolShorter;
+}
 cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Scan& sc, cudaStream_t st) {
   const u64 total = na + nb;
   const ColumnProducer prod = na >= nb ? ColumnProducer{a, na, b, nb} : ColumnProducer{b, nb, a, na};
-  if (total <= kSchoolClusterTile * kSchoolClusterCtas && prod.nb <= kSchoolShorter) {
+  if (school_whole(na, nb)) {
     static DeviceOnce once;  // clusters of more than eight CTAs want asking
     cudaError_t e = kernel_attribute(once, school_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;

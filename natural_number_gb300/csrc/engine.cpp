@@ -573,6 +573,29 @@ bool base_case(u64 na, u64 nb) {
   return !(nb >= 256 || (nb >= 96 && na + nb > 1024) || (nb >= 32 && na >= 16384));
 }
 
+// Base-case product.  Tiles of a longer one write limbs while others still read
+// operands: an operand that lies in the output's limbs (a product in place, which
+// the transforms take as it is) is copied first.
+nn_status base_product(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b, u64 nb) {
+  auto lies = [&](const u64* x, u64 n) { return x < d_out + (na + nb) && d_out < x + n; };
+  u64* copy = nullptr;
+  if (!nn::school_whole(na, nb) && (lies(a, na) || lies(b, nb))) {
+    NN_CK(c, cudaMallocAsync((void**)&copy, (na + nb) * 8, c->stream), "operands in place");
+    cudaError_t e = cudaMemcpyAsync(copy, a, na * 8, cudaMemcpyDeviceToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(copy + na, b, nb * 8, cudaMemcpyDeviceToDevice, c->stream);
+    if (e != cudaSuccess) {
+      cudaFreeAsync(copy, c->stream);
+      return fail(c, e, "operands in place");
+    }
+    a = copy;
+    b = copy + na;
+  }
+  const cudaError_t e = nn::school_mul(a, na, b, nb, d_out, c->scan, c->stream);
+  if (copy) cudaFreeAsync(copy, c->stream);
+  NN_CK(c, e, "base-case product");
+  return NN_OK;
+}
+
 // A product of fewer than kNttMulThreshold limbs needs no memory as the base
 // case: it takes that where the transforms' would not fit the budget, and while
 // the stream is captured, where their memory would be a part of the graph (which
@@ -582,9 +605,7 @@ nn_status short_product(nn_context* c, u64* d_out, const nn::SixOperands& op, in
     const nn_status st = six_product(c, d_out, op, s);
     if (!short_of_memory(st)) return st;
   }
-  const u64* b = op.b ? op.b : op.a;
-  NN_CK(c, nn::school_mul(op.a, op.na, b, op.nb, d_out, c->scan, c->stream), "base-case product");
-  return NN_OK;
+  return base_product(c, d_out, op.a, op.na, op.b ? op.b : op.a, op.nb);
 }
 
 nn_status mul_impl(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b, u64 nb) {
@@ -596,10 +617,7 @@ nn_status mul_impl(nn_context* c, u64* d_out, const u64* a, u64 na, const u64* b
     std::swap(a, b);
     std::swap(na, nb);
   }
-  if (base_case(na, nb)) {  // natural.h:445-446 -> _mul_base
-    NN_CK(c, nn::school_mul(a, na, b, nb, d_out, c->scan, c->stream), "base-case product");
-    return NN_OK;
-  }
+  if (base_case(na, nb)) return base_product(c, d_out, a, na, b, nb);  // natural.h:445-446 -> _mul_base
   // natural::_mul_NTT (natural.h:391-419) cuts the longer operand in two when
   // that lowers the scale; here it may go in any number of pieces.
   u64 piece, pieces;
@@ -614,10 +632,7 @@ nn_status sqr_impl(nn_context* c, u64* d_out, const u64* a, u64 n) {
     c->err = "sqr: null pointer or empty operand";
     return NN_ERR_INVALID;
   }
-  if (base_case(n, n)) {  // natural.h:530-531 -> _sqr_base
-    NN_CK(c, nn::school_mul(a, n, a, n, d_out, c->scan, c->stream), "base-case square");
-    return NN_OK;
-  }
+  if (base_case(n, n)) return base_product(c, d_out, a, n, a, n);  // natural.h:530-531 -> _sqr_base
   // natural::_sqr_NTT (natural.h:433-442): one transform.
   const int s = ntt_scale(n, n);
   if (s > nn::kSixMaxScale) return ntt_product(c, d_out, a, n, a, n, s, 2 * n, nullptr);
@@ -1197,8 +1212,7 @@ nn_status nn_ntt_mul(nn_context* c, uint64_t* d_out, const uint64_t* a, uint64_t
 nn_status nn_mul_base(nn_context* c, uint64_t* d_out, const uint64_t* a, uint64_t na, const uint64_t* b,
                       uint64_t nb) {
   if (!c || !d_out || !a || !b || !na || !nb) return NN_ERR_INVALID;
-  NN_CK(c, nn::school_mul(a, na, b, nb, d_out, c->scan, c->stream), "base-case product");
-  return NN_OK;
+  return base_product(c, d_out, a, na, b, nb);
 }
 
 nn_status nn_mul_host(nn_context* c, uint64_t* out, uint64_t* out_n, const uint64_t* a, uint64_t na,

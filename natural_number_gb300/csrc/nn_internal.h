@@ -229,7 +229,10 @@ cudaError_t six_to_three(const u32* res, int s, u64* out, cudaStream_t st);
 // B^L - 1 in L limbs when size-1 > L (ntt_info.h:237-248).  Returns the
 // number of limbs written through *written (host value).
 cudaError_t ntt_save(const u64* res, int s, u64* out, u64 size, Scan& sc, u64* written, cudaStream_t st);
-// Schoolbook product by column sums + carry scan: out[0..na+nb).
+// Schoolbook product by column sums + carry scan: out[0..na+nb), apart from the
+// operands but where school_whole says that they are read before any limb is
+// written.
+bool school_whole(u64 na, u64 nb);
 cudaError_t school_mul(const u64* a, u64 na, const u64* b, u64 nb, u64* out, Scan& sc, cudaStream_t st);
 // out[0..n) = x (nx limbs) + y (ny limbs) shifted up by `shift` limbs; the
 // carry out of limb n-1 is dropped.  out must not alias x or y (a tile
