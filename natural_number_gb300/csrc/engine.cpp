@@ -712,9 +712,9 @@ nn_status batch_plan(nn_context* c, nn_batch* B, const u64* na, const u64* nb, c
   // CTAs a job, under a wave), and where the batch has launches of two passes
   // anyhow, products of up to 2^14 limbs are not split.  (Contexts with a budget,
   // or "batch_few" 0, keep the smaller arenas.)  With and without, us: 64 jobs of
-  // 8 to 1024 limbs 38 and 45, one of 2000 x 2000 limbs beside 150 of 64 x 200 43
-  // and 50, beside 150 of 120 x 120 42 and 48, 111 of 44 to 6439 limbs 120 and 144.
-  // Unsplit by themselves five products of 16000 x 300 limbs take 137, split 31.
+  // 8 to 1024 limbs 38 and 45, one of 2000 x 2000 limbs beside 150 of 64 x 200 42
+  // and 49, beside 150 of 500 x 500 42 and 54, 111 of 44 to 6439 limbs 114 and 140.
+  // Unsplit by themselves five products of 16000 x 300 limbs take 79, split 32.
   constexpr int kOnePass = 12, kFewWhole = 14;
   const bool few = c->batch_few && count <= 152 && !c->budget;
   int few_s = 0, whole = 0;
@@ -1455,8 +1455,8 @@ nn_status nn_batch_launch(nn_context* c, nn_batch* B, const nn_mul_job* jobs) {
 
 // A plan's first run goes launch by launch, later ones as a graph: making that
 // costs more than it saves one run.  Plan, run and release together, us, first run
-// as a graph / so: one product of 8 to 1024 limbs 180 / 39, 153 of them 272 / 95,
-// 400 of 300 to 5000 507 / 266, 4096 of 64 to 2^18 20080 / 19700.
+// as a graph / so: one product of 8 to 1024 limbs 180 / 40, 153 of them 272 / 98,
+// 400 of 300 to 5000 507 / 274, 4096 of 64 to 2^18 20080 / 19870.
 nn_status nn_batch_run(nn_context* c, nn_batch* B, const nn_mul_job* jobs) {
   if (!c || !B || !jobs) return NN_ERR_INVALID;
   if (B->pending) NN_CK(c, cudaEventSynchronize(B->ran), "previous batch run");
